@@ -24,7 +24,7 @@ _HAS_GPTQ_FUSED_KERNEL = is_gptq_cuda_available()
 
 
 def _tileable(bits, groupsize):
-    kb = {2: 128, 4: 64}.get(bits)
+    kb = {2: 128, 3: 64, 4: 64}.get(bits)
     return kb is not None and groupsize is not None and groupsize > 0 and groupsize % kb == 0
 
 
@@ -70,9 +70,12 @@ class GLoRCQLinear(nn.Module):
 
     # ---- loaders (inference/quantized_linear.py:195-269) ---------------------------------
     def load_gptq(self, packed_data, device="cuda", keep_raw=False, check_range=True):
-        """Integer codes + per-group scale/zero.  2- and 4-bit codes with a group size that is a
-        multiple of 128 (64 for 4-bit) are re-tiled for the fused kernel; anything else keeps the
-        (N,K) codes and runs through the int8 drop-in kernel."""
+        """Integer codes + per-group scale/zero.  2-, 3- and 4-bit codes with a group size that is a
+        multiple of 128 (64 for 3- and 4-bit) are re-tiled for the fused kernel; anything else keeps the
+        (N,K) codes and runs through the int8 drop-in kernel.  3-bit codes take the 4-bit fields: half the
+        bytes of the int8 codes, and one launch where the int8 route needs six (2 rows of 2048 x 2048 with
+        rank 64: 117 -> 26 us per eager call).  Their range is checked whatever `check_range` says: codes
+        outside it (the int8 kernel takes any int8 value) keep the int8 route."""
         self.quant_type = "gptq"
         q = packed_data["qweight_int"].to(device)
         self.scales = packed_data["scales"].to(device).to(torch.float16)
@@ -81,7 +84,7 @@ class GLoRCQLinear(nn.Module):
         self.gptq_groupsize = packed_data["groupsize"]
         self.gptq_sym = packed_data.get("sym", False)
         in_range = True
-        if check_range and _tileable(self.gptq_bits, self.gptq_groupsize):
+        if (check_range or self.gptq_bits == 3) and _tileable(self.gptq_bits, self.gptq_groupsize):
             in_range = bool(((q >= 0) & (q < 2 ** self.gptq_bits)).all())   # load time only
         if _tileable(self.gptq_bits, self.gptq_groupsize) and in_range:
             self._tiled = TiledWeight.from_gptq(q, self.scales, self.zeros, self.gptq_bits,
@@ -208,8 +211,13 @@ class GLoRCQLinear(nn.Module):
         if self._tiled is None and self._dense is not None:
             y = self._forward_dense(x, a)
         elif self.quant_type == "gptq":
-            if self._tiled is not None:
+            if self._tiled is not None and (self.gptq_bits != 3 or x.shape[0] <= 32):
                 y = tiled.linear_forward(self._tiled, x, ut=self._ut, a=a)
+            elif self._tiled is not None:
+                # 3-bit codes stay on the integer product, which keeps (q - z) * s unrounded as the int8 kernel does
+                # (the GEMM above 32 rows rounds it to fp16): 32 rows at a time
+                y = torch.cat([tiled.linear_forward(self._tiled, x[i:i + 32], ut=self._ut, a=None if a is None else a[i:i + 32])
+                               for i in range(0, x.shape[0], 32)])
             else:
                 y = gptq_dequant_matmul_fused(x, self.qweight_int, self.scales, self.zeros,
                                               self.gptq_groupsize, self.gptq_sym, lora_USV=None)

@@ -67,7 +67,8 @@ class TiledWeight:
         s = scales.to(torch.float16).contiguous()
         z = None if (sym or zeros is None) else zeros.to(torch.float16).contiguous()
         with torch.cuda.device(self.codes.device):
-            _lib.check(_lib.lib().glq_pack_gptq(q32.data_ptr(), s.data_ptr(), _ptr(z), bits, N, K, self.group_size,
+            # (3-bit codes sit in the 4-bit fields)
+            _lib.check(_lib.lib().glq_pack_gptq(q32.data_ptr(), s.data_ptr(), _ptr(z), 2 if bits == 2 else 4, N, K, self.group_size,
                                                 self.codes.data_ptr(), slot, self.count,
                                                 _stream_ptr(self.codes.device)), "pack_gptq")
 
@@ -119,8 +120,8 @@ class TiledWeight:
     # ---- constructors -------------------------------------------------------------------
     @staticmethod
     def _gptq_fmt(bits, groupsize):
-        if bits not in (2, 4):
-            raise RuntimeError(f"tiled layout covers 2- and 4-bit codes, got bits={bits}")
+        if bits not in (2, 3, 4):
+            raise RuntimeError(f"tiled layout covers 2-, 3- and 4-bit codes, got bits={bits}")
         kb = 128 if bits == 2 else 64
         if groupsize <= 0 or groupsize % kb != 0:
             raise RuntimeError(f"group size {groupsize} must be a positive multiple of {kb} for {bits}-bit codes")

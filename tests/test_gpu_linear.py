@@ -34,6 +34,21 @@ def test_gptq_tiles_bit_exact(dev, N, K, bits, gs, int_zeros):
     assert torch.equal(W, ref)
 
 
+@pytest.mark.parametrize("B", [1, 9, 32, 33])
+@pytest.mark.parametrize("N,K,gs", [(2048, 2048, 128), (40, 192, 64)])
+def test_3bit_codes_in_4bit_tiles(dev, N, K, gs, B):
+    d = cases.make_linear(31 * N + B, N, K, rank=16, fmt="gptq", bits=3, groupsize=gs)
+    lin = cases.to_b200_linear(d, dev)
+    assert lin._tiled is not None
+    assert torch.equal(lin._dequant_gptq().cpu(), O.gptq_tile_fp16(d["qweight_int"], d["scales"], d["zeros"], gs))
+    x = cases.make_x(N + B, B, K)
+    assert cases.rel_l2(lin(x.to(dev)).cpu(), O.linear_forward(cases.to_oracle_linear(d), x, x_rot_half=True)) <= REL
+    d["qweight_int"][0, 0] = 9          # outside 3 bits: the int8 kernel
+    lin = cases.to_b200_linear(d, dev)
+    assert lin._tiled is None
+    assert cases.rel_l2(lin(x.to(dev)).cpu(), O.linear_forward(cases.to_oracle_linear(d), x, x_rot_half=True)) <= REL
+
+
 @pytest.mark.parametrize("N,K", [(1408, 2048), (72, 256), (19, 132), (64, 64)])
 def test_turbo_tiles_bit_exact(dev, N, K):
     from glorcq_b200.tiled import TiledWeight
