@@ -110,6 +110,9 @@ _SIGS = {
     "glq_linear_workspace_bytes": (C.c_size_t, [C.c_int, C.c_int, C.POINTER(Weight), C.c_int]),
     "glq_linear_forward": (C.c_int, [C.c_int, C.c_int, C.POINTER(Weight), vp, vp, C.c_int64, vp, vp, C.c_int64,
                                      C.c_int, vp, C.c_size_t, vp, C.c_size_t, vp]),
+    "glq_linear_rht_workspace_bytes": (C.c_size_t, [C.c_int, C.c_int, C.POINTER(Weight), C.c_int]),
+    "glq_linear_rht_forward": (C.c_int, [C.c_int, C.c_int, C.POINTER(Weight), vp, vp, vp, C.c_int64, vp, vp, C.c_int64,
+                                         C.c_int, vp, C.c_size_t, vp, C.c_size_t, vp]),
     "glq_moe_fused_trace": (C.c_int, [vp, C.c_int]),
     "glq_moe_uses_fused_kernel": (C.c_int, [C.POINTER(MoeDesc), C.c_int]),
     "glq_moe_workspace_bytes": (C.c_size_t, [C.POINTER(MoeDesc), C.c_int]),
@@ -140,6 +143,25 @@ def lib():
             fn.argtypes = args
         _lib = L
     return _lib
+
+
+_native = None
+
+
+def native():
+    """The host path's native module (csrc/native.cpp) bound to the loaded library; RuntimeError when it has not been built."""
+    global _native
+    if _native is None:
+        L = lib()
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        try:
+            from . import _native as mod
+        except ImportError as e:
+            raise RuntimeError("glorcq_b200/_native is missing or was built for another torch: build it with "
+                               "`python -m glorcq_b200._build`") from e
+        mod.bind({n: C.cast(getattr(L, n), vp).value for n in mod.names()})
+        _native = mod
+    return _native
 
 
 def exported_symbols():

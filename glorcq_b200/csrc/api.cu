@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -811,9 +812,10 @@ extern "C" size_t glq_linear_counters(int fmt, int group_size, const glq_weight_
     return total;
 }
 
-extern "C" int glq_linear_forward(int fmt, int group_size, const glq_weight_t* w, const void* ut, const void* x,
-                                  int64_t ldx, const void* a, void* y, int64_t ldy, int B, void* workspace,
-                                  size_t workspace_bytes, int32_t* counters, size_t n_counters, void* stream) {
+// x: rows of the low-rank term, xq: rows of the quantized product
+static int linear_forward(int fmt, int group_size, const glq_weight_t* w, const void* ut, const void* x, int64_t ldx,
+                          const void* xq, int64_t ldxq, const void* a, void* y, int64_t ldy, int B, void* workspace,
+                          size_t workspace_bytes, int32_t* counters, size_t n_counters, void* stream) {
     if (!w || !x || !y || B < 0) return GLQ_ERR_ARG;
     if (B == 0 || w->N == 0) return GLQ_OK;
     glq_mm_args_t m;
@@ -844,8 +846,8 @@ extern "C" int glq_linear_forward(int fmt, int group_size, const glq_weight_t* w
     }
     if (main_ws > 0 && (!ws || workspace_bytes < main_ws)) return GLQ_ERR_WORKSPACE;
     if (main_ctr > 0 && (!counters || n_counters < main_ctr)) return GLQ_ERR_WORKSPACE;
-    m.x = x;
-    m.ldx = ldx;
+    m.x = xq;
+    m.ldx = ldxq;
     m.a0 = a_use;
     m.lda = w->rank;
     m.y = y;
@@ -858,6 +860,33 @@ extern "C" int glq_linear_forward(int fmt, int group_size, const glq_weight_t* w
     // x.U was just launched above and is needed only in the epilogue; x itself is older
     if (a_use != nullptr && a_use != a) m.flags = GLQ_MM_A_FROM_PREVIOUS_LAUNCH;
     return glq_grouped_matmul(&m, stream);
+}
+
+extern "C" int glq_linear_forward(int fmt, int group_size, const glq_weight_t* w, const void* ut, const void* x,
+                                  int64_t ldx, const void* a, void* y, int64_t ldy, int B, void* workspace,
+                                  size_t workspace_bytes, int32_t* counters, size_t n_counters, void* stream) {
+    return linear_forward(fmt, group_size, w, ut, x, ldx, x, ldx, a, y, ldy, B, workspace, workspace_bytes, counters, n_counters,
+                          stream);
+}
+
+// the quantized product sees the rotated rows, the low-rank term the rows as given: rotation, x.U, product.  The
+// rotation goes first: the product may then start while x.U still runs (it needs x.U only in its epilogue)
+extern "C" size_t glq_linear_rht_workspace_bytes(int fmt, int group_size, const glq_weight_t* w, int B) {
+    if (!w || B <= 0) return 0;
+    return glq_linear_workspace_bytes(fmt, group_size, w, B) + up256((size_t)B * w->K * sizeof(__half));
+}
+
+extern "C" int glq_linear_rht_forward(int fmt, int group_size, const glq_weight_t* w, const void* ut, const float* signs,
+                                      const void* x, int64_t ldx, const void* a, void* y, int64_t ldy, int B, void* workspace,
+                                      size_t workspace_bytes, int32_t* counters, size_t n_counters, void* stream) {
+    if (!w || !x || !y || !signs || B < 0) return GLQ_ERR_ARG;
+    if (B == 0 || w->N == 0) return GLQ_OK;
+    const size_t rot = up256((size_t)B * w->K * sizeof(__half));
+    if (!workspace || workspace_bytes < rot) return GLQ_ERR_WORKSPACE;
+    int rc = glq_rht_forward(x, 0, ldx, signs, B, w->K, 1.0f / sqrtf((float)w->K), workspace, 0, w->K, stream);
+    if (rc != GLQ_OK) return rc;
+    return linear_forward(fmt, group_size, w, ut, x, ldx, workspace, w->K, a, y, ldy, B, static_cast<char*>(workspace) + rot,
+                          workspace_bytes - rot, counters, n_counters, stream);
 }
 
 // ---------------------------------------------------------------------------------------------

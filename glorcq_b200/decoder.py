@@ -81,13 +81,7 @@ def _add_rmsnorm(x, delta, weight, eps):
     if not (x.is_cuda and x.dtype == torch.float16 and delta.dtype == torch.float16 and H % 8 == 0 and H <= 8192):
         y = x + delta
         return y, F.rms_norm(y, (H,), weight, eps)
-    x, delta = x.contiguous(), delta.contiguous()
-    x_out, h_out = torch.empty_like(x), torch.empty_like(x)
-    with torch.cuda.device(x.device):
-        _lib.check(_lib.lib().glq_add_rmsnorm(x.data_ptr(), delta.data_ptr(), weight.data_ptr(), float(eps),
-                                              x.numel() // H, H, x_out.data_ptr(), h_out.data_ptr(),
-                                              tiled._stream_ptr(x.device)), "add_rmsnorm")
-    return x_out, h_out
+    return _lib.native().add_rmsnorm(x.contiguous(), delta.contiguous(), weight, eps)
 
 
 class _Attention(nn.Module):

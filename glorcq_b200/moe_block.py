@@ -61,25 +61,6 @@ def _table(descs: List[Weight], device) -> torch.Tensor:
     return torch.frombuffer(bytearray(raw), dtype=torch.uint8).to(device)
 
 
-_SHARED_WS_FROM = 256 << 20       # scratch sizes above this come from the per-device pool below
-_BIG_WS = {}
-
-
-def _shared_big_workspace(device, nbytes, ncounters):
-    """Scratch and arrival counters for prompt-sized calls, one pair per device (grown on demand, never shrunk).
-    The counters are zero before a call and every kernel leaves them zero."""
-    key = torch.device(device).index or 0
-    ws, ctr = _BIG_WS.get(key, (None, None))
-    if ws is None or ws.numel() < nbytes:
-        ws = None
-        _BIG_WS.pop(key, None)
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-    if ctr is None or ctr.numel() < ncounters:
-        ctr = torch.zeros(ncounters, dtype=torch.int32, device=device)
-    _BIG_WS[key] = (ws, ctr)
-    return ws, ctr
-
-
 class GraphCompatibleMoeBlock(nn.Module):
     """Drop-in replacement for Qwen2MoeSparseMoeBlock running on the fused kernels."""
 
@@ -97,7 +78,8 @@ class GraphCompatibleMoeBlock(nn.Module):
         self._built = False
         self._keep = []                  # tensors the descriptor tables point into
         self._desc: Optional[MoeDesc] = None
-        self._ws = {}
+        self._entries = {}               # expert parallel: exchange buffers, one per token count
+        self._native = None              # native handle of the built block
         self.parallel_shared_expert = True   # shared expert on a side stream, as the reference's side-stream LoRA
         self._side = None
         self.last_selected_experts = None
@@ -305,6 +287,11 @@ class GraphCompatibleMoeBlock(nn.Module):
         ``next_norm = (weight or None, eps)`` folds the decoder's next steps into the combine kernel: the
         first result becomes ``residual + block output`` (``residual`` (B, S, H), optional) and a third result
         is its RMS norm times ``weight``: ((B, S, H), logits, (B, S, H))."""
+        if self._native is not None and top_k_index is None and residual is None and next_norm is None and self.gate is not None \
+                and self._ep[1] == 1 and hidden_states.dtype is torch.float16 and hidden_states.is_contiguous():
+            out, logits, self.last_selected_experts, self.last_routing_weights, _ = _lib.native().moe(
+                self._block(hidden_states.device), hidden_states, None, None, None, None, None)
+            return out, logits
         batch_size, sequence_length, hidden_dim = hidden_states.shape
         x = hidden_states.reshape(-1, hidden_dim)
         if x.dtype != torch.float16:
@@ -316,104 +303,96 @@ class GraphCompatibleMoeBlock(nn.Module):
             self._build(x.device)
         d = self._desc
         n = x.shape[0]
-        out = torch.empty(n, d.H, dtype=torch.float16, device=x.device)
         given = top_k_index is not None
         if given != (self.gate is None):
             raise RuntimeError("routing must be passed exactly when the block has no router")
-        logits = None if given else torch.empty(n, d.E, dtype=torch.float16, device=x.device)
+        sel_in = wts_in = eps = nw = res2 = None
         if given:
             sel_in = top_k_index.to(device=x.device, dtype=torch.int32).contiguous()
             wts_in = top_k_weights.to(device=x.device, dtype=torch.float16).contiguous()
             if sel_in.shape != (n, d.top_k) or wts_in.shape != (n, d.top_k):
                 raise RuntimeError(f"top_k_index / top_k_weights must have shape ({n}, {d.top_k})")
-        sel = torch.empty(n, d.top_k, dtype=torch.int32, device=x.device)
-        wts = torch.empty(n, d.top_k, dtype=torch.float16, device=x.device)
-        normed = res2 = nw = None
         if next_norm is not None:
             nw, eps = next_norm
-            normed = torch.empty(n, d.H, dtype=torch.float16, device=x.device)
+            eps = float(eps)
             if nw is not None:
                 nw = nw.to(device=x.device, dtype=torch.float16).contiguous()
             if residual is not None:
                 res2 = residual.reshape(-1, hidden_dim).to(torch.float16).contiguous()
         elif residual is not None:
             raise RuntimeError("a residual is folded in only together with next_norm")
-        if n > 0:
-            L = _lib.lib()
-            with torch.cuda.device(x.device):
-                # one workspace per token count: a block's calls run one after another (it is not re-entrant across
-                # streams), and a workspace made by the warm-up call must be the one a later capture finds -- an
-                # allocation inside a capture would put its zero fill into the graph, once per replay
-                key = n
-                if key not in self._ws:
-                    nbytes = L.glq_moe_workspace_bytes(C.byref(d), n)
-                    nctr = L.glq_moe_counters(C.byref(d), n)
-                    if nbytes > _SHARED_WS_FROM and not torch.cuda.is_current_stream_capturing():
-                        # prompt-sized calls: one scratch per device for all blocks (they run one after another;
-                        # a private copy per block of a 32-layer model would not fit the device)
-                        ws, ctr = _shared_big_workspace(x.device, nbytes + 256, max(nctr, 1))
-                    else:
-                        self._ws[key] = (torch.empty(nbytes + 256, dtype=torch.uint8, device=x.device),
-                                         torch.zeros(max(nctr, 1), dtype=torch.int32, device=x.device))
-                if key in self._ws:
-                    ws, ctr = self._ws[key]
-                base = (ws.data_ptr() + 255) // 256 * 256
-                aux = fork = join = None
-                if self.parallel_shared_expert and d.I_shared > 0:
-                    if self._side is None:
-                        self._side = (torch.cuda.Stream(device=x.device), torch.cuda.Event(), torch.cuda.Event())
-                    aux, fork, join = self._side[0].cuda_stream, self._side[1], self._side[2]
-                    # torch creates events lazily: record once so that the handles exist
-                    if not getattr(self, "_events_ready", False):
-                        fork.record()
-                        join.record()
-                        self._events_ready = True
-                    fork, join = fork.cuda_event, join.cuda_event
-                ep_rank, ep_world, group = self._ep
-
-                def call(ep):
-                    if (given or normed is not None) and ep is None:
-                        ep = MoeEp(0, 1, _lib.MOE_PHASE_ALL, 0, None, None, None)
-                    if given:
-                        ep.sel_in, ep.weight_in = sel_in.data_ptr(), wts_in.data_ptr()
-                    if normed is not None:
-                        ep.normed_out, ep.norm_eps = normed.data_ptr(), float(eps)
-                        ep.residual = None if res2 is None else res2.data_ptr()
-                        ep.norm_weight = None if nw is None else nw.data_ptr()
-                    _lib.check(L.glq_moe_forward_ep(C.byref(d), x.data_ptr(), n, out.data_ptr(),
-                                                    None if logits is None else logits.data_ptr(),
-                                                    sel.data_ptr(), wts.data_ptr(), base,
-                                                    ws.numel() - (base - ws.data_ptr()), ctr.data_ptr(), ctr.numel(),
-                                                    tiled._stream_ptr(x.device), aux, fork, join,
-                                                    None if ep is None else C.byref(ep)),
-                               "moe_forward")
-                if ep_world == 1:
-                    call(None)
-                else:
-                    ekey = ("entries", n)
-                    if ekey not in self._ws:
-                        self._ws[ekey] = torch.empty(n * d.top_k, d.H, dtype=torch.float16, device=x.device)
-                    entries = self._ws[ekey]
-                    by_peers = 0 < n <= self.peer_exchange_max_tokens
-                    ep = MoeEp(ep_rank, ep_world, _lib.MOE_PHASE_EXPERTS, _lib.MOE_EP_NO_ZERO_FILL if by_peers else 0,
-                               entries.data_ptr(), None, None)
-                    call(ep)
-                    if by_peers:
-                        # this library's exchange kernel: peer stores into every rank's buffer, then flags
-                        if self._peers is None:
-                            self._peers = parallel.PeerExchange.get(
-                                group, x.device, self.peer_exchange_max_tokens * d.top_k, d.H)
-                        px = self._peers
-                        ep.phase, ep.peers = _lib.MOE_PHASE_EXCHANGE, C.pointer(px.peers)
-                        call(ep)
-                        ep.phase, ep.entry_out = _lib.MOE_PHASE_COMBINE, px.local_ptr
-                        call(ep)
-                    else:
-                        self._exchange(entries, group)
-                        ep.phase = _lib.MOE_PHASE_COMBINE
-                        call(ep)
+        if self._ep[1] == 1:
+            out, logits, sel, wts, normed = _lib.native().moe(self._block(x.device), x, res2, nw, eps, sel_in, wts_in)
+        else:
+            out, logits, sel, wts, normed = self._forward_sharded(x, n, res2, nw, eps, sel_in, wts_in)
         self.last_selected_experts, self.last_routing_weights = sel, wts
+        shape = hidden_states.shape
         if normed is not None:
-            return (out.reshape(batch_size, sequence_length, hidden_dim), logits,
-                    normed.reshape(batch_size, sequence_length, hidden_dim))
-        return out.reshape(batch_size, sequence_length, hidden_dim), logits
+            return out.view(shape), logits, normed.view(shape)
+        return out.view(shape), logits
+
+    def _block(self, device):
+        """The native handle: descriptor, and the stream and events of the shared expert's branch."""
+        side = self.parallel_shared_expert and self._desc.I_shared > 0
+        if self._native is None or self._native[1] != side:
+            handles = (0, 0, 0)
+            if side:
+                if self._side is None:
+                    with torch.cuda.device(device):
+                        self._side = (torch.cuda.Stream(device=device), torch.cuda.Event(), torch.cuda.Event())
+                        for ev in self._side[1:]:       # torch creates events lazily: record once so that the handles exist
+                            ev.record()
+                handles = (self._side[0].cuda_stream, self._side[1].cuda_event, self._side[2].cuda_event)
+            self._native = (_lib.native().block(C.addressof(self._desc), torch.device(device).index or 0, *handles), side, handles)
+        return self._native[0]
+
+    def _forward_sharded(self, x, n, res2, nw, eps, sel_in, wts_in):
+        """Expert parallel: this rank's experts, the exchange of their rows, the combine."""
+        d, L = self._desc, _lib.lib()
+        out = torch.empty(n, d.H, dtype=torch.float16, device=x.device)
+        logits = None if sel_in is not None else torch.empty(n, d.E, dtype=torch.float16, device=x.device)
+        sel = torch.empty(n, d.top_k, dtype=torch.int32, device=x.device)
+        wts = torch.empty(n, d.top_k, dtype=torch.float16, device=x.device)
+        normed = None if eps is None else torch.empty(n, d.H, dtype=torch.float16, device=x.device)
+        if n == 0:
+            return out, logits, sel, wts, normed
+        with torch.cuda.device(x.device):
+            ws, ctr = _lib.native().block_scratch(self._block(x.device), n)
+            base = (ws.data_ptr() + 255) // 256 * 256
+            aux, fork, join = (h or None for h in self._native[2])
+            ep_rank, ep_world, group = self._ep
+
+            def call(ep):
+                if sel_in is not None:
+                    ep.sel_in, ep.weight_in = sel_in.data_ptr(), wts_in.data_ptr()
+                if normed is not None:
+                    ep.normed_out, ep.norm_eps = normed.data_ptr(), eps
+                    ep.residual = None if res2 is None else res2.data_ptr()
+                    ep.norm_weight = None if nw is None else nw.data_ptr()
+                _lib.check(L.glq_moe_forward_ep(C.byref(d), x.data_ptr(), n, out.data_ptr(),
+                                                None if logits is None else logits.data_ptr(),
+                                                sel.data_ptr(), wts.data_ptr(), base,
+                                                ws.numel() - (base - ws.data_ptr()), ctr.data_ptr(), ctr.numel(),
+                                                tiled._stream_ptr(x.device), aux, fork, join, C.byref(ep)), "moe_forward")
+
+            if n not in self._entries:
+                self._entries[n] = torch.empty(n * d.top_k, d.H, dtype=torch.float16, device=x.device)
+            entries = self._entries[n]
+            by_peers = n <= self.peer_exchange_max_tokens
+            ep = MoeEp(ep_rank, ep_world, _lib.MOE_PHASE_EXPERTS, _lib.MOE_EP_NO_ZERO_FILL if by_peers else 0,
+                       entries.data_ptr(), None, None)
+            call(ep)
+            if by_peers:
+                # this library's exchange kernel: peer stores into every rank's buffer, then flags
+                if self._peers is None:
+                    self._peers = parallel.PeerExchange.get(group, x.device, self.peer_exchange_max_tokens * d.top_k, d.H)
+                px = self._peers
+                ep.phase, ep.peers = _lib.MOE_PHASE_EXCHANGE, C.pointer(px.peers)
+                call(ep)
+                ep.phase, ep.entry_out = _lib.MOE_PHASE_COMBINE, px.local_ptr
+                call(ep)
+            else:
+                self._exchange(entries, group)
+                ep.phase = _lib.MOE_PHASE_COMBINE
+                call(ep)
+        return out, logits, sel, wts, normed

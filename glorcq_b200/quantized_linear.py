@@ -197,6 +197,15 @@ class GLoRCQLinear(nn.Module):
         return y
 
     def forward(self, x, precomputed_xU=None, precomputed_x_rot=None):
+        t = self._tiled
+        if t is not None and precomputed_xU is None and precomputed_x_rot is None and x.dtype is torch.float16 and x.is_contiguous():
+            # everything from the re-tiled weights and the rows as they are: one native call
+            if self.quant_type == "turbo":
+                signs = self._rht_signs
+                if signs is not None and signs.dtype is torch.float32 and signs.is_cuda:
+                    return tiled.linear_forward(t, x, self._ut, None, signs)
+            elif self.gptq_bits != 3 or x.numel() <= 32 * self.in_features:
+                return tiled.linear_forward(t, x, self._ut)
         orig_shape = x.shape
         in_dtype = x.dtype
         if x.dim() != 2:

@@ -41,7 +41,7 @@ class TiledWeight:
         self.fmt, self.N, self.K, self.group_size, self.count = fmt, N, K, group_size, count
         self.codes = self.norms = self.centroids = self.sv = self.bias = None
         self.rank = 0
-        self._desc = None
+        self._desc = self._native = None
         self._device = device
         L = _lib.lib()
         if fmt == FMT_F16:
@@ -170,6 +170,13 @@ class TiledWeight:
                                 _ptr(self.sv), _ptr(self.bias), self.N, self.K, self.rank, 0)
         return self._desc
 
+    @property
+    def native(self):
+        """The descriptor as the native host path holds it."""
+        if self._desc is None or self._native is None:
+            self._native = _lib.native().layer(self.fmt, self.group_size, self.desc_bytes())
+        return self._native
+
     def desc_bytes(self) -> bytes:
         return bytes(self.desc)
 
@@ -230,29 +237,12 @@ def clear_pool():
 
 
 # ---- workspaces ------------------------------------------------------------------------------
-_WS: Dict[Tuple[int, int], Tuple[torch.Tensor, torch.Tensor]] = {}
-
-
 def workspace(device, nbytes: int, ncounters: int = 0):
     """(scratch, counters) for the current stream of `device`.  The scratch holds split-k partial
     sums and small intermediates and needs no initialisation.  The counters are arrival counters:
     they must be zero before a call and every kernel leaves them zero, so they are cleared only
     when the array is (re)allocated."""
-    key = (torch.device(device).index or 0, _stream_ptr(device))
-    ws, ctr = _WS.get(key, (None, None))
-    if (ws is None or ctr is None) and torch.cuda.is_current_stream_capturing():
-        # no allocation (and no zero fill) inside a capture: the workspace of the warm-up calls on this device serves
-        # the captured calls too (they run in stream order after them)
-        for (dev_idx, _), (ows, octr) in _WS.items():
-            if dev_idx == key[0] and ows.numel() >= nbytes and octr.numel() >= ncounters:
-                ws, ctr = ows, octr
-                break
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-    if ctr is None or ctr.numel() < ncounters:
-        ctr = torch.zeros(max(ncounters, 1 << 16), dtype=torch.int32, device=device)
-    _WS[key] = (ws, ctr)
-    return ws, ctr
+    return _lib.native().workspace(torch.device(device).index or 0, nbytes, ncounters)
 
 
 def debug_error(clear: bool = True):
@@ -265,30 +255,10 @@ def debug_error(clear: bool = True):
 
 # ---- calls -----------------------------------------------------------------------------------
 def linear_forward(w: TiledWeight, x: torch.Tensor, ut: Optional[TiledWeight] = None,
-                   a: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """y = Q(x) + a . SV^T + bias on (B, K) fp16 rows; a = x . U is taken from `a`, or computed
-    from `ut`, or absent."""
-    if x.dtype != torch.float16:
-        raise RuntimeError("x must be fp16")
-    _need_cuda(x, "x")
-    B = x.shape[0]
-    y = torch.empty(B, w.N, dtype=torch.float16, device=x.device)
-    if B == 0 or w.N == 0:
-        return y
-    L = _lib.lib()
-    if a is not None:
-        if a.dtype != torch.float16 or a.shape != (B, w.rank):
-            raise RuntimeError("precomputed x@U must be fp16 of shape (B, rank)")
-        a = a.contiguous()
-    with torch.cuda.device(x.device):
-        nbytes = L.glq_linear_workspace_bytes(w.fmt, w.group_size, C.byref(w.desc), B)
-        nctr = L.glq_linear_counters(w.fmt, w.group_size, C.byref(w.desc), B)
-        ws, ctr = workspace(x.device, nbytes, nctr)
-        _lib.check(L.glq_linear_forward(w.fmt, w.group_size, C.byref(w.desc), None if ut is None else _ptr(ut.codes),
-                                        x.data_ptr(), x.stride(0), _ptr(a), y.data_ptr(), w.N, B,
-                                        ws.data_ptr(), ws.numel(), ctr.data_ptr(), ctr.numel(),
-                                        _stream_ptr(x.device)), "linear_forward")
-    return y
+                   a: Optional[torch.Tensor] = None, signs: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """y = Q(x) + a . SV^T + bias on (..., K) fp16 rows; a = x . U is taken from `a`, or computed
+    from `ut`, or absent.  With `signs` the quantized product sees the Hadamard-rotated rows."""
+    return _lib.native().linear(w.native, x, None if ut is None else ut.codes, signs, a)
 
 
 def dense_matmul(w: TiledWeight, x: torch.Tensor) -> torch.Tensor:
@@ -313,41 +283,8 @@ class GroupedLinear:
         if self.uts:
             descs = [_lib.Weight(u.codes.data_ptr(), None, None, None, None, None, u.N, u.K, 0, 0) for u in self.uts]
             self._ut_table = torch.frombuffer(bytearray(b"".join(bytes(d) for d in descs)), dtype=torch.uint8).to(dev)
-        self._rows = {}
+        self._native = _lib.native().group(w0.fmt, w0.group_size, len(self.weights), w0.N, w0.K, w0.rank, self._table.data_ptr(),
+                                           0 if self._ut_table is None else self._ut_table.data_ptr())
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
-        w0, P = self.weights[0], len(self.weights)
-        B = x.shape[0]
-        dev = x.device
-        L = _lib.lib()
-        if B not in self._rows:     # every problem reads the same B activation rows
-            self._rows[B] = torch.arange(B, dtype=torch.int32, device=dev).repeat(P)
-        rows = self._rows[B]
-        y = torch.empty(P, B, w0.N, dtype=torch.float16, device=dev)
-        st = _stream_ptr(dev)
-
-        def call(fmt, gs, table, N, K, rank, out, a):
-            m = _lib.MMArgs()
-            if a is not None:
-                m.flags = 1      # GLQ_MM_A_FROM_PREVIOUS_LAUNCH: x.U was launched directly before
-            m.fmt, m.group_size, m.epilogue, m.n_problems, m.max_rows, m.rows_stride = fmt, gs, 0, P, B, B
-            m.N, m.K, m.rank, m.total_rows = N, K, rank, P * B
-            m.w_table = table.data_ptr()
-            m.entry_row = rows.data_ptr()
-            m.x, m.ldx = x.data_ptr(), x.stride(0)
-            if a is not None:
-                m.a0, m.lda = a.data_ptr(), a.shape[-1]
-            m.y, m.ldy = out.data_ptr(), N
-            nbytes, nctr = L.glq_mm_workspace_bytes(C.byref(m)), L.glq_mm_counters(C.byref(m))
-            ws, ctr = workspace(dev, nbytes, nctr)
-            m.workspace, m.workspace_bytes = ws.data_ptr(), ws.numel()
-            m.counters, m.n_counters = ctr.data_ptr(), ctr.numel()
-            _lib.check(L.glq_grouped_matmul(C.byref(m), st), "grouped_matmul")
-
-        with torch.cuda.device(dev):
-            a = None
-            if self._ut_table is not None and w0.rank > 0:
-                a = torch.empty(P, B, w0.rank, dtype=torch.float16, device=dev)
-                call(_lib.FMT_F16, 0, self._ut_table, w0.rank, w0.K, 0, a, None)
-            call(w0.fmt, w0.group_size, self._table, w0.N, w0.K, w0.rank if a is not None else 0, y, a)
-        return y
+        return _lib.native().grouped_linear(self._native, x)

@@ -228,6 +228,14 @@ int glq_linear_forward(int fmt, int group_size, const glq_weight_t* w, const voi
 size_t glq_linear_workspace_bytes(int fmt, int group_size, const glq_weight_t* w, int B);
 size_t glq_linear_counters(int fmt, int group_size, const glq_weight_t* w, int B);
 
+/* The same layer behind a randomized Hadamard rotation (codebook format): y = Q(R(x)) + a . SV^T + bias with
+ * R(x) = glq_rht_forward(x, signs, 1/sqrt(K)) rounded to fp16 and a = x . U of the rows as given.  Arrival counters as
+ * glq_linear_counters. */
+int glq_linear_rht_forward(int fmt, int group_size, const glq_weight_t* w, const void* ut, const float* signs,
+                           const void* x, int64_t ldx, const void* a, void* y, int64_t ldy, int B, void* workspace,
+                           size_t workspace_bytes, int32_t* counters, size_t n_counters, void* stream);
+size_t glq_linear_rht_workspace_bytes(int fmt, int group_size, const glq_weight_t* w, int B);
+
 /* ---------------------------------------------------------------------------------------------
  * MoE block forward (GraphCompatibleMoeBlock.forward, inference/moe_block.py:381-436), entirely on
  * the device: router matmul, softmax in fp32, top-k, optional renormalisation, per-expert token

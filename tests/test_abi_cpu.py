@@ -93,3 +93,20 @@ def test_no_fallback_without_gpu():
     d = cases.make_linear(1, 32, 128, rank=16)
     with pytest.raises((RuntimeError, AssertionError)):
         cases.to_b200_linear(d, device="cpu")
+
+
+def test_native_host_path_binds_and_refuses_cpu_tensors(libpath):
+    import torch
+    from glorcq_b200 import _lib
+    nat = _lib.native()
+    assert set(nat.names()) <= set(_lib.exported_symbols())
+    w = _lib.Weight(None, None, None, None, None, None, 16, 128, 0, 0)
+    layer = nat.layer(_lib.FMT_Q2, 128, bytes(w))
+    with pytest.raises(RuntimeError, match="x must be a CUDA tensor"):
+        nat.linear(layer, torch.zeros(1, 128, dtype=torch.float16), None, None, None)
+    with pytest.raises(RuntimeError, match="x must be fp16"):
+        nat.linear(layer, torch.zeros(1, 128), None, None, None)
+    with pytest.raises(TypeError):
+        nat.linear(layer)
+    with pytest.raises(RuntimeError, match="x_rot must be a CUDA tensor"):
+        nat.turbo_matmul(*[torch.zeros(1, 4, dtype=torch.float16)] * 4)
