@@ -13,6 +13,7 @@
 #include "stream_mm.cuh"
 #include "tc_mm.cuh"
 #include "tc_ps.cuh"
+#include "xu_mm.cuh"
 
 using namespace glq;
 
@@ -442,6 +443,13 @@ static bool tc_disabled() {
     static const bool v = std::getenv("GLQ_NO_TC") != nullptr;
     return v;
 }
+// entries of all problems together: the upper bound that sizes grids and the token operand
+static long long total_entries(const glq_mm_args_t* a) {
+    const long long stride = a->rows_stride > 0 ? a->rows_stride : a->max_rows;
+    const long long total = a->total_rows > 0 ? a->total_rows : (long long)a->n_problems * (a->slot_offset ? a->max_rows : stride);
+    return a->slot_offset ? total : std::max(total, (long long)(a->n_problems - 1) * stride + a->max_rows);
+}
+
 // true when the tcgen05 kernel takes the call: 2-bit affine codes, more rows than the streaming kernel stages
 static bool plan_tc(const glq_mm_args_t* a, TcGeom* out) {
     if (tc_disabled() || a->max_rows <= 32) return false;
@@ -454,9 +462,7 @@ static bool plan_tc(const glq_mm_args_t* a, TcGeom* out) {
         return false;
     }
     TcGeom g{};
-    const long long stride = a->rows_stride > 0 ? a->rows_stride : a->max_rows;
-    long long total = a->total_rows > 0 ? a->total_rows : (long long)a->n_problems * (a->slot_offset ? a->max_rows : stride);
-    if (!a->slot_offset) total = std::max(total, (long long)(a->n_problems - 1) * stride + a->max_rows);
+    const long long total = total_entries(a);
     g.tn = (total / a->n_problems > 64) ? 128 : 64;
     // 256-token tiles: tensor-memory variant, plain epilogue (2-bit codes), long problems only
     static const char* tn_env = std::getenv("GLQ_TC_TN");
@@ -538,10 +544,8 @@ static int launch_tc_ps_t(const TcParams& p, cudaStream_t st) {
     return GLQ_OK;
 }
 
-static int launch_tc(const glq_mm_args_t* a, const TcGeom& g, cudaStream_t st, int min_rows = 0) {
-    if (!a->workspace || a->workspace_bytes < g.xp_bytes) return GLQ_ERR_WORKSPACE;
-    if ((reinterpret_cast<uintptr_t>(a->workspace) & 127u) != 0) return GLQ_ERR_ALIGN;
-    TcParams p{};
+// operands and alignment facts of the many-row kernels; the geometry is filled in by the launchers
+static void fill_tc_operands(const glq_mm_args_t* a, TcParams& p) {
     p.w = a->w;
     p.table = a->w_table;
     p.slot_index = a->slot_index;
@@ -557,26 +561,85 @@ static int launch_tc(const glq_mm_args_t* a, const TcGeom& g, cudaStream_t st, i
     p.lda = a->lda;
     p.y = reinterpret_cast<__half*>(a->y);
     p.ldy = a->ldy;
-    p.xp = reinterpret_cast<unsigned char*>(a->workspace);
-    p.tile_bytes = g.tile_bytes;
     p.n_problems = a->n_problems;
     p.max_rows = a->max_rows;
     p.rows_stride = a->rows_stride > 0 ? a->rows_stride : a->max_rows;
     p.K = a->K;
+    p.N = a->N;
     p.rank = (a->a0 != nullptr) ? a->rank : 0;
+    p.fmt = a->fmt;
+    p.x_vec = ((reinterpret_cast<uintptr_t>(a->x) & 7u) == 0 && a->ldx % 4 == 0) ? 1 : 0;
+    p.x_vec16 = ((reinterpret_cast<uintptr_t>(a->x) & 15u) == 0 && a->ldx % 8 == 0) ? 1 : 0;
+    p.y_vec = ((reinterpret_cast<uintptr_t>(a->y) & 15u) == 0 && a->ldy % 8 == 0 && a->N % 8 == 0) ? 1 : 0;
+}
+
+// Dense products with few columns (xu_mm.cuh).  From 9 rows: up to 8 rows one pass of the skinny kernel takes them all.
+// Up to 512 columns: every 64-column slice reads x again (from L2), and a wide W fills the tcgen05 kernel's tiles.
+static bool xu_takes(const glq_mm_args_t* a) {
+    return a->fmt == GLQ_FMT_F16 && a->max_rows > 8 && a->N > 0 && a->N <= 512 && a->K > 0 && a->K % 8 == 0 && a->n_problems > 0 &&
+           a->epilogue == GLQ_EPI_LINEAR && !a->entry_scale && !(a->rank > 0 && a->a0) && aligned16(a->x) && a->ldx % 8 == 0 &&
+           total_entries(a) / kXuRows + a->n_problems + 1 <= 65535;
+}
+
+static int launch_xu(const glq_mm_args_t* a, cudaStream_t st, bool dependent) {
+    if (!a->w_table && !a->w.codes) return GLQ_ERR_ARG;
+    TcParams p{};
+    fill_tc_operands(a, p);
+    p.nkb = cdiv(a->K, 64);
+    const long long total = total_entries(a);
+    const bool one = a->n_problems == 1 && !a->slot_offset && !a->n_slots;
+    p.tiles_max = one ? cdiv(a->max_rows, kXuRows) : (int)(total / kXuRows + a->n_problems + 1);
+    const int slices = cdiv(a->N, kXuCols);
+    // tiles that will have rows: every problem has one when there are entries enough, whole tiles otherwise
+    const long long live = one ? p.tiles_max : std::max(total / kXuRows, std::min<long long>(a->n_problems, total));
+    // CTAs per tile along K: as many as keep the grid within one wave (two CTAs per SM) and every warp one block of K
+    int cs = 1;
+    while (cs < 8 && live * slices * cs * 2 <= 2 * num_sms() && p.nkb >= 2 * cs * kWarpsPerCta) cs *= 2;
+    static bool configured[64] = {};
+    int dev = 0;
+    GLQ_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        GLQ_CUDA(cudaFuncSetAttribute(xu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kXuSmem));
+        if (dev >= 0 && dev < 64) configured[dev] = true;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cs, slices, p.tiles_max);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kXuSmem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int na = 0;
+    if (cs > 1) {
+        attr[na].id = cudaLaunchAttributeClusterDimension;
+        attr[na].val.clusterDim.x = cs;
+        attr[na].val.clusterDim.y = attr[na].val.clusterDim.z = 1;
+        ++na;
+    }
+    if (dependent) {
+        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[na++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = na;
+    GLQ_CUDA(cudaLaunchKernelEx(&cfg, xu_kernel, p));
+    return GLQ_OK;
+}
+
+static int launch_tc(const glq_mm_args_t* a, const TcGeom& g, cudaStream_t st, int min_rows = 0) {
+    if (!a->workspace || a->workspace_bytes < g.xp_bytes) return GLQ_ERR_WORKSPACE;
+    if ((reinterpret_cast<uintptr_t>(a->workspace) & 127u) != 0) return GLQ_ERR_ALIGN;
+    TcParams p{};
+    fill_tc_operands(a, p);
+    p.xp = reinterpret_cast<unsigned char*>(a->workspace);
+    p.tile_bytes = g.tile_bytes;
     p.nkb = g.nkb;
     p.ns = p.rank > 0 ? g.ns : 0;
     p.na = g.na;
     p.tiles_max = g.tiles_max;
-    p.x_vec = ((reinterpret_cast<uintptr_t>(a->x) & 7u) == 0 && a->ldx % 4 == 0) ? 1 : 0;
-    p.fmt = a->fmt;
     p.min_rows = min_rows;
     const bool sw = a->epilogue == GLQ_EPI_SWIGLU;
     const bool big = g.tn == 128;
-    p.N = a->N;
     p.n_ft = cdiv(a->N, kTcFeat);
-    p.y_vec = ((reinterpret_cast<uintptr_t>(a->y) & 15u) == 0 && a->ldy % 8 == 0 && a->N % 8 == 0) ? 1 : 0;
-    p.x_vec16 = ((reinterpret_cast<uintptr_t>(a->x) & 15u) == 0 && a->ldx % 8 == 0) ? 1 : 0;
     p.tile_ctr = nullptr;
     if (a->fmt == GLQ_FMT_Q2 && !ts_disabled()) {
         p.ts = 1;
@@ -637,6 +700,8 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
     if (a->rank > 0 && (a->a0 || a->a1) && (a->lda % 8 != 0 || !aligned16(a->a0) || !aligned16(a->a1)))
         return GLQ_ERR_ALIGN;
     t_share_sm = (a->flags & GLQ_MM_SHARE_SM) != 0;
+    if (xu_takes(a))
+        return launch_xu(a, reinterpret_cast<cudaStream_t>(stream), (a->flags & GLQ_MM_AFTER_KERNEL) != 0 && !pdl_disabled());
     TcGeom tg;
     const bool use_tc = plan_tc(a, &tg);
     if (use_tc && !tg.hybrid) {

@@ -313,6 +313,20 @@ def test_gptq_i8_dropin(dev, B, N, K, sym, lora):
 
 
 # ---- routes around the packed formats ----------------------------------------------------------------
+@pytest.mark.parametrize("N,K", [(64, 2048), (192, 4096), (8, 264), (72, 64), (512, 1408), (520, 256)])
+def test_dense_few_columns(dev, N, K):
+    """x . W^T on 9 and more rows: row tiles of 32, column slices of 64, K over warps and clusters of CTAs."""
+    from glorcq_b200 import tiled
+    W = torch.randn(N, K, generator=torch.Generator().manual_seed(N + K)).half()
+    tw = tiled.TiledWeight.from_dense(W.to(dev))
+    for B in (9, 32, 33, 333, 5000):
+        x = cases.make_x(B + K, B, K)
+        y = tiled.dense_matmul(tw, x.to(dev))
+        assert cases.rel_l2(y.cpu(), x.float() @ W.float().T) <= REL, B
+        assert torch.equal(y, tiled.dense_matmul(tw, x.to(dev))), B
+    assert tiled.debug_error() is None
+
+
 def test_dense_weight_route_dtype_and_reference_op_names(dev):
     """Pre-dequantised weights (a checkpoint's ``weight_quant`` records and the legacy load_turbo_predequant)
     run dense through the fp16 kernels with the low-rank term; a bf16 / fp32 input gets its own dtype back;
