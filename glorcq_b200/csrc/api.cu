@@ -431,10 +431,6 @@ struct TcGeom {
     long long tile_bytes;
     size_t xp_bytes;
 };
-static bool ts_disabled() {
-    static const bool v = std::getenv("GLQ_NO_TS") != nullptr;
-    return v;
-}
 static bool hybrid_disabled() {
     static const bool v = std::getenv("GLQ_NO_HYBRID") != nullptr;
     return v;
@@ -450,7 +446,7 @@ static long long total_entries(const glq_mm_args_t* a) {
     return a->slot_offset ? total : std::max(total, (long long)(a->n_problems - 1) * stride + a->max_rows);
 }
 
-// true when the tcgen05 kernel takes the call: 2-bit affine codes, more rows than the streaming kernel stages
+// true when a tcgen05 kernel takes the call: more rows than the streaming kernel stages
 static bool plan_tc(const glq_mm_args_t* a, TcGeom* out) {
     if (tc_disabled() || a->max_rows <= 32) return false;
     if (a->N <= 0 || a->K <= 0 || a->n_problems <= 0 || a->rank < 0 || a->rank % 16 != 0) return false;
@@ -464,9 +460,9 @@ static bool plan_tc(const glq_mm_args_t* a, TcGeom* out) {
     TcGeom g{};
     const long long total = total_entries(a);
     g.tn = (total / a->n_problems > 64) ? 128 : 64;
-    // 256-token tiles: tensor-memory variant, plain epilogue (2-bit codes), long problems only
+    // 256-token tiles: packed codes, plain epilogue, long problems only
     static const char* tn_env = std::getenv("GLQ_TC_TN");
-    const bool wide_ok = a->fmt == GLQ_FMT_Q2 && a->epilogue == GLQ_EPI_LINEAR && !ts_disabled();
+    const bool wide_ok = a->fmt != GLQ_FMT_F16 && a->epilogue == GLQ_EPI_LINEAR;
     const int wide_from = tn_env ? std::atoi(tn_env) : 512;      // rows per problem from which the wide tile is used
     if (wide_ok && wide_from > 0 && total / a->n_problems >= wide_from) g.tn = 256;
     g.nkb = cdiv(a->K, 128);
@@ -485,63 +481,55 @@ static bool plan_tc(const glq_mm_args_t* a, TcGeom* out) {
     return true;
 }
 
-template <int FMT, int TN, bool SW>
-static int launch_tc_t(const TcParams& p, int N, cudaStream_t st) {
-    using C = TcCfg<TN, SW>;
-    static bool configured[64] = {};
+template <typename Kern>
+static int allow_smem(Kern kern, bool (&configured)[64], size_t smem) {
     int dev = 0;
     GLQ_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !configured[dev]) {
-        GLQ_CUDA(cudaFuncSetAttribute(tc_kernel<FMT, TN, SW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
+        GLQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
+    return GLQ_OK;
+}
+
+// dense fp16 weights
+template <int TN>
+static int launch_tc_t(const TcParams& p, cudaStream_t st) {
+    using C = TcCfg<TN>;
+    static bool configured[64] = {};
+    const int rc = allow_smem(tc_kernel<TN>, configured, C::SMEM);
+    if (rc != GLQ_OK) return rc;
     tc_pack_b_kernel<TN><<<dim3(p.tiles_max, p.nkb + p.ns), 256, 0, st>>>(p);
     GLQ_CUDA(cudaGetLastError());
-    tc_kernel<FMT, TN, SW><<<dim3(cdiv(N, kTcFeat), p.tiles_max), kTcThreads, C::SMEM, st>>>(p);
+    tc_kernel<TN><<<dim3(p.n_ft, p.tiles_max), kTcThreads, C::SMEM, st>>>(p);
     GLQ_CUDA(cudaGetLastError());
     return GLQ_OK;
 }
 
-// variant with the weight operand in tensor memory (2-bit affine codes)
-template <int TN, bool SW>
-static int launch_tc_ts_t(const TcParams& p, int N, cudaStream_t st) {
-    using C = TcTsCfg<TN, SW>;
+// packed codes: one CTA per SM over all (token tile, feature tile) items
+template <int FMT, int TN, int NM, bool SW>
+static int launch_tc_ps_t(TcParams& p, cudaStream_t st) {
+    using C = TcPsCfg<TN, NM, SW>;
     static bool configured[64] = {};
-    int dev = 0;
-    GLQ_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        GLQ_CUDA(cudaFuncSetAttribute(tc_ts_kernel<TN, SW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
-    tc_pack_b_kernel<TN><<<dim3(p.tiles_max, p.nkb + p.ns), 256, 0, st>>>(p);
-    GLQ_CUDA(cudaGetLastError());
-    tc_ts_kernel<TN, SW><<<dim3(cdiv(N, kTcFeat), p.tiles_max), kTcThreads, C::SMEM, st>>>(p);
-    GLQ_CUDA(cudaGetLastError());
-    return GLQ_OK;
-}
-
-// persistent form of the tensor-memory variant: one CTA per SM over all (token tile, feature tile) items
-static bool ps_disabled() {
-    static const bool v = std::getenv("GLQ_NO_TC_PERSISTENT") != nullptr;
-    return v;
-}
-template <int TN, bool SW>
-static int launch_tc_ps_t(const TcParams& p, cudaStream_t st) {
-    using C = TcPsCfg<TN, SW>;
-    static bool configured[64] = {};
-    int dev = 0;
-    GLQ_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        GLQ_CUDA(cudaFuncSetAttribute(tc_ps_kernel<TN, SW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
+    const int rc = allow_smem(tc_ps_kernel<FMT, TN, NM, SW>, configured, C::SMEM);
+    if (rc != GLQ_OK) return rc;
+    p.n_ft = cdiv(p.N, kTcFeat * C::NOUT);
     tc_pack_b_kernel<TN><<<dim3(p.tiles_max, p.nkb + p.ns), 256, 0, st>>>(p);
     GLQ_CUDA(cudaGetLastError());
     const long work = (long)p.n_ft * p.tiles_max;
-    const int grid = (int)std::min<long>(work, num_sms());
-    tc_ps_kernel<TN, SW><<<grid, kTcThreads, C::SMEM, st>>>(p);
+    tc_ps_kernel<FMT, TN, NM, SW><<<(int)std::min<long>(work, num_sms()), kPsThreads, C::SMEM, st>>>(p);
     GLQ_CUDA(cudaGetLastError());
     return GLQ_OK;
+}
+// live_tiles: token tiles that will have rows, as far as the host can tell
+template <int FMT>
+static int launch_tc_ps(TcParams& p, int tn, bool sw, long live_tiles, cudaStream_t st) {
+    if (tn == 256) return launch_tc_ps_t<FMT, 256, 1, false>(p, st);
+    if (tn == 128) return sw ? launch_tc_ps_t<FMT, 128, 2, true>(p, st) : launch_tc_ps_t<FMT, 128, 1, false>(p, st);
+    if (sw) return launch_tc_ps_t<FMT, 64, 2, true>(p, st);
+    // 256 features per item cost the producers fewer instructions per code; below two items per SM they leave SMs idle
+    if (live_tiles * cdiv(p.N, 2 * kTcFeat) >= 2 * num_sms()) return launch_tc_ps_t<FMT, 64, 2, false>(p, st);
+    return launch_tc_ps_t<FMT, 64, 1, false>(p, st);
 }
 
 // operands and alignment facts of the many-row kernels; the geometry is filled in by the launchers
@@ -568,7 +556,6 @@ static void fill_tc_operands(const glq_mm_args_t* a, TcParams& p) {
     p.N = a->N;
     p.rank = (a->a0 != nullptr) ? a->rank : 0;
     p.fmt = a->fmt;
-    p.x_vec = ((reinterpret_cast<uintptr_t>(a->x) & 7u) == 0 && a->ldx % 4 == 0) ? 1 : 0;
     p.x_vec16 = ((reinterpret_cast<uintptr_t>(a->x) & 15u) == 0 && a->ldx % 8 == 0) ? 1 : 0;
     p.y_vec = ((reinterpret_cast<uintptr_t>(a->y) & 15u) == 0 && a->ldy % 8 == 0 && a->N % 8 == 0) ? 1 : 0;
 }
@@ -638,32 +625,15 @@ static int launch_tc(const glq_mm_args_t* a, const TcGeom& g, cudaStream_t st, i
     p.tiles_max = g.tiles_max;
     p.min_rows = min_rows;
     const bool sw = a->epilogue == GLQ_EPI_SWIGLU;
-    const bool big = g.tn == 128;
     p.n_ft = cdiv(a->N, kTcFeat);
-    p.tile_ctr = nullptr;
-    if (a->fmt == GLQ_FMT_Q2 && !ts_disabled()) {
-        p.ts = 1;
-        if (!ps_disabled()) {
-            p.tile_ctr = reinterpret_cast<int*>(p.xp + (g.xp_bytes - 256));
-            if (g.tn == 256) return launch_tc_ps_t<256, false>(p, st);
-            if (big) return sw ? launch_tc_ps_t<128, true>(p, st) : launch_tc_ps_t<128, false>(p, st);
-            return sw ? launch_tc_ps_t<64, true>(p, st) : launch_tc_ps_t<64, false>(p, st);
-        }
-        if (g.tn == 256) return launch_tc_ts_t<256, false>(p, a->N, st);
-        if (big) return sw ? launch_tc_ts_t<128, true>(p, a->N, st) : launch_tc_ts_t<128, false>(p, a->N, st);
-        return sw ? launch_tc_ts_t<64, true>(p, a->N, st) : launch_tc_ts_t<64, false>(p, a->N, st);
-    }
+    if (a->fmt == GLQ_FMT_F16) return g.tn == 128 ? launch_tc_t<128>(p, st) : launch_tc_t<64>(p, st);
+    p.ts = 1;
+    const long live_tiles = std::max<long>(total_entries(a) / g.tn, std::min<long>(a->n_problems, total_entries(a)));
+    p.tile_ctr = reinterpret_cast<int*>(p.xp + (g.xp_bytes - 256));
     switch (a->fmt) {
-#define GLQ_TC_CASE(F)                                                                                       \
-    case F:                                                                                                  \
-        if (big) return sw ? launch_tc_t<F, 128, true>(p, a->N, st) : launch_tc_t<F, 128, false>(p, a->N, st); \
-        return sw ? launch_tc_t<F, 64, true>(p, a->N, st) : launch_tc_t<F, 64, false>(p, a->N, st);
-        GLQ_TC_CASE(GLQ_FMT_Q2)
-        GLQ_TC_CASE(GLQ_FMT_Q4)
-        GLQ_TC_CASE(GLQ_FMT_T2)
-#undef GLQ_TC_CASE
-        case GLQ_FMT_F16:
-            return big ? launch_tc_t<GLQ_FMT_F16, 128, false>(p, a->N, st) : launch_tc_t<GLQ_FMT_F16, 64, false>(p, a->N, st);
+        case GLQ_FMT_Q2: return launch_tc_ps<GLQ_FMT_Q2>(p, g.tn, sw, live_tiles, st);
+        case GLQ_FMT_Q4: return launch_tc_ps<GLQ_FMT_Q4>(p, g.tn, sw, live_tiles, st);
+        case GLQ_FMT_T2: return launch_tc_ps<GLQ_FMT_T2>(p, g.tn, sw, live_tiles, st);
     }
     return GLQ_ERR_UNSUPPORTED;
 }

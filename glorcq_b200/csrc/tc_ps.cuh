@@ -1,20 +1,38 @@
 // SPDX-License-Identifier: Apache-2.0
 //
-// Persistent form of the tensor-memory dequant-GEMM (2-bit affine codes, tc_ts_kernel).
+// Grouped dequant-GEMM with the weight operand in tensor memory: 2-bit, 4-bit and codebook codes.
+//
+// An SS-operand MMA reads both operands from shared memory (8 KB per 128x128x16 instruction, the whole
+// 128 B/clk port) while producers would store the unpacked weights and the bulk copy write the token
+// operand through the same port.  Here the producers write the unpacked fp16 values straight into
+// tensor memory (tcgen05.st, 16 lanes x 256 bit shape, which matches the (g, t) ownership of the code
+// tiles: lane (g, t) holds rows g and g+8 and four consecutive K positions of every 16) and the MMA
+// takes A from there; only the token operand uses shared memory.
+//
+// Tensor memory (512 columns): accumulators first (TN columns, twice for gate|up), then a ring of S
+// stages of 64 columns (128 K positions x fp16) per matrix.
 //
 // One CTA per SM works through the list of (token tile, 128-feature tile) items; the warps keep their roles
 // over all of a CTA's items, so barrier set-up, the TMEM allocation and the pipeline fill are paid once per
-// CTA instead of once per tile.  Roles, stage layout and the epilogue arithmetic are those of tc_ts_kernel:
-// 16 producer warps unpack the codes of a 128-channel stage into the tensor-memory ring, one warp issues
-// the MMAs, one thread bulk-copies the token operand.
+// CTA instead of once per tile.  16 producer warps unpack the codes of a 128-channel stage into the
+// tensor-memory ring, one warp issues the MMAs, one bulk-copies the token operand.
 //
-//  * Work items are drawn from a grid-wide counter (zeroed by the pre-pass) by the loader warp and handed
-//    to the other warps through a small queue in shared memory, so an SM that runs faster takes more items.
+//  * Work items are drawn from a grid-wide counter (zeroed by the pre-pass) by the loader warp one item ahead;
+//    it looks the problem up and hands the operands' addresses to the other warps through a small queue in
+//    shared memory, so an SM that runs faster takes more items and nobody else walks the dependent loads.
 //  * The rings run on across item boundaries: the loader fetches the next item's token operand while the
-//    producers still finish the current one.
+//    producers still finish the current one, and the producers request the next item's first codes before
+//    they turn to the finished accumulator.
 //  * A finished accumulator is read into registers (epilogue arithmetic, fp16 pairs) and released at once;
 //    the results go to y after the weight ring of the next item is full again, through a staging tile in
 //    shared memory ([token][feature], two passes) with 16-byte row-contiguous stores.
+//
+// What bounds it: with few tokens per problem (an expert of a prompt sees some tens of rows) the producers' issue
+// slots.  A first form spent 253 instructions per warp, matrix and stage (one shift per pair of codes, both
+// roundings of the dequantisation computed and one selected, every warp looking up its item): 142 us for the gate|up
+// product of 60 experts x 34 rows (1408 x 2048, 2-bit), scheduler slots 57 % used, DRAM 12 %.  Now 140 instructions
+// and 99 us; 97 -> 60 us for the down product (2048 x 1408).  The half-precision and the integer pipes (one warp
+// instruction every two cycles each) are 60 % busy; the unpack alone, without the loop around it, would take 55 us.
 //
 // Every wait is bounded (tc_wait); a wait that runs out marks the CTA dead, all roles leave their loops
 // and the kernel ends.
@@ -22,44 +40,161 @@
 
 #include "tc_mm.cuh"
 
-#ifndef GLQ_PS_FLUSH_AT
-#define GLQ_PS_FLUSH_AT (S - 1)
-#endif
-#ifndef GLQ_PS_FLUSH_GAP
-#define GLQ_PS_FLUSH_GAP 0
-#endif
-
 namespace glq {
 
 constexpr int kPsQueue = 4;        // work items the loader may be ahead of the slowest warp
 
-template <int TN, bool SW> struct TcPsCfg {
-    using T = TcTsCfg<TN, SW>;
-    static constexpr int NH = TN >= 128 ? 2 : 1;                 // the results leave in NH passes over a staging tile
-    static constexpr int TH = TN / NH;                           // tokens per pass
-    static constexpr int OUT_BYTES = TH * 256;                   // staged results [TH][128] fp16
-    static constexpr size_t SMEM = (size_t)T::S * T::B_BYTES + OUT_BYTES + 1024;
-    static_assert(SMEM <= 227 * 1024, "shared memory");
+__device__ __forceinline__ void tc_st_x4(uint32_t taddr, const uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.16x256b.x4.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tc_st_x2(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
+                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+__device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D (TMEM) += A (TMEM, 128 lanes x 8 columns = 16 fp16 per row) * B (shared memory descriptor).  The whole warp comes here
+// with the same operands and one elected lane issues: in code that one lane runs alone the operands of every instruction go
+// through R2UR, and the issuing warp, not the tensor pipe, set the pace (113 to 117 cycles per MMA of any N up to 128).
+__device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n .reg .pred p, e;\n setp.ne.b32 p, %4, 0;\n elect.sync _|e, 0xffffffff;\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(acc)
+        : "memory");
+}
+__device__ __forceinline__ void tc_commit_warp(uint32_t bar) {
+    asm volatile(
+        "{\n .reg .pred e;\n elect.sync _|e, 0xffffffff;\n"
+        " @e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar)
+        : "memory");
+}
+
+constexpr int kPsRows = 64;                                      // tokens of a result pass
+constexpr int kPsOut = kPsRows * 256;                            // its staging tile [token][128 features] fp16, two of them
+constexpr int kPsThreads = (kTcProducers + 3) * 32;
+
+template <int TN, int NM, bool SW> struct TcPsCfg {
+    static constexpr int NOUT = SW ? 1 : NM;                     // 128-feature output tiles of an item
+    static constexpr int ACC = NM * TN;                          // accumulator columns
+    static constexpr int B_BYTES = TN * 256;
+    static constexpr int NPASS = NOUT * (TN / kPsRows);          // passes in which an item's results leave
+    // ring stages: what tensor memory and shared memory both hold, at most 6
+    static constexpr int S_TMEM = (512 - ACC) / (NM * 64), S_SMEM = (225 * 1024 - 2 * kPsOut) / B_BYTES;
+    static constexpr int S0 = S_TMEM < S_SMEM ? S_TMEM : S_SMEM, S = S0 < 6 ? S0 : 6;
+    static constexpr size_t SMEM = (size_t)S * B_BYTES + 2 * kPsOut + 1024;
+    static_assert(S >= 2 && SMEM <= 227 * 1024, "shared memory");
 };
 
-template <int TN, bool SW>
-__global__ void __launch_bounds__(kTcThreads, 1) tc_ps_kernel(const TcParams p) {
-    using C = TcTsCfg<TN, SW>;
-    using P = TcPsCfg<TN, SW>;
-    constexpr int S = C::S, NM = C::NM;
+// tc_wait of a whole warp: the barrier is tried before anything else is looked at (the common case costs one instruction)
+__device__ __forceinline__ bool ps_wait_warp(uint32_t bar, uint32_t parity, volatile int* dead, int code) {
+    return __all_sync(0xffffffffu, mbar_try_wait(bar, parity) || tc_wait(bar, parity, dead, code));
+}
+
+// A work item as the loader hands it out; ft < 0 ends the list.
+struct PsItem {
+    const unsigned char *codes, *sv;
+    const __half* bias;
+    const float *norms, *centroids;
+    int ft, lt, cnt, e0;
+};
+
+// One row's 16 codes of a stage -> eight fp16 pairs in K position order (tc_ts_channel_of).
+// Affine codes: the code bits are put into the mantissa of an fp16 number of a known offset, one subtraction of
+// offset + z -- exact for every zero point that the sum keeps whole, which integer zero points, the quantizer's
+// output, always are -- yields fp16(q - z), one product the same fp16(fp16(q - z) * s) as the reference's tiles.
+// Three instructions per pair; another zero point takes (offset + code - offset) - z.
+template <int FMT> struct PsUnpack;
+template <> struct PsUnpack<GLQ_FMT_Q2> {
+    static __device__ __forceinline__ constexpr float off(int c) { return c == 0 ? 64.f : (c == 1 ? 16.f : 4.f); }
+    static constexpr float kTop = 64.f;        // the largest offset
+    // offset class of pair j (see unpack_q2)
+    static __device__ __forceinline__ constexpr int cls(int j) { return (j == 4 || j == 7) ? 2 : ((j == 1 || j == 3 || j == 6) ? 1 : 0); }
+    static __device__ __forceinline__ void pairs(const uint32_t (&w)[2], uint32_t (&h)[8]) { unpack_q2(w[0], h); }
+};
+template <> struct PsUnpack<GLQ_FMT_Q4> {
+    static __device__ __forceinline__ constexpr float off(int c) { return c == 0 ? 1024.f : 64.f; }
+    static constexpr float kTop = 1024.f;
+    static __device__ __forceinline__ constexpr int cls(int j) { return j & 1; }
+    // pair j of a word = codes (j, j + 4): nibbles 0, 4 at mantissa bit 0, nibbles 1, 5 at bit 4, the rest after one shift
+    static __device__ __forceinline__ void pairs(const uint32_t (&w)[2], uint32_t (&h)[8]) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const uint32_t v = w[u], v8 = w[u] >> 8;
+            h[4 * u + 0] = and_or(v, 0x000F000Fu, 0x64006400u);
+            h[4 * u + 1] = and_or(v, 0x00F000F0u, 0x54005400u);
+            h[4 * u + 2] = and_or(v8, 0x000F000Fu, 0x64006400u);
+            h[4 * u + 3] = and_or(v8, 0x00F000F0u, 0x54005400u);
+        }
+    }
+};
+
+// Both rows (g, g + 8) of a lane: words w[row][..], (scale, zero) pairs sz[row] -> the 16 registers of tc_st_x4.
+template <int FMT>
+__device__ __forceinline__ void ps_affine(const uint32_t (&w)[2][2], const uint32_t (&sz)[2], uint32_t (&r)[16]) {
+    using U = PsUnpack<FMT>;
+    const uint32_t zb = __byte_perm(sz[0], sz[1], 0x7632);        // (z of row g, z of row g + 8)
+    const __half2 z2 = *reinterpret_cast<const __half2*>(&zb);
+    __half2 zo[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) zo[i] = __hadd2(z2, __float2half2_rn(U::off(i)));
+    // the largest offset keeps every bit of both zero points (the smaller ones then do, for |z| <= 1024)
+    const __half2 top = __hadd2(z2, __float2half2_rn(U::kTop));
+    const bool whole = __hbeq2(__hsub2(top, __float2half2_rn(U::kTop)), z2) && __hble2(__habs2(z2), __float2half2_rn(1024.f));
+    const bool fast = __all_sync(0xffffffffu, whole);
+#pragma unroll
+    for (int hrow = 0; hrow < 2; ++hrow) {
+        uint32_t h[8];
+        U::pairs(w[hrow], h);
+        const __half2 s2 = __half2half2(__ushort_as_half((unsigned short)(sz[hrow] & 0xffffu)));
+        if (fast) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const __half2 zc = zo[U::cls(j)];
+                const __half2 zr = hrow ? __high2half2(zc) : __low2half2(zc);
+                const __half2 v = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&h[j]), zr), s2);
+                r[4 * (j >> 1) + 2 * hrow + (j & 1)] = *reinterpret_cast<const uint32_t*>(&v);
+            }
+        } else {
+            const __half2 zr = hrow ? __high2half2(z2) : __low2half2(z2);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const __half2 q = __hsub2(*reinterpret_cast<const __half2*>(&h[j]), __float2half2_rn(U::off(U::cls(j))));
+                const __half2 v = __hmul2(__hsub2(q, zr), s2);
+                r[4 * (j >> 1) + 2 * hrow + (j & 1)] = *reinterpret_cast<const uint32_t*>(&v);
+            }
+        }
+    }
+}
+
+// NM = 2: an item is 128 features of gate and of up (SW), or two adjacent 128-feature tiles of a plain product; a producer
+// warp then unpacks all 128 channels of its 16-row tile of one matrix.  NM = 1 (few items, or token tiles so wide that one
+// accumulator fills half of tensor memory): two warps share a tile, one per half of the lanes' channels.
+template <int FMT, int TN, int NM, bool SW>
+__global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) {
+    using C = TcPsCfg<TN, NM, SW>;
+    constexpr int S = C::S;
+    static_assert(!SW || NM == 2, "gate|up items hold two matrices");
+    constexpr bool AFFINE = FMT != GLQ_FMT_T2;
+    constexpr int BB = FMT == GLQ_FMT_T2 ? 512 : 576;       // bytes of a (tile, k block)
+    constexpr int HALVES = NM;                              // halves of the lanes' channels that a warp unpacks
     extern __shared__ unsigned char tc_smem_raw[];
-    __shared__ __align__(8) unsigned long long bars[2 * S + 4 + 2 * kPsQueue];
+    __shared__ __align__(8) unsigned long long bars[2 * S + 6 + 2 * kPsQueue];
     __shared__ uint32_t s_tmem;
     __shared__ int s_dead;
-    __shared__ int s_tile[kPsQueue];          // work items in the order the loader drew them; -1 ends the list
+    __shared__ PsItem s_item[kPsQueue];       // work items in the order the loader drew them
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t sbase = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
-    const uint32_t obase = sbase + (uint32_t)S * C::B_BYTES;      // staging tile of the results
+    const uint32_t obase = sbase + (uint32_t)S * C::B_BYTES;      // two staging tiles of the results
     const uint32_t bar_full = smem_u32(bars), bar_empty = bar_full + 8 * S;
     const uint32_t bar_acc = bar_full + 16 * S, bar_acc_free = bar_acc + 8;
-    const uint32_t bar_drained = bar_acc + 16, bar_stored = bar_acc + 24;   // staging tile written / read by all producers
-    const uint32_t bar_tq_full = bar_acc + 32, bar_tq_empty = bar_tq_full + 8 * kPsQueue;
+    const uint32_t bar_staged = bar_acc + 16, bar_stored = bar_acc + 32;   // per staging tile: written by the producers / read
+    const uint32_t bar_tq_full = bar_acc + 48, bar_tq_empty = bar_tq_full + 8 * kPsQueue;
     volatile int* dead = &s_dead;
 
     if (threadIdx.x == 0) {
@@ -69,11 +204,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_ps_kernel(const TcParams p) 
         }
         mbar_init(bar_acc, 1);
         mbar_init(bar_acc_free, kTcProducers);
-        mbar_init(bar_drained, kTcProducers);
-        mbar_init(bar_stored, kTcProducers);
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(bar_staged + 8 * i, kTcProducers);
+            mbar_init(bar_stored + 8 * i, 1);
+        }
         for (int i = 0; i < kPsQueue; ++i) {
             mbar_init(bar_tq_full + 8 * i, 1);
-            mbar_init(bar_tq_empty + 8 * i, kTcProducers + 1);
+            mbar_init(bar_tq_empty + 8 * i, kTcProducers + 2);
         }
         s_dead = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -89,314 +226,385 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_ps_kernel(const TcParams p) 
     const bool has_lr = p.rank > 0 && p.a[0] != nullptr;
     const int nst = p.nkb + (has_lr ? p.ns : 0);
     const int n_work = p.n_ft * p.tiles_max;
-    // next work item of this CTA (every consumer warp calls it with all lanes): -1 = none left or the CTA is dead
-    auto next_item = [&](int n) -> int {
+    // Work item n of this CTA (all lanes of a consumer warp call it): false when there is none left, or the CTA is dead.
+    // Its slot is the caller's until release_item.
+    auto have_item = [&](int n) -> bool {
         const int qi = n % kPsQueue;
         const bool got = __all_sync(0xffffffffu, tc_wait(bar_tq_full + 8 * qi, (uint32_t)((n / kPsQueue) & 1), dead, 108));
-        int wk = -1;
-        if (got) wk = *reinterpret_cast<volatile int*>(&s_tile[qi]);
+        return got && s_item[qi].ft >= 0;
+    };
+    auto release_item = [&](int n) {
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_tq_empty + 8 * qi);
-        return wk;
+        if (lane == 0) mbar_arrive(bar_tq_empty + 8 * (n % kPsQueue));
     };
 
     if (warp < kTcProducers) {
         // ================= producers: unpack into tensor memory, then the tile's epilogue =================
         const int g = lane >> 2, t = lane & 3;
-        const int q = warp & 3, sub = warp >> 2;
-        const int tl = 2 * q + (sub & 1), wh = sub >> 1;
+        const int q = warp & 3, sub = warp >> 2;                   // a warp reaches the tensor-memory lanes of its quarter q
+        const int tl = 2 * q + (sub & 1);                          // its 16-row tile of the 128
+        const int mx = NM == 2 ? sub >> 1 : 0, wh0 = NM == 2 ? 0 : sub >> 1;   // its matrix / its half of the channels
         const uint32_t lane_base = (uint32_t)(16 * tl) << 16;
+        const int nblk = FMT == GLQ_FMT_Q4 ? (p.K + 63) / 64 : p.nkb;
         int s = 0;
         uint32_t ph = 0;
-        int it = 0;
-        const int part = warp >> 2;                                // quarter of a pass's token columns
-        const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
-        const uint32_t orow = obase + (uint32_t)(q * 32 + lane) * 2u;
-        // results of the tile before, fp16 pairs of this thread's feature: columns h*TH + part*TH/4 + 2i, +1
-        constexpr int PK = TN / 8;
-        constexpr int kFlushAt = GLQ_PS_FLUSH_AT, kFlushGap = GLQ_PS_FLUSH_GAP;
-        uint32_t packed[PK];
-        bool st_ok = true;
-        int pv_ft = 0, pv_lt = 0, pv_cnt = 0, pv_e0 = 0, pass = 0;
-
-        // write the held results to y: per pass, staging tile [token][feature] in shared memory, then 16 lanes
-        // per 256-byte token row; bounded handshakes between the sixteen warps around the staging tile
-        int pend = 0;                 // passes of the tile before that are still to be written
-        auto flush_pass = [&]() {
-            const int f0 = pv_ft * kTcFeat;
-            const int nf = min(kTcFeat, N - f0);
-            const int hcur = P::NH - pend;
-            if (pass > 0) st_ok = __all_sync(0xffffffffu, st_ok && tc_wait(bar_stored, (uint32_t)((pass - 1) & 1), dead, 106));
-#pragma unroll
-            for (int h = 0; h < P::NH; ++h) {
-                if (h == hcur) {
-#pragma unroll
-                    for (int i = 0; i < P::TH / 8; ++i) {
-                        const uint32_t v = packed[h * (P::TH / 8) + i];
-                        const uint32_t a = orow + (uint32_t)(part * (P::TH / 4) + 2 * i) * 256u;
-                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(a), "h"((unsigned short)(v & 0xffffu)) : "memory");
-                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(a + 256u), "h"((unsigned short)(v >> 16)) : "memory");
-                    }
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_drained);
-            st_ok = __all_sync(0xffffffffu, st_ok && tc_wait(bar_drained, (uint32_t)(pass & 1), dead, 107));
-            if (st_ok) {
-                const int tid = threadIdx.x;
-                for (int r = tid >> 4; r < P::TH; r += kTcProducers * 2) {
-                    const int rr = pv_lt * TN + hcur * P::TH + r;
-                    if (rr >= pv_cnt) break;
-                    const int c8 = (tid & 15) * 8;
-                    __half* dst = p.y + (size_t)(pv_e0 + rr) * p.ldy + f0 + c8;
-                    if (p.y_vec) {
-                        if (c8 < nf) *reinterpret_cast<uint4*>(dst) = lds128(obase + (uint32_t)r * 256u + (uint32_t)c8 * 2u);
-                    } else {
-                        for (int i = 0; i < 8 && c8 + i < nf; ++i) {
-                            unsigned short hv;
-                            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hv) : "r"(obase + (uint32_t)r * 256u + (uint32_t)(c8 + i) * 2u) : "memory");
-                            dst[i] = __ushort_as_half(hv);
-                        }
-                    }
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_stored);
-            ++pass;
-            --pend;
-        };
-
-        for (;;) {
-            const int wk = next_item(it);
-            if (wk < 0) break;
-            const int gt = wk / p.n_ft, ft = wk - gt * p.n_ft;
-            int slot, lt, cnt, e0;
-            if (!tc_find_tile<TN>(p, gt, slot, lt, cnt, e0)) break;        // the loader publishes live tiles only
-            const int widx = p.slot_index ? __ldg(p.slot_index + slot) : slot;
-            const glq_weight_t W = p.table ? p.table[widx] : p.w;
-            const int tile16 = ft * 8 + tl;
-            const bool live = tile16 < (N + 15) / 16;
-            const unsigned char* blk[NM];
-#pragma unroll
-            for (int m = 0; m < NM; ++m) {
-                const int d = SW ? tile16 * 2 + m : tile16;
-                blk[m] = reinterpret_cast<const unsigned char*>(W.codes) + ((size_t)(d >> 1) * p.nkb * 2 + (d & 1)) * 576;
-            }
-            constexpr int D = 4;
-            uint32_t cq[D][NM][2], csz[D][NM][2];     // word `wh` of row g and of row g+8; their (scale, zero) pairs
-            auto fetch = [&](int st, uint32_t (&qv)[NM][2], uint32_t (&zv)[NM][2]) {
-#pragma unroll
-                for (int m = 0; m < NM; ++m) {
-                    const bool in = live && st < p.nkb;
-                    const unsigned char* src = blk[m] + (size_t)st * 2 * 576;
-                    const uint32_t* wsrc = reinterpret_cast<const uint32_t*>(src) + lane * 4 + wh;
-                    qv[m][0] = in ? __ldg(wsrc) : 0u;
-                    qv[m][1] = in ? __ldg(wsrc + 2) : 0u;
-                    const uint2 z = in ? __ldg(reinterpret_cast<const uint2*>(src + 512) + g) : make_uint2(0, 0);
-                    zv[m][0] = z.x;
-                    zv[m][1] = z.y;
-                }
-            };
-#pragma unroll
-            for (int d = 0; d < D; ++d) fetch(d, cq[d], csz[d]);
-
-            bool ok = true;
-            for (int st0 = 0; st0 < nst; st0 += D) {
-#pragma unroll
-                for (int d = 0; d < D; ++d) {
-                    const int st = st0 + d;
-                    if (st < nst) {
-                        ok = __all_sync(0xffffffffu, ok && tc_wait(bar_empty + 8 * s, ph ^ 1u, dead, 100));
-                        tc_fence_after();
-                        const uint32_t acol = ring + (uint32_t)(s * NM * 64);
-                        if (ok && st < p.nkb) {
-#pragma unroll
-                            for (int m = 0; m < NM; ++m) {
-                                // regs of repeat n: {row g: positions 4t..4t+3 of k step 4*wh + n}, {row g+8: the same}
-                                uint32_t r[16];
-#pragma unroll
-                                for (int hrow = 0; hrow < 2; ++hrow) {
-                                    const TcAffine af(csz[d][m][hrow], 1024.f);
-                                    const uint32_t w = cq[d][m][hrow];
-#pragma unroll
-                                    for (int n = 0; n < 4; ++n)
-#pragma unroll
-                                        for (int e = 0; e < 2; ++e) {
-                                            const uint32_t h = and_or(w >> (2 * (2 * n + e)), 0x00030003u, 0x64006400u);
-                                            r[4 * n + 2 * hrow + e] = af.integral ? af.exact(h) : af.general(h);
-                                        }
-                                }
-                                tc_st_x4(acol + (uint32_t)(m * 64 + wh * 32) + lane_base, r);
-                            }
-                            fetch(st + D, cq[d], csz[d]);
-                        } else if (ok) {
-                            // low-rank stage: SV rows in natural K order; this warp stores k steps 2*wh, 2*wh+1
-                            const int sl = st - p.nkb;
-#pragma unroll
-                            for (int m = 0; m < NM; ++m) {
-                                const int dt = SW ? tile16 * 2 + m : tile16;
-                                uint32_t r[8];
-#pragma unroll
-                                for (int n = 0; n < 2; ++n)
-#pragma unroll
-                                    for (int hrow = 0; hrow < 2; ++hrow) {
-                                        const int row = g + 8 * hrow;
-                                        const uint2* src = reinterpret_cast<const uint2*>(
-                                            reinterpret_cast<const unsigned char*>(W.sv) +
-                                            ((((size_t)(dt >> 1) * p.ns + sl) * 32) + (dt & 1) * 16 + row) * 128 +
-                                            (2 * wh + n) * 32 + t * 8);
-                                        const uint2 v = (live && W.sv) ? __ldg(src) : make_uint2(0, 0);
-                                        r[4 * n + 2 * hrow] = v.x;
-                                        r[4 * n + 2 * hrow + 1] = v.y;
-                                    }
-                                tc_st_x2(acol + (uint32_t)(m * 64 + wh * 16) + lane_base, r);
-                            }
-                        }
-                        tc_st_wait();
-                        tc_fence_before();
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar_full + 8 * s);
-                        if (++s == S) {
-                            s = 0;
-                            ph ^= 1u;
-                        }
-                        // the ring is full again: the tensor pipe has work while the tile before goes to memory
-                        if (pend > 0 && st == kFlushAt + kFlushGap * (P::NH - pend)) flush_pass();
-                    }
-                }
-            }
-            while (pend > 0) flush_pass();     // tiles with few stages
-
-            // ---- accumulator -> registers (epilogue arithmetic, fp16 pairs); then it is free for the next tile ----
-            const bool acc_ok = __all_sync(0xffffffffu, ok && tc_wait(bar_acc, (uint32_t)(it & 1), dead, 101));
+        // ---- results of item n: accumulator -> epilogue arithmetic -> staging tile [token][feature], 64 tokens per pass;
+        // the store warp takes the tiles from there.  Done while the ring of item n + 1 is already full, so that neither the
+        // producers wait for the last products of item n nor the tensor pipe for the producers.
+        const int part = warp >> 2;                                // this warp's 16 tokens of a pass
+        const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(part * 16);
+        const uint32_t orow = obase + (uint32_t)(part * 16) * 256u + (uint32_t)(q * 32 + lane) * 2u;
+        int pass = 0;
+        auto results = [&](int n) -> bool {
+            const volatile PsItem& im = s_item[n % kPsQueue];
+            bool ok = ps_wait_warp(bar_acc, (uint32_t)(n & 1), dead, 101);
             tc_fence_after();
-            {
-                const int f = ft * kTcFeat + q * 32 + lane;
-                const __half* bias = reinterpret_cast<const __half*>(W.bias);
+#pragma unroll
+            for (int h = 0; h < C::NPASS; ++h) {
+                const int o = h / (TN / kPsRows), c0 = (h % (TN / kPsRows)) * kPsRows;
+                const int f = (im.ft * C::NOUT + o) * kTcFeat + q * 32 + lane;
+                uint32_t vg[16], vu[16];
+                tc_ld16(trow + (uint32_t)(o * TN + c0), vg);
+                if (SW) tc_ld16(trow + (uint32_t)(TN + c0), vu);
+                const __half* bias = im.bias;
                 const float bv = (!SW && bias && f < N) ? __half2float(__ldg(bias + f)) : 0.f;
-#pragma unroll
-                for (int h = 0; h < P::NH; ++h) {
-#pragma unroll
-                    for (int k = 0; k < P::TH / 64; ++k) {
-                        const int c0 = h * P::TH + part * (P::TH / 4) + 16 * k;
-                        uint32_t vg[16], vu[16];
-                        tc_ld16(trow + (uint32_t)c0, vg);
-                        if (SW) tc_ld16(trow + (uint32_t)(TN + c0), vu);
-                        tc_ld_wait();
-                        if (!SW && !bias && !p.entry_scale) {
-                            // plain product: one rounding, two values per conversion
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                const __half2 h2 = __floats2half2_rn(__uint_as_float(vg[2 * j]), __uint_as_float(vg[2 * j + 1]));
-                                packed[h * (P::TH / 8) + 8 * k + j] = *reinterpret_cast<const uint32_t*>(&h2);
-                            }
-                        } else {
-                            unsigned short hv[16];
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                const int rr = lt * TN + c0 + j;
-                                float v = round16(__uint_as_float(vg[j]));
-                                if (SW) {
-                                    v = round16(silu16(v) * round16(__uint_as_float(vu[j])));
-                                } else {
-                                    if (bias) v = round16(v + bv);
-                                    if (p.entry_scale && rr < cnt) v = round16(__half2float(__ldg(p.entry_scale + e0 + rr)) * v);
-                                }
-                                hv[j] = __half_as_ushort(__float2half_rn(v));
-                            }
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                packed[h * (P::TH / 8) + 8 * k + j] = (uint32_t)hv[2 * j] | ((uint32_t)hv[2 * j + 1] << 16);
-                        }
+                float nrm_g = 1.f, nrm_u = 1.f;     // codebook format: per-row norms, in tile order
+                if constexpr (!AFFINE) {
+                    if (f < N) {
+                        const int t16 = f >> 4, r16 = f & 15;
+                        nrm_g = __ldg(im.norms + (size_t)(SW ? 2 * t16 : t16) * 16 + r16);
+                        if (SW) nrm_u = __ldg(im.norms + (size_t)(2 * t16 + 1) * 16 + r16);
                     }
                 }
+                const int b = pass & 1;
+                if (pass > 1) ok = ps_wait_warp(bar_stored + 8 * b, (uint32_t)((pass >> 1) & 1) ^ 1u, dead, 106) && ok;
+                tc_ld_wait();
+                const uint32_t dst = orow + (uint32_t)(b * kPsOut);
+                const int r0 = im.lt * TN + c0 + part * 16, cnt = im.cnt;
+                const __half* scale = SW || !p.entry_scale ? nullptr : p.entry_scale + im.e0 + r0;
+                if (ok && r0 < cnt) {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        float v = __uint_as_float(vg[j]);
+                        if constexpr (!AFFINE) v *= nrm_g;
+                        if constexpr (SW) {
+                            float u = __uint_as_float(vu[j]);
+                            if constexpr (!AFFINE) u *= nrm_u;
+                            v = silu16(round16(v)) * round16(u);
+                        } else {
+                            if (bias) v = round16(v) + bv;
+                            if (scale && r0 + j < cnt) v = __half2float(__ldg(scale + j)) * round16(v);
+                        }
+                        const unsigned short hv = __half_as_ushort(__float2half_rn(v));
+                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(dst + (uint32_t)j * 256u), "h"(hv) : "memory");
+                    }
+                }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_staged + 8 * b);
+                ++pass;
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar_acc_free);
-            pend = P::NH;
-            pv_ft = ft;
-            pv_lt = lt;
-            pv_cnt = cnt;
-            pv_e0 = e0;
-            ++it;
-            if (!acc_ok || !st_ok) break;
+            release_item(n);
+            return ok;
+        };
+
+        // ---- codes: requested D stages ahead (the first ones of an item before the previous item's epilogue).  Lane (g, t)
+        // holds rows g and g + 8 of its tile.  Half h of the channels: Q2/T2 word h of a row, Q4 both words of k block h.
+        // (D <= S: the stages of a group find room in the ring before the results of the item before are taken)
+        constexpr int D0 = HALVES == 2 ? (FMT == GLQ_FMT_Q4 ? 2 : 3) : 4, D = D0 < S ? D0 : S;
+        constexpr int NSZ = FMT == GLQ_FMT_Q4 ? HALVES : 1;        // (scale, zero) sets per stage
+        uint32_t cq[D][HALVES][2][2], csz[D][NSZ][2];              // [stage][half][row][word]
+        const unsigned char* blk = nullptr;                        // of the next stage to request
+        int left = 0;                                              // k blocks of the item still to request
+        bool live = false;
+        auto fetch = [&](uint32_t (&qv)[HALVES][2][2], uint32_t (&zv)[NSZ][2]) {
+            if constexpr (FMT == GLQ_FMT_Q4) {
+#pragma unroll
+                for (int h = 0; h < HALVES; ++h) {
+                    const bool in = wh0 + h < left;
+                    const unsigned char* src = blk + (wh0 + h) * (2 * BB);
+                    const uint4 v = in ? __ldg(reinterpret_cast<const uint4*>(src) + lane) : make_uint4(0, 0, 0, 0);
+                    const uint2 z = in ? __ldg(reinterpret_cast<const uint2*>(src + 512) + g) : make_uint2(0, 0);
+                    qv[h][0][0] = v.x, qv[h][0][1] = v.y, qv[h][1][0] = v.z, qv[h][1][1] = v.w;
+                    zv[h][0] = z.x, zv[h][1] = z.y;
+                }
+                left -= 2;
+                blk += 4 * BB;
+            } else {
+                const bool in = left > 0;
+                if constexpr (HALVES == 2) {
+                    const uint4 v = in ? __ldg(reinterpret_cast<const uint4*>(blk) + lane) : make_uint4(0, 0, 0, 0);
+                    qv[0][0][0] = v.x, qv[1][0][0] = v.y, qv[0][1][0] = v.z, qv[1][1][0] = v.w;
+                } else {
+                    const uint32_t* wsrc = reinterpret_cast<const uint32_t*>(blk) + lane * 4 + wh0;
+                    qv[0][0][0] = in ? __ldg(wsrc) : 0u;
+                    qv[0][1][0] = in ? __ldg(wsrc + 2) : 0u;
+                }
+                if constexpr (AFFINE) {
+                    const uint2 z = in ? __ldg(reinterpret_cast<const uint2*>(blk + 512) + g) : make_uint2(0, 0);
+                    zv[0][0] = z.x, zv[0][1] = z.y;
+                }
+                --left;
+                blk += 2 * BB;
+            }
+        };
+        uint32_t TL = 0, TH = 0;                  // codebook tables
+        // tile of the matrix (destination tile of the fused layout for gate|up) that this warp unpacks in an item
+        auto tile_of = [&](int ft) { return SW ? (ft * 8 + tl) * 2 + mx : (ft * NM + mx) * 8 + tl; };
+        const int n_tiles = SW ? 2 * ((N + 15) / 16) : (N + 15) / 16;
+        auto open_item = [&](int n) {
+            const volatile PsItem& im = s_item[n % kPsQueue];
+            const int d16 = tile_of(im.ft);
+            live = d16 < n_tiles;
+            left = live ? nblk : 0;
+            blk = im.codes + ((size_t)(d16 >> 1) * nblk * 2 + (d16 & 1)) * BB;
+            if constexpr (!AFFINE) make_t2_tables(im.centroids + (SW ? 4 * mx : 0), TL, TH);
+#pragma unroll
+            for (int d = 0; d < D; ++d) fetch(cq[d], csz[d]);
+            // the low-rank rows come last: into L2 by then (each lane one of its 128-byte rows)
+            if (live && im.sv && lane < 16)
+                for (int sl = 0; sl < nst - p.nkb; ++sl)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(im.sv + ((((size_t)(d16 >> 1) * p.ns + sl) * 32) + (d16 & 1) * 16 + lane) * 128));
+        };
+        // the 16 registers of a half's store: for k step n of the half {row g: positions 4t..4t+3, row g+8: the same}
+        auto unpack = [&](const uint32_t (&qv)[2][2], const uint32_t (&zv)[2], uint32_t (&r)[16]) {
+            if constexpr (AFFINE) {
+                ps_affine<FMT>(qv, zv, r);
+            } else {
+#pragma unroll
+                for (int hrow = 0; hrow < 2; ++hrow) {
+                    uint32_t h[8];
+                    unpack_t2(qv[hrow][0], TL, TH, h);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) r[4 * (j >> 1) + 2 * hrow + (j & 1)] = h[j];
+                }
+            }
+        };
+        // low-rank slice sl: SV rows in natural K order, four k steps per 64 columns
+        auto load_sv = [&](const volatile PsItem& im, int sl, uint32_t (&v)[HALVES][8]) {
+            const int d16 = tile_of(im.ft);
+            const unsigned char* sv = im.sv;
+#pragma unroll
+            for (int h = 0; h < HALVES; ++h)
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+#pragma unroll
+                    for (int hrow = 0; hrow < 2; ++hrow) {
+                        const int row = g + 8 * hrow;
+                        const uint2* src = reinterpret_cast<const uint2*>(
+                            sv + ((((size_t)(d16 >> 1) * p.ns + sl) * 32) + (d16 & 1) * 16 + row) * 128 + (2 * (wh0 + h) + n) * 32 + t * 8);
+                        uint2 u = (live && sv) ? __ldg(src) : make_uint2(0, 0);
+                        if constexpr (!AFFINE) {
+                            // the epilogue scales by the row norm: the low-rank rows go in divided by it
+                            const float nv = live ? __ldg(im.norms + (size_t)d16 * 16 + row) : 0.f;
+                            const float inv = nv != 0.f ? 1.f / nv : 0.f;
+                            __half2* hp = reinterpret_cast<__half2*>(&u);
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                const float2 f = __half22float2(hp[i]);
+                                hp[i] = __floats2half2_rn(f.x * inv, f.y * inv);
+                            }
+                        }
+                        v[h][4 * n + 2 * hrow] = u.x;
+                        v[h][4 * n + 2 * hrow + 1] = u.y;
+                    }
+        };
+        const int n_sv = nst - p.nkb;
+        auto publish_stage = [&]() {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_full + 8 * s);
+            if (++s == S) {
+                s = 0;
+                ph ^= 1u;
+            }
+        };
+
+        bool ok = true, more = have_item(0), pending = false;      // pending: the results of the item before are still to be taken
+        if (more) open_item(0);
+        for (int it = 0; more || pending; ++it) {
+            const volatile PsItem& im = s_item[it % kPsQueue];
+            const int nk = more ? p.nkb : 0;
+            // Software pipeline: a stage's first half is unpacked while the stores of the stage before are on their way to
+            // tensor memory, and before its ring slot is free.
+            uint32_t r[16];
+            unpack(cq[0][0], csz[0][0], r);
+            for (int st0 = 0;; st0 += D) {
+                if (pending && (st0 > 0 || nk == 0)) {
+                    ok = results(it - 1) && ok;
+                    pending = false;
+                }
+                if (st0 >= nk) break;
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    const int st = st0 + d;
+                    if (st < nk) {
+                        ok = ps_wait_warp(bar_empty + 8 * s, ph ^ 1u, dead, 100) && ok;
+                        tc_fence_after();
+                        if (ok) {
+                            const uint32_t acol = ring + (uint32_t)(s * NM * 64 + mx * 64 + wh0 * 32) + lane_base;
+                            tc_st_x4(acol, r);
+                            if constexpr (HALVES == 2) {
+                                uint32_t r2[16];
+                                unpack(cq[d][1], csz[d][NSZ - 1], r2);
+                                tc_st_x4(acol + 32, r2);
+                            }
+                            fetch(cq[d], csz[d]);
+                            unpack(cq[(d + 1) % D][0], csz[(d + 1) % D][0], r);
+                            tc_st_wait();
+                        }
+                        publish_stage();
+                    }
+                }
+            }
+            if (!more) break;
+            for (int sl = 0; sl < n_sv; ++sl) {
+                uint32_t v[HALVES][8];
+                load_sv(im, sl, v);
+                ok = ps_wait_warp(bar_empty + 8 * s, ph ^ 1u, dead, 100) && ok;
+                tc_fence_after();
+                if (ok) {
+#pragma unroll
+                    for (int h = 0; h < HALVES; ++h)
+                        tc_st_x2(ring + (uint32_t)(s * NM * 64 + mx * 64 + (wh0 + h) * 16) + lane_base, v[h]);
+                    tc_st_wait();
+                }
+                publish_stage();
+            }
+            if (!ok) break;
+            pending = true;
+            more = have_item(it + 1);
+            if (more) open_item(it + 1);
         }
-        while (pend > 0 && st_ok && !__any_sync(0xffffffffu, *dead != 0)) flush_pass();
         tc_fence_before();
     } else if (warp == kTcProducers) {
         // ================= MMA issuer =================
         constexpr uint32_t idesc = tc_idesc(TN);
+        constexpr uint32_t kAtom = TN * 128 / 16;            // an atom of the token operand in descriptor units
+        const uint64_t bdesc0 = tc_smem_desc(sbase);
         int s = 0;
         uint32_t ph = 0;
-        int it = 0;
-        for (;;) {
-            const int wk = next_item(it);
-            if (wk < 0) break;
-            if (lane == 0) {
-                bool ok = true;
-                for (int st = 0; st < nst && ok; ++st) {
-                    ok = tc_wait(bar_full + 8 * s, ph, dead, 103);
-                    if (ok && st == 0 && it > 0) ok = tc_wait(bar_acc_free, (uint32_t)((it - 1) & 1), dead, 104);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t acol = ring + (uint32_t)(s * NM * 64);
-                    const uint32_t bbase = sbase + (uint32_t)s * C::B_BYTES;
-                    if (st < p.nkb) {
+        bool ok = true;
+        for (int it = 0; ok; ++it) {
+            const bool more = have_item(it);
+            release_item(it);
+            if (!more) break;
+            for (int st = 0; st < nst && ok; ++st) {
+                ok = ps_wait_warp(bar_full + 8 * s, ph, dead, 103);
+                if (ok && st == 0 && it > 0) ok = ps_wait_warp(bar_acc_free, (uint32_t)((it - 1) & 1), dead, 104);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t acol = ring + (uint32_t)(s * NM * 64);
+                const uint64_t bd = bdesc0 + (uint32_t)(s * (C::B_BYTES / 16));
+                if (st < p.nkb) {
 #pragma unroll
-                        for (int kk = 0; kk < 8; ++kk) {
-                            const uint64_t bd = tc_smem_desc(bbase + (uint32_t)(kk >> 2) * (TN * 128) + (uint32_t)(kk & 3) * 32u);
-                            tc_mma_f16_ts(tmem, acol + 8 * kk, bd, idesc, (st | kk) != 0);
-                            if (SW) tc_mma_f16_ts(tmem + TN, acol + 64 + 8 * kk, bd, idesc, (st | kk) != 0);
-                        }
-                    } else {
-#pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {
-                            tc_mma_f16_ts(tmem, acol + 8 * kk, tc_smem_desc(bbase + (uint32_t)kk * 32u), idesc, 1);
-                            if (SW) tc_mma_f16_ts(tmem + TN, acol + 64 + 8 * kk, tc_smem_desc(bbase + TN * 128 + (uint32_t)kk * 32u), idesc, 1);
-                        }
+                    for (int kk = 0; kk < 8; ++kk) {
+                        const uint64_t b = bd + (uint32_t)((kk >> 2) * kAtom + (kk & 3) * 2);
+                        const uint32_t acc = kk == 0 ? (uint32_t)(st != 0) : 1u;
+                        tc_mma_f16_ts(tmem, acol + 8 * kk, b, idesc, acc);
+                        if (NM == 2) tc_mma_f16_ts(tmem + TN, acol + 64 + 8 * kk, b, idesc, acc);
                     }
-                    tc_commit(bar_empty + 8 * s);
-                    if (++s == S) {
-                        s = 0;
-                        ph ^= 1u;
+                } else {
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk) {
+                        tc_mma_f16_ts(tmem, acol + 8 * kk, bd + 2 * kk, idesc, 1);
+                        if (NM == 2) tc_mma_f16_ts(tmem + TN, acol + 64 + 8 * kk, bd + (SW ? kAtom : 0) + 2 * kk, idesc, 1);
                     }
                 }
-                if (ok) tc_commit(bar_acc);
+                tc_commit_warp(bar_empty + 8 * s);
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1u;
+                }
             }
-            // every lane keeps the ring position of lane 0
-            s = __shfl_sync(0xffffffffu, s, 0);
-            ph = __shfl_sync(0xffffffffu, ph, 0);
-            ++it;
+            if (ok) tc_commit_warp(bar_acc);
         }
+    } else if (warp == kTcProducers + 1) {
+        // ================= results: staging tiles -> y, one 256-byte copy per token row =================
+        int pass = 0;
+        for (int it = 0; have_item(it); ++it) {
+            const volatile PsItem& im = s_item[it % kPsQueue];
+            const int ft = im.ft, lt = im.lt, cnt = im.cnt, e0 = im.e0;
+            bool ok = true;
+            for (int h = 0; h < C::NPASS && ok; ++h, ++pass) {
+                const int b = pass & 1, f0 = (ft * C::NOUT + h / (TN / kPsRows)) * kTcFeat, nf = min(kTcFeat, N - f0);
+                const int r0 = lt * TN + (h % (TN / kPsRows)) * kPsRows, rows = min(kPsRows, cnt - r0);
+                // (the producers come to an item's results an item later: a longer limit)
+                ok = __all_sync(0xffffffffu, tc_wait(bar_staged + 8 * b, (uint32_t)(pass >> 1) & 1u, dead, 107, 50000000ull));
+                if (!ok) break;
+                const uint32_t src = obase + (uint32_t)(b * kPsOut);
+                if (nf > 0) {
+                    for (int r = lane; r < rows; r += 32) {
+                        __half* dst = p.y + (size_t)(e0 + r0 + r) * p.ldy + f0;
+                        if (p.y_vec) {
+                            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src + (uint32_t)r * 256u), "r"(nf * 2) : "memory");
+                        } else {
+                            for (int i = 0; i < nf; ++i) {
+                                unsigned short hv;
+                                asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hv) : "r"(src + (uint32_t)r * 256u + (uint32_t)i * 2u) : "memory");
+                                dst[i] = __ushort_as_half(hv);
+                            }
+                        }
+                    }
+                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_stored + 8 * b);
+            }
+            release_item(it);
+            if (!ok) break;
+        }
+        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else {
         // ================= loader of the token operand =================
         int s = 0;
         uint32_t ph = 0;
         int issued = 0;
-        for (int n = 0;; ++n) {
-            // draw the next live work item from the grid-wide counter and publish it to the other warps
+        // Draw work item n (the first one is the CTA's number, the others come from the grid-wide counter), look its
+        // problem up and publish it; returns its token tile, -1 at the end of the list.  Item n + 1 is published before
+        // the copies of item n are issued: these wait for the ring, and the producers want the addresses early.
+        auto publish = [&](int n) -> int {
             const int qi = n % kPsQueue;
             const bool room = __all_sync(0xffffffffu, tc_wait(bar_tq_empty + 8 * qi, (uint32_t)(((n / kPsQueue) & 1) ^ 1), dead, 109));
-            int wk = -1, gt = 0;
-            while (room) {
-                int w = 0;
-                if (lane == 0) w = atomicAdd(p.tile_ctr, 1);
-                w = __shfl_sync(0xffffffffu, w, 0);
+            PsItem im;
+            im.ft = -1;
+            int gt = -1;
+            for (bool first = n == 0; room; first = false) {
+                int w = blockIdx.x;
+                if (!first) {
+                    if (lane == 0) w = atomicAdd(p.tile_ctr, 1) + gridDim.x;
+                    w = __shfl_sync(0xffffffffu, w, 0);
+                }
                 if (w >= n_work) break;
-                gt = w / p.n_ft;
-                int slot, lt, cnt, e0;
-                if (tc_find_tile<TN>(p, gt, slot, lt, cnt, e0)) {
-                    wk = w;
+                const int tile = w / p.n_ft;
+                int slot;
+                if (tc_find_tile<TN>(p, tile, slot, im.lt, im.cnt, im.e0)) {
+                    const int widx = p.slot_index ? __ldg(p.slot_index + slot) : slot;
+                    const glq_weight_t* W = p.table ? p.table + widx : &p.w;
+                    im.codes = reinterpret_cast<const unsigned char*>(W->codes);
+                    im.sv = reinterpret_cast<const unsigned char*>(W->sv);
+                    im.bias = reinterpret_cast<const __half*>(W->bias);
+                    im.norms = W->norms;
+                    im.centroids = W->centroids;
+                    gt = tile;
+                    im.ft = w - tile * p.n_ft;
                     break;
                 }
             }
             if (lane == 0) {
-                *reinterpret_cast<volatile int*>(&s_tile[qi]) = wk;
+                s_item[qi] = im;
                 mbar_arrive(bar_tq_full + 8 * qi);
             }
             __syncwarp();
-            if (wk < 0) break;
+            return gt;
+        };
+        int gt = publish(0), nxt = -1;
+        for (int n = 0; gt >= 0; ++n, gt = nxt) {
+            nxt = publish(n + 1);
             if (lane == 0) {
                 const unsigned char* tile = p.xp + (size_t)gt * p.tile_bytes;
                 for (int st = 0; st < nst; ++st) {

@@ -313,6 +313,21 @@ def test_gptq_i8_dropin(dev, B, N, K, sym, lora):
 
 
 # ---- routes around the packed formats ----------------------------------------------------------------
+@pytest.mark.parametrize("B", [33, 64, 65, 130, 515])
+@pytest.mark.parametrize("fmt,bits,gs,N,K,rank", [("gptq", 2, 128, 264, 384, 16), ("gptq", 4, 64, 264, 320, 80), ("gptq", 4, 128, 40, 64, 0),
+                                                  ("turbo", 2, 0, 392, 256, 64), ("gptq", 2, 256, 100, 200, 16)])
+def test_many_rows_every_format(dev, fmt, bits, gs, N, K, rank, B):
+    """The tensor-memory GEMM at the edges of its tiles: token tiles of 64, 128 and 256, ragged features and channels, a
+    half-filled last stage, more than one low-rank slice, zero points that are not whole numbers."""
+    from glorcq_b200 import tiled
+    d = cases.make_linear(N + K + B, N, K, rank=max(rank, 16), fmt=fmt, bits=bits, groupsize=gs or 128, with_lora=rank > 0,
+                          int_zeros=B != 65)
+    x = cases.make_x(N + B, B, K)
+    y = cases.to_b200_linear(d, dev)(x.to(dev)).cpu()
+    assert cases.rel_l2(y, O.linear_forward(cases.to_oracle_linear(d), x, x_rot_half=True)) <= REL
+    assert tiled.debug_error() is None
+
+
 @pytest.mark.parametrize("N,K", [(64, 2048), (192, 4096), (8, 264), (72, 64), (512, 1408), (520, 256)])
 def test_dense_few_columns(dev, N, K):
     """x . W^T on 9 and more rows: row tiles of 32, column slices of 64, K over warps and clusters of CTAs."""
