@@ -226,7 +226,8 @@ static void fill_geometry(SkinnyParams& p, const Geometry& g) {
 // streaming kernel: eligibility, geometry, launch
 // ---------------------------------------------------------------------------------------------
 struct StreamGeom {
-    int i8, nt, ntc, nkb, sk, kb_per_split, npairs, ips, stages, stage_bytes, swiglu;
+    int i8, nt, ntc, nkb, nw, kc, kb_per_chunk, cb, sk, kb_per_split, npairs, ips, stages, stage_bytes, swiglu;
+    size_t scratch_bytes, n_counters;    // of the k chunks
     int off_xs, off_ox, off_as, off_ring, off_red;
     size_t smem;
     int grid;
@@ -285,73 +286,93 @@ static bool plan_stream(int fmt, int epilogue, int N, int K, int rank, int group
     }
     const int ntiles = cdiv(N, kRowTile);
     g.npairs = g.swiglu ? ntiles : cdiv(ntiles, 2);
-    // k splits (warps of one CTA): enough iterations to give every SM one; splits on group boundaries
-    const int units = cdiv(g.nkb, group_blocks);
-    int sk = 1;
-    const long want_iters = (long)kStreamCtasPerSm * num_sms();
-    while (sk < 8 && (long)n_problems * cdiv(g.npairs * sk, kWarpsPerCta) < want_iters && units >= 2 * sk) sk *= 2;
-    int ctas_per_sm = kStreamCtasPerSm;
-    for (;; sk /= 2) {
-        g.sk = sk;
-        g.kb_per_split = cdiv(units, sk) * group_blocks;
-        g.ips = cdiv(g.npairs * sk, kWarpsPerCta);
-        g.stage_bytes = std::max(kStreamCB * 2 * block_bytes_of(fmt), 4096);
-        size_t off = kWarpsPerCta * kMaxStages * 8;
+    const int units = cdiv(g.nkb, group_blocks);      // splits lie on group boundaries
+    // Warps per CTA, k chunks over CTAs and ring stages: of the forms that fit shared memory beside the staged activations,
+    // the one with the least work per CTA slot -- rounds of iterations, each as long as the k blocks of a warp item and
+    // about six more for its prologue, low-rank term and epilogue.  Two CTAs of eight warps are the rule; one CTA of eight
+    // leaves room for the sums of more k splits (a small problem), one of sixteen shares its activations among all warps
+    // of an SM (long rows), k chunks cut what one does not hold.  Stages hold four k blocks, two when that is what it takes.
+    auto fits = [&](int nw, int kc, int cb, size_t cap) {
+        g.nw = nw;
+        g.cb = cb;
+        g.kb_per_chunk = cdiv(units, kc) * group_blocks;
+        g.kc = cdiv(g.nkb, g.kb_per_chunk);
+        // k splits (warps of one CTA): enough iterations to give every CTA slot one
+        const long want = nw == 8 ? (long)kStreamCtasPerSm * num_sms() : num_sms();
+        const int cunits = g.kb_per_chunk / group_blocks;
+        int sk = 1;
+        while (sk < 8 && (long)n_problems * g.kc * cdiv(g.npairs * sk, nw) < want && cunits >= 2 * sk) sk *= 2;
+        g.stage_bytes = std::max(cb * 2 * block_bytes_of(fmt), 4096);
+        const int nkb = g.kb_per_chunk;
+        size_t off = (size_t)nw * kMaxStages * 8;
         off = (off + 127) / 128 * 128;
         g.off_xs = (int)off;
         if (g.i8) {
             const int p8 = fmt == GLQ_FMT_Q4 ? 1 : 2;
-            off += (size_t)g.nkb * p8 * (2 * rows) * 4 * 16;
+            off += (size_t)nkb * p8 * (2 * rows) * 4 * 16;
             g.off_ox = (int)off;
-            off += (size_t)g.nkb * rows * 8;
+            off += (size_t)nkb * rows * 8;
         } else {
             const int xs_u4 = (fmt == GLQ_FMT_Q4) ? 8 : 16;
-            off += (size_t)g.nkb * xs_u4 * g.ntc * 16;
+            off += (size_t)nkb * xs_u4 * g.ntc * 16;
             g.off_ox = (int)off;
-            off += (size_t)g.nkb * g.ntc * 8;
+            off += (size_t)nkb * g.ntc * 8;
         }
         off = (off + 15) / 16 * 16;
         g.off_as = (int)off;
         off += (size_t)(g.swiglu ? 2 : 1) * rows * std::max(rank, 16) * 2;
         off = (off + 127) / 128 * 128;
         g.off_ring = (int)off;
-        const size_t red = sk > 1 ? (size_t)2 * kWarpsPerCta * 2 * g.nt * 32 * 16 : 0;
-        // two CTAs per SM when the staged activations leave room for it, else one
-        size_t cap = (size_t)(kStreamCtasPerSm == 1 ? 220 : 110) * 1024;
-        ctas_per_sm = kStreamCtasPerSm;
-        if (off + red + (size_t)kWarpsPerCta * 2 * g.stage_bytes > cap) {
-            cap = 220 * 1024;
-            ctas_per_sm = 1;
+        const size_t stage = (size_t)nw * g.stage_bytes;
+        for (;; sk /= 2) {
+            const size_t red = sk > 1 ? (size_t)2 * nw * 2 * g.nt * 32 * (g.i8 ? 8 : 16) : 0;
+            if (off + red + 2 * stage > cap) {
+                if (sk > 1) continue;
+                return false;
+            }
+            g.sk = sk;
+            g.kb_per_split = cdiv(cunits, sk) * group_blocks;
+            g.ips = cdiv(g.npairs * sk, nw);
+            g.stages = std::min((int)((cap - off - red) / stage), kMaxStages);
+            g.off_red = (int)(off + g.stages * stage);
+            g.smem = g.off_red + red;
+            return true;
         }
-        if (off + red + (size_t)kWarpsPerCta * 2 * g.stage_bytes > cap) {
-            if (sk > 1) continue;
-            return false;
+    };
+    const size_t half = (size_t)110 * 1024, full = (size_t)225 * 1024;
+    const int sms = num_sms();
+    StreamGeom best{};
+    long best_cost = -1;
+    auto consider = [&](int nw, int kc, int cb, size_t cap, int slots) {
+        if (!fits(nw, kc, cb, cap)) return;
+        const long iters = (long)n_problems * g.kc * g.ips;
+        const long cost = (iters + slots - 1) / slots * (g.kb_per_split + 6 + (g.kc > 1 ? 3 : 0));
+        if (best_cost >= 0 && cost >= best_cost) return;
+        best_cost = cost;
+        best = g;
+        best.grid = (int)std::min<long>(iters, slots);
+    };
+    consider(8, 1, 4, half, kStreamCtasPerSm * sms);
+    consider(8, 1, 4, full, sms);
+    if (g.i8)
+        for (int kc = 1; kc <= 16 && kc <= units && (best_cost < 0 || kc <= 2); ++kc) {
+            consider(16, kc, 4, full, sms);
+            if (best_cost < 0) consider(16, kc, 2, full, sms);
         }
-        int stages = (int)((cap - off - red) / ((size_t)kWarpsPerCta * g.stage_bytes));
-        g.stages = std::min(stages, kMaxStages);
-        off += (size_t)kWarpsPerCta * g.stages * g.stage_bytes;
-        g.off_red = (int)off;
-        off += red;
-        g.smem = off;
-        // the k-split reduction buffer may be what pushes the CTA over half an SM's shared memory: fewer
-        // splits with two CTAs per SM stream better, as long as every SM still gets work
-        if (ctas_per_sm == 1 && sk > 1 && kStreamCtasPerSm == 2 &&
-            (size_t)g.off_ring + (size_t)kWarpsPerCta * 2 * g.stage_bytes <= (size_t)110 * 1024 &&
-            (long)n_problems * cdiv(g.npairs, kWarpsPerCta) >= num_sms()) {
-            sk = 2;      // -> one split: no reduction buffer
-            continue;
-        }
-        break;
+    if (best_cost < 0) return false;
+    g = best;
+    if (g.kc > 1) {
+        const int nm = cdiv(rows, 8);
+        g.n_counters = (size_t)n_problems * g.npairs;
+        g.scratch_bytes = g.n_counters * (size_t)(g.kc * 4 * g.nt + 8 * nm) * 32 * sizeof(float);
     }
-    const long iters = (long)n_problems * g.ips;
-    g.grid = (int)std::min<long>(iters, (long)ctas_per_sm * num_sms());
     *out = g;
     return g.grid > 0;
 }
 
-template <int FMT, bool I8, int NT>
+template <int FMT, bool I8, int NT, int NW = 8>
 static int launch_stream_one(const StreamParams& sp, const StreamGeom& g, cudaStream_t st) {
-    auto kern = stream_kernel<FMT, I8, NT>;
+    auto kern = stream_kernel<FMT, I8, NT, NW>;
     static size_t configured[16] = {0};
     int dev = 0;
     GLQ_CUDA(cudaGetDevice(&dev));
@@ -359,14 +380,16 @@ static int launch_stream_one(const StreamParams& sp, const StreamGeom& g, cudaSt
         GLQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
         if (dev >= 0 && dev < 16) configured[dev] = g.smem;
     }
-    if (sp.a_late || sp.dependent) return launch_dependent(kern, dim3(g.grid), dim3(kThreads), g.smem, st, sp);
-    kern<<<g.grid, kThreads, g.smem, st>>>(sp);
+    if (sp.a_late || sp.dependent) return launch_dependent(kern, dim3(g.grid), dim3(NW * 32), g.smem, st, sp);
+    kern<<<g.grid, NW * 32, g.smem, st>>>(sp);
     GLQ_CUDA(cudaGetLastError());
     return GLQ_OK;
 }
 
 template <int FMT>
 static int launch_stream_fmt(const StreamParams& sp, const StreamGeom& g, cudaStream_t st) {
+    if (g.i8 && g.nw == 16)
+        return g.nt == 1 ? launch_stream_one<FMT, true, 1, 16>(sp, g, st) : launch_stream_one<FMT, true, 2, 16>(sp, g, st);
     if (g.i8) {
         if (g.nt == 1) return launch_stream_one<FMT, true, 1>(sp, g, st);
         return launch_stream_one<FMT, true, 2>(sp, g, st);
@@ -376,9 +399,12 @@ static int launch_stream_fmt(const StreamParams& sp, const StreamGeom& g, cudaSt
     return launch_stream_one<FMT, false, 4>(sp, g, st);
 }
 
-static int launch_stream(int fmt, SkinnyParams& p, const StreamGeom& g, int N, int K, int rank, int n_problems,
-                         cudaStream_t st, bool a_late = false, bool dependent = false, int cnt_lo = 0,
+static int launch_stream(const glq_mm_args_t* a, SkinnyParams& p, const StreamGeom& g, cudaStream_t st, bool a_late = false, bool dependent = false, int cnt_lo = 0,
                          int cnt_hi = 0x7fffffff) {
+    const int fmt = a->fmt, N = a->N, K = a->K, rank = a->rank, n_problems = a->n_problems;
+    if (g.kc > 1 && (!a->workspace || !aligned16(a->workspace) || a->workspace_bytes < g.scratch_bytes || !a->counters ||
+                     a->n_counters < g.n_counters))
+        return GLQ_ERR_WORKSPACE;
     StreamParams sp{};
     sp.cnt_lo = cnt_lo;
     sp.cnt_hi = cnt_hi;
@@ -398,6 +424,9 @@ static int launch_stream(int fmt, SkinnyParams& p, const StreamGeom& g, int N, i
     sp.sk = g.sk;
     sp.sk_log2 = g.sk == 1 ? 0 : (g.sk == 2 ? 1 : (g.sk == 4 ? 2 : 3));
     sp.kb_per_split = g.kb_per_split;
+    sp.kc = g.kc;
+    sp.kb_per_chunk = g.kb_per_chunk;
+    sp.cb = g.cb;
     sp.npairs = g.npairs;
     sp.ips = g.ips;
     sp.stages = g.stages;
@@ -560,7 +589,8 @@ static void fill_tc_operands(const glq_mm_args_t* a, TcParams& p) {
     p.y_vec = ((reinterpret_cast<uintptr_t>(a->y) & 15u) == 0 && a->ldy % 8 == 0 && a->N % 8 == 0) ? 1 : 0;
 }
 
-// Dense products with few columns (xu_mm.cuh).  From 9 rows: up to 8 rows one pass of the skinny kernel takes them all.
+// Dense products with few columns (xu_mm.cuh).  From 9 rows: up to 8 rows one pass of
+// the skinny kernel takes them all and is faster (5 rows of 2048: 4.4 us where xu_kernel takes 5.9).
 // Up to 512 columns: every 64-column slice reads x again (from L2), and a wide W fills the tcgen05 kernel's tiles.
 static bool xu_takes(const glq_mm_args_t* a) {
     return a->fmt == GLQ_FMT_F16 && a->max_rows > 8 && a->N > 0 && a->N <= 512 && a->K > 0 && a->K % 8 == 0 && a->n_problems > 0 &&
@@ -638,28 +668,41 @@ static int launch_tc(const glq_mm_args_t* a, const TcGeom& g, cudaStream_t st, i
     return GLQ_ERR_UNSUPPORTED;
 }
 
-extern "C" size_t glq_mm_workspace_bytes(const glq_mm_args_t* a) {
-    if (!a) return 0;
+// Scratch and counters of every launch a call may be cut into: k chunks of the streaming kernel at each row class, the
+// tcgen05 kernel's token operand, the general kernel's split.  The launches follow one another, so they share.
+static void mm_needs(const glq_mm_args_t* a, size_t* bytes, size_t* counters) {
+    *bytes = *counters = 0;
+    if (!a) return;
     TcGeom tg;
-    if (plan_tc(a, &tg)) return tg.xp_bytes;
-    StreamGeom sg;
-    if (plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, a->max_rows, &sg)) return 0;
+    const bool tc = plan_tc(a, &tg);
+    if (tc) *bytes = tg.xp_bytes;
+    bool stream = false;
+    for (int rows : {4, 8, 16, 32}) {
+        StreamGeom sg;
+        rows = std::min(rows, a->max_rows);
+        if ((!tc || tg.hybrid) && plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, rows, &sg)) {
+            *bytes = std::max(*bytes, sg.scratch_bytes);
+            *counters = std::max(*counters, sg.n_counters);
+            stream = stream || rows == std::min(a->max_rows, 32);
+        }
+        if (rows == a->max_rows) break;
+    }
     Geometry g;
-    if (plan_geometry(a->fmt, a->epilogue, a->N, a->K, a->group_size, a->n_problems, a->max_rows, true, &g) != GLQ_OK)
-        return 0;
-    return g.scratch_bytes;
+    if (!tc && !stream &&
+        plan_geometry(a->fmt, a->epilogue, a->N, a->K, a->group_size, a->n_problems, a->max_rows, true, &g) == GLQ_OK) {
+        *bytes = std::max(*bytes, g.scratch_bytes);
+        *counters = std::max(*counters, g.n_counters);
+    }
 }
-
+extern "C" size_t glq_mm_workspace_bytes(const glq_mm_args_t* a) {
+    size_t b, c;
+    mm_needs(a, &b, &c);
+    return b;
+}
 extern "C" size_t glq_mm_counters(const glq_mm_args_t* a) {
-    if (!a) return 0;
-    TcGeom tg;
-    if (plan_tc(a, &tg)) return 0;
-    StreamGeom sg;
-    if (plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, a->max_rows, &sg)) return 0;
-    Geometry g;
-    if (plan_geometry(a->fmt, a->epilogue, a->N, a->K, a->group_size, a->n_problems, a->max_rows, true, &g) != GLQ_OK)
-        return 0;
-    return g.n_counters;
+    size_t b, c;
+    mm_needs(a, &b, &c);
+    return c;
 }
 
 extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
@@ -678,23 +721,26 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
         if (!a->w_table && !a->w.codes) return GLQ_ERR_ARG;
         return launch_tc(a, tg, reinterpret_cast<cudaStream_t>(stream));
     }
-    // 9..32 rows of the same problems, counts known on the host: the integer path stages at most 8 rows (4 when the
-    // staged activations of a long reduction leave no room for 8) and streams at a multiple of the fp16 path's rate,
-    // so it runs over chunks of rows; after the first chunk the weights come from L2 where they fit
+    // 9..32 rows of the same problems, counts known on the host: the integer path stages at most 8 rows and streams at a
+    // multiple of the fp16 path's rate, so it runs over chunks of rows; after the first chunk the weights come from L2
+    // where they fit
     if (!use_tc && !a->slot_count && !a->slot_offset && a->max_rows > 8 && a->max_rows <= 32 && !i8_disabled() &&
         (a->fmt == GLQ_FMT_Q2 || a->fmt == GLQ_FMT_Q4)) {
         int chunk = 0;
+        bool shares = false;      // its k chunks use the scratch: the launches of two row chunks must not overlap
         for (int c : {8, 4}) {
             StreamGeom cg;
             if (plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, c, &cg) && cg.i8) {
                 chunk = c;
+                shares = cg.kc > 1;
                 break;
             }
         }
-        if (chunk) {
+        if (chunk && chunk < a->max_rows) {
             for (int r0 = 0; r0 < a->max_rows; r0 += chunk) {
                 glq_mm_args_t b = *a;
                 b.max_rows = std::min(chunk, a->max_rows - r0);
+                if (r0 > 0 && shares) b.flags &= ~(GLQ_MM_A_FROM_PREVIOUS_LAUNCH | GLQ_MM_AFTER_KERNEL);
                 b.rows_stride = a->rows_stride > 0 ? a->rows_stride : a->max_rows;
                 if (a->entry_row) b.entry_row = a->entry_row + r0;
                 else b.x = static_cast<const char*>(a->x) + (size_t)r0 * a->ldx * 2;
@@ -716,7 +762,7 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
     StreamGeom sg8, sg16;
     const int cap = use_tc ? 16 : std::min(a->max_rows, 32);
     bool use_stream = plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, cap, &sg);
-    const bool classes = use_stream && a->slot_count != nullptr && a->max_rows > 8 && !sg.i8 && !hybrid_disabled();
+    const bool classes = use_stream && a->slot_count != nullptr && a->max_rows > 8 && !hybrid_disabled();
     const bool split8 = classes && plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, 8, &sg8) &&
                         sg8.i8;
     const bool split16 = classes && cap > 16 &&
@@ -763,7 +809,7 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
     if (use_stream) {
         cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
         const bool a_late = (a->flags & GLQ_MM_A_FROM_PREVIOUS_LAUNCH) != 0, dep = (a->flags & GLQ_MM_AFTER_KERNEL) != 0;
-        if (!split8 && !split16 && !use_tc) return launch_stream(a->fmt, p, sg, a->N, a->K, a->rank, a->n_problems, st, a_late, dep);
+        if (!split8 && !split16 && !use_tc) return launch_stream(a, p, sg, st, a_late, dep);
         // one launch per class; only the first may depend programmatically on the producer of x.U (the
         // later ones start after it has finished)
         int lo = 0;
@@ -771,8 +817,7 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
         auto one = [&](const StreamGeom& gg, int rows, int hi) {
             SkinnyParams pp = p;
             pp.max_rows = rows;
-            const int r2 = launch_stream(a->fmt, pp, gg, a->N, a->K, a->rank, a->n_problems, st, first && a_late, first && dep,
-                                         lo, hi);
+            const int r2 = launch_stream(a, pp, gg, st, first && a_late, first && dep, lo, hi);
             first = false;
             lo = hi;
             return r2;

@@ -52,8 +52,7 @@ struct MoeLayout {
 inline int moe_chunk(const glq_moe_desc_t* d, int n) {
     static const bool off = std::getenv("GLQ_NO_CHUNK") != nullptr;
     const long long nk = (long long)n * d->top_k;
-    const bool affine = d->fmt == GLQ_FMT_Q2 || d->fmt == GLQ_FMT_Q4;
-    return (!off && affine && n > 8 && nk <= 24ll * d->E) ? 8 : 0;
+    return (!off && n > 8 && nk <= 24ll * d->E) ? 8 : 0;
 }
 inline int moe_slots(const glq_moe_desc_t* d, int n) {
     const long long nk = (long long)n * d->top_k;

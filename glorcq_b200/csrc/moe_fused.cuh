@@ -835,7 +835,7 @@ __global__ void __launch_bounds__(kFT, 1) moe_fused_kernel(const FusedParams p) 
                                 const uint4 q = lds128(blk + lane * 16);
                                 const uint2 szv = lds64(blk + 512 + g * 8);
                                 int ci[1][4];
-                                tile_block_i8<FMT, 1>(q, bx, ci);
+                                tile_block_i8<FMT, 1>(q, bx, ci, 1);
                                 const __half2 sz0 = *reinterpret_cast<const __half2*>(&szv.x);
                                 const __half2 sz1 = *reinterpret_cast<const __half2*>(&szv.y);
                                 const float s0 = __low2float(sz0), z0 = __high2float(sz0);

@@ -19,10 +19,19 @@
 //     -> s32 tensor-core op (m16n8k32) does the dot products exactly; scale, zero point and the digit
 //     weights are applied in fp32 per k block.  More rows (and the codebook format) use the fp16 op;
 //   * k splits of a pair are warps of one CTA, reduced through shared memory in a fixed order
-//     (named barrier per pair): no global scratch, no atomics, deterministic.
+//     (named barrier per pair): no global scratch, no atomics, deterministic;
+//   * when two CTAs of eight warps with their own copies of the staged activations do not fit an SM (8 rows of 4096
+//     channels: 65 KB), one CTA of sixteen warps shares one copy -- one of eight left the SM at a quarter of its warps and
+//     took 18.4 us for 8 rows of a 4-bit 4096 x 4096, the one of sixteen 13.0;
+//   * reductions whose activations do not fit at all (14336 channels) are cut into k chunks that go to different CTAs; a
+//     pair's chunks meet in global scratch, the warp that arrives last adds them in chunk order (deterministic) and runs
+//     the epilogue.  The general kernel (skinny_mm.cuh) took these before: 152 us for the down products of 16 tokens over
+//     8 experts (14336 -> 4096), now 75.
 // Every mbarrier wait is bounded in time; a wait that runs out records an error word and the warp
 // stops waiting, so the kernel always terminates.  No cluster launch, no multicast.
 #pragma once
+
+#include <type_traits>
 
 #include "skinny_mm.cuh"
 
@@ -32,7 +41,7 @@ constexpr int kMaxStages = 6;
 #ifndef GLQ_STREAM_CB
 #define GLQ_STREAM_CB 4
 #endif
-constexpr int kStreamCB = GLQ_STREAM_CB;  // k blocks per ring stage
+constexpr int kStreamCB = GLQ_STREAM_CB;  // k blocks per ring stage (most; StreamParams::cb)
 #ifndef GLQ_STREAM_CTAS
 #define GLQ_STREAM_CTAS 2
 #endif
@@ -46,8 +55,10 @@ struct StreamParams {
     int sk;            // k splits (warps of one CTA): 1, 2, 4 or 8
     int sk_log2;
     int kb_per_split;
+    int kc, kb_per_chunk;   // k chunks over CTAs (1: none) and their k blocks
+    int cb;            // k blocks per ring stage
     int npairs;        // tile pairs per problem
-    int ips;           // iterations (8 warp items) per problem
+    int ips;           // iterations (one item per warp of the CTA) per problem and k chunk
     int stages;        // ring depth
     int stage_bytes;
     int off_xs, off_ox, off_as, off_ring, off_red;  // shared memory carve-up (bytes)
@@ -144,39 +155,48 @@ __device__ __forceinline__ void imma16832(int (&d)[4], uint32_t a0, uint32_t a1,
 // {2m, 2m+4, 2m+8, 2m+12}, b1 = codes {2m+1, ...} (2-bit); word u: b0 = even codes, b1 = odd codes
 // (4-bit).  Layout: xs[kb][piece][col = 2*row + digit][t] of uint4, piece = u (2-bit) / 0 (4-bit);
 // ox[kb][row] = (2^-sh, sum of x).
-template <int FMT>
-__device__ __forceinline__ void stage_x_i8(const SkinnyParams& p, uint4* xs, float2* ox, int nkb, int ncol, int e0,
+template <int FMT, int THREADS>
+__device__ __forceinline__ void stage_x_i8(const SkinnyParams& p, uint4* xs, float2* ox, int kb0, int nkb, int ncol, int e0,
                                            int cnt, int K) {
     using F = Fmt<FMT>;
     constexpr int P8 = F::UPK / 4;  // pieces per block: 2 (2-bit), 1 (4-bit)
     const int nrow = ncol >> 1;
     // only the live rows are staged; columns of absent rows keep stale (finite or not) data, and the
     // outputs computed from them are never stored
-    const int total = min(nrow, cnt) * nkb * F::UPK;
-    for (int base = 0; base < total; base += kThreads) {
+    const int per = nkb * F::UPK, total = min(nrow, cnt) * per;
+    // unit u = 16 channels of a row; the loads of a thread's next unit are under way while it converts one
+    auto load = [&](int u, int row, int rem, uint4 (&v)[2]) {
+        v[0] = v[1] = make_uint4(0, 0, 0, 0);
+        const int k0 = kb0 * F::KB + rem * 16;
+        if (u >= total || k0 >= K) return;
+        const int entry = e0 + row;
+        const long long xr = p.entry_row ? __ldg(p.entry_row + entry) : entry;
+        const __half* src = p.x + xr * p.ldx + k0;
+        if (p.x_vec && k0 + 16 <= K) {
+            v[0] = __ldg(reinterpret_cast<const uint4*>(src));
+            v[1] = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+        } else {
+            __align__(16) __half h[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) h[j] = (k0 + j < K) ? src[j] : __float2half(0.f);
+            v[0] = reinterpret_cast<const uint4*>(h)[0];
+            v[1] = reinterpret_cast<const uint4*>(h)[1];
+        }
+    };
+    int row = 0, rem = threadIdx.x;
+    while (rem >= per) rem -= per, ++row;
+    uint4 nv[2];
+    load(threadIdx.x, row, rem, nv);
+    for (int base = 0; base < total; base += THREADS) {
         const int u = base + (int)threadIdx.x;
         const bool valid = u < total;
-        const int row = valid ? u / (nkb * F::UPK) : 0;
-        const int rem = valid ? u % (nkb * F::UPK) : 0;
-        const int kb = rem / F::UPK, wi = rem % F::UPK;
-        const int k0 = kb * F::KB + wi * 16;
+        const int crow = row, kb = rem / F::UPK, wi = rem % F::UPK;
         __align__(16) __half v[16];
-        const bool live = valid && row < cnt && k0 < K;
-        if (live) {
-            const int entry = e0 + row;
-            const long long xr = p.entry_row ? p.entry_row[entry] : entry;
-            const __half* src = p.x + xr * p.ldx + k0;
-            if (p.x_vec && k0 + 16 <= K) {
-                *reinterpret_cast<uint4*>(&v[0]) = __ldg(reinterpret_cast<const uint4*>(src));
-                *reinterpret_cast<uint4*>(&v[8]) = __ldg(reinterpret_cast<const uint4*>(src) + 1);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = (k0 + j < K) ? src[j] : __float2half(0.f);
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __float2half(0.f);
-        }
+        reinterpret_cast<uint4*>(v)[0] = nv[0];
+        reinterpret_cast<uint4*>(v)[1] = nv[1];
+        rem += THREADS;
+        while (rem >= per) rem -= per, ++row;
+        load(u + THREADS, row, rem, nv);
         float f[16], mx = 0.f, sx = 0.f;
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
@@ -223,9 +243,9 @@ __device__ __forceinline__ void stage_x_i8(const SkinnyParams& p, uint4* xs, flo
                 hi = make_uint4(pack4(d1, 0, 2, 4, 6), pack4(d1, 1, 3, 5, 7), pack4(d1, 8, 10, 12, 14),
                                 pack4(d1, 9, 11, 13, 15));
             }
-            xs[((size_t)(kb * P8 + piece) * ncol + 2 * row) * 4 + t] = lo;
-            xs[((size_t)(kb * P8 + piece) * ncol + 2 * row + 1) * 4 + t] = hi;
-            if (wi == 0) ox[kb * nrow + row] = make_float2(ldexpf(1.f, -sh), sx);
+            xs[((size_t)(kb * P8 + piece) * ncol + 2 * crow) * 4 + t] = lo;
+            xs[((size_t)(kb * P8 + piece) * ncol + 2 * crow + 1) * 4 + t] = hi;
+            if (wi == 0) ox[kb * nrow + crow] = make_float2(ldexpf(1.f, -sh), sx);
         }
     }
 }
@@ -275,7 +295,7 @@ __device__ __forceinline__ void tile_block(const uint4 q, const uint4 (&bx)[NTT]
 
 // ---- integer path: one k block of one tile; bx[nt][piece] are the digit fragments ------------------
 template <int FMT, int NT>
-__device__ __forceinline__ void tile_block_i8(const uint4 q, const uint4 (&bx)[NT][2], int (&c)[NT][4]) {
+__device__ __forceinline__ void tile_block_i8(const uint4 q, const uint4 (&bx)[NT][2], int (&c)[NT][4], int nt_live) {
     if constexpr (FMT == GLQ_FMT_Q2) {
         const uint32_t m = 0x03030303u;
         const uint32_t wa[2] = {q.x, q.y}, wb[2] = {q.z, q.w};
@@ -285,6 +305,7 @@ __device__ __forceinline__ void tile_block_i8(const uint4 q, const uint4 (&bx)[N
             const uint32_t b0 = wb[u] & m, b1 = (wb[u] >> 2) & m, b2 = (wb[u] >> 4) & m, b3 = (wb[u] >> 6) & m;
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
+                if (nt >= nt_live) continue;      // activation tiles beyond the problem's rows (warp-uniform)
                 const uint4 x = bx[nt][u];
                 if (u == 0)
                     imma16832(c[nt], a0, b0, a1, b1, x.x, x.y, 0, 0, 0, 0);
@@ -299,6 +320,7 @@ __device__ __forceinline__ void tile_block_i8(const uint4 q, const uint4 (&bx)[N
         const uint32_t b0 = q.z & m, b1 = (q.z >> 4) & m, b2 = q.w & m, b3 = (q.w >> 4) & m;
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
+            if (nt >= nt_live) continue;
             const uint4 x = bx[nt][0];
             imma16832(c[nt], a0, b0, a1, b1, x.x, x.y, 0, 0, 0, 0);
             imma16832(c[nt], a2, b2, a3, b3, x.z, x.w, c[nt][0], c[nt][1], c[nt][2], c[nt][3]);
@@ -356,10 +378,12 @@ __device__ __forceinline__ void tile_block_t2_i8(const uint4 q, const uint4 (&bx
 // ---- the kernel -----------------------------------------------------------------------------------
 // I8 = true : NT tiles of 4 activation rows (integer path: affine formats and the 2-bit codebook)
 // I8 = false: NT tiles of 8 activation rows (fp16 path)
-template <int FMT, bool I8, int NT>
-__global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(const StreamParams sp) {
+// NW = 8: two CTAs per SM; NW = 16 (integer path only): one
+template <int FMT, bool I8, int NT, int NW>
+__global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) stream_kernel(const StreamParams sp) {
     using F = Fmt<FMT>;
     static_assert(FMT != GLQ_FMT_F16, "dense weights use the fallback kernel");
+    static_assert(I8 || NW == 8, "the fp16 path stages with the threads of eight warps");
     constexpr bool kAffine = (FMT == GLQ_FMT_Q2 || FMT == GLQ_FMT_Q4);
     constexpr int BB = block_bytes<FMT>();
     constexpr int kPieces = I8 ? F::UPK / 4 : F::XS / 4;  // uint4 fragments per k block, lane and column
@@ -372,7 +396,7 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
     const int g = lane >> 2, t = lane & 3;
     const int N = sp.N, K = sp.K, rank = sp.rank;
     const int nkb = p.nkb, ntc = p.ntc;
-    const int S = sp.stages, sk = sp.sk;
+    const int S = sp.stages, sk = sp.sk, kc = sp.kc, cb = sp.cb;
     const bool swiglu = sp.swiglu != 0;
     const int ns = (rank + 63) / 64;
 
@@ -381,7 +405,7 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
     if (!sp.a_late) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int n_live = p.n_slots ? min(__ldg(p.n_slots), sp.n_problems) : sp.n_problems;
-    const long total = (long)n_live * sp.ips;
+    const long total = (long)n_live * kc * sp.ips;
     const int it_lo = (int)((long)blockIdx.x * total / gridDim.x);
     const int it_hi = (int)((long)(blockIdx.x + 1) * total / gridDim.x);
     if (it_lo >= it_hi) {
@@ -395,7 +419,8 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
     uint4* xs = reinterpret_cast<uint4*>(smem + sp.off_xs);
     float2* ox = reinterpret_cast<float2*>(smem + sp.off_ox);
     __half* as = reinterpret_cast<__half*>(smem + sp.off_as);
-    float4* red = reinterpret_cast<float4*>(smem + sp.off_red);
+    using Red = std::conditional_t<I8, float2, float4>;       // the integer path uses two of a fragment's four sums
+    Red* red = reinterpret_cast<Red*>(smem + sp.off_red);
     const uint32_t xs_a = smem_u32(xs), ox_a = smem_u32(ox);
     const uint32_t ring_a = smem_u32(smem + sp.off_ring) + (uint32_t)(w * S * sp.stage_bytes);
     const uint32_t bar_a = smem_u32(bars) + (uint32_t)(w * kMaxStages * 8);
@@ -433,19 +458,20 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
     };
     // item of warp w in iteration it: (slot, pair, split) -> k range and chunk counts
     struct Item {
-        int slot, pair, s, kb_lo, kb_hi, ncode, nch;
+        int slot, chunk, pair, s, kb_lo, kb_hi, ncode, nch;
         bool valid;
     };
-    auto make_item = [&](Item& im, const Slot& sc, int slot, int rem) {   // iteration = slot * ips + rem
-        const int local = rem * kWarpsPerCta + w;
+    auto make_item = [&](Item& im, const Slot& sc, int slot, int chunk, int rem) {   // iteration = (slot * kc + chunk) * ips + rem
+        const int local = rem * NW + w;
         im.slot = slot;
+        im.chunk = chunk;
         im.pair = local >> sp.sk_log2;
         im.s = local & (sk - 1);
         im.valid = im.pair < sp.npairs && sc.cnt > 0;
-        im.kb_lo = im.s * sp.kb_per_split;
-        im.kb_hi = min(nkb, im.kb_lo + sp.kb_per_split);
-        im.ncode = im.kb_hi > im.kb_lo ? (im.kb_hi - im.kb_lo + kStreamCB - 1) / kStreamCB : 0;
-        im.nch = im.ncode + ((im.s == 0 && sc.sv != nullptr) ? ns : 0);
+        im.kb_lo = chunk * sp.kb_per_chunk + im.s * sp.kb_per_split;
+        im.kb_hi = min(min(nkb, (chunk + 1) * sp.kb_per_chunk), im.kb_lo + sp.kb_per_split);
+        im.ncode = im.kb_hi > im.kb_lo ? (im.kb_hi - im.kb_lo + cb - 1) >> (cb == 4 ? 2 : 1) : 0;
+        im.nch = im.ncode + ((im.s == 0 && chunk == 0 && sc.sv != nullptr) ? ns : 0);
     };
 
     // ---- fetch cursor: runs over the same (item, chunk) sequence as the compute loop, S stages ahead
@@ -453,7 +479,13 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
     Slot fs, cs;
     Item fi;
     // cursors keep (iteration, slot, iteration within the slot) and ring positions incrementally: no divisions
-    int f_it = it_lo, f_slot = it_lo / sp.ips, f_rem = it_lo % sp.ips, f_c = 0;
+    int f_it = it_lo, f_rem = it_lo % sp.ips, f_chunk = (it_lo / sp.ips) % kc, f_slot = it_lo / sp.ips / kc, f_c = 0;
+    auto step = [&](int& slot, int& chunk, int& rem) {
+        if (++rem == sp.ips) {
+            rem = 0;
+            if (++chunk == kc) chunk = 0, ++slot;
+        }
+    };
     int f_stage = 0, f_inflight = 0;      // next stage to fill, chunks issued and not yet consumed
     int c_stage = 0;                      // next stage to consume
     uint32_t c_phase = 0;                 // its mbarrier phase parity
@@ -462,13 +494,13 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
         f_live = false;
         while (f_it < it_hi) {
             load_slot(fs, f_slot);
-            make_item(fi, fs, f_slot, f_rem);
+            make_item(fi, fs, f_slot, f_chunk, f_rem);
             if (fi.valid && fi.nch > 0) {
                 f_live = true;
                 return;
             }
             ++f_it;
-            if (++f_rem == sp.ips) f_rem = 0, ++f_slot;
+            step(f_slot, f_chunk, f_rem);
         }
     };
     auto fetch_one = [&]() {
@@ -479,8 +511,8 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
             const void* src;
             uint32_t bytes;
             if (f_c < fi.ncode) {
-                const int kb0 = fi.kb_lo + f_c * kStreamCB;
-                bytes = (uint32_t)(min(kStreamCB, fi.kb_hi - kb0) * 2 * BB);
+                const int kb0 = fi.kb_lo + f_c * cb;
+                bytes = (uint32_t)(min(cb, fi.kb_hi - kb0) * 2 * BB);
                 src = fs.codes + ((size_t)fi.pair * nkb + kb0) * (2 * BB);
             } else {
                 bytes = 4096;
@@ -494,7 +526,7 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
         if (++f_c >= fi.nch) {
             f_c = 0;
             ++f_it;
-            if (++f_rem == sp.ips) f_rem = 0, ++f_slot;
+            step(f_slot, f_chunk, f_rem);
             fetch_seek();
         }
     };
@@ -516,28 +548,29 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
     // integer path of the codebook format: coefficients of the two tiles' codebooks (tile_block_t2_i8)
     float cb_c0[2] = {0.f, 0.f}, cb_d0[2] = {0.f, 0.f}, cb_dh[2] = {0.f, 0.f}, cb_e[2] = {0.f, 0.f};
     bool cb_cross = false;
-    int staged_slot = -1, red_par = 0;
+    int staged_slot = -1, staged_chunk = -1, red_par = 0;
     bool dep_waited = false;
     constexpr int ncol_i8 = 2 * kRows;  // digit columns staged on the integer path
 
-    int c_slot = it_lo / sp.ips, c_rem = it_lo % sp.ips;
-    for (int it = it_lo; it < it_hi; ++it, c_rem = (c_rem + 1 == sp.ips ? 0 : c_rem + 1), c_slot += (c_rem == 0)) {
+    int c_rem = it_lo % sp.ips, c_chunk = (it_lo / sp.ips) % kc, c_slot = it_lo / sp.ips / kc;
+    for (int it = it_lo; it < it_hi; ++it, step(c_slot, c_chunk, c_rem)) {
         load_slot(cs, c_slot);
         Item im;
-        make_item(im, cs, c_slot, c_rem);
+        make_item(im, cs, c_slot, c_chunk, c_rem);
+        const int kb_base = c_chunk * sp.kb_per_chunk;      // first staged k block
         const int cnt = cs.cnt, e0 = cs.e0;
 
         // ---- activations of a new problem: staged once per CTA ----
-        if (im.slot != staged_slot) {
+        if (im.slot != staged_slot || c_chunk != staged_chunk) {
             __syncthreads();
             if (cnt > 0) {
                 if constexpr (I8)
-                    stage_x_i8<FMT>(p, xs, ox, nkb, ncol_i8, e0, cnt, K);
+                    stage_x_i8<FMT, NW * 32>(p, xs, ox, kb_base, min(nkb - kb_base, sp.kb_per_chunk), ncol_i8, e0, cnt, K);
                 else
                     stage_x<FMT>(p, xs, ox, 0, nkb, e0, 0, cnt, K);
                 if (cs.sv != nullptr && !sp.a_late) {
                     const int na = swiglu ? 2 : 1, r8 = rank / 8;
-                    for (int idx = tid; idx < na * kRows * r8; idx += kThreads) {
+                    for (int idx = tid; idx < na * kRows * r8; idx += NW * 32) {
                         const int i = idx / (kRows * r8), rem = idx % (kRows * r8);
                         const int row = rem / r8, ch = rem % r8;
                         uint4 v = make_uint4(0, 0, 0, 0);
@@ -549,6 +582,7 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
             }
             __syncthreads();
             staged_slot = im.slot;
+            staged_chunk = c_chunk;
             if constexpr (FMT == GLQ_FMT_T2) {
                 // a fused gate|up weight carries two codebooks (4 floats each)
                 if constexpr (I8) {
@@ -576,7 +610,7 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
             }
         }
         if (!im.valid) continue;
-        const int nt_live = I8 ? NT : min(NT, (cnt + 7) >> 3);     // fp16 path: activation tiles that hold rows
+        const int nt_live = NT == 1 ? 1 : min(NT, I8 ? (cnt + 3) >> 2 : (cnt + 7) >> 3);     // activation tiles that hold rows
 
         // accumulators [tile in pair][activation tile]: {row g: 2 values, row g+8: 2 values}.
         // fp16 path: the two values are activation rows 2t, 2t+1 of the tile; integer path: only
@@ -592,17 +626,18 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
         // ---- code chunks ----
         for (int c = 0; c < im.ncode; ++c) {
             const uint32_t st = ring_wait();
-            const int kb0 = im.kb_lo + c * kStreamCB;
-            const int nblk = min(kStreamCB, im.kb_hi - kb0);
+            const int kb0 = im.kb_lo + c * cb;
+            const int nblk = min(cb, im.kb_hi - kb0);
 #pragma unroll
             for (int b = 0; b < kStreamCB; ++b) {
                 if (b >= nblk) break;
-                const int kb = kb0 + b;
+                const int kb = kb0 + b - kb_base;     // among the staged ones
                 if constexpr (I8) {
                     uint4 bx[NT][2];
                     float2 o[NT];
 #pragma unroll
                     for (int nt = 0; nt < NT; ++nt) {
+                        if (nt >= nt_live) continue;
 #pragma unroll
                         for (int i = 0; i < kPieces; ++i)
                             bx[nt][i] = lds128(
@@ -636,13 +671,14 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
                         } else {
                             const uint2 szv = lds64(blk + 512 + g * 8);
                             int ci[NT][4];
-                            tile_block_i8<FMT, NT>(q, bx, ci);
+                            tile_block_i8<FMT, NT>(q, bx, ci, nt_live);
                             const __half2 sz0 = *reinterpret_cast<const __half2*>(&szv.x);
                             const __half2 sz1 = *reinterpret_cast<const __half2*>(&szv.y);
                             const float s0 = __low2float(sz0), z0 = __high2float(sz0);
                             const float s1 = __low2float(sz1), z1 = __high2float(sz1);
 #pragma unroll
                             for (int nt = 0; nt < NT; ++nt) {
+                                if (nt >= nt_live) continue;
                                 const float f0 = (float)(ci[nt][0] + (ci[nt][1] << 8)) * o[nt].x;
                                 const float f1 = (float)(ci[nt][2] + (ci[nt][3] << 8)) * o[nt].x;
                                 acc[j][nt][0] = fmaf(s0, fmaf(-z0, o[nt].y, f0), acc[j][nt][0]);
@@ -700,14 +736,18 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
 
         // ---- k splits of this pair: fixed-order reduction through shared memory ----
         if (sk > 1) {
-            float4* rbuf = red + (size_t)red_par * (kWarpsPerCta * 2 * NT * 32);
+            Red* rbuf = red + (size_t)red_par * (NW * 2 * NT * 32);
             if (im.s != 0) {
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
 #pragma unroll
-                    for (int nt = 0; nt < NT; ++nt)
-                        rbuf[((w * 2 + j) * NT + nt) * 32 + lane] =
-                            make_float4(acc[j][nt][0], acc[j][nt][1], acc[j][nt][2], acc[j][nt][3]);
+                    for (int nt = 0; nt < NT; ++nt) {
+                        if constexpr (I8)
+                            rbuf[((w * 2 + j) * NT + nt) * 32 + lane] = make_float2(acc[j][nt][0], acc[j][nt][2]);
+                        else
+                            rbuf[((w * 2 + j) * NT + nt) * 32 + lane] =
+                                make_float4(acc[j][nt][0], acc[j][nt][1], acc[j][nt][2], acc[j][nt][3]);
+                    }
             }
             named_bar_sync(1 + w / sk, sk * 32);
             if (im.s == 0) {
@@ -716,11 +756,16 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
                     for (int j = 0; j < 2; ++j)
 #pragma unroll
                         for (int nt = 0; nt < NT; ++nt) {
-                            const float4 v = rbuf[(((w + s2) * 2 + j) * NT + nt) * 32 + lane];
-                            acc[j][nt][0] += v.x;
-                            acc[j][nt][1] += v.y;
-                            acc[j][nt][2] += v.z;
-                            acc[j][nt][3] += v.w;
+                            const Red v = rbuf[(((w + s2) * 2 + j) * NT + nt) * 32 + lane];
+                            if constexpr (I8) {
+                                acc[j][nt][0] += v.x;
+                                acc[j][nt][2] += v.y;
+                            } else {
+                                acc[j][nt][0] += v.x;
+                                acc[j][nt][1] += v.y;
+                                acc[j][nt][2] += v.z;
+                                acc[j][nt][3] += v.w;
+                            }
                         }
             }
             red_par ^= 1;
@@ -778,6 +823,52 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
             ring_release();
         }
 
+        // ---- k chunks of this pair: records in global scratch, added in chunk order by the warp that arrives last ----
+        bool low_rank = nsv > 0;
+        if constexpr (I8) {
+            if (kc > 1) {
+                constexpr int REC = 2 * NT * 2, LOREC = 2 * NM * 4;       // floats per lane of a chunk's record, of the low-rank term
+                low_rank = cs.sv != nullptr;
+                const size_t item = (size_t)im.slot * sp.npairs + im.pair;
+                float* rec = reinterpret_cast<float*>(p.scratch) + item * (size_t)((kc * REC + LOREC) * 32) + lane;
+                float* mine = rec + (LOREC + im.chunk * REC) * 32;
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) {
+                        __stcg(mine + ((j * NT + nt) * 2) * 32, acc[j][nt][0]);
+                        __stcg(mine + ((j * NT + nt) * 2 + 1) * 32, acc[j][nt][2]);
+                    }
+                if (im.chunk == 0 && low_rank)
+#pragma unroll
+                    for (int i = 0; i < LOREC; ++i) __stcg(rec + i * 32, lo[i / (NM * 4)][(i / 4) % NM][i % 4]);
+                __threadfence();
+                __syncwarp();
+                int last = 0;
+                if (lane == 0) last = atomicAdd(p.counters + item, 1) == kc - 1;
+                if (!__shfl_sync(0xffffffffu, last, 0)) continue;
+                __threadfence();
+                if (lane == 0) p.counters[item] = 0;
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) acc[j][nt][0] = acc[j][nt][2] = 0.f;
+                for (int c = 0; c < kc; ++c) {
+                    const float* r = rec + (LOREC + c * REC) * 32;
+#pragma unroll
+                    for (int j = 0; j < 2; ++j)
+#pragma unroll
+                        for (int nt = 0; nt < NT; ++nt) {
+                            acc[j][nt][0] += __ldcg(r + ((j * NT + nt) * 2) * 32);
+                            acc[j][nt][2] += __ldcg(r + ((j * NT + nt) * 2 + 1) * 32);
+                        }
+                }
+                if (low_rank)
+#pragma unroll
+                    for (int i = 0; i < LOREC; ++i) lo[i / (NM * 4)][(i / 4) % NM][i % 4] = __ldcg(rec + i * 32);
+            }
+        }
+
         // ---- epilogue: this lane's activation rows, weight rows g and g+8 of both tiles ----
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
@@ -795,15 +886,15 @@ __global__ void __launch_bounds__(kThreads, kStreamCtasPerSm) stream_kernel(cons
                     }
                     float v0 = round16(acc[j][nt][I8 ? 0 : e] * n0);
                     float v1 = round16(acc[j][nt][I8 ? 2 : 2 + e] * n1);
-                    if (nsv > 0) {
+                    if (low_rank) {
                         float l0, l1;
                         if constexpr (I8) {
                             // the low-rank op holds rows 2t', 2t'+1 in lane t': fetch this lane's row
                             const int src = (g << 2) | ((row & 7) >> 1);
-                            const float a0 = __shfl_sync(0xffffffffu, lo[j][0][0], src);
-                            const float a1 = __shfl_sync(0xffffffffu, lo[j][0][1], src);
-                            const float b0 = __shfl_sync(0xffffffffu, lo[j][0][2], src);
-                            const float b1 = __shfl_sync(0xffffffffu, lo[j][0][3], src);
+                            const float a0 = __shfl_sync(0xffffffffu, lo[j][nt >> 1][0], src);
+                            const float a1 = __shfl_sync(0xffffffffu, lo[j][nt >> 1][1], src);
+                            const float b0 = __shfl_sync(0xffffffffu, lo[j][nt >> 1][2], src);
+                            const float b1 = __shfl_sync(0xffffffffu, lo[j][nt >> 1][3], src);
                             l0 = (row & 1) ? a1 : a0;
                             l1 = (row & 1) ? b1 : b0;
                         } else {

@@ -328,6 +328,23 @@ def test_many_rows_every_format(dev, fmt, bits, gs, N, K, rank, B):
     assert tiled.debug_error() is None
 
 
+@pytest.mark.parametrize("B", [1, 5, 8, 13])
+@pytest.mark.parametrize("fmt,bits,N,K", [("gptq", 2, 72, 14336), ("gptq", 4, 4096, 4096), ("turbo", 2, 1000, 8192), ("gptq", 2, 4096, 24576)])
+def test_long_reductions(dev, fmt, bits, N, K, B):
+    """Rows too long for two CTAs' copies of them: one CTA of sixteen warps, and k chunks that meet in global scratch."""
+    from glorcq_b200 import tiled
+    if N * K > 20_000_000 and B > 5:
+        pytest.skip("the longest rows on few of them")
+    d = cases.make_linear(N + K, N, K, rank=16, fmt=fmt, bits=bits)
+    lin = cases.to_b200_linear(d, dev)
+    x = cases.make_x(K + B, B, K)
+    y = lin(x.to(dev))
+    assert cases.rel_l2(y.cpu(), O.linear_forward(cases.to_oracle_linear(d), x, x_rot_half=True)) <= REL
+    for _ in range(3):
+        assert torch.equal(y, lin(x.to(dev)))
+    assert tiled.debug_error() is None
+
+
 @pytest.mark.parametrize("N,K", [(64, 2048), (192, 4096), (8, 264), (72, 64), (512, 1408), (520, 256)])
 def test_dense_few_columns(dev, N, K):
     """x . W^T on 9 and more rows: row tiles of 32, column slices of 64, K over warps and clusters of CTAs."""
