@@ -226,8 +226,7 @@ static void fill_geometry(SkinnyParams& p, const Geometry& g) {
 // streaming kernel: eligibility, geometry, launch
 // ---------------------------------------------------------------------------------------------
 struct StreamGeom {
-    int i8, nt, ntc, nkb, nw, kc, kb_per_chunk, cb, sk, kb_per_split, npairs, ips, stages, stage_bytes, swiglu;
-    size_t scratch_bytes, n_counters;    // of the k chunks
+    int i8, nt, ntc, nkb, nw, cb, sk, kb_per_split, npairs, ips, stages, stage_bytes, swiglu;
     int off_xs, off_ox, off_as, off_ring, off_red;
     size_t smem;
     int grid;
@@ -252,6 +251,23 @@ static bool i8_disabled() {
         v = (e && e[0] == '1') ? 1 : 0;
     }
     return v == 1;
+}
+
+// k splits of a pair, -1 when the call is not the streaming kernel's.  The splits fix the order of the sums, which deep models
+// amplify, so they follow the problem and the memory of CTAs of eight warps alone, whatever form of CTA then runs it:
+// enough iterations to give every CTA slot one, as few as fit beside the staged activations (`base` bytes up to the ring) with
+// two ring stages and four floats per lane, tile and split for their sums.
+static int stream_splits(size_t base, size_t stage, int nt, int npairs, int units, int n_problems) {
+    int sk = 1;
+    const long want = (long)kStreamCtasPerSm * num_sms();
+    while (sk < 8 && (long)n_problems * cdiv(npairs * sk, kWarpsPerCta) < want && units >= 2 * sk) sk *= 2;
+    const size_t half = (size_t)110 * 1024, full = (size_t)220 * 1024, ring = 2 * kWarpsPerCta * stage;
+    const auto sums = [&](int k) { return k > 1 ? (size_t)2 * kWarpsPerCta * 2 * nt * 32 * 16 : 0; };
+    while (sk > 1 && base + sums(sk) + ring > full) sk /= 2;
+    if (base + sums(sk) + ring > full) return -1;
+    // (fewer splits with two CTAs per SM stream better, as long as every SM still gets work)
+    if (sk > 1 && base + sums(sk) + ring > half && base + ring <= half && (long)n_problems * cdiv(npairs, kWarpsPerCta) >= num_sms()) sk = 1;
+    return sk;
 }
 
 // returns true when the streaming kernel covers this call
@@ -287,87 +303,65 @@ static bool plan_stream(int fmt, int epilogue, int N, int K, int rank, int group
     const int ntiles = cdiv(N, kRowTile);
     g.npairs = g.swiglu ? ntiles : cdiv(ntiles, 2);
     const int units = cdiv(g.nkb, group_blocks);      // splits lie on group boundaries
-    // Warps per CTA, k chunks over CTAs and ring stages: of the forms that fit shared memory beside the staged activations,
-    // the one with the least work per CTA slot -- rounds of iterations, each as long as the k blocks of a warp item and
-    // about six more for its prologue, low-rank term and epilogue.  Two CTAs of eight warps are the rule; one CTA of eight
-    // leaves room for the sums of more k splits (a small problem), one of sixteen shares its activations among all warps
-    // of an SM (long rows), k chunks cut what one does not hold.  Stages hold four k blocks, two when that is what it takes.
-    auto fits = [&](int nw, int kc, int cb, size_t cap) {
-        g.nw = nw;
-        g.cb = cb;
-        g.kb_per_chunk = cdiv(units, kc) * group_blocks;
-        g.kc = cdiv(g.nkb, g.kb_per_chunk);
-        // k splits (warps of one CTA): enough iterations to give every CTA slot one
-        const long want = nw == 8 ? (long)kStreamCtasPerSm * num_sms() : num_sms();
-        const int cunits = g.kb_per_chunk / group_blocks;
-        int sk = 1;
-        while (sk < 8 && (long)n_problems * g.kc * cdiv(g.npairs * sk, nw) < want && cunits >= 2 * sk) sk *= 2;
-        g.stage_bytes = std::max(cb * 2 * block_bytes_of(fmt), 4096);
-        const int nkb = g.kb_per_chunk;
+    // shared memory up to the ring, for CTAs of nw warps
+    auto base_bytes = [&](int nw) {
         size_t off = (size_t)nw * kMaxStages * 8;
         off = (off + 127) / 128 * 128;
         g.off_xs = (int)off;
         if (g.i8) {
             const int p8 = fmt == GLQ_FMT_Q4 ? 1 : 2;
-            off += (size_t)nkb * p8 * (2 * rows) * 4 * 16;
+            off += (size_t)g.nkb * p8 * (2 * rows) * 4 * 16;
             g.off_ox = (int)off;
-            off += (size_t)nkb * rows * 8;
+            off += (size_t)g.nkb * rows * 8;
         } else {
             const int xs_u4 = (fmt == GLQ_FMT_Q4) ? 8 : 16;
-            off += (size_t)nkb * xs_u4 * g.ntc * 16;
+            off += (size_t)g.nkb * xs_u4 * g.ntc * 16;
             g.off_ox = (int)off;
-            off += (size_t)nkb * g.ntc * 8;
+            off += (size_t)g.nkb * g.ntc * 8;
         }
         off = (off + 15) / 16 * 16;
         g.off_as = (int)off;
         off += (size_t)(g.swiglu ? 2 : 1) * rows * std::max(rank, 16) * 2;
-        off = (off + 127) / 128 * 128;
-        g.off_ring = (int)off;
-        const size_t stage = (size_t)nw * g.stage_bytes;
-        for (;; sk /= 2) {
-            const size_t red = sk > 1 ? (size_t)2 * nw * 2 * g.nt * 32 * (g.i8 ? 8 : 16) : 0;
-            if (off + red + 2 * stage > cap) {
-                if (sk > 1) continue;
-                return false;
-            }
-            g.sk = sk;
-            g.kb_per_split = cdiv(cunits, sk) * group_blocks;
-            g.ips = cdiv(g.npairs * sk, nw);
-            g.stages = std::min((int)((cap - off - red) / stage), kMaxStages);
-            g.off_red = (int)(off + g.stages * stage);
-            g.smem = g.off_red + red;
-            return true;
-        }
+        return (off + 127) / 128 * 128;
     };
-    const size_t half = (size_t)110 * 1024, full = (size_t)225 * 1024;
+    const size_t stage4 = std::max<size_t>(4 * 2 * block_bytes_of(fmt), 4096);
+    g.sk = stream_splits(base_bytes(kWarpsPerCta), stage4, g.nt, g.npairs, units, n_problems);
+    if (g.sk < 0) return false;
+    g.kb_per_split = cdiv(units, g.sk) * group_blocks;
+    // Form of the CTAs: of those that fit beside the staged activations, the one with the fewest rounds of iterations over its
+    // slots.  Two CTAs of eight warps per SM are the rule; one of eight leaves room for the sums of many splits; one of
+    // sixteen shares its activations among all warps of an SM.  Stages hold four k blocks, two when that is what it takes.
     const int sms = num_sms();
     StreamGeom best{};
-    long best_cost = -1;
-    auto consider = [&](int nw, int kc, int cb, size_t cap, int slots) {
-        if (!fits(nw, kc, cb, cap)) return;
-        const long iters = (long)n_problems * g.kc * g.ips;
-        const long cost = (iters + slots - 1) / slots * (g.kb_per_split + 6 + (g.kc > 1 ? 3 : 0));
-        if (best_cost >= 0 && cost >= best_cost) return;
-        best_cost = cost;
+    long best_rounds = -1;
+    auto consider = [&](int nw, int cb, size_t cap, int slots) {
+        const size_t off = base_bytes(nw), stage = (size_t)nw * std::max(cb * 2 * block_bytes_of(fmt), 4096);
+        const size_t red = g.sk > 1 ? (size_t)2 * nw * 2 * g.nt * 32 * (g.i8 ? 8 : 16) : 0;
+        if (off + red + 2 * stage > cap) return;
+        g.nw = nw;
+        g.cb = cb;
+        g.ips = cdiv(g.npairs * g.sk, nw);
+        const long iters = (long)n_problems * g.ips, rounds = (iters + slots - 1) / slots;      // (ties: the form named first)
+        if (best_rounds >= 0 && rounds >= best_rounds) return;
+        g.stage_bytes = (int)(stage / nw);
+        g.off_ring = (int)off;
+        g.stages = std::min((int)((cap - off - red) / stage), kMaxStages);
+        g.off_red = (int)(off + g.stages * stage);
+        g.smem = g.off_red + red;
+        g.grid = (int)std::min<long>(iters, slots);
+        best_rounds = rounds;
         best = g;
-        best.grid = (int)std::min<long>(iters, slots);
     };
-    consider(8, 1, 4, half, kStreamCtasPerSm * sms);
-    consider(8, 1, 4, full, sms);
-    if (g.i8)
-        for (int kc = 1; kc <= 16 && kc <= units && (best_cost < 0 || kc <= 2); ++kc) {
-            consider(16, kc, 4, full, sms);
-            if (best_cost < 0) consider(16, kc, 2, full, sms);
-        }
-    if (best_cost < 0) return false;
-    g = best;
-    if (g.kc > 1) {
-        const int nm = cdiv(rows, 8);
-        g.n_counters = (size_t)n_problems * g.npairs;
-        g.scratch_bytes = g.n_counters * (size_t)(g.kc * 4 * g.nt + 8 * nm) * 32 * sizeof(float);
+    const size_t half = (size_t)110 * 1024, full = (size_t)225 * 1024;
+    consider(8, 4, half, kStreamCtasPerSm * sms);
+    if (g.i8) {
+        consider(16, 4, full, sms);
+        consider(16, 2, full, sms);
     }
-    *out = g;
-    return g.grid > 0;
+    consider(8, 4, full, sms);
+    if (best_rounds < 0) return false;
+    *out = best;
+    return best.grid > 0;
 }
 
 template <int FMT, bool I8, int NT, int NW = 8>
@@ -402,9 +396,6 @@ static int launch_stream_fmt(const StreamParams& sp, const StreamGeom& g, cudaSt
 static int launch_stream(const glq_mm_args_t* a, SkinnyParams& p, const StreamGeom& g, cudaStream_t st, bool a_late = false, bool dependent = false, int cnt_lo = 0,
                          int cnt_hi = 0x7fffffff) {
     const int fmt = a->fmt, N = a->N, K = a->K, rank = a->rank, n_problems = a->n_problems;
-    if (g.kc > 1 && (!a->workspace || !aligned16(a->workspace) || a->workspace_bytes < g.scratch_bytes || !a->counters ||
-                     a->n_counters < g.n_counters))
-        return GLQ_ERR_WORKSPACE;
     StreamParams sp{};
     sp.cnt_lo = cnt_lo;
     sp.cnt_hi = cnt_hi;
@@ -424,8 +415,6 @@ static int launch_stream(const glq_mm_args_t* a, SkinnyParams& p, const StreamGe
     sp.sk = g.sk;
     sp.sk_log2 = g.sk == 1 ? 0 : (g.sk == 2 ? 1 : (g.sk == 4 ? 2 : 3));
     sp.kb_per_split = g.kb_per_split;
-    sp.kc = g.kc;
-    sp.kb_per_chunk = g.kb_per_chunk;
     sp.cb = g.cb;
     sp.npairs = g.npairs;
     sp.ips = g.ips;
@@ -451,11 +440,22 @@ static int launch_stream(const glq_mm_args_t* a, SkinnyParams& p, const StreamGe
 // ---------------------------------------------------------------------------------------------
 // glq_grouped_matmul
 // ---------------------------------------------------------------------------------------------
+template <typename Kern>
+static int allow_smem(Kern kern, bool (&configured)[64], size_t smem) {
+    int dev = 0;
+    GLQ_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !configured[dev]) {
+        GLQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (dev >= 0 && dev < 64) configured[dev] = true;
+    }
+    return GLQ_OK;
+}
+
 // ---------------------------------------------------------------------------------------------
 // tensor-core path (tc_mm.cuh): many rows per problem
 // ---------------------------------------------------------------------------------------------
 struct TcGeom {
-    int tn, nkb, ns, na, tiles_max;
+    int tn, nm, nkb, ns, na, tiles_max;    // nm: accumulators of an item of the tensor-memory kernel
     bool hybrid;
     long long tile_bytes;
     size_t xp_bytes;
@@ -475,6 +475,29 @@ static long long total_entries(const glq_mm_args_t* a) {
     return a->slot_offset ? total : std::max(total, (long long)(a->n_problems - 1) * stride + a->max_rows);
 }
 
+// Token tile (and, for a plain product, one or two 128-feature tiles per item) of the tcgen05 kernels: the least time of the
+// fullest SM, rounds of items x (stages x time of a stage + time around an item), in units of 0.4 us.  Stages measured on
+// B200 with packed codes: one accumulator 1 / 1.1 / 1.5 at 64 / 128 / 256 tokens (unpack-bound up to 128), two 1.8 / 2.0;
+// around an item five, and two for every 64 tokens of results.  A problem's rows fill ceil(rows / tile) tiles; with device-side
+// counts half a tile more than their mean.
+static void choose_tile(const glq_mm_args_t* a, long long total, int stages, TcGeom* g) {
+    const double rows = (double)total / a->n_problems;
+    if (a->fmt == GLQ_FMT_F16) {
+        g->tn = rows > 64 ? 128 : 64;
+        g->nm = 1;
+        return;
+    }
+    const bool sw = a->epilogue == GLQ_EPI_SWIGLU;
+    struct Form { int tn, nm; double stage; };
+    static const Form plain[] = {{64, 1, 1.0}, {64, 2, 1.8}, {128, 1, 1.1}, {256, 1, 1.5}}, fused[] = {{64, 2, 1.8}, {128, 2, 2.0}};
+    double best = -1;
+    for (const Form* f = sw ? fused : plain; f != (sw ? fused + 2 : plain + 4); ++f) {
+        const double tiles = a->slot_count ? (rows <= 0.75 * f->tn ? 1.0 : rows / f->tn + 0.5) : std::ceil(rows / f->tn);
+        const double items = a->n_problems * tiles * cdiv(a->N, kTcFeat * (sw ? 1 : f->nm));
+        const double t = std::ceil(items / num_sms()) * (stages * f->stage + 5 + 2 * (f->tn / 64) * (sw ? 1 : f->nm));
+        if (best < 0 || t < best) best = t, g->tn = f->tn, g->nm = f->nm;
+    }
+}
 // true when a tcgen05 kernel takes the call: more rows than the streaming kernel stages
 static bool plan_tc(const glq_mm_args_t* a, TcGeom* out) {
     if (tc_disabled() || a->max_rows <= 32) return false;
@@ -488,15 +511,10 @@ static bool plan_tc(const glq_mm_args_t* a, TcGeom* out) {
     }
     TcGeom g{};
     const long long total = total_entries(a);
-    g.tn = (total / a->n_problems > 64) ? 128 : 64;
-    // 256-token tiles: packed codes, plain epilogue, long problems only
-    static const char* tn_env = std::getenv("GLQ_TC_TN");
-    const bool wide_ok = a->fmt != GLQ_FMT_F16 && a->epilogue == GLQ_EPI_LINEAR;
-    const int wide_from = tn_env ? std::atoi(tn_env) : 512;      // rows per problem from which the wide tile is used
-    if (wide_ok && wide_from > 0 && total / a->n_problems >= wide_from) g.tn = 256;
     g.nkb = cdiv(a->K, 128);
     g.ns = a->rank > 0 ? cdiv(a->rank, 64) : 0;
     g.na = a->epilogue == GLQ_EPI_SWIGLU ? 2 : 1;
+    choose_tile(a, total, g.nkb + g.ns, &g);
     const long long tiles = total / g.tn + a->n_problems + 1;
     if (tiles > 65535) return false;
     g.tiles_max = (int)tiles;
@@ -508,17 +526,6 @@ static bool plan_tc(const glq_mm_args_t* a, TcGeom* out) {
     g.hybrid = a->slot_count != nullptr && a->fmt != GLQ_FMT_F16 && total / a->n_problems <= 24 && !hybrid_disabled();
     *out = g;
     return true;
-}
-
-template <typename Kern>
-static int allow_smem(Kern kern, bool (&configured)[64], size_t smem) {
-    int dev = 0;
-    GLQ_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        GLQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
-    return GLQ_OK;
 }
 
 // dense fp16 weights
@@ -550,15 +557,12 @@ static int launch_tc_ps_t(TcParams& p, cudaStream_t st) {
     GLQ_CUDA(cudaGetLastError());
     return GLQ_OK;
 }
-// live_tiles: token tiles that will have rows, as far as the host can tell
 template <int FMT>
-static int launch_tc_ps(TcParams& p, int tn, bool sw, long live_tiles, cudaStream_t st) {
-    if (tn == 256) return launch_tc_ps_t<FMT, 256, 1, false>(p, st);
-    if (tn == 128) return sw ? launch_tc_ps_t<FMT, 128, 2, true>(p, st) : launch_tc_ps_t<FMT, 128, 1, false>(p, st);
-    if (sw) return launch_tc_ps_t<FMT, 64, 2, true>(p, st);
-    // 256 features per item cost the producers fewer instructions per code; below two items per SM they leave SMs idle
-    if (live_tiles * cdiv(p.N, 2 * kTcFeat) >= 2 * num_sms()) return launch_tc_ps_t<FMT, 64, 2, false>(p, st);
-    return launch_tc_ps_t<FMT, 64, 1, false>(p, st);
+static int launch_tc_ps(TcParams& p, const TcGeom& g, bool sw, cudaStream_t st) {
+    if (sw) return g.tn == 128 ? launch_tc_ps_t<FMT, 128, 2, true>(p, st) : launch_tc_ps_t<FMT, 64, 2, true>(p, st);
+    if (g.tn == 256) return launch_tc_ps_t<FMT, 256, 1, false>(p, st);
+    if (g.tn == 128) return launch_tc_ps_t<FMT, 128, 1, false>(p, st);
+    return g.nm == 2 ? launch_tc_ps_t<FMT, 64, 2, false>(p, st) : launch_tc_ps_t<FMT, 64, 1, false>(p, st);
 }
 
 // operands and alignment facts of the many-row kernels; the geometry is filled in by the launchers
@@ -589,57 +593,33 @@ static void fill_tc_operands(const glq_mm_args_t* a, TcParams& p) {
     p.y_vec = ((reinterpret_cast<uintptr_t>(a->y) & 15u) == 0 && a->ldy % 8 == 0 && a->N % 8 == 0) ? 1 : 0;
 }
 
-// Dense products with few columns (xu_mm.cuh).  From 9 rows: up to 8 rows one pass of
-// the skinny kernel takes them all and is faster (5 rows of 2048: 4.4 us where xu_kernel takes 5.9).
-// Up to 512 columns: every 64-column slice reads x again (from L2), and a wide W fills the tcgen05 kernel's tiles.
+// Dense products with few columns (xu_mm.cuh).  Above 32 rows, where the order of the sums is the tcgen05 kernel's.  Up to 512
+// columns: every 64-column slice reads x again (from L2), and a wide W fills the tcgen05 kernel's tiles.
 static bool xu_takes(const glq_mm_args_t* a) {
-    return a->fmt == GLQ_FMT_F16 && a->max_rows > 8 && a->N > 0 && a->N <= 512 && a->K > 0 && a->K % 8 == 0 && a->n_problems > 0 &&
-           a->epilogue == GLQ_EPI_LINEAR && !a->entry_scale && !(a->rank > 0 && a->a0) && aligned16(a->x) && a->ldx % 8 == 0 &&
-           total_entries(a) / kXuRows + a->n_problems + 1 <= 65535;
+    return a->fmt == GLQ_FMT_F16 && a->max_rows > 32 && a->N > 0 && a->N <= 512 && a->K > 0 && a->K % 8 == 0 && a->n_problems > 0 &&
+           a->epilogue == GLQ_EPI_LINEAR && !a->entry_scale && !(a->rank > 0 && a->a0) && aligned16(a->x) && a->ldx % 8 == 0;
 }
 
-static int launch_xu(const glq_mm_args_t* a, cudaStream_t st, bool dependent) {
+template <int NT>
+static int launch_xu_t(TcParams& p, const glq_mm_args_t* a, cudaStream_t st) {
+    using C = XuCfg<NT>;
+    static bool configured[64] = {};
+    const int rc = allow_smem(xu_kernel<NT>, configured, C::SMEM);
+    if (rc != GLQ_OK) return rc;
+    const bool one = a->n_problems == 1 && !a->slot_offset && !a->n_slots;
+    p.tiles_max = one ? cdiv(a->max_rows, C::ROWS) : (int)(total_entries(a) / C::ROWS + a->n_problems + 1);
+    xu_kernel<NT><<<dim3(p.tiles_max, cdiv(a->N, kXuCols)), kXuThreads, C::SMEM, st>>>(p);
+    GLQ_CUDA(cudaGetLastError());
+    return GLQ_OK;
+}
+static int launch_xu(const glq_mm_args_t* a, cudaStream_t st) {
     if (!a->w_table && !a->w.codes) return GLQ_ERR_ARG;
     TcParams p{};
     fill_tc_operands(a, p);
     p.nkb = cdiv(a->K, 64);
-    const long long total = total_entries(a);
-    const bool one = a->n_problems == 1 && !a->slot_offset && !a->n_slots;
-    p.tiles_max = one ? cdiv(a->max_rows, kXuRows) : (int)(total / kXuRows + a->n_problems + 1);
-    const int slices = cdiv(a->N, kXuCols);
-    // tiles that will have rows: every problem has one when there are entries enough, whole tiles otherwise
-    const long long live = one ? p.tiles_max : std::max(total / kXuRows, std::min<long long>(a->n_problems, total));
-    // CTAs per tile along K: as many as keep the grid within one wave (two CTAs per SM) and every warp one block of K
-    int cs = 1;
-    while (cs < 8 && live * slices * cs * 2 <= 2 * num_sms() && p.nkb >= 2 * cs * kWarpsPerCta) cs *= 2;
-    static bool configured[64] = {};
-    int dev = 0;
-    GLQ_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        GLQ_CUDA(cudaFuncSetAttribute(xu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kXuSmem));
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(cs, slices, p.tiles_max);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = kXuSmem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[2];
-    int na = 0;
-    if (cs > 1) {
-        attr[na].id = cudaLaunchAttributeClusterDimension;
-        attr[na].val.clusterDim.x = cs;
-        attr[na].val.clusterDim.y = attr[na].val.clusterDim.z = 1;
-        ++na;
-    }
-    if (dependent) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na++].val.programmaticStreamSerializationAllowed = 1;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = na;
-    GLQ_CUDA(cudaLaunchKernelEx(&cfg, xu_kernel, p));
-    return GLQ_OK;
+    // 64 rows per CTA read W half as often; 32 where the smaller tiles still leave CTA slots free
+    const long long total = total_entries(a), tiles = std::max(total / 32, std::min<long long>(a->n_problems, total));
+    return tiles * cdiv(a->N, kXuCols) > 3 * num_sms() ? launch_xu_t<8>(p, a, st) : launch_xu_t<4>(p, a, st);
 }
 
 static int launch_tc(const glq_mm_args_t* a, const TcGeom& g, cudaStream_t st, int min_rows = 0) {
@@ -658,51 +638,37 @@ static int launch_tc(const glq_mm_args_t* a, const TcGeom& g, cudaStream_t st, i
     p.n_ft = cdiv(a->N, kTcFeat);
     if (a->fmt == GLQ_FMT_F16) return g.tn == 128 ? launch_tc_t<128>(p, st) : launch_tc_t<64>(p, st);
     p.ts = 1;
-    const long live_tiles = std::max<long>(total_entries(a) / g.tn, std::min<long>(a->n_problems, total_entries(a)));
     p.tile_ctr = reinterpret_cast<int*>(p.xp + (g.xp_bytes - 256));
     switch (a->fmt) {
-        case GLQ_FMT_Q2: return launch_tc_ps<GLQ_FMT_Q2>(p, g.tn, sw, live_tiles, st);
-        case GLQ_FMT_Q4: return launch_tc_ps<GLQ_FMT_Q4>(p, g.tn, sw, live_tiles, st);
-        case GLQ_FMT_T2: return launch_tc_ps<GLQ_FMT_T2>(p, g.tn, sw, live_tiles, st);
+        case GLQ_FMT_Q2: return launch_tc_ps<GLQ_FMT_Q2>(p, g, sw, st);
+        case GLQ_FMT_Q4: return launch_tc_ps<GLQ_FMT_Q4>(p, g, sw, st);
+        case GLQ_FMT_T2: return launch_tc_ps<GLQ_FMT_T2>(p, g, sw, st);
     }
     return GLQ_ERR_UNSUPPORTED;
 }
 
-// Scratch and counters of every launch a call may be cut into: k chunks of the streaming kernel at each row class, the
-// tcgen05 kernel's token operand, the general kernel's split.  The launches follow one another, so they share.
-static void mm_needs(const glq_mm_args_t* a, size_t* bytes, size_t* counters) {
-    *bytes = *counters = 0;
-    if (!a) return;
-    TcGeom tg;
-    const bool tc = plan_tc(a, &tg);
-    if (tc) *bytes = tg.xp_bytes;
-    bool stream = false;
-    for (int rows : {4, 8, 16, 32}) {
-        StreamGeom sg;
-        rows = std::min(rows, a->max_rows);
-        if ((!tc || tg.hybrid) && plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, rows, &sg)) {
-            *bytes = std::max(*bytes, sg.scratch_bytes);
-            *counters = std::max(*counters, sg.n_counters);
-            stream = stream || rows == std::min(a->max_rows, 32);
-        }
-        if (rows == a->max_rows) break;
-    }
-    Geometry g;
-    if (!tc && !stream &&
-        plan_geometry(a->fmt, a->epilogue, a->N, a->K, a->group_size, a->n_problems, a->max_rows, true, &g) == GLQ_OK) {
-        *bytes = std::max(*bytes, g.scratch_bytes);
-        *counters = std::max(*counters, g.n_counters);
-    }
-}
 extern "C" size_t glq_mm_workspace_bytes(const glq_mm_args_t* a) {
-    size_t b, c;
-    mm_needs(a, &b, &c);
-    return b;
+    if (!a) return 0;
+    TcGeom tg;
+    if (plan_tc(a, &tg)) return tg.xp_bytes;
+    StreamGeom sg;
+    if (plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, a->max_rows, &sg)) return 0;
+    Geometry g;
+    if (plan_geometry(a->fmt, a->epilogue, a->N, a->K, a->group_size, a->n_problems, a->max_rows, true, &g) != GLQ_OK)
+        return 0;
+    return g.scratch_bytes;
 }
+
 extern "C" size_t glq_mm_counters(const glq_mm_args_t* a) {
-    size_t b, c;
-    mm_needs(a, &b, &c);
-    return c;
+    if (!a) return 0;
+    TcGeom tg;
+    if (plan_tc(a, &tg)) return 0;
+    StreamGeom sg;
+    if (plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, a->max_rows, &sg)) return 0;
+    Geometry g;
+    if (plan_geometry(a->fmt, a->epilogue, a->N, a->K, a->group_size, a->n_problems, a->max_rows, true, &g) != GLQ_OK)
+        return 0;
+    return g.n_counters;
 }
 
 extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
@@ -714,7 +680,7 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
         return GLQ_ERR_ALIGN;
     t_share_sm = (a->flags & GLQ_MM_SHARE_SM) != 0;
     if (xu_takes(a))
-        return launch_xu(a, reinterpret_cast<cudaStream_t>(stream), (a->flags & GLQ_MM_AFTER_KERNEL) != 0 && !pdl_disabled());
+        return launch_xu(a, reinterpret_cast<cudaStream_t>(stream));
     TcGeom tg;
     const bool use_tc = plan_tc(a, &tg);
     if (use_tc && !tg.hybrid) {
@@ -727,12 +693,10 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
     if (!use_tc && !a->slot_count && !a->slot_offset && a->max_rows > 8 && a->max_rows <= 32 && !i8_disabled() &&
         (a->fmt == GLQ_FMT_Q2 || a->fmt == GLQ_FMT_Q4)) {
         int chunk = 0;
-        bool shares = false;      // its k chunks use the scratch: the launches of two row chunks must not overlap
         for (int c : {8, 4}) {
             StreamGeom cg;
             if (plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, c, &cg) && cg.i8) {
                 chunk = c;
-                shares = cg.kc > 1;
                 break;
             }
         }
@@ -740,7 +704,6 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
             for (int r0 = 0; r0 < a->max_rows; r0 += chunk) {
                 glq_mm_args_t b = *a;
                 b.max_rows = std::min(chunk, a->max_rows - r0);
-                if (r0 > 0 && shares) b.flags &= ~(GLQ_MM_A_FROM_PREVIOUS_LAUNCH | GLQ_MM_AFTER_KERNEL);
                 b.rows_stride = a->rows_stride > 0 ? a->rows_stride : a->max_rows;
                 if (a->entry_row) b.entry_row = a->entry_row + r0;
                 else b.x = static_cast<const char*>(a->x) + (size_t)r0 * a->ldx * 2;

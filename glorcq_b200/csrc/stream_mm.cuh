@@ -21,12 +21,8 @@
 //   * k splits of a pair are warps of one CTA, reduced through shared memory in a fixed order
 //     (named barrier per pair): no global scratch, no atomics, deterministic;
 //   * when two CTAs of eight warps with their own copies of the staged activations do not fit an SM (8 rows of 4096
-//     channels: 65 KB), one CTA of sixteen warps shares one copy -- one of eight left the SM at a quarter of its warps and
-//     took 18.4 us for 8 rows of a 4-bit 4096 x 4096, the one of sixteen 13.0;
-//   * reductions whose activations do not fit at all (14336 channels) are cut into k chunks that go to different CTAs; a
-//     pair's chunks meet in global scratch, the warp that arrives last adds them in chunk order (deterministic) and runs
-//     the epilogue.  The general kernel (skinny_mm.cuh) took these before: 152 us for the down products of 16 tokens over
-//     8 experts (14336 -> 4096), now 75.
+//     channels: 65 KB), one CTA of sixteen warps shares one copy: 8 rows of a 4-bit 4096 x 4096 took 18.4 us with eight
+//     warps on an SM, 13.0 with sixteen.
 // Every mbarrier wait is bounded in time; a wait that runs out records an error word and the warp
 // stops waiting, so the kernel always terminates.  No cluster launch, no multicast.
 #pragma once
@@ -55,10 +51,9 @@ struct StreamParams {
     int sk;            // k splits (warps of one CTA): 1, 2, 4 or 8
     int sk_log2;
     int kb_per_split;
-    int kc, kb_per_chunk;   // k chunks over CTAs (1: none) and their k blocks
     int cb;            // k blocks per ring stage
     int npairs;        // tile pairs per problem
-    int ips;           // iterations (one item per warp of the CTA) per problem and k chunk
+    int ips;           // iterations (one item per warp of the CTA) per problem
     int stages;        // ring depth
     int stage_bytes;
     int off_xs, off_ox, off_as, off_ring, off_red;  // shared memory carve-up (bytes)
@@ -156,8 +151,8 @@ __device__ __forceinline__ void imma16832(int (&d)[4], uint32_t a0, uint32_t a1,
 // (4-bit).  Layout: xs[kb][piece][col = 2*row + digit][t] of uint4, piece = u (2-bit) / 0 (4-bit);
 // ox[kb][row] = (2^-sh, sum of x).
 template <int FMT, int THREADS>
-__device__ __forceinline__ void stage_x_i8(const SkinnyParams& p, uint4* xs, float2* ox, int kb0, int nkb, int ncol, int e0,
-                                           int cnt, int K) {
+__device__ __forceinline__ void stage_x_i8(const SkinnyParams& p, uint4* xs, float2* ox, int nkb, int ncol, int e0, int cnt,
+                                           int K) {
     using F = Fmt<FMT>;
     constexpr int P8 = F::UPK / 4;  // pieces per block: 2 (2-bit), 1 (4-bit)
     const int nrow = ncol >> 1;
@@ -167,7 +162,7 @@ __device__ __forceinline__ void stage_x_i8(const SkinnyParams& p, uint4* xs, flo
     // unit u = 16 channels of a row; the loads of a thread's next unit are under way while it converts one
     auto load = [&](int u, int row, int rem, uint4 (&v)[2]) {
         v[0] = v[1] = make_uint4(0, 0, 0, 0);
-        const int k0 = kb0 * F::KB + rem * 16;
+        const int k0 = rem * 16;
         if (u >= total || k0 >= K) return;
         const int entry = e0 + row;
         const long long xr = p.entry_row ? __ldg(p.entry_row + entry) : entry;
@@ -396,7 +391,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
     const int g = lane >> 2, t = lane & 3;
     const int N = sp.N, K = sp.K, rank = sp.rank;
     const int nkb = p.nkb, ntc = p.ntc;
-    const int S = sp.stages, sk = sp.sk, kc = sp.kc, cb = sp.cb;
+    const int S = sp.stages, sk = sp.sk, cb = sp.cb;
     const bool swiglu = sp.swiglu != 0;
     const int ns = (rank + 63) / 64;
 
@@ -405,7 +400,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
     if (!sp.a_late) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int n_live = p.n_slots ? min(__ldg(p.n_slots), sp.n_problems) : sp.n_problems;
-    const long total = (long)n_live * kc * sp.ips;
+    const long total = (long)n_live * sp.ips;
     const int it_lo = (int)((long)blockIdx.x * total / gridDim.x);
     const int it_hi = (int)((long)(blockIdx.x + 1) * total / gridDim.x);
     if (it_lo >= it_hi) {
@@ -458,20 +453,19 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
     };
     // item of warp w in iteration it: (slot, pair, split) -> k range and chunk counts
     struct Item {
-        int slot, chunk, pair, s, kb_lo, kb_hi, ncode, nch;
+        int slot, pair, s, kb_lo, kb_hi, ncode, nch;
         bool valid;
     };
-    auto make_item = [&](Item& im, const Slot& sc, int slot, int chunk, int rem) {   // iteration = (slot * kc + chunk) * ips + rem
+    auto make_item = [&](Item& im, const Slot& sc, int slot, int rem) {   // iteration = slot * ips + rem
         const int local = rem * NW + w;
         im.slot = slot;
-        im.chunk = chunk;
         im.pair = local >> sp.sk_log2;
         im.s = local & (sk - 1);
         im.valid = im.pair < sp.npairs && sc.cnt > 0;
-        im.kb_lo = chunk * sp.kb_per_chunk + im.s * sp.kb_per_split;
-        im.kb_hi = min(min(nkb, (chunk + 1) * sp.kb_per_chunk), im.kb_lo + sp.kb_per_split);
+        im.kb_lo = im.s * sp.kb_per_split;
+        im.kb_hi = min(nkb, im.kb_lo + sp.kb_per_split);
         im.ncode = im.kb_hi > im.kb_lo ? (im.kb_hi - im.kb_lo + cb - 1) >> (cb == 4 ? 2 : 1) : 0;
-        im.nch = im.ncode + ((im.s == 0 && chunk == 0 && sc.sv != nullptr) ? ns : 0);
+        im.nch = im.ncode + ((im.s == 0 && sc.sv != nullptr) ? ns : 0);
     };
 
     // ---- fetch cursor: runs over the same (item, chunk) sequence as the compute loop, S stages ahead
@@ -479,13 +473,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
     Slot fs, cs;
     Item fi;
     // cursors keep (iteration, slot, iteration within the slot) and ring positions incrementally: no divisions
-    int f_it = it_lo, f_rem = it_lo % sp.ips, f_chunk = (it_lo / sp.ips) % kc, f_slot = it_lo / sp.ips / kc, f_c = 0;
-    auto step = [&](int& slot, int& chunk, int& rem) {
-        if (++rem == sp.ips) {
-            rem = 0;
-            if (++chunk == kc) chunk = 0, ++slot;
-        }
-    };
+    int f_it = it_lo, f_slot = it_lo / sp.ips, f_rem = it_lo % sp.ips, f_c = 0;
     int f_stage = 0, f_inflight = 0;      // next stage to fill, chunks issued and not yet consumed
     int c_stage = 0;                      // next stage to consume
     uint32_t c_phase = 0;                 // its mbarrier phase parity
@@ -494,13 +482,13 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
         f_live = false;
         while (f_it < it_hi) {
             load_slot(fs, f_slot);
-            make_item(fi, fs, f_slot, f_chunk, f_rem);
+            make_item(fi, fs, f_slot, f_rem);
             if (fi.valid && fi.nch > 0) {
                 f_live = true;
                 return;
             }
             ++f_it;
-            step(f_slot, f_chunk, f_rem);
+            if (++f_rem == sp.ips) f_rem = 0, ++f_slot;
         }
     };
     auto fetch_one = [&]() {
@@ -526,7 +514,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
         if (++f_c >= fi.nch) {
             f_c = 0;
             ++f_it;
-            step(f_slot, f_chunk, f_rem);
+            if (++f_rem == sp.ips) f_rem = 0, ++f_slot;
             fetch_seek();
         }
     };
@@ -548,24 +536,23 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
     // integer path of the codebook format: coefficients of the two tiles' codebooks (tile_block_t2_i8)
     float cb_c0[2] = {0.f, 0.f}, cb_d0[2] = {0.f, 0.f}, cb_dh[2] = {0.f, 0.f}, cb_e[2] = {0.f, 0.f};
     bool cb_cross = false;
-    int staged_slot = -1, staged_chunk = -1, red_par = 0;
+    int staged_slot = -1, red_par = 0;
     bool dep_waited = false;
     constexpr int ncol_i8 = 2 * kRows;  // digit columns staged on the integer path
 
-    int c_rem = it_lo % sp.ips, c_chunk = (it_lo / sp.ips) % kc, c_slot = it_lo / sp.ips / kc;
-    for (int it = it_lo; it < it_hi; ++it, step(c_slot, c_chunk, c_rem)) {
+    int c_slot = it_lo / sp.ips, c_rem = it_lo % sp.ips;
+    for (int it = it_lo; it < it_hi; ++it, c_rem = (c_rem + 1 == sp.ips ? 0 : c_rem + 1), c_slot += (c_rem == 0)) {
         load_slot(cs, c_slot);
         Item im;
-        make_item(im, cs, c_slot, c_chunk, c_rem);
-        const int kb_base = c_chunk * sp.kb_per_chunk;      // first staged k block
+        make_item(im, cs, c_slot, c_rem);
         const int cnt = cs.cnt, e0 = cs.e0;
 
         // ---- activations of a new problem: staged once per CTA ----
-        if (im.slot != staged_slot || c_chunk != staged_chunk) {
+        if (im.slot != staged_slot) {
             __syncthreads();
             if (cnt > 0) {
                 if constexpr (I8)
-                    stage_x_i8<FMT, NW * 32>(p, xs, ox, kb_base, min(nkb - kb_base, sp.kb_per_chunk), ncol_i8, e0, cnt, K);
+                    stage_x_i8<FMT, NW * 32>(p, xs, ox, nkb, ncol_i8, e0, cnt, K);
                 else
                     stage_x<FMT>(p, xs, ox, 0, nkb, e0, 0, cnt, K);
                 if (cs.sv != nullptr && !sp.a_late) {
@@ -582,7 +569,6 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
             }
             __syncthreads();
             staged_slot = im.slot;
-            staged_chunk = c_chunk;
             if constexpr (FMT == GLQ_FMT_T2) {
                 // a fused gate|up weight carries two codebooks (4 floats each)
                 if constexpr (I8) {
@@ -631,7 +617,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
 #pragma unroll
             for (int b = 0; b < kStreamCB; ++b) {
                 if (b >= nblk) break;
-                const int kb = kb0 + b - kb_base;     // among the staged ones
+                const int kb = kb0 + b;
                 if constexpr (I8) {
                     uint4 bx[NT][2];
                     float2 o[NT];
@@ -823,52 +809,6 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
             ring_release();
         }
 
-        // ---- k chunks of this pair: records in global scratch, added in chunk order by the warp that arrives last ----
-        bool low_rank = nsv > 0;
-        if constexpr (I8) {
-            if (kc > 1) {
-                constexpr int REC = 2 * NT * 2, LOREC = 2 * NM * 4;       // floats per lane of a chunk's record, of the low-rank term
-                low_rank = cs.sv != nullptr;
-                const size_t item = (size_t)im.slot * sp.npairs + im.pair;
-                float* rec = reinterpret_cast<float*>(p.scratch) + item * (size_t)((kc * REC + LOREC) * 32) + lane;
-                float* mine = rec + (LOREC + im.chunk * REC) * 32;
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-#pragma unroll
-                    for (int nt = 0; nt < NT; ++nt) {
-                        __stcg(mine + ((j * NT + nt) * 2) * 32, acc[j][nt][0]);
-                        __stcg(mine + ((j * NT + nt) * 2 + 1) * 32, acc[j][nt][2]);
-                    }
-                if (im.chunk == 0 && low_rank)
-#pragma unroll
-                    for (int i = 0; i < LOREC; ++i) __stcg(rec + i * 32, lo[i / (NM * 4)][(i / 4) % NM][i % 4]);
-                __threadfence();
-                __syncwarp();
-                int last = 0;
-                if (lane == 0) last = atomicAdd(p.counters + item, 1) == kc - 1;
-                if (!__shfl_sync(0xffffffffu, last, 0)) continue;
-                __threadfence();
-                if (lane == 0) p.counters[item] = 0;
-#pragma unroll
-                for (int j = 0; j < 2; ++j)
-#pragma unroll
-                    for (int nt = 0; nt < NT; ++nt) acc[j][nt][0] = acc[j][nt][2] = 0.f;
-                for (int c = 0; c < kc; ++c) {
-                    const float* r = rec + (LOREC + c * REC) * 32;
-#pragma unroll
-                    for (int j = 0; j < 2; ++j)
-#pragma unroll
-                        for (int nt = 0; nt < NT; ++nt) {
-                            acc[j][nt][0] += __ldcg(r + ((j * NT + nt) * 2) * 32);
-                            acc[j][nt][2] += __ldcg(r + ((j * NT + nt) * 2 + 1) * 32);
-                        }
-                }
-                if (low_rank)
-#pragma unroll
-                    for (int i = 0; i < LOREC; ++i) lo[i / (NM * 4)][(i / 4) % NM][i % 4] = __ldcg(rec + i * 32);
-            }
-        }
-
         // ---- epilogue: this lane's activation rows, weight rows g and g+8 of both tiles ----
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt) {
@@ -886,15 +826,15 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
                     }
                     float v0 = round16(acc[j][nt][I8 ? 0 : e] * n0);
                     float v1 = round16(acc[j][nt][I8 ? 2 : 2 + e] * n1);
-                    if (low_rank) {
+                    if (nsv > 0) {
                         float l0, l1;
                         if constexpr (I8) {
                             // the low-rank op holds rows 2t', 2t'+1 in lane t': fetch this lane's row
                             const int src = (g << 2) | ((row & 7) >> 1);
-                            const float a0 = __shfl_sync(0xffffffffu, lo[j][nt >> 1][0], src);
-                            const float a1 = __shfl_sync(0xffffffffu, lo[j][nt >> 1][1], src);
-                            const float b0 = __shfl_sync(0xffffffffu, lo[j][nt >> 1][2], src);
-                            const float b1 = __shfl_sync(0xffffffffu, lo[j][nt >> 1][3], src);
+                            const float a0 = __shfl_sync(0xffffffffu, lo[j][0][0], src);
+                            const float a1 = __shfl_sync(0xffffffffu, lo[j][0][1], src);
+                            const float b0 = __shfl_sync(0xffffffffu, lo[j][0][2], src);
+                            const float b1 = __shfl_sync(0xffffffffu, lo[j][0][3], src);
                             l0 = (row & 1) ? a1 : a0;
                             l1 = (row & 1) ? b1 : b0;
                         } else {

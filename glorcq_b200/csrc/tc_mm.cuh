@@ -90,10 +90,12 @@ __device__ __forceinline__ bool tc_find_tile(const TcParams& p, int gt, int& slo
 
 // K position -> channel of the tensor-memory kernel (tc_ps.cuh).  Position P = 64*w + 16*n + 4*t + i of a 128-channel
 // stage (w: producer half, n: repeat of its tensor-memory store = k step inside the half, t: lane mod 4, i: 0..3) holds
-// value i & 1 of the pair 2*n + (i >> 1) that the format's unpack yields from the lane's 16 codes of that half.
+// value i & 1 of the pair 2*n + (i >> 1) that the format's unpack yields from the lane's 16 codes of that half; 4-bit: of pair
+// 2*(t & 1) + (i >> 1) of word t >> 1 of the 16 consecutive channels 16*n.. of k block w, so that a k step is 16 consecutive
+// channels in order (the order of the sums of the kernel for dense weights).
 __host__ __device__ __forceinline__ int tc_ts_channel_of(int fmt, int P) {
     const int w = P >> 6, n = (P >> 4) & 3, t = (P >> 2) & 3, j = 2 * n + ((P >> 1) & 1), b = P & 1;
-    if (fmt == GLQ_FMT_Q4) return 64 * w + 16 * t + 8 * (j >> 2) + (j & 3) + 4 * b;
+    if (fmt == GLQ_FMT_Q4) return 64 * w + 16 * n + 8 * (t >> 1) + 2 * (t & 1) + (j & 1) + 4 * b;
     const int c = fmt == GLQ_FMT_Q2 ? j + 8 * b : 4 * (j & 3) + (j >> 2) + 2 * b;
     return 32 * t + 16 * w + c;
 }
@@ -110,9 +112,9 @@ __global__ void __launch_bounds__(256) tc_pack_b_kernel(const TcParams p) {
     unsigned char* tile = p.xp + (size_t)blockIdx.x * p.tile_bytes;
     const int st = blockIdx.y;
     if (st < p.nkb && p.ts && p.x_vec16 && st * 128 + 128 <= p.K) {
-        // tensor-memory order, whole stage inside K: a thread takes the 16 consecutive channels (two 16-byte
-        // loads) of one row that half w of lane t unpacks, and writes the four 8-byte pieces that k steps 0..3 of
-        // atom w hold for lane t
+        // tensor-memory order, whole stage inside K: a thread takes 16 consecutive channels (two 16-byte loads) of one
+        // row.  Q2/T2: those that half w of lane t unpacks, in four 8-byte pieces, one for each of k steps 0..3 of atom w;
+        // Q4: k step n of atom w, in four 8-byte pieces, one for each lane t.
         unsigned char* sdst = tile + (size_t)st * TN * 256;
 #pragma unroll 2
         for (int idx = threadIdx.x; idx < TN * 8; idx += 256) {
@@ -126,22 +128,31 @@ __global__ void __launch_bounds__(256) tc_pack_b_kernel(const TcParams p) {
                 hi = __ldg(src + 1);
             }
             const uint32_t a[4] = {lo.x, lo.y, lo.z, lo.w}, b[4] = {hi.x, hi.y, hi.z, hi.w};
-            unsigned char* rdst = sdst + (size_t)w * (TN * 128) + (size_t)r * 128 + (t & 1) * 8;
+            unsigned char* rdst = sdst + (size_t)w * (TN * 128) + (size_t)r * 128;
+            if (p.fmt == GLQ_FMT_Q4) {
+                // (c, c+4), (c+1, c+5): c = 0, 2 of the lower, of the upper eight channels for lanes 0..3 of step n = t
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t(&u)[4] = h ? b : a;
+                    const int c = (2 * t + h) ^ (r & 7);
+                    *reinterpret_cast<uint4*>(rdst + c * 16) =
+                        make_uint4(__byte_perm(u[0], u[2], 0x5410), __byte_perm(u[0], u[2], 0x7632), __byte_perm(u[1], u[3], 0x5410),
+                                   __byte_perm(u[1], u[3], 0x7632));
+                }
+                continue;
+            }
 #pragma unroll
             for (int n = 0; n < 4; ++n) {
                 const int c = (2 * n + (t >> 1)) ^ (r & 7);
                 uint2 v;
                 if (p.fmt == GLQ_FMT_Q2) {            // (2n, 2n+8), (2n+1, 2n+9)
                     v = make_uint2(__byte_perm(a[n], b[n], 0x5410), __byte_perm(a[n], b[n], 0x7632));
-                } else if (p.fmt == GLQ_FMT_Q4) {     // (c, c+4), (c+1, c+5), c = 8 (n/2) + 2 (n%2)
-                    const uint32_t(&u)[4] = n < 2 ? a : b;
-                    v = make_uint2(__byte_perm(u[n & 1], u[(n & 1) + 2], 0x5410), __byte_perm(u[n & 1], u[(n & 1) + 2], 0x7632));
                 } else {                              // even (n < 2) or odd codes of eight: (c, c+2), (c+4, c+6)
                     const uint32_t(&u)[4] = n & 1 ? b : a;
                     const uint32_t sel = n < 2 ? 0x5410u : 0x7632u;
                     v = make_uint2(__byte_perm(u[0], u[1], sel), __byte_perm(u[2], u[3], sel));
                 }
-                *reinterpret_cast<uint2*>(rdst + c * 16) = v;
+                *reinterpret_cast<uint2*>(rdst + (t & 1) * 8 + c * 16) = v;
             }
         }
     } else if (st < p.nkb) {

@@ -114,28 +114,29 @@ template <> struct PsUnpack<GLQ_FMT_Q2> {
     static constexpr float kTop = 64.f;        // the largest offset
     // offset class of pair j (see unpack_q2)
     static __device__ __forceinline__ constexpr int cls(int j) { return (j == 4 || j == 7) ? 2 : ((j == 1 || j == 3 || j == 6) ? 1 : 0); }
-    static __device__ __forceinline__ void pairs(const uint32_t (&w)[2], uint32_t (&h)[8]) { unpack_q2(w[0], h); }
+    static constexpr int WORDS = 1;             // 32-bit words that hold a row's 16 codes of a half
+    static __device__ __forceinline__ void pairs(const uint32_t (&w)[1], int, uint32_t (&h)[8]) { unpack_q2(w[0], h); }
 };
 template <> struct PsUnpack<GLQ_FMT_Q4> {
     static __device__ __forceinline__ constexpr float off(int c) { return c == 0 ? 1024.f : 64.f; }
     static constexpr float kTop = 1024.f;
     static __device__ __forceinline__ constexpr int cls(int j) { return j & 1; }
-    // pair j of a word = codes (j, j + 4): nibbles 0, 4 at mantissa bit 0, nibbles 1, 5 at bit 4, the rest after one shift
-    static __device__ __forceinline__ void pairs(const uint32_t (&w)[2], uint32_t (&h)[8]) {
+    static constexpr int WORDS = 4;             // word t >> 1 of each of the block's four groups of 16 channels
+    // codes (c, c + 4), (c + 1, c + 5) of every word, c = 2 (t & 1); sh = 8 (t & 1)
+    static __device__ __forceinline__ void pairs(const uint32_t (&w)[4], int sh, uint32_t (&h)[8]) {
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const uint32_t v = w[u], v8 = w[u] >> 8;
-            h[4 * u + 0] = and_or(v, 0x000F000Fu, 0x64006400u);
-            h[4 * u + 1] = and_or(v, 0x00F000F0u, 0x54005400u);
-            h[4 * u + 2] = and_or(v8, 0x000F000Fu, 0x64006400u);
-            h[4 * u + 3] = and_or(v8, 0x00F000F0u, 0x54005400u);
+        for (int n = 0; n < 4; ++n) {
+            const uint32_t v = w[n] >> sh;
+            h[2 * n] = and_or(v, 0x000F000Fu, 0x64006400u);
+            h[2 * n + 1] = and_or(v, 0x00F000F0u, 0x54005400u);
         }
     }
 };
+template <> struct PsUnpack<GLQ_FMT_T2> { static constexpr int WORDS = 1; };
 
 // Both rows (g, g + 8) of a lane: words w[row][..], (scale, zero) pairs sz[row] -> the 16 registers of tc_st_x4.
 template <int FMT>
-__device__ __forceinline__ void ps_affine(const uint32_t (&w)[2][2], const uint32_t (&sz)[2], uint32_t (&r)[16]) {
+__device__ __forceinline__ void ps_affine(const uint32_t (&w)[2][PsUnpack<FMT>::WORDS], const uint32_t (&sz)[2], int sh, uint32_t (&r)[16]) {
     using U = PsUnpack<FMT>;
     const uint32_t zb = __byte_perm(sz[0], sz[1], 0x7632);        // (z of row g, z of row g + 8)
     const __half2 z2 = *reinterpret_cast<const __half2*>(&zb);
@@ -149,7 +150,7 @@ __device__ __forceinline__ void ps_affine(const uint32_t (&w)[2][2], const uint3
 #pragma unroll
     for (int hrow = 0; hrow < 2; ++hrow) {
         uint32_t h[8];
-        U::pairs(w[hrow], h);
+        U::pairs(w[hrow], sh, h);
         const __half2 s2 = __half2half2(__ushort_as_half((unsigned short)(sz[hrow] & 0xffffu)));
         if (fast) {
 #pragma unroll
@@ -312,23 +313,29 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
         };
 
         // ---- codes: requested D stages ahead (the first ones of an item before the previous item's epilogue).  Lane (g, t)
-        // holds rows g and g + 8 of its tile.  Half h of the channels: Q2/T2 word h of a row, Q4 both words of k block h.
+        // holds rows g and g + 8 of its tile.  Half h of the channels: Q2/T2 word h of its own 16 bytes' rows, Q4 a word of each
+        // of the four lanes of its row in k block h (see tc_ts_channel_of).
         // (D <= S: the stages of a group find room in the ring before the results of the item before are taken)
-        constexpr int D0 = HALVES == 2 ? (FMT == GLQ_FMT_Q4 ? 2 : 3) : 4, D = D0 < S ? D0 : S;
+        constexpr int WPR = PsUnpack<FMT>::WORDS;                  // words per half and row
+        constexpr int D0 = (HALVES == 2 ? 3 : 4) - (FMT == GLQ_FMT_Q4 ? 1 : 0), D = D0 < S ? D0 : S;
         constexpr int NSZ = FMT == GLQ_FMT_Q4 ? HALVES : 1;        // (scale, zero) sets per stage
-        uint32_t cq[D][HALVES][2][2], csz[D][NSZ][2];              // [stage][half][row][word]
+        uint32_t cq[D][HALVES][2][WPR], csz[D][NSZ][2];              // [stage][half][row][word]
         const unsigned char* blk = nullptr;                        // of the next stage to request
         int left = 0;                                              // k blocks of the item still to request
         bool live = false;
-        auto fetch = [&](uint32_t (&qv)[HALVES][2][2], uint32_t (&zv)[NSZ][2]) {
+        auto fetch = [&](uint32_t (&qv)[HALVES][2][WPR], uint32_t (&zv)[NSZ][2]) {
             if constexpr (FMT == GLQ_FMT_Q4) {
 #pragma unroll
                 for (int h = 0; h < HALVES; ++h) {
                     const bool in = wh0 + h < left;
                     const unsigned char* src = blk + (wh0 + h) * (2 * BB);
-                    const uint4 v = in ? __ldg(reinterpret_cast<const uint4*>(src) + lane) : make_uint4(0, 0, 0, 0);
+                    const uint32_t* wsrc = reinterpret_cast<const uint32_t*>(src) + g * 16 + (t >> 1);
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        qv[h][0][n] = in ? __ldg(wsrc + 4 * n) : 0u;
+                        qv[h][1][n] = in ? __ldg(wsrc + 4 * n + 2) : 0u;
+                    }
                     const uint2 z = in ? __ldg(reinterpret_cast<const uint2*>(src + 512) + g) : make_uint2(0, 0);
-                    qv[h][0][0] = v.x, qv[h][0][1] = v.y, qv[h][1][0] = v.z, qv[h][1][1] = v.w;
                     zv[h][0] = z.x, zv[h][1] = z.y;
                 }
                 left -= 2;
@@ -370,9 +377,9 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(im.sv + ((((size_t)(d16 >> 1) * p.ns + sl) * 32) + (d16 & 1) * 16 + lane) * 128));
         };
         // the 16 registers of a half's store: for k step n of the half {row g: positions 4t..4t+3, row g+8: the same}
-        auto unpack = [&](const uint32_t (&qv)[2][2], const uint32_t (&zv)[2], uint32_t (&r)[16]) {
+        auto unpack = [&](const uint32_t (&qv)[2][WPR], const uint32_t (&zv)[2], uint32_t (&r)[16]) {
             if constexpr (AFFINE) {
-                ps_affine<FMT>(qv, zv, r);
+                ps_affine<FMT>(qv, zv, 8 * (t & 1), r);
             } else {
 #pragma unroll
                 for (int hrow = 0; hrow < 2; ++hrow) {

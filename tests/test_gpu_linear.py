@@ -331,7 +331,7 @@ def test_many_rows_every_format(dev, fmt, bits, gs, N, K, rank, B):
 @pytest.mark.parametrize("B", [1, 5, 8, 13])
 @pytest.mark.parametrize("fmt,bits,N,K", [("gptq", 2, 72, 14336), ("gptq", 4, 4096, 4096), ("turbo", 2, 1000, 8192), ("gptq", 2, 4096, 24576)])
 def test_long_reductions(dev, fmt, bits, N, K, B):
-    """Rows too long for two CTAs' copies of them: one CTA of sixteen warps, and k chunks that meet in global scratch."""
+    """Rows too long for two CTAs' copies of them: one CTA of eight or sixteen warps, or the general kernel."""
     from glorcq_b200 import tiled
     if N * K > 20_000_000 and B > 5:
         pytest.skip("the longest rows on few of them")
@@ -347,7 +347,7 @@ def test_long_reductions(dev, fmt, bits, N, K, B):
 
 @pytest.mark.parametrize("N,K", [(64, 2048), (192, 4096), (8, 264), (72, 64), (512, 1408), (520, 256)])
 def test_dense_few_columns(dev, N, K):
-    """x . W^T on 9 and more rows: row tiles of 32, column slices of 64, K over warps and clusters of CTAs."""
+    """x . W^T with few columns on both sides of 32 rows: row tiles of 32 and 64, column slices of 64."""
     from glorcq_b200 import tiled
     W = torch.randn(N, K, generator=torch.Generator().manual_seed(N + K)).half()
     tw = tiled.TiledWeight.from_dense(W.to(dev))
