@@ -80,7 +80,7 @@ extern "C" size_t glq_tiled_f16_bytes(int N, int K) {
 // launch geometry of the skinny kernel (shared by the workspace query and the launcher)
 // ---------------------------------------------------------------------------------------------
 struct Geometry {
-    int nw, ntt, ntc, nkb, group_blocks, tile_groups, sk, kb_per_split, kb_chunk, max_passes;
+    int nw, ntt, ntc, nkb, group_blocks, tile_groups, tgn, sk, kb_per_split, kb_chunk, max_passes;
     size_t smem, n_counters, scratch_bytes;
 };
 
@@ -134,6 +134,10 @@ static int plan_geometry(int fmt, int epilogue, int N, int K, int group_size, in
     g.kb_chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)std::min(g.kb_per_split, g.nkb),
                                                              (smem_cap - fixed) / per_kb));
     g.smem = skinny_smem_bytes(fmt, g.kb_chunk, g.ntc, g.nw, g.ntt);
+    // rows too long to stage at once are staged again by every CTA: four tile groups share a staging when that still leaves
+    // a CTA for every slot
+    g.tgn = ((fmt == GLQ_FMT_Q2 || fmt == GLQ_FMT_Q4) && g.nw == 1 && g.ntt == 1 && g.sk == 1 && g.kb_chunk < g.nkb &&
+             (long)n_problems * g.tile_groups >= 4L * 2 * num_sms()) ? 4 : 1;
     const size_t tiles = (size_t)n_problems * g.tile_groups * g.max_passes;
     g.n_counters = g.sk > 1 ? tiles : 0;
     g.scratch_bytes = g.sk > 1 ? tiles * g.sk * (size_t)(kRW * g.nw * g.ntt * 32) * sizeof(float4) : 0;
@@ -161,9 +165,9 @@ static int launch_dependent(Kern kern, dim3 grid, dim3 block, size_t smem, cudaS
     return GLQ_OK;
 }
 
-template <int FMT, int NW, int NTT, bool RM>
+template <int FMT, int NW, int NTT, bool RM, int TGN = 1>
 static int launch_one(const SkinnyParams& p, int grid, size_t smem, cudaStream_t st) {
-    auto kern = skinny_kernel<FMT, NW, NTT, RM>;
+    auto kern = skinny_kernel<FMT, NW, NTT, RM, TGN>;
     if (smem > 48 * 1024) {
         static size_t configured[16] = {0};
         int dev = 0;
@@ -189,6 +193,8 @@ static int launch_fmt(const SkinnyParams& p, const Geometry& g, int grid, cudaSt
             return launch_one<FMT, 2, 2, false>(p, grid, g.smem, st);
         }
     }
+    if constexpr (!RM && (FMT == GLQ_FMT_Q2 || FMT == GLQ_FMT_Q4))
+        if (g.tgn == 4) return launch_one<FMT, 1, 1, false, 4>(p, grid, g.smem, st);
     if (g.ntt == 1) return launch_one<FMT, 1, 1, RM>(p, grid, g.smem, st);
     if (g.ntt == 2) return launch_one<FMT, 1, 2, RM>(p, grid, g.smem, st);
     return launch_one<FMT, 1, 4, RM>(p, grid, g.smem, st);
@@ -196,7 +202,7 @@ static int launch_fmt(const SkinnyParams& p, const Geometry& g, int grid, cudaSt
 
 static int launch_skinny(int fmt, bool rowmajor, const SkinnyParams& p, const Geometry& g, int n_problems,
                          cudaStream_t st) {
-    const long grid = (long)n_problems * g.tile_groups * g.sk;
+    const long grid = (long)n_problems * cdiv(g.tile_groups, g.tgn) * g.sk;
     if (grid <= 0 || grid > 0x7fffffffL) return GLQ_ERR_UNSUPPORTED;
     if (rowmajor) {
         if (fmt != GLQ_FMT_T2) return GLQ_ERR_UNSUPPORTED;
@@ -226,7 +232,7 @@ static void fill_geometry(SkinnyParams& p, const Geometry& g) {
 // streaming kernel: eligibility, geometry, launch
 // ---------------------------------------------------------------------------------------------
 struct StreamGeom {
-    int i8, nt, ntc, nkb, nw, cb, sk, kb_per_split, npairs, ips, stages, stage_bytes, swiglu;
+    int i8, nt, ntc, nkb, nw, cb, chunks, sk, kb_per_split, npairs, ips, stages, stage_bytes, swiglu;
     int off_xs, off_ox, off_as, off_ring, off_red;
     size_t smem;
     int grid;
@@ -271,8 +277,9 @@ static int stream_splits(size_t base, size_t stage, int nt, int npairs, int unit
 }
 
 // returns true when the streaming kernel covers this call
+// chunks: slots that a problem's rows are cut into
 static bool plan_stream(int fmt, int epilogue, int N, int K, int rank, int group_size, int n_problems, int max_rows,
-                        StreamGeom* out) {
+                        StreamGeom* out, int chunks = 1) {
     if (stream_disabled()) return false;
     if (fmt != GLQ_FMT_Q2 && fmt != GLQ_FMT_Q4 && fmt != GLQ_FMT_T2) return false;
     if (N <= 0 || K <= 0 || n_problems <= 0 || max_rows <= 0 || rank < 0 || rank % 16 != 0) return false;
@@ -332,6 +339,7 @@ static bool plan_stream(int fmt, int epilogue, int N, int K, int rank, int group
     // slots.  Two CTAs of eight warps per SM are the rule; one of eight leaves room for the sums of many splits; one of
     // sixteen shares its activations among all warps of an SM.  Stages hold four k blocks, two when that is what it takes.
     const int sms = num_sms();
+    g.chunks = chunks;
     StreamGeom best{};
     long best_rounds = -1;
     auto consider = [&](int nw, int cb, size_t cap, int slots) {
@@ -341,7 +349,7 @@ static bool plan_stream(int fmt, int epilogue, int N, int K, int rank, int group
         g.nw = nw;
         g.cb = cb;
         g.ips = cdiv(g.npairs * g.sk, nw);
-        const long iters = (long)n_problems * g.ips, rounds = (iters + slots - 1) / slots;      // (ties: the form named first)
+        const long iters = (long)n_problems * chunks * g.ips, rounds = (iters + slots - 1) / slots;      // (ties: the form named first)
         if (best_rounds >= 0 && rounds >= best_rounds) return;
         g.stage_bytes = (int)(stage / nw);
         g.off_ring = (int)off;
@@ -410,7 +418,10 @@ static int launch_stream(const glq_mm_args_t* a, SkinnyParams& p, const StreamGe
     sp.N = N;
     sp.K = K;
     sp.rank = rank;
-    sp.n_problems = n_problems;
+    sp.n_problems = n_problems * g.chunks;
+    sp.chunks = g.chunks;
+    sp.chunk_rows = p.max_rows;
+    sp.prob_rows = a->max_rows;
     sp.swiglu = g.swiglu;
     sp.sk = g.sk;
     sp.sk_log2 = g.sk == 1 ? 0 : (g.sk == 2 ? 1 : (g.sk == 4 ? 2 : 3));
@@ -687,44 +698,27 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
         if (!a->w_table && !a->w.codes) return GLQ_ERR_ARG;
         return launch_tc(a, tg, reinterpret_cast<cudaStream_t>(stream));
     }
-    // 9..32 rows of the same problems, counts known on the host: the integer path stages at most 8 rows and streams at a
-    // multiple of the fp16 path's rate, so it runs over chunks of rows; after the first chunk the weights come from L2
-    // where they fit
-    if (!use_tc && !a->slot_count && !a->slot_offset && a->max_rows > 8 && a->max_rows <= 32 && !i8_disabled() &&
-        (a->fmt == GLQ_FMT_Q2 || a->fmt == GLQ_FMT_Q4)) {
-        int chunk = 0;
-        for (int c : {8, 4}) {
-            StreamGeom cg;
-            if (plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, c, &cg) && cg.i8) {
-                chunk = c;
-                break;
-            }
-        }
-        if (chunk && chunk < a->max_rows) {
-            for (int r0 = 0; r0 < a->max_rows; r0 += chunk) {
-                glq_mm_args_t b = *a;
-                b.max_rows = std::min(chunk, a->max_rows - r0);
-                b.rows_stride = a->rows_stride > 0 ? a->rows_stride : a->max_rows;
-                if (a->entry_row) b.entry_row = a->entry_row + r0;
-                else b.x = static_cast<const char*>(a->x) + (size_t)r0 * a->ldx * 2;
-                if (a->entry_scale) b.entry_scale = static_cast<const char*>(a->entry_scale) + (size_t)r0 * 2;
-                if (a->a0) b.a0 = static_cast<const char*>(a->a0) + (size_t)r0 * a->lda * 2;
-                if (a->a1) b.a1 = static_cast<const char*>(a->a1) + (size_t)r0 * a->lda * 2;
-                b.y = static_cast<char*>(a->y) + (size_t)r0 * a->ldy * 2;
-                const int rc = glq_grouped_matmul(&b, stream);
-                if (rc != GLQ_OK) return rc;
-            }
-            return GLQ_OK;
-        }
-    }
     StreamGeom sg;
     // Row-count classes (device-side counts): slots with <= 8 rows go to the integer path, 9..16 to the
     // fp16 path with two activation tiles, and above that to the tcgen05 kernel when the call may have
     // more than 32 rows per slot, else to the fp16 path with four tiles.  Each class is one launch that
     // skips the slots of the others.
     StreamGeom sg8, sg16;
-    const int cap = use_tc ? 16 : std::min(a->max_rows, 32);
-    bool use_stream = plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, cap, &sg);
+    // 9..32 rows, counts known on the host: the integer path stages at most 8 rows (4 when the staged activations of a long
+    // reduction leave no room for 8) and streams at a multiple of the fp16 path's rate, so the rows are cut into chunks, the
+    // slots of ONE launch (a launch per chunk took 17.7 us for each 8 of 16 rows of a 4-bit 4096 x 4096); the chunks read
+    // the weights at about the same time, once from memory and then from L2.
+    int cap = use_tc ? 16 : std::min(a->max_rows, 32);
+    bool chunked = false;
+    if (!use_tc && !a->slot_count && !a->slot_offset && !a->slot_index && a->max_rows > 8 && a->max_rows <= 32 && !i8_disabled() &&
+        (a->fmt == GLQ_FMT_Q2 || a->fmt == GLQ_FMT_Q4))
+        for (int c : {8, 4})
+            if (!chunked && plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, c, &sg, cdiv(a->max_rows, c)) &&
+                sg.i8) {
+                chunked = true;
+                cap = c;
+            }
+    bool use_stream = chunked || plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, cap, &sg);
     const bool classes = use_stream && a->slot_count != nullptr && a->max_rows > 8 && !hybrid_disabled();
     const bool split8 = classes && plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, 8, &sg8) &&
                         sg8.i8;
@@ -769,6 +763,7 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
     p.rows_stride = a->rows_stride > 0 ? a->rows_stride : a->max_rows;
     p.epilogue = a->epilogue;
     p.x_vec = (aligned16(a->x) && a->ldx % 8 == 0) ? 1 : 0;
+    if (chunked) p.max_rows = cap;
     if (use_stream) {
         cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
         const bool a_late = (a->flags & GLQ_MM_A_FROM_PREVIOUS_LAUNCH) != 0, dep = (a->flags & GLQ_MM_AFTER_KERNEL) != 0;

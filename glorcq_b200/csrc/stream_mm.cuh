@@ -52,6 +52,7 @@ struct StreamParams {
     int sk_log2;
     int kb_per_split;
     int cb;            // k blocks per ring stage
+    int chunks, chunk_rows, prob_rows;  // chunks > 1: a slot is a chunk of the prob_rows rows of problem slot / chunks
     int npairs;        // tile pairs per problem
     int ips;           // iterations (one item per warp of the CTA) per problem
     int stages;        // ring depth
@@ -439,11 +440,18 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
     auto load_slot = [&](Slot& sc, int slot) {
         if (slot == sc.slot) return;
         sc.slot = slot;
+        int prob = slot;
         sc.cnt = p.slot_count ? __ldg(p.slot_count + slot) : p.max_rows;
         if (sc.cnt <= sp.cnt_lo || sc.cnt > sp.cnt_hi) sc.cnt = 0;     // not this launch's slot: skipped like an empty one
         sc.cnt = min(sc.cnt, p.max_rows);
         sc.e0 = p.slot_offset ? __ldg(p.slot_offset + slot) : slot * p.rows_stride;
-        const int widx = p.slot_index ? __ldg(p.slot_index + slot) : slot;
+        if (sp.chunks > 1) {
+            prob = slot / sp.chunks;
+            const int r0 = (slot - prob * sp.chunks) * sp.chunk_rows;
+            sc.cnt = min(sp.chunk_rows, sp.prob_rows - r0);
+            sc.e0 = prob * p.rows_stride + r0;
+        }
+        const int widx = p.slot_index ? __ldg(p.slot_index + prob) : prob;
         const glq_weight_t* W = p.table ? p.table + widx : &p.w;
         sc.codes = reinterpret_cast<const unsigned char*>(W->codes);
         sc.sv = (rank > 0 && p.a[0] != nullptr) ? reinterpret_cast<const unsigned char*>(W->sv) : nullptr;

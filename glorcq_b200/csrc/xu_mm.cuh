@@ -3,7 +3,7 @@
 //
 // What bounds it: one pass over the rows of x (and over W, which stays in L2).  The tcgen05 kernel (tc_mm.cuh) gives a
 // product with 64 columns ONE 128-feature tile per 128 rows -- three CTAs for 333 rows -- whose producers set the pace
-// (0.9 us per 128 channels), after a pre-pass that re-tiles x: 35.6 + 5.3 us for 333 x 4096 x 64, here XU_MEASURED.
+// (0.9 us per 128 channels), after a pre-pass that re-tiles x: 35.6 + 5.3 us for 333 x 4096 x 64, here 22.4; 21.6 + 6 and 13.7 in a 512-token prompt.
 //   * a CTA owns 16 NT / 2 rows x 64 columns: four warps, each 16 columns (the M side, one operand fragment of W per step) against
 //     NT tiles of 8 rows; a problem with few live rows skips whole operand tiles;
 //   * x (rows gathered through entry_row, 128-byte swizzle) and the fragments of W, which are tiled in operand order, arrive by
