@@ -1175,15 +1175,26 @@ extern "C" int glq_dequant_tiled(int fmt, const void* tiled, const float* norms_
 // ---------------------------------------------------------------------------------------------
 // randomized Hadamard rotation
 // ---------------------------------------------------------------------------------------------
-template <typename TI, typename TO>
-static int launch_rht(const void* x, int64_t ldx, const float* signs, int rows, int d, int n, float scale, void* y,
-                      int64_t ldy, cudaStream_t st) {
-    const size_t smem = (size_t)n * sizeof(float);
-    auto kern = rht_kernel<TI, TO>;
+template <int E, typename TI, typename TO>
+static int launch_rht_e(const void* x, int64_t ldx, const float* signs, int rows, int d, int n, float scale, void* y, int64_t ldy, cudaStream_t st) {
+    const int threads = std::max(32, n >> E);
+    const size_t smem = threads > 32 ? (size_t)n * sizeof(float) : 0;
+    auto kern = rht_kernel<E, TI, TO>;
     if (smem > 48 * 1024) GLQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<rows, 256, smem, st>>>(reinterpret_cast<const TI*>(x), ldx, signs, d, n, scale, reinterpret_cast<TO*>(y), ldy);
+    const int vec = aligned16(x) && ldx % 8 == 0 ? 1 : 0;
+    kern<<<rows, threads, smem, st>>>(reinterpret_cast<const TI*>(x), ldx, signs, d, n, scale, reinterpret_cast<TO*>(y), ldy, vec);
     GLQ_CUDA(cudaGetLastError());
     return GLQ_OK;
+}
+// values per thread: the smallest power whose exponent covers the stages between warps (log2(n) <= 2 E + 5)
+template <typename TI, typename TO>
+static int launch_rht(const void* x, int64_t ldx, const float* signs, int rows, int d, int n, float scale, void* y, int64_t ldy, cudaStream_t st) {
+    if (n <= 32) return launch_rht_e<0, TI, TO>(x, ldx, signs, rows, d, n, scale, y, ldy, st);
+    if (n <= 128) return launch_rht_e<1, TI, TO>(x, ldx, signs, rows, d, n, scale, y, ldy, st);
+    if (n <= 512) return launch_rht_e<2, TI, TO>(x, ldx, signs, rows, d, n, scale, y, ldy, st);
+    if (n <= 2048) return launch_rht_e<3, TI, TO>(x, ldx, signs, rows, d, n, scale, y, ldy, st);
+    if (n <= 8192) return launch_rht_e<4, TI, TO>(x, ldx, signs, rows, d, n, scale, y, ldy, st);
+    return launch_rht_e<5, TI, TO>(x, ldx, signs, rows, d, n, scale, y, ldy, st);
 }
 
 extern "C" int glq_rht_forward(const void* x, int x_is_f32, int64_t ldx, const float* signs, int rows, int d, float scale,

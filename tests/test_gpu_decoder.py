@@ -34,6 +34,15 @@ def dev():
     return torch.device("cuda:0")
 
 
+@pytest.mark.parametrize("d", [1, 5, 32, 33, 100, 300, 1000, 4100, 5632, 14336, 32768])
+def test_rht_every_length(dev, d):
+    """Every number of values per thread, and rows that do not start at 16 bytes."""
+    from glorcq_b200.hadamard_rotation import generate_rht_signs, rht_forward_half
+    x = cases.make_x(70 + d, 3, d, torch.float16)
+    y = rht_forward_half(x.to(dev), generate_rht_signs(d, seed=d, device=dev))
+    assert cases.rel_l2(y.cpu(), O.rht_forward(x.float(), O.generate_rht_signs(d, d))) <= 5e-4
+
+
 @pytest.mark.parametrize("d", [2048, 1408, 768, 64, 48])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
 def test_rht_forward(dev, d, dtype):
