@@ -102,6 +102,7 @@ _SIGS = {
                                   C.c_float, vp, C.c_size_t, vp, C.c_size_t, vp]),
     "glq_lm_head_workspace_bytes": (C.c_size_t, []),
     "glq_lm_head": (C.c_int, [vp, C.c_int64, vp, C.c_int, C.c_int, C.c_int, vp, C.c_int64, vp, vp, C.c_size_t, vp, vp]),
+    "glq_lm_head_rows": (C.c_int, [vp, C.c_int64, vp, C.c_int, C.c_int, C.c_int, vp, C.c_int64, vp, vp, C.c_size_t, vp, vp]),
     "glq_rht_forward": (C.c_int, [vp, C.c_int, C.c_int64, vp, C.c_int, C.c_int, C.c_float, vp, C.c_int, C.c_int64, vp]),
     "glq_mm_workspace_bytes": (C.c_size_t, [C.POINTER(MMArgs)]),
     "glq_mm_counters": (C.c_size_t, [C.POINTER(MMArgs)]),

@@ -10,7 +10,7 @@ shared expert) layouts.
 
 The quantized projections and the MoE block run on this package's kernels, and so does the attention
 of a decode step (``glq_attn_decode``: q/k norms, rotary embedding, cache write and attention over the
-live positions in one launch) and the fp16 ``lm_head`` product of up to 64 rows (``glq_lm_head``: a streaming
+live positions in one launch) and the fp16 ``lm_head`` product of up to 64 rows (``glq_lm_head_rows``: a streaming
 kernel over the row-major vocabulary matrix with the greedy arg-max folded in).  A prompt written at positions
 0..T-1 runs its norms, rotary embedding and cache write in ``glq_rope_prefill`` and its causal attention in
 ``glq_attn_prefill`` (head sizes 64 and 128; prompts of 2048 tokens and more, where the library's kernel is
@@ -309,8 +309,8 @@ class GLoRCQDecoder(nn.Module):
         return self._rope
 
     def _lm_head(self, x):
-        """(rows, H) fp16 -> (rows, V) logits; up to 64 rows go through this package's streaming kernel (8 rows
-        per pass of the weights) with the greedy arg-max of every row folded in (kept in ``last_argmax``),
+        """(rows, H) fp16 -> (rows, V) logits; up to 64 rows go through this package's streaming kernel (up to
+        32 rows per pass of the weights) with the greedy arg-max of every row folded in (kept in ``last_argmax``),
         longer inputs (the logits of a whole prompt) through a dense library product."""
         rows, H = x.shape
         V = self.lm_head.shape[0]
@@ -327,12 +327,10 @@ class GLoRCQDecoder(nn.Module):
                 self._lm_ws[key] = (torch.empty(L.glq_lm_head_workspace_bytes() + 16, dtype=torch.uint8, device=x.device),
                                     torch.zeros(1, dtype=torch.int32, device=x.device))
             ws, ctr = self._lm_ws[key]
-            for r0 in range(0, rows, 8):
-                nb = min(8, rows - r0)
-                _lib.check(L.glq_lm_head(x[r0:].data_ptr(), x.stride(0), self.lm_head.data_ptr(), nb, V, H,
-                                         logits[r0:].data_ptr(), V, best[r0:].data_ptr(),
-                                         (ws.data_ptr() + 15) // 16 * 16, ws.numel() - 16, ctr.data_ptr(),
-                                         tiled._stream_ptr(x.device)), "lm_head")
+            _lib.check(L.glq_lm_head_rows(x.data_ptr(), x.stride(0), self.lm_head.data_ptr(), rows, V, H,
+                                          logits.data_ptr(), V, best.data_ptr(),
+                                          (ws.data_ptr() + 15) // 16 * 16, ws.numel() - 16, ctr.data_ptr(),
+                                          tiled._stream_ptr(x.device)), "lm_head")
         self.last_argmax = best
         return logits
 

@@ -408,6 +408,9 @@ int glq_add_rmsnorm(const void* x, const void* delta, const void* weight, float 
 size_t glq_lm_head_workspace_bytes(void);
 int glq_lm_head(const void* x, int64_t ldx, const void* W, int B, int V, int H, void* logits, int64_t ldl,
                 int64_t* argmax_out, void* workspace, size_t workspace_bytes, int32_t* counter, void* stream);
+/* the same for any number of rows: up to 32 per pass over W, as many as fit in shared memory beside each other */
+int glq_lm_head_rows(const void* x, int64_t ldx, const void* W, int B, int V, int H, void* logits, int64_t ldl,
+                     int64_t* argmax_out, void* workspace, size_t workspace_bytes, int32_t* counter, void* stream);
 
 #ifdef __cplusplus
 }

@@ -254,6 +254,25 @@ def test_lm_head_logits_and_argmax(dev, B, V, H):
     assert L.glq_lm_head(x.data_ptr(), H, W.data_ptr(), 9, V, H, logits2.data_ptr(), V, None, None, 0, None, st) == -3
 
 
+
+@pytest.mark.parametrize("B,V,H", [(1, 40, 32), (9, 1000, 96), (16, 32000, 4096), (17, 5000, 8192), (33, 2500, 1056), (64, 9000, 2048)])
+def test_lm_head_many_rows(dev, B, V, H):
+    """Up to 32 rows per pass, as many as fit beside each other; chunks of H that fill no whole group, ragged last tiles."""
+    from glorcq_b200 import _lib
+    L = _lib.lib()
+    g = torch.Generator().manual_seed(B + V + H)
+    W = (torch.randn(V, H, generator=g) * 0.02).half().to(dev)
+    x = torch.randn(B, H, generator=g).half().to(dev)
+    ws = torch.empty(L.glq_lm_head_workspace_bytes(), dtype=torch.uint8, device=dev)
+    ctr = torch.zeros(1, dtype=torch.int32, device=dev)
+    logits = torch.full((B, V), float("nan"), dtype=torch.float16, device=dev)
+    best = torch.full((B,), -1, dtype=torch.int64, device=dev)
+    _lib.check(L.glq_lm_head_rows(x.data_ptr(), H, W.data_ptr(), B, V, H, logits.data_ptr(), V, best.data_ptr(), ws.data_ptr(),
+                                  ws.numel(), ctr.data_ptr(), torch.cuda.current_stream().cuda_stream), "lm_head")
+    assert int(ctr) == 0
+    assert cases.rel_l2(logits.cpu(), (x.float() @ W.float().t()).cpu()) <= 1e-3
+    assert torch.equal(best, torch.argmax(logits, dim=-1))
+
 QWEN15_SHAPE = dict(hidden_size=2048, num_hidden_layers=2, num_attention_heads=16, num_key_value_heads=16,
                     vocab_size=151936, num_experts=60, num_experts_per_tok=4, moe_intermediate_size=1408,
                     shared_expert_intermediate_size=5632, norm_topk_prob=False, rms_norm_eps=1e-6,
