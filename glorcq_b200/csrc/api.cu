@@ -451,6 +451,15 @@ static int launch_stream(const glq_mm_args_t* a, SkinnyParams& p, const StreamGe
 // ---------------------------------------------------------------------------------------------
 // glq_grouped_matmul
 // ---------------------------------------------------------------------------------------------
+// <<<>>> with programmatic stream serialization when `dependent`
+template <typename Kern, typename Params>
+static int launch_maybe_dependent(bool dependent, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Params& p) {
+    if (dependent) return launch_dependent(kern, grid, block, smem, st, p);
+    kern<<<grid, block, smem, st>>>(p);
+    GLQ_CUDA(cudaGetLastError());
+    return GLQ_OK;
+}
+
 template <typename Kern>
 static int allow_smem(Kern kern, bool (&configured)[64], size_t smem) {
     int dev = 0;
@@ -561,12 +570,11 @@ static int launch_tc_ps_t(TcParams& p, cudaStream_t st) {
     const int rc = allow_smem(tc_ps_kernel<FMT, TN, NM, SW>, configured, C::SMEM);
     if (rc != GLQ_OK) return rc;
     p.n_ft = cdiv(p.N, kTcFeat * C::NOUT);
-    tc_pack_b_kernel<TN><<<dim3(p.tiles_max, p.nkb + p.ns), 256, 0, st>>>(p);
-    GLQ_CUDA(cudaGetLastError());
+    const int rp = launch_maybe_dependent(p.a_late != 0, tc_pack_b_kernel<TN>, dim3(p.tiles_max, p.nkb + p.ns), dim3(256), 0, st, p);
+    if (rp != GLQ_OK) return rp;
     const long work = (long)p.n_ft * p.tiles_max;
-    tc_ps_kernel<FMT, TN, NM, SW><<<(int)std::min<long>(work, num_sms()), kPsThreads, C::SMEM, st>>>(p);
-    GLQ_CUDA(cudaGetLastError());
-    return GLQ_OK;
+    return launch_maybe_dependent(!pdl_disabled(), tc_ps_kernel<FMT, TN, NM, SW>, dim3((int)std::min<long>(work, num_sms())),
+                                  dim3(kPsThreads), C::SMEM, st, p);
 }
 template <int FMT>
 static int launch_tc_ps(TcParams& p, const TcGeom& g, bool sw, cudaStream_t st) {
@@ -633,7 +641,10 @@ static int launch_xu(const glq_mm_args_t* a, cudaStream_t st) {
     return tiles * cdiv(a->N, kXuCols) > 3 * num_sms() ? launch_xu_t<8>(p, a, st) : launch_xu_t<4>(p, a, st);
 }
 
-static int launch_tc(const glq_mm_args_t* a, const TcGeom& g, cudaStream_t st, int min_rows = 0) {
+// output of the x.U product that this thread launched last, if xu_kernel took it and no other product has come since
+static thread_local const void* t_xu_out = nullptr;
+
+static int launch_tc(const glq_mm_args_t* a, const TcGeom& g, cudaStream_t st, const void* xu_out, int min_rows = 0) {
     if (!a->workspace || a->workspace_bytes < g.xp_bytes) return GLQ_ERR_WORKSPACE;
     if ((reinterpret_cast<uintptr_t>(a->workspace) & 127u) != 0) return GLQ_ERR_ALIGN;
     TcParams p{};
@@ -647,6 +658,11 @@ static int launch_tc(const glq_mm_args_t* a, const TcGeom& g, cudaStream_t st, i
     p.min_rows = min_rows;
     const bool sw = a->epilogue == GLQ_EPI_SWIGLU;
     p.n_ft = cdiv(a->N, kTcFeat);
+    // The pre-pass may run beside x.U only when that is xu_kernel: it uses no workspace, and the caller's workspace is often the
+    // same memory for both products.
+    p.a_late = (a->flags & GLQ_MM_A_FROM_PREVIOUS_LAUNCH) != 0 && xu_out != nullptr && xu_out == a->a0 && p.ns > 0 && min_rows == 0 &&
+                       a->fmt != GLQ_FMT_F16 && !pdl_disabled()
+                   ? 1 : 0;
     if (a->fmt == GLQ_FMT_F16) return g.tn == 128 ? launch_tc_t<128>(p, st) : launch_tc_t<64>(p, st);
     p.ts = 1;
     p.tile_ctr = reinterpret_cast<int*>(p.xp + (g.xp_bytes - 256));
@@ -690,13 +706,18 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
     if (a->rank > 0 && (a->a0 || a->a1) && (a->lda % 8 != 0 || !aligned16(a->a0) || !aligned16(a->a1)))
         return GLQ_ERR_ALIGN;
     t_share_sm = (a->flags & GLQ_MM_SHARE_SM) != 0;
-    if (xu_takes(a))
-        return launch_xu(a, reinterpret_cast<cudaStream_t>(stream));
+    const void* const xu_out = t_xu_out;
+    t_xu_out = nullptr;
+    if (xu_takes(a)) {
+        const int r = launch_xu(a, reinterpret_cast<cudaStream_t>(stream));
+        if (r == GLQ_OK) t_xu_out = a->y;
+        return r;
+    }
     TcGeom tg;
     const bool use_tc = plan_tc(a, &tg);
     if (use_tc && !tg.hybrid) {
         if (!a->w_table && !a->w.codes) return GLQ_ERR_ARG;
-        return launch_tc(a, tg, reinterpret_cast<cudaStream_t>(stream));
+        return launch_tc(a, tg, reinterpret_cast<cudaStream_t>(stream), xu_out);
     }
     StreamGeom sg;
     // Row-count classes (device-side counts): slots with <= 8 rows go to the integer path, 9..16 to the
@@ -711,7 +732,7 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
     int cap = use_tc ? 16 : std::min(a->max_rows, 32);
     bool chunked = false;
     if (!use_tc && !a->slot_count && !a->slot_offset && !a->slot_index && a->max_rows > 8 && a->max_rows <= 32 && !i8_disabled() &&
-        (a->fmt == GLQ_FMT_Q2 || a->fmt == GLQ_FMT_Q4))
+        a->fmt != GLQ_FMT_F16)
         for (int c : {8, 4})
             if (!chunked && plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, c, &sg, cdiv(a->max_rows, c)) &&
                 sg.i8) {
@@ -726,7 +747,7 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
                          plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, 16, &sg16);
     if (use_tc && !use_stream) {
         if (!a->w_table && !a->w.codes) return GLQ_ERR_ARG;
-        return launch_tc(a, tg, reinterpret_cast<cudaStream_t>(stream));
+        return launch_tc(a, tg, reinterpret_cast<cudaStream_t>(stream), nullptr);
     }
     Geometry g{};
     int rc = use_stream ? GLQ_OK
@@ -783,7 +804,7 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
         if (split8 && (rc = one(sg8, 8, 8)) != GLQ_OK) return rc;
         if (split16 && (rc = one(sg16, 16, 16)) != GLQ_OK) return rc;
         if ((rc = one(sg, cap, cap)) != GLQ_OK) return rc;
-        if (use_tc) return launch_tc(a, tg, st, cap);
+        if (use_tc) return launch_tc(a, tg, st, nullptr, cap);
         return GLQ_OK;
     }
     fill_geometry(p, g);

@@ -54,6 +54,7 @@ struct TcParams {
     int N, n_ft;              // output features of every problem; 128-feature tiles (persistent kernel)
     int y_vec;                // y rows allow 16-byte bulk stores
     int x_vec16;              // x rows allow 16-byte loads
+    int a_late;               // 1: a[] is written by the launch before this one, nothing else the call reads is
     int* tile_ctr;            // work-item counter of the persistent kernel (in the workspace, zeroed by the pre-pass)
 };
 
@@ -106,6 +107,10 @@ __host__ __device__ __forceinline__ int tc_ts_channel_of(int fmt, int P) {
 // position c ^ (r & 7) (the 128-byte swizzle).  grid = (tiles_max, nkb + ns), 256 threads.
 template <int TN>
 __global__ void __launch_bounds__(256) tc_pack_b_kernel(const TcParams p) {
+    // Programmatic dependent launch: only the low-rank blocks read what the launch before this one writes (x.U); the blocks that
+    // re-tile x run beside it.  They wait for it, so this grid ends after that one has.
+    if ((int)blockIdx.y >= p.nkb || !p.a_late) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (p.tile_ctr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *p.tile_ctr = 0;
     int slot, lt, cnt, e0;
     if (!tc_find_tile<TN>(p, blockIdx.x, slot, lt, cnt, e0)) return;

@@ -583,6 +583,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
             for (bool first = n == 0; room; first = false) {
                 int w = blockIdx.x;
                 if (!first) {
+                    if (n == 0) asm volatile("griddepcontrol.wait;" ::: "memory");     // (a padding tile came first)
                     if (lane == 0) w = atomicAdd(p.tile_ctr, 1) + gridDim.x;
                     w = __shfl_sync(0xffffffffu, w, 0);
                 }
@@ -609,7 +610,11 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
             __syncwarp();
             return gt;
         };
+        // launched beside the pre-pass: its tiles and the zeroed counter are needed from here on (the other warps' first codes
+        // and addresses are not its work)
         int gt = publish(0), nxt = -1;
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
         for (int n = 0; gt >= 0; ++n, gt = nxt) {
             nxt = publish(n + 1);
             if (lane == 0) {

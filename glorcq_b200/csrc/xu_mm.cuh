@@ -3,11 +3,13 @@
 //
 // What bounds it: one pass over the rows of x (and over W, which stays in L2).  The tcgen05 kernel (tc_mm.cuh) gives a
 // product with 64 columns ONE 128-feature tile per 128 rows -- three CTAs for 333 rows -- whose producers set the pace
-// (0.9 us per 128 channels), after a pre-pass that re-tiles x: 35.6 + 5.3 us for 333 x 4096 x 64, here 22.4; 21.6 + 6 and 13.7 in a 512-token prompt.
+// (0.9 us per 128 channels), after a pre-pass that re-tiles x: 35.6 + 5.3 us for 333 x 4096 x 64, here 17.0;
+// 21.6 + 6 and 12.6 in a 512-token prompt.  Stages of 64 channels paid the wait, the barrier and the first fragments' latency
+// twice as often: 22.4 us, and 75 against 59 for the 65536 rows of a 4096-token prompt's h.U.
 //   * a CTA owns 16 NT / 2 rows x 64 columns: four warps, each 16 columns (the M side, one operand fragment of W per step) against
 //     NT tiles of 8 rows; a problem with few live rows skips whole operand tiles;
 //   * x (rows gathered through entry_row, 128-byte swizzle) and the fragments of W, which are tiled in operand order, arrive by
-//     cp.async in stages of 64 channels;
+//     cp.async in stages of 128 channels;
 //   * K is walked in ascending steps of 16 into one fp32 accumulator, no splits.  That is the order of the tcgen05 kernel, and
 //     m16n8k16 and tcgen05.mma round alike (no output of 1.4 million differed), so the kernels agree bit for bit and
 //     a prompt's results do not depend on which one took a product.  The chain of 128 steps for 2048 channels takes
@@ -19,10 +21,10 @@
 namespace glq {
 
 constexpr int kXuCols = 64, kXuThreads = 128;
-constexpr int kXuW = 4 * 4 * 512;                             // bytes of a stage's W fragments: 4 column tiles x 4 steps
+constexpr int kXuW = 4 * 8 * 512;                             // bytes of a stage's W fragments: 4 column tiles x 8 steps
 template <int NT> struct XuCfg {
     // stages: about 100 KB, two CTAs per SM -- a copy takes a microsecond to arrive, a stage's products an eighth of that
-    static constexpr int ROWS = 8 * NT, X = ROWS * 128, STAGE = X + kXuW, S = NT == 4 ? 8 : 6;
+    static constexpr int ROWS = 8 * NT, X = ROWS * 256, STAGE = X + kXuW, S = NT == 4 ? 4 : 3;
     static constexpr size_t SMEM = (size_t)S * STAGE;
 };
 
@@ -60,22 +62,28 @@ __global__ void __launch_bounds__(kXuThreads) xu_kernel(const TcParams p) {
     }
     const unsigned char* wsrc = reinterpret_cast<const unsigned char*>(W->codes);
     const uint32_t base = smem_u32(smem);
-    auto issue = [&](int s, int kb) {
-        if (kb < nkb) {
-            const uint32_t st = base + (uint32_t)(s * C::STAGE);
-            const int k = kb * 64;
-            const bool in = k + (tid & 7) * 8 < p.K;
+    // stage of k blocks 2 st, 2 st + 1: two x tiles [ROWS][128 B], then per column tile the fragments of eight steps
+    const int nst = (nkb + 1) / 2;
+    auto issue = [&](int slot, int stg) {
+        if (stg < nst) {
+            const uint32_t dst = base + (uint32_t)(slot * C::STAGE);
 #pragma unroll
-            for (int i = 0; i < NT / 2; ++i) {
-                const int r = (tid >> 3) + 16 * i;
-                const bool ok = in && src[i] != nullptr;
-                cp_async16_zfill(st + (uint32_t)(r * 128 + (((tid & 7) ^ (r & 7)) << 4)), ok ? src[i] + k : p.x, ok ? 16 : 0);
-            }
+            for (int u = 0; u < 2; ++u) {
+                const int kb = 2 * stg + u, k = kb * 64;
+                const bool in = k + (tid & 7) * 8 < p.K;
 #pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const int tile = blockIdx.y * 4 + m;
-                const bool ok = tile < n_mt;
-                cp_async16_zfill(st + C::X + (uint32_t)(m * 2048 + tid * 16), wsrc + ((size_t)(ok ? tile : 0) * nkb + kb) * 2048 + tid * 16, ok ? 16 : 0);
+                for (int i = 0; i < NT / 2; ++i) {
+                    const int r = (tid >> 3) + 16 * i;
+                    const bool ok = in && src[i] != nullptr;
+                    cp_async16_zfill(dst + (uint32_t)(u * (C::X / 2) + r * 128 + (((tid & 7) ^ (r & 7)) << 4)), ok ? src[i] + k : p.x, ok ? 16 : 0);
+                }
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const int tile = blockIdx.y * 4 + m;
+                    const bool ok = tile < n_mt && kb < nkb;
+                    cp_async16_zfill(dst + C::X + (uint32_t)(m * 4096 + u * 2048 + tid * 16),
+                                     wsrc + ((size_t)(ok ? tile : 0) * nkb + (ok ? kb : 0)) * 2048 + tid * 16, ok ? 16 : 0);
+                }
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -86,26 +94,35 @@ __global__ void __launch_bounds__(kXuThreads) xu_kernel(const TcParams p) {
 #pragma unroll
         for (int q = 0; q < 4; ++q) acc[n][q] = 0.f;
 #pragma unroll
-    for (int s = 0; s < C::S - 1; ++s) issue(s, s);
+    for (int i = 0; i < C::S - 1; ++i) issue(i, i);
     int s = 0;
-    for (int kb = 0; kb < nkb; ++kb) {
+    uint4 a[2][2];
+    uint32_t b[2][NT][4];
+    for (int stg = 0; stg < nst; ++stg) {
         asm volatile("cp.async.wait_group %0;" ::"n"(C::S - 2) : "memory");
         __syncthreads();
-        issue(s == 0 ? C::S - 1 : s - 1, kb + C::S - 1);
-        const uint32_t st = base + (uint32_t)(s * C::STAGE), wst = st + C::X + (uint32_t)(w * 2048 + lane * 16);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint4 a0 = lds128(wst + h * 1024), a1 = lds128(wst + h * 1024 + 512);
-            uint32_t b[NT][4];
+        const uint32_t st = base + (uint32_t)(s * C::STAGE), wst = st + C::X + (uint32_t)(w * 4096 + lane * 16);
+        auto frags = [&](int h, uint4 (&fa)[2], uint32_t (&fb)[NT][4]) {       // two steps: quarter h of the stage
+            fa[0] = lds128(wst + h * 1024);
+            fa[1] = lds128(wst + h * 1024 + 512);
 #pragma unroll
             for (int n = 0; n < NT; ++n)
-                if (n < nt_live) ldsm_x4(st + (uint32_t)((n * 8 + (lane & 7)) * 128 + (((4 * h + (lane >> 3)) ^ (lane & 7)) << 4)), b[n]);
+                if (n < nt_live)
+                    ldsm_x4(st + (uint32_t)((h >> 1) * (C::X / 2) + (n * 8 + (lane & 7)) * 128 + (((4 * (h & 1) + (lane >> 3)) ^ (lane & 7)) << 4)), fb[n]);
+        };
+        frags(0, a[0], b[0]);
+        issue(s == 0 ? C::S - 1 : s - 1, stg + C::S - 1);
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            if (h < 3) frags(h + 1, a[(h + 1) & 1], b[(h + 1) & 1]);
+            const uint4(&fa)[2] = a[h & 1];
+            const uint32_t(&fb)[NT][4] = b[h & 1];
 #pragma unroll
             for (int n = 0; n < NT; ++n)
-                if (n < nt_live) mma16816(acc[n], a0.x, a0.y, a0.z, a0.w, b[n][0], b[n][1]);
+                if (n < nt_live) mma16816(acc[n], fa[0].x, fa[0].y, fa[0].z, fa[0].w, fb[n][0], fb[n][1]);
 #pragma unroll
             for (int n = 0; n < NT; ++n)
-                if (n < nt_live) mma16816(acc[n], a1.x, a1.y, a1.z, a1.w, b[n][2], b[n][3]);
+                if (n < nt_live) mma16816(acc[n], fa[1].x, fa[1].y, fa[1].z, fa[1].w, fb[n][2], fb[n][3]);
         }
         s = s + 1 == C::S ? 0 : s + 1;
     }
