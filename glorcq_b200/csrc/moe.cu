@@ -31,10 +31,6 @@ inline bool share_sm() {
     static const bool v = std::getenv("GLQ_NO_SHARE_SM") == nullptr;
     return v;
 }
-inline bool no_dependent_launch() {
-    static const bool v = std::getenv("GLQ_NO_PDL") != nullptr;
-    return v;
-}
 
 // ---- workspace carve-up ---------------------------------------------------------------------------
 struct MoeLayout {

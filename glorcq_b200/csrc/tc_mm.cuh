@@ -52,7 +52,7 @@ struct TcParams {
     int min_rows;             // only problems with more rows than this are this launch's
     int ts;                   // 1: K positions of a stage in the order of the tensor-memory kernel, 0: F16 fragment order
     int N, n_ft;              // output features of every problem; 128-feature tiles (persistent kernel)
-    int y_vec;                // y rows allow 16-byte bulk stores
+    int y_vec;                // y rows allow 16-byte stores
     int x_vec16;              // x rows allow 16-byte loads
     int a_late;               // 1: a[] is written by the launch before this one, nothing else the call reads is
     int* tile_ctr;            // work-item counter of the persistent kernel (in the workspace, zeroed by the pre-pass)

@@ -25,14 +25,17 @@
 //    they turn to the finished accumulator.
 //  * A finished accumulator is read into registers (epilogue arithmetic, fp16 pairs) and released at once;
 //    the results go to y after the weight ring of the next item is full again, through a staging tile in
-//    shared memory ([token][feature], two passes) with 16-byte row-contiguous stores.
+//    shared memory ([token][feature], two passes) with 16-byte row-contiguous stores.  With one accumulator the tensor
+//    pipe waits for this: 128 experts x 256 rows, 2048 x 768, took 228 us with a bulk copy per row and the output scales read
+//    by every lane, and 161 with plain stores and the scales requested before the wait.
 //
 // What bounds it: with few tokens per problem (an expert of a prompt sees some tens of rows) the producers' issue
 // slots.  A first form spent 253 instructions per warp, matrix and stage (one shift per pair of codes, both
 // roundings of the dequantisation computed and one selected, every warp looking up its item): 142 us for the gate|up
 // product of 60 experts x 34 rows (1408 x 2048, 2-bit), scheduler slots 57 % used, DRAM 12 %.  Now 140 instructions
-// and 99 us; 97 -> 60 us for the down product (2048 x 1408).  The half-precision and the integer pipes (one warp
-// instruction every two cycles each) are 60 % busy; the unpack alone, without the loop around it, would take 55 us.
+// and 99 us; 97 -> 60 us for the down product (2048 x 1408).  With one multiply-add per pair of 2-bit codes and one election
+// per four MMAs 95 and 54 us.  No pipe is full (integer 45 %, issue slots 49 %, tensor 40 %): what is left is the latency
+// of a warp's own chain through a stage, of which four warps per scheduler cover only a part.
 //
 // Every wait is bounded (tc_wait); a wait that runs out marks the CTA dead, all roles leave their loops
 // and the kernel ends.
@@ -57,13 +60,22 @@ __device__ __forceinline__ void tc_st_x2(uint32_t taddr, const uint32_t (&r)[8])
                  : "memory");
 }
 __device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// D (TMEM) += A (TMEM, 128 lanes x 8 columns = 16 fp16 per row) * B (shared memory descriptor).  The whole warp comes here
-// with the same operands and one elected lane issues: in code that one lane runs alone the operands of every instruction go
-// through R2UR, and the issuing warp, not the tensor pipe, set the pace (113 to 117 cycles per MMA of any N up to 128).
-__device__ __forceinline__ void tc_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
+// D (TMEM) += A (TMEM, 128 lanes x 8 columns = 16 fp16 per row) * B (shared memory descriptor), a run of four k steps: A
+// advances by 8 columns, B by 32 bytes.  The whole warp comes here with the same operands and one elected lane issues: in code
+// that one lane runs alone the operands of every instruction go through R2UR, and the issuing warp, not the tensor pipe,
+// set the pace (113 to 117 cycles per MMA of any N up to 128).  One election serves the four (one for each still left 70
+// to 90 cycles between MMAs of 64 columns, which the tensor pipe does in 32).
+__device__ __forceinline__ void tc_mma4_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
     asm volatile(
-        "{\n .reg .pred p, e;\n setp.ne.b32 p, %4, 0;\n elect.sync _|e, 0xffffffff;\n"
-        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+        "{\n .reg .pred p, o, e;\n .reg .b32 a1, a2, a3;\n .reg .b64 b1, b2, b3;\n"
+        " setp.ne.b32 p, %4, 0;\n setp.eq.b32 o, 0, 0;\n"
+        " add.u32 a1, %1, 8;\n add.u32 a2, %1, 16;\n add.u32 a3, %1, 24;\n"
+        " add.u64 b1, %2, 2;\n add.u64 b2, %2, 4;\n add.u64 b3, %2, 6;\n"
+        " elect.sync _|e, 0xffffffff;\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, o;\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, o;\n"
+        " @e tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, o;\n}\n" ::"r"(d_tmem),
         "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(acc)
         : "memory");
 }
@@ -134,6 +146,34 @@ template <> struct PsUnpack<GLQ_FMT_Q4> {
 };
 template <> struct PsUnpack<GLQ_FMT_T2> { static constexpr int WORDS = 1; };
 
+// 2-bit codes, the usual case: a field masked out of its word, with nothing or-ed in, IS an fp16 number, the subnormal
+// q 2^-18 (bits 6, 7) or q 2^-16 (bits 8, 9).  With s 2^18 / s 2^16 as the factor and -z s as the addend, one multiply-add
+// yields fp16((q - z) s): the product is exact, and so is z s for z = 0, 1, 2 (z = 3: the codes are inverted, 3 - q, and the
+// factor's sign with them), so that the one rounding is that of the reference's product.  Two instructions per pair and two
+// of the half-precision pipe's slots fewer.  |s| < 1/4 keeps the factors finite.
+struct PsQ2 {
+    uint32_t f6, f8, c, flip;         // (row g, row g + 8): s 2^18, s 2^16, -z s; inversion mask
+    bool fast;                        // the whole warp's rows allow this
+};
+__device__ __forceinline__ PsQ2 ps_q2_setup(const uint32_t (&sz)[2]) {
+    auto h2 = [](uint32_t v) { return *reinterpret_cast<const __half2*>(&v); };
+    auto u = [](__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); };
+    PsQ2 r;
+    const uint32_t zb = __byte_perm(sz[0], sz[1], 0x7632), sb = __byte_perm(sz[0], sz[1], 0x5410);
+    r.flip = __heq2_mask(h2(zb), __float2half2_rn(3.f));
+    const __half2 z = h2(zb & ~r.flip), big = __float2half2_rn(1024.f);
+    // z one of 0, 1, 2: 1024 + z keeps it, and it lies in the range
+    const bool ok = __hbeq2(__hsub2(__hadd2(z, big), big), z) && __hbeq2(__hmax2(__hmin2(z, __float2half2_rn(2.f)), __float2half2_rn(0.f)), z) &&
+                    __hblt2(__habs2(h2(sb)), __float2half2_rn(0.25f));
+    r.fast = __all_sync(0xffffffffu, ok);
+    const __half2 s = h2(sb ^ (r.flip & 0x80008000u));
+    const __half2 f8 = __hmul2(__hmul2(s, __float2half2_rn(256.f)), __float2half2_rn(256.f));
+    r.f8 = u(f8);
+    r.f6 = u(__hmul2(f8, __float2half2_rn(4.f)));
+    r.c = u(__hneg2(__hmul2(z, h2(sb))));
+    return r;
+}
+
 // Both rows (g, g + 8) of a lane: words w[row][..], (scale, zero) pairs sz[row] -> the 16 registers of tc_st_x4.
 template <int FMT>
 __device__ __forceinline__ void ps_affine(const uint32_t (&w)[2][PsUnpack<FMT>::WORDS], const uint32_t (&sz)[2], int sh, uint32_t (&r)[16]) {
@@ -168,6 +208,27 @@ __device__ __forceinline__ void ps_affine(const uint32_t (&w)[2][PsUnpack<FMT>::
                 const __half2 v = __hmul2(__hsub2(q, zr), s2);
                 r[4 * (j >> 1) + 2 * hrow + (j & 1)] = *reinterpret_cast<const uint32_t*>(&v);
             }
+        }
+    }
+}
+
+__device__ __forceinline__ void ps_q2_fast(const uint32_t (&w)[2][1], const PsQ2& q, uint32_t (&r)[16]) {
+#pragma unroll
+    for (int hrow = 0; hrow < 2; ++hrow) {
+        auto sel = [&](uint32_t v) {
+            const __half2 h = *reinterpret_cast<const __half2*>(&v);
+            return hrow ? __high2half2(h) : __low2half2(h);
+        };
+        const __half2 f6 = sel(q.f6), f8 = sel(q.f8), c = sel(q.c);
+        const uint32_t v = w[hrow][0] ^ __byte_perm(q.flip, 0, hrow ? 0x3232 : 0x1010);
+        // fields 0..7 of either half of the word, moved to bits 6 or 8
+        const uint32_t h[8] = {(v << 6) & 0x00C000C0u, (v << 6) & 0x03000300u, (v << 4) & 0x03000300u, v & 0x00C000C0u,
+                               v & 0x03000300u, (v >> 4) & 0x00C000C0u, (v >> 4) & 0x03000300u, (v >> 6) & 0x03000300u};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const bool low = j == 0 || j == 3 || j == 5;
+            const __half2 y = __hfma2(*reinterpret_cast<const __half2*>(&h[j]), low ? f6 : f8, c);
+            r[4 * (j >> 1) + 2 * hrow + (j & 1)] = *reinterpret_cast<const uint32_t*>(&y);
         }
     }
 }
@@ -258,6 +319,14 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
         int pass = 0;
         auto results = [&](int n) -> bool {
             const volatile PsItem& im = s_item[n % kPsQueue];
+            // the tokens' output scales, lane j that of token j, all requested before the wait
+            const bool scaled = !SW && p.entry_scale;
+            __half sc_h[TN / kPsRows];
+#pragma unroll
+            for (int i = 0; i < TN / kPsRows; ++i) {
+                const int r = im.lt * TN + i * kPsRows + part * 16 + (lane & 15);
+                sc_h[i] = scaled && r < im.cnt ? __ldg(p.entry_scale + im.e0 + r) : __float2half(0.f);
+            }
             bool ok = ps_wait_warp(bar_acc, (uint32_t)(n & 1), dead, 101);
             tc_fence_after();
 #pragma unroll
@@ -282,7 +351,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
                 tc_ld_wait();
                 const uint32_t dst = orow + (uint32_t)(b * kPsOut);
                 const int r0 = im.lt * TN + c0 + part * 16, cnt = im.cnt;
-                const __half* scale = SW || !p.entry_scale ? nullptr : p.entry_scale + im.e0 + r0;
+                const float scv = __half2float(sc_h[h % (TN / kPsRows)]);
                 if (ok && r0 < cnt) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
@@ -294,13 +363,12 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
                             v = silu16(round16(v)) * round16(u);
                         } else {
                             if (bias) v = round16(v) + bv;
-                            if (scale && r0 + j < cnt) v = __half2float(__ldg(scale + j)) * round16(v);
+                            if (scaled) v = __shfl_sync(0xffffffffu, scv, j) * round16(v);
                         }
                         const unsigned short hv = __half_as_ushort(__float2half_rn(v));
                         asm volatile("st.shared.u16 [%0], %1;" ::"r"(dst + (uint32_t)j * 256u), "h"(hv) : "memory");
                     }
                 }
-                fence_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_staged + 8 * b);
                 ++pass;
@@ -377,8 +445,13 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(im.sv + ((((size_t)(d16 >> 1) * p.ns + sl) * 32) + (d16 & 1) * 16 + lane) * 128));
         };
         // the 16 registers of a half's store: for k step n of the half {row g: positions 4t..4t+3, row g+8: the same}
-        auto unpack = [&](const uint32_t (&qv)[2][WPR], const uint32_t (&zv)[2], uint32_t (&r)[16]) {
-            if constexpr (AFFINE) {
+        PsQ2 q2{};                                // of the stage in work (2-bit codes)
+        auto unpack = [&](const uint32_t (&qv)[2][WPR], const uint32_t (&zv)[2], uint32_t (&r)[16], bool first) {
+            if constexpr (FMT == GLQ_FMT_Q2) {
+                if (first) q2 = ps_q2_setup(zv);
+                if (q2.fast) ps_q2_fast(qv, q2, r);
+                else ps_affine<FMT>(qv, zv, 0, r);
+            } else if constexpr (AFFINE) {
                 ps_affine<FMT>(qv, zv, 8 * (t & 1), r);
             } else {
 #pragma unroll
@@ -438,7 +511,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
             // Software pipeline: a stage's first half is unpacked while the stores of the stage before are on their way to
             // tensor memory, and before its ring slot is free.
             uint32_t r[16];
-            unpack(cq[0][0], csz[0][0], r);
+            unpack(cq[0][0], csz[0][0], r, true);
             for (int st0 = 0;; st0 += D) {
                 if (pending && (st0 > 0 || nk == 0)) {
                     ok = results(it - 1) && ok;
@@ -456,11 +529,11 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
                             tc_st_x4(acol, r);
                             if constexpr (HALVES == 2) {
                                 uint32_t r2[16];
-                                unpack(cq[d][1], csz[d][NSZ - 1], r2);
+                                unpack(cq[d][1], csz[d][NSZ - 1], r2, false);
                                 tc_st_x4(acol + 32, r2);
                             }
                             fetch(cq[d], csz[d]);
-                            unpack(cq[(d + 1) % D][0], csz[(d + 1) % D][0], r);
+                            unpack(cq[(d + 1) % D][0], csz[(d + 1) % D][0], r, true);
                             tc_st_wait();
                         }
                         publish_stage();
@@ -508,18 +581,14 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
                 const uint64_t bd = bdesc0 + (uint32_t)(s * (C::B_BYTES / 16));
                 if (st < p.nkb) {
 #pragma unroll
-                    for (int kk = 0; kk < 8; ++kk) {
-                        const uint64_t b = bd + (uint32_t)((kk >> 2) * kAtom + (kk & 3) * 2);
-                        const uint32_t acc = kk == 0 ? (uint32_t)(st != 0) : 1u;
-                        tc_mma_f16_ts(tmem, acol + 8 * kk, b, idesc, acc);
-                        if (NM == 2) tc_mma_f16_ts(tmem + TN, acol + 64 + 8 * kk, b, idesc, acc);
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t acc = h == 0 ? (uint32_t)(st != 0) : 1u;
+                        tc_mma4_f16_ts(tmem, acol + 32 * h, bd + (uint32_t)(h * kAtom), idesc, acc);
+                        if (NM == 2) tc_mma4_f16_ts(tmem + TN, acol + 64 + 32 * h, bd + (uint32_t)(h * kAtom), idesc, acc);
                     }
                 } else {
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        tc_mma_f16_ts(tmem, acol + 8 * kk, bd + 2 * kk, idesc, 1);
-                        if (NM == 2) tc_mma_f16_ts(tmem + TN, acol + 64 + 8 * kk, bd + (SW ? kAtom : 0) + 2 * kk, idesc, 1);
-                    }
+                    tc_mma4_f16_ts(tmem, acol, bd, idesc, 1);
+                    if (NM == 2) tc_mma4_f16_ts(tmem + TN, acol + 64, bd + (SW ? kAtom : 0), idesc, 1);
                 }
                 tc_commit_warp(bar_empty + 8 * s);
                 if (++s == S) {
@@ -544,20 +613,23 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
                 if (!ok) break;
                 const uint32_t src = obase + (uint32_t)(b * kPsOut);
                 if (nf > 0) {
-                    for (int r = lane; r < rows; r += 32) {
-                        __half* dst = p.y + (size_t)(e0 + r0 + r) * p.ldy + f0;
-                        if (p.y_vec) {
-                            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src + (uint32_t)r * 256u), "r"(nf * 2) : "memory");
-                        } else {
+                    __half* y = p.y + (size_t)(e0 + r0) * p.ldy + f0;
+                    if (p.y_vec) {
+                        // 16 bytes per lane, two token rows per instruction.  (A bulk copy of 256 bytes per row kept the pass
+                        // 3600 cycles, 64 copies one after the other, and the tensor pipe idle behind it.)
+                        const int c = lane & 15;
+                        if (8 * c < nf)
+#pragma unroll 8
+                            for (int r = lane >> 4; r < rows; r += 2)
+                                *reinterpret_cast<uint4*>(y + (size_t)r * p.ldy + 8 * c) = lds128(src + (uint32_t)(r * 256 + c * 16));
+                    } else {
+                        for (int r = lane; r < rows; r += 32)
                             for (int i = 0; i < nf; ++i) {
                                 unsigned short hv;
                                 asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hv) : "r"(src + (uint32_t)r * 256u + (uint32_t)i * 2u) : "memory");
-                                dst[i] = __ushort_as_half(hv);
+                                y[(size_t)r * p.ldy + i] = __ushort_as_half(hv);
                             }
-                        }
                     }
-                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
                 }
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_stored + 8 * b);
@@ -565,7 +637,6 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
             release_item(it);
             if (!ok) break;
         }
-        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else {
         // ================= loader of the token operand =================
         int s = 0;
