@@ -40,164 +40,6 @@ __device__ __forceinline__ void rope_norm(float (&v)[EPL], const __half* __restr
     }
 }
 
-template <int EPL>
-__global__ void __launch_bounds__(kAttnWarps * 32) attn_decode_kernel(
-    const __half* __restrict__ q, const __half* __restrict__ k_new, const __half* __restrict__ v_new,
-    const __half* __restrict__ cos_t, const __half* __restrict__ sin_t, const long long* __restrict__ pos_p,
-    __half* __restrict__ k_cache, __half* __restrict__ v_cache, __half* __restrict__ out, int n_heads, int n_kv, int max_len,
-    const __half* __restrict__ q_norm_w, const __half* __restrict__ k_norm_w, float eps, float* __restrict__ partial,
-    int* __restrict__ arrivals) {
-    constexpr int HD = EPL * 32;
-    const int h = blockIdx.x, b = blockIdx.y, z = blockIdx.z, nsplit = gridDim.z;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int group = n_heads / n_kv, kvh = h / group;
-    long long pos = *pos_p;
-    if (pos < 0) pos = 0;
-    if (pos >= max_len) pos = max_len - 1;
-    float cs[EPL], sn[EPL];
-#pragma unroll
-    for (int i = 0; i < EPL; ++i) {
-        cs[i] = __half2float(cos_t[(size_t)pos * HD + lane * EPL + i]);
-        sn[i] = __half2float(sin_t[(size_t)pos * HD + lane * EPL + i]);
-    }
-
-    float qv[EPL], kn[EPL], vn[EPL];
-#pragma unroll
-    for (int i = 0; i < EPL; ++i) {
-        qv[i] = __half2float(q[((size_t)b * n_heads + h) * HD + lane * EPL + i]);
-        kn[i] = __half2float(k_new[((size_t)b * n_kv + kvh) * HD + lane * EPL + i]);
-        vn[i] = __half2float(v_new[((size_t)b * n_kv + kvh) * HD + lane * EPL + i]);
-    }
-    rope_norm<EPL>(qv, q_norm_w, eps, HD, cs, sn, lane);
-    rope_norm<EPL>(kn, k_norm_w, eps, HD, cs, sn, lane);
-    __half* kc = k_cache + ((size_t)b * n_kv + kvh) * max_len * HD;
-    __half* vc = v_cache + ((size_t)b * n_kv + kvh) * max_len * HD;
-    if (h % group == 0 && warp == 0 && z == 0) {     // one CTA per key/value head stores the new entry
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) {
-            kc[(size_t)pos * HD + lane * EPL + i] = __float2half_rn(kn[i]);
-            vc[(size_t)pos * HD + lane * EPL + i] = __float2half_rn(vn[i]);
-        }
-    }
-    const float scale = rsqrtf((float)HD);
-    // online softmax per warp over its share of positions 0..pos-1 (the new position is warp 0's, from
-    // registers: other CTAs of the group may not have stored it yet)
-    float m = -INFINITY, l = 0.f, o[EPL];
-#pragma unroll
-    for (int i = 0; i < EPL; ++i) o[i] = 0.f;
-    auto visit = [&](const float (&kk)[EPL], const float (&vv)[EPL]) {
-        float s = 0.f;
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) s += qv[i] * kk[i];
-        s = warp_sum(s) * scale;
-        const float mn = fmaxf(m, s);
-        const float a = __expf(m - mn), p = __expf(s - mn);
-        l = l * a + p;
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) o[i] = o[i] * a + p * vv[i];
-        m = mn;
-    };
-    // this CTA's share of the cached positions (the grid's z dimension splits them)
-    const long long per = (pos + nsplit - 1) / nsplit;
-    const long long t_lo = (long long)z * per, t_hi = t_lo + per < pos ? t_lo + per : pos;
-    // the rows of up to kAhead positions are requested before the first of them is used: the loop is a chain of
-    // dependent updates, and one cache round trip per position would set its pace
-    constexpr int kAhead = 8;
-    for (long long t0 = t_lo + warp; t0 < t_hi; t0 += (long long)kAttnWarps * kAhead) {
-        __half kr[kAhead][EPL], vr[kAhead][EPL];
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            const long long t = t0 + (long long)u * kAttnWarps;
-            if (t < t_hi) {
-                if constexpr (EPL == 4) {
-                    *reinterpret_cast<uint2*>(kr[u]) = *reinterpret_cast<const uint2*>(kc + (size_t)t * HD + lane * EPL);
-                    *reinterpret_cast<uint2*>(vr[u]) = *reinterpret_cast<const uint2*>(vc + (size_t)t * HD + lane * EPL);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < EPL; ++i) {
-                        kr[u][i] = kc[(size_t)t * HD + lane * EPL + i];
-                        vr[u][i] = vc[(size_t)t * HD + lane * EPL + i];
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            const long long t = t0 + (long long)u * kAttnWarps;
-            if (t < t_hi) {
-                float kk[EPL], vv[EPL];
-#pragma unroll
-                for (int i = 0; i < EPL; ++i) {
-                    kk[i] = __half2float(kr[u][i]);
-                    vv[i] = __half2float(vr[u][i]);
-                }
-                visit(kk, vv);
-            }
-        }
-    }
-    if (warp == 0 && z == 0) visit(kn, vn);
-    // combine the warps
-    __shared__ float sm_m[kAttnWarps], sm_l[kAttnWarps], sm_o[kAttnWarps][HD];
-    if (lane == 0) {
-        sm_m[warp] = m;
-        sm_l[warp] = l;
-    }
-#pragma unroll
-    for (int i = 0; i < EPL; ++i) sm_o[warp][lane * EPL + i] = o[i];
-    __syncthreads();
-    __shared__ int s_last;
-    if (warp == 0) {
-        float mm = -INFINITY;
-        for (int w = 0; w < kAttnWarps; ++w) mm = fmaxf(mm, sm_m[w]);
-        float ll = 0.f, oo[EPL];
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) oo[i] = 0.f;
-        for (int w = 0; w < kAttnWarps; ++w) {
-            const float a = sm_m[w] == -INFINITY ? 0.f : __expf(sm_m[w] - mm);
-            ll += sm_l[w] * a;
-#pragma unroll
-            for (int i = 0; i < EPL; ++i) oo[i] += sm_o[w][lane * EPL + i] * a;
-        }
-        if (nsplit == 1) {
-#pragma unroll
-            for (int i = 0; i < EPL; ++i) out[((size_t)b * n_heads + h) * HD + lane * EPL + i] = __float2half_rn(oo[i] / ll);
-            return;
-        }
-        // several CTAs per head: leave (max, sum, weighted values) of this share; the CTA that arrives last
-        // (counter per head, reset by it) merges the shares in a fixed order
-        float* mine = partial + (((size_t)b * n_heads + h) * nsplit + z) * (HD + 2);
-        if (lane == 0) {
-            mine[0] = mm;
-            mine[1] = ll;
-        }
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) mine[2 + lane * EPL + i] = oo[i];
-        __threadfence();
-        __syncwarp();
-        if (lane == 0) s_last = atomicAdd(arrivals + (size_t)b * n_heads + h, 1) == nsplit - 1;
-        __syncwarp();
-        if (!s_last) return;
-        __threadfence();
-        const float* all = partial + ((size_t)b * n_heads + h) * nsplit * (HD + 2);
-        float gm = -INFINITY;
-        for (int s2 = 0; s2 < nsplit; ++s2) gm = fmaxf(gm, __ldcg(all + (size_t)s2 * (HD + 2)));
-        float gl = 0.f, go[EPL];
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) go[i] = 0.f;
-        for (int s2 = 0; s2 < nsplit; ++s2) {
-            const float* pp = all + (size_t)s2 * (HD + 2);
-            const float pm = __ldcg(pp);
-            const float a = pm == -INFINITY ? 0.f : __expf(pm - gm);
-            gl += __ldcg(pp + 1) * a;
-#pragma unroll
-            for (int i = 0; i < EPL; ++i) go[i] += __ldcg(pp + 2 + lane * EPL + i) * a;
-        }
-#pragma unroll
-        for (int i = 0; i < EPL; ++i) out[((size_t)b * n_heads + h) * HD + lane * EPL + i] = __float2half_rn(go[i] / gl);
-        if (lane == 0) arrivals[(size_t)b * n_heads + h] = 0;
-    }
-}
-
 // EPL consecutive values of a row; vec: every row starts at an 8-byte boundary
 template <int EPL>
 __device__ __forceinline__ void load_row(const __half* p, bool vec, __half (&h)[EPL]) {
@@ -212,6 +54,243 @@ __device__ __forceinline__ void store_row(__half* p, bool vec, const __half (&h)
     else
 #pragma unroll
         for (int i = 0; i < EPL; ++i) p[i] = h[i];
+}
+
+// What bounds it: a warp's chain of positions (few heads), instruction issue (many).  One position at a time, every score
+// waited for five shuffles and every update for two exponentials.  Now eight positions make one step: their partial scores are
+// summed by a transposing butterfly (the same pairs of lanes in the same order, so the same bits), the running maximum is
+// a scan, each exponential is taken once per position instead of by every lane, only l and o are chains, and the rows of
+// the next step are requested before this one's are used.  G = 2 heads that share their keys and values read and convert
+// them once.  16 x 32 heads x 1024 positions, 8 key heads: 72 -> 40 us (46 with rows selected by 64-bit positions, 74 with one
+// head per CTA); 9 x 32 x 500: 25 -> 15; 16 heads x 512 in a decode step: 8.2 -> 7.5; 64 x 16 x 300 without sharing: 45 -> 42
+// (four CTAs per SM: with three, 46).  G = 4 leaves too few warps: 64 x 32 x 500 took 82 us, 75 with G = 2, 97 before.
+template <int EPL, int G>
+__global__ void __launch_bounds__(kAttnWarps * 32, EPL == 4 && G == 1 ? 4 : 1) attn_decode_kernel(
+    const __half* __restrict__ q, const __half* __restrict__ k_new, const __half* __restrict__ v_new,
+    const __half* __restrict__ cos_t, const __half* __restrict__ sin_t, const long long* __restrict__ pos_p,
+    __half* __restrict__ k_cache, __half* __restrict__ v_cache, __half* __restrict__ out, int n_heads, int n_kv, int max_len,
+    const __half* __restrict__ q_norm_w, const __half* __restrict__ k_norm_w, float eps, float* __restrict__ partial,
+    int* __restrict__ arrivals) {
+    constexpr int HD = EPL * 32;
+    const int h = blockIdx.x * G, b = blockIdx.y, z = blockIdx.z, nsplit = gridDim.z;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int group = n_heads / n_kv, kvh = h / group;
+    long long pos = *pos_p;
+    if (pos < 0) pos = 0;
+    if (pos >= max_len) pos = max_len - 1;
+    __half* kc = k_cache + ((size_t)b * n_kv + kvh) * max_len * HD;
+    __half* vc = v_cache + ((size_t)b * n_kv + kvh) * max_len * HD;
+    // this CTA's share of the cached positions (the grid's z dimension splits them), interleaved over its warps; a step is
+    // kAhead of a warp's positions, its keys and values at constant distances from one row
+    const int per = ((int)pos + nsplit - 1) / nsplit;
+    const int t_lo = z * per, t_hi = min(t_lo + per, (int)pos);
+    constexpr int kAhead = 8;
+    __half kr[kAhead][EPL], vr[kAhead][EPL];
+    auto live_from = [&](int t0) { return t0 < t_hi ? min(kAhead, (t_hi - t0 + kAttnWarps - 1) / kAttnWarps) : 0; };
+    // rows of the step at t0: n of them
+    auto request = [&](const __half* cache, int t0, int n, __half (&r)[kAhead][EPL]) {
+        const __half* row = cache + (size_t)t0 * HD + lane * EPL;
+        if (n == kAhead) {
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) load_row<EPL>(row + u * (kAttnWarps * HD), true, r[u]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (u < n) load_row<EPL>(row + u * (kAttnWarps * HD), true, r[u]);
+        }
+    };
+    int nv = live_from(t_lo + warp);
+    request(kc, t_lo + warp, nv, kr);
+    request(vc, t_lo + warp, nv, vr);
+    float cs[EPL], sn[EPL];
+#pragma unroll
+    for (int i = 0; i < EPL; ++i) {
+        cs[i] = __half2float(cos_t[(size_t)pos * HD + lane * EPL + i]);
+        sn[i] = __half2float(sin_t[(size_t)pos * HD + lane * EPL + i]);
+    }
+
+    float qv[G][EPL], kn[EPL], vn[EPL];
+#pragma unroll
+    for (int i = 0; i < EPL; ++i) {
+#pragma unroll
+        for (int j = 0; j < G; ++j) qv[j][i] = __half2float(q[((size_t)b * n_heads + h + j) * HD + lane * EPL + i]);
+        kn[i] = __half2float(k_new[((size_t)b * n_kv + kvh) * HD + lane * EPL + i]);
+        vn[i] = __half2float(v_new[((size_t)b * n_kv + kvh) * HD + lane * EPL + i]);
+    }
+#pragma unroll
+    for (int j = 0; j < G; ++j) rope_norm<EPL>(qv[j], q_norm_w, eps, HD, cs, sn, lane);
+    rope_norm<EPL>(kn, k_norm_w, eps, HD, cs, sn, lane);
+    if (h % group == 0 && warp == 0 && z == 0) {     // one CTA per key/value head stores the new entry
+#pragma unroll
+        for (int i = 0; i < EPL; ++i) {
+            kc[(size_t)pos * HD + lane * EPL + i] = __float2half_rn(kn[i]);
+            vc[(size_t)pos * HD + lane * EPL + i] = __float2half_rn(vn[i]);
+        }
+    }
+    const float scale = rsqrtf((float)HD);
+    // online softmax per warp over its share of positions 0..pos-1 (the new position is warp 0's, from
+    // registers: other CTAs of the group may not have stored it yet)
+    float m[G], l[G], o[G][EPL];
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+        m[j] = -INFINITY;
+        l[j] = 0.f;
+#pragma unroll
+        for (int i = 0; i < EPL; ++i) o[j][i] = 0.f;
+    }
+    const bool b16 = (lane & 16) != 0, b8 = (lane & 8) != 0, b4 = (lane & 4) != 0;
+    for (int t0 = t_lo + warp; nv > 0; t0 += kAttnWarps * kAhead) {
+        const int t1 = t0 + kAttnWarps * kAhead, nv1 = live_from(t1);      // the next step
+        float s[G][kAhead], ea[G], ep[G];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u)
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                s[j][u] = 0.f;
+#pragma unroll
+                for (int i = 0; i < EPL; ++i) s[j][u] += qv[j][i] * __half2float(kr[u][i]);
+            }
+        request(kc, t1, nv1, kr);
+#pragma unroll
+        for (int j = 0; j < G; ++j) {
+            // sums over the lanes, in warp_sum's order; lanes 4 u .. 4 u + 3 end up with position u
+            float r4[4], r2[2], v;
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+                r4[n] = (b16 ? s[j][n + 4] : s[j][n]) + __shfl_xor_sync(0xffffffffu, b16 ? s[j][n] : s[j][n + 4], 16);
+#pragma unroll
+            for (int n = 0; n < 2; ++n) r2[n] = (b8 ? r4[n + 2] : r4[n]) + __shfl_xor_sync(0xffffffffu, b8 ? r4[n] : r4[n + 2], 8);
+            v = (b4 ? r2[1] : r2[0]) + __shfl_xor_sync(0xffffffffu, b4 ? r2[0] : r2[1], 4);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v = (lane >> 2) < nv ? v * scale : -INFINITY;
+            // running maximum up to and including, and before, each position
+            float mi = fmaxf(m[j], v);
+#pragma unroll
+            for (int d = 4; d < 32; d <<= 1) {
+                const float o2 = __shfl_up_sync(0xffffffffu, mi, d);
+                if (lane >= d) mi = fmaxf(mi, o2);
+            }
+            float mp = __shfl_up_sync(0xffffffffu, mi, 4);
+            if (lane < 4) mp = m[j];
+            ea[j] = __expf(mp - mi);
+            ep[j] = __expf(v - mi);
+            m[j] = __shfl_sync(0xffffffffu, mi, 31);
+        }
+        auto take = [&](int u) {
+#pragma unroll
+            for (int j = 0; j < G; ++j) {
+                const float a = __shfl_sync(0xffffffffu, ea[j], 4 * u), p = __shfl_sync(0xffffffffu, ep[j], 4 * u);
+                l[j] = l[j] * a + p;
+#pragma unroll
+                for (int i = 0; i < EPL; ++i) o[j][i] = o[j][i] * a + p * __half2float(vr[u][i]);
+            }
+        };
+        if (nv == kAhead) {
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u) take(u);
+        } else {
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (u < nv) take(u);
+        }
+        request(vc, t1, nv1, vr);
+        nv = nv1;
+    }
+    if (warp == 0 && z == 0) {
+#pragma unroll
+        for (int j = 0; j < G; ++j) {
+            float s = 0.f;
+#pragma unroll
+            for (int i = 0; i < EPL; ++i) s += qv[j][i] * kn[i];
+            s = warp_sum(s) * scale;
+            const float mn = fmaxf(m[j], s);
+            const float a = __expf(m[j] - mn), p = __expf(s - mn);
+            l[j] = l[j] * a + p;
+#pragma unroll
+            for (int i = 0; i < EPL; ++i) o[j][i] = o[j][i] * a + p * vn[i];
+            m[j] = mn;
+        }
+    }
+    // combine the warps
+    __shared__ float sm_ml[G][kAttnWarps][2], sm_ov[G][kAttnWarps][HD];
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+        if (lane == 0) {
+            sm_ml[j][warp][0] = m[j];
+            sm_ml[j][warp][1] = l[j];
+        }
+#pragma unroll
+        for (int i = 0; i < EPL; ++i) sm_ov[j][warp][lane * EPL + i] = o[j][i];
+    }
+    __syncthreads();
+    if (warp < G) {                                  // warp j merges head j
+        const int hj = h + warp;
+        const float(*sm_o)[HD] = sm_ov[warp];
+        const float(*ml)[2] = sm_ml[warp];
+        float mm = -INFINITY;
+        for (int w = 0; w < kAttnWarps; ++w) mm = fmaxf(mm, ml[w][0]);
+        float ll = 0.f, oo[EPL];
+#pragma unroll
+        for (int i = 0; i < EPL; ++i) oo[i] = 0.f;
+        for (int w = 0; w < kAttnWarps; ++w) {
+            const float a = ml[w][0] == -INFINITY ? 0.f : __expf(ml[w][0] - mm);
+            ll += ml[w][1] * a;
+#pragma unroll
+            for (int i = 0; i < EPL; ++i) oo[i] += sm_o[w][lane * EPL + i] * a;
+        }
+        if (nsplit == 1) {
+#pragma unroll
+            for (int i = 0; i < EPL; ++i) out[((size_t)b * n_heads + hj) * HD + lane * EPL + i] = __float2half_rn(oo[i] / ll);
+            return;
+        }
+        // several CTAs per head: leave (max, sum, weighted values) of this share; the CTA that arrives last
+        // (counter per head, reset by it) merges the shares in a fixed order
+        float* mine = partial + (((size_t)b * n_heads + hj) * nsplit + z) * (HD + 2);
+        if (lane == 0) {
+            mine[0] = mm;
+            mine[1] = ll;
+        }
+#pragma unroll
+        for (int i = 0; i < EPL; ++i) mine[2 + lane * EPL + i] = oo[i];
+        __threadfence();
+        __syncwarp();
+        int last = 0;
+        if (lane == 0) last = atomicAdd(arrivals + (size_t)b * n_heads + hj, 1) == nsplit - 1;
+        if (!__shfl_sync(0xffffffffu, last, 0)) return;
+        __threadfence();
+        const float* all = partial + ((size_t)b * n_heads + hj) * nsplit * (HD + 2);
+        // (at most 16 shares: lane s2 takes the maximum and the sum of share s2)
+        const float pm = lane < nsplit ? __ldcg(all + (size_t)lane * (HD + 2)) : -INFINITY;
+        const float pl = lane < nsplit ? __ldcg(all + (size_t)lane * (HD + 2) + 1) : 0.f;
+        float gm = pm;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) gm = fmaxf(gm, __shfl_xor_sync(0xffffffffu, gm, d));
+        const float pa = pm == -INFINITY ? 0.f : __expf(pm - gm);
+        float gl = 0.f, go[EPL];
+#pragma unroll
+        for (int i = 0; i < EPL; ++i) go[i] = 0.f;
+        for (int s0 = 0; s0 < nsplit; s0 += 8) {
+            float pv[8][EPL];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+#pragma unroll
+                for (int i = 0; i < EPL; ++i)
+                    pv[u][i] = s0 + u < nsplit ? __ldcg(all + (size_t)(s0 + u) * (HD + 2) + 2 + lane * EPL + i) : 0.f;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const float a = __shfl_sync(0xffffffffu, pa, s0 + u), ls = __shfl_sync(0xffffffffu, pl, s0 + u);
+                if (s0 + u < nsplit) {
+                    gl += ls * a;
+#pragma unroll
+                    for (int i = 0; i < EPL; ++i) go[i] += pv[u][i] * a;
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < EPL; ++i) out[((size_t)b * n_heads + hj) * HD + lane * EPL + i] = __float2half_rn(go[i] / gl);
+        if (lane == 0) arrivals[(size_t)b * n_heads + hj] = 0;
+    }
 }
 
 // The prompt's form of the first half of attn_decode_kernel: per (token, head) one warp applies the optional RMS norm
@@ -533,9 +612,13 @@ extern "C" int glq_add_rmsnorm(const void* x, const void* delta, const void* wei
 }
 
 // position splits per head: enough CTAs to fill the device for long caches
-static int attn_splits(int B, int n_heads, int max_len) {
+static int attn_sms() {
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+static int attn_splits(int B, int n_heads, int max_len) {
+    const int sms = attn_sms();
     int s = (2 * sms + B * n_heads - 1) / (B * n_heads);
     s = std::max(1, std::min(s, 16));
     return std::min(s, std::max(1, max_len / 64));
@@ -561,19 +644,26 @@ extern "C" int glq_attn_decode(const void* q, const void* k_new, const void* v_n
         if (!workspace || workspace_bytes < glq_attn_decode_workspace_bytes(B, n_heads, head_dim, max_len)) return GLQ_ERR_WORKSPACE;
         if (!counters || n_counters < (size_t)B * n_heads) return GLQ_ERR_WORKSPACE;
     }
-    const dim3 grid(n_heads, B, nsplit), block(kAttnWarps * 32);
-#define GLQ_ATTN(EPL)                                                                                              \
-    attn_decode_kernel<EPL><<<grid, block, 0, st>>>(                                                               \
+    // Heads of a CTA: two that share their keys and values read and convert these once, as long as that leaves a CTA for every
+    // SM; with fewer a warp's own chain sets the pace.
+    const bool two = head_dim == 128 && (n_heads / n_kv) % 2 == 0 && (long long)B * n_heads * nsplit >= 2 * attn_sms();
+    const int heads = two ? 2 : 1;
+    const dim3 grid(n_heads / heads, B, nsplit), block(kAttnWarps * 32);
+#define GLQ_ATTN(EPL, G)                                                                                           \
+    attn_decode_kernel<EPL, G><<<grid, block, 0, st>>>(                                                            \
         reinterpret_cast<const __half*>(q), reinterpret_cast<const __half*>(k_new), reinterpret_cast<const __half*>(v_new), \
         reinterpret_cast<const __half*>(cos_t), reinterpret_cast<const __half*>(sin_t),                           \
         reinterpret_cast<const long long*>(pos), reinterpret_cast<__half*>(k_cache), reinterpret_cast<__half*>(v_cache), \
         reinterpret_cast<__half*>(out), n_heads, n_kv, max_len, reinterpret_cast<const __half*>(q_norm_w),         \
         reinterpret_cast<const __half*>(k_norm_w), eps, reinterpret_cast<float*>(workspace), counters)
     switch (head_dim) {
-        case 32: GLQ_ATTN(1); break;
-        case 64: GLQ_ATTN(2); break;
-        case 128: GLQ_ATTN(4); break;
-        case 256: GLQ_ATTN(8); break;
+        case 32: GLQ_ATTN(1, 1); break;
+        case 64: GLQ_ATTN(2, 1); break;
+        case 128:
+            if (two) GLQ_ATTN(4, 2);
+            else GLQ_ATTN(4, 1);
+            break;
+        case 256: GLQ_ATTN(8, 1); break;
         default: return GLQ_ERR_UNSUPPORTED;
     }
 #undef GLQ_ATTN

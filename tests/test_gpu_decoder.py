@@ -192,6 +192,37 @@ def test_rope_prefill_matches_tensor_ops(dev, B, T, nh, nkv, hd, norms):
     assert not kc[:, :, rest].any() and not vc[:, :, rest].any()
 
 
+@pytest.mark.parametrize("B,nh,nkv,hd,max_len,pos", [(1, 16, 16, 128, 576, 511), (16, 32, 8, 128, 130, 101), (16, 32, 8, 128, 64, 0),
+                                                     (64, 32, 4, 128, 40, 33), (3, 8, 2, 64, 320, 257), (2, 4, 1, 32, 80, 63),
+                                                     (2, 4, 4, 256, 70, 69)])
+def test_attn_decode_matches_fp32_attention(dev, B, nh, nkv, hd, max_len, pos):
+    """One, two and four heads per CTA, split and unsplit positions, ragged last steps, the first position, every head size."""
+    from glorcq_b200 import _lib, tiled
+    from glorcq_b200.decoder import _rope_tables, _rotate_half
+    L = _lib.lib()
+    g = torch.Generator().manual_seed(B * 1000 + pos)
+    q, k, v = (torch.randn(B, n, hd, generator=g).half().to(dev) for n in (nh, nkv, nkv))
+    kc, vc = (torch.randn(B, nkv, max_len, hd, generator=g).half().to(dev) for _ in range(2))
+    cos, sin = _rope_tables(hd, max_len, 10000.0, dev)
+    qr, kr = q * cos[pos] + _rotate_half(q) * sin[pos], k * cos[pos] + _rotate_half(k) * sin[pos]
+    kf, vf = kc.float().clone(), vc.float().clone()
+    kf[:, :, pos], vf[:, :, pos] = kr.float(), v.float()
+    rep = nh // nkv
+    kf, vf = kf[:, :, : pos + 1].repeat_interleave(rep, 1), vf[:, :, : pos + 1].repeat_interleave(rep, 1)
+    s = (qr.float().unsqueeze(2) @ kf.transpose(-1, -2)) * hd ** -0.5
+    ref = (torch.softmax(s, -1) @ vf).squeeze(2)
+    y = torch.full_like(q, float("nan"))
+    ws = torch.empty(max(L.glq_attn_decode_workspace_bytes(B, nh, hd, max_len), 16), dtype=torch.uint8, device=dev)
+    ctr = torch.zeros(B * nh, dtype=torch.int32, device=dev)
+    p = torch.tensor([pos], device=dev)
+    for _ in range(2):
+        _lib.check(L.glq_attn_decode(q.data_ptr(), k.data_ptr(), v.data_ptr(), cos.data_ptr(), sin.data_ptr(), p.data_ptr(),
+                                     kc.data_ptr(), vc.data_ptr(), y.data_ptr(), B, nh, nkv, hd, max_len, None, None, 1e-6,
+                                     ws.data_ptr(), ws.numel(), ctr.data_ptr(), ctr.numel(), tiled._stream_ptr(dev)), "attn_decode")
+        assert cases.rel_l2(y.cpu(), ref.cpu()) <= 2e-3
+        assert torch.equal(kc[:, :, pos], kr) and torch.equal(vc[:, :, pos], v) and not ctr.any()
+
+
 @pytest.mark.parametrize("B,T,nh,nkv,hd", [(1, 1, 2, 2, 128), (2, 200, 4, 2, 128), (1, 64, 2, 2, 64), (1, 513, 16, 16, 128),
                                           (3, 65, 8, 2, 64), (1, 1031, 4, 1, 128)])
 def test_attn_prefill_matches_fp32_attention(dev, B, T, nh, nkv, hd):
