@@ -521,16 +521,30 @@ __global__ void __launch_bounds__(1024) moe_exchange_kernel(const __half* __rest
 }
 
 // ---- combine ------------------------------------------------------------------------------------------
-// A token's rows are added in `order`, rounded to fp16 after each; the rows of four are requested before the first is used
-// (one row at a time, 4096 tokens of 8 rows took 72 us, 57 now).
-__device__ __forceinline__ void combine_rows(const __half* __restrict__ yd, const int* __restrict__ entries, const int (&order)[16],
-                                             int k, int n_entries, int H, int c0, float (&acc)[8]) {
+// The entries of a token in the order in which their rows are added (slots, or experts ascending and slots within one), by
+// one warp: a lane's rank is the number of slots that come before its own.  (A sort of the slots by every thread, with its
+// dependent reads of sel, held each of the 4096 CTAs of a long prompt up longer than the rows themselves: 56 us.)
+__device__ __forceinline__ void ordered_entries(const int* __restrict__ sel, const int* __restrict__ entries, int k, bool by_expert, int* s_entry) {
+    if (threadIdx.x < 32) {
+        const int s = threadIdx.x, e = by_expert && s < k ? __ldg(sel + s) : 0, entry = s < k ? __ldg(entries + s) : -1;
+        int rank = 0;
+        for (int j = 0; j < k; ++j) {
+            const int ej = __shfl_sync(0xffffffffu, e, j);
+            rank += ej < e || (ej == e && j < s) ? 1 : 0;
+        }
+        if (s < k) s_entry[rank] = entry;
+    }
+    __syncthreads();
+}
+// A token's rows are added in that order, rounded to fp16 after each; the rows of four are requested before the first is used
+// (one row at a time, 4096 tokens of 8 rows took 72 us instead of 57).
+__device__ __forceinline__ void combine_rows(const __half* __restrict__ yd, const int* entries, int k, int n_entries, int H, int c0, float (&acc)[8]) {
     for (int s0 = 0; s0 < k; s0 += 4) {
         uint4 v[4];
         bool live[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int entry = s0 + u < k ? __ldg(entries + order[s0 + u]) : -1;
+            const int entry = s0 + u < k ? entries[s0 + u] : -1;
             live[u] = entry >= 0 && entry < n_entries;          // a dropped slot adds nothing
             v[u] = live[u] ? __ldg(reinterpret_cast<const uint4*>(yd + (size_t)entry * H + c0)) : make_uint4(0, 0, 0, 0);
         }
@@ -554,25 +568,13 @@ __global__ void moe_combine_kernel(const __half* __restrict__ yd, const int* __r
     if (epoch) yd += (size_t)(*epoch & 1) * half_elems;            // the half the last exchange filled
     const int t = blockIdx.y;
     const int c0 = (blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    __shared__ int s_entry[16];
+    ordered_entries(sel + t * k, tok_entries + t * k, k, by_expert != 0, s_entry);
     if (c0 >= H) return;
-    int order[16];
-    for (int s = 0; s < k; ++s) order[s] = s;
-    if (by_expert) {
-        for (int i = 1; i < k; ++i) {
-            const int v = order[i];
-            const int ev = sel[t * k + v];
-            int j = i - 1;
-            while (j >= 0 && sel[t * k + order[j]] > ev) {
-                order[j + 1] = order[j];
-                --j;
-            }
-            order[j + 1] = v;
-        }
-    }
     float acc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-    combine_rows(yd, tok_entries + t * k, order, k, n_entries, H, c0, acc);
+    combine_rows(yd, s_entry, k, n_entries, H, c0, acc);
     if (ysh) {
         const float gate = gate_col >= 0 ? sigmoid16(__half2float(logits[(size_t)t * ldl + gate_col])) : 1.f;
         __align__(16) __half v[8];
@@ -587,8 +589,11 @@ __global__ void moe_combine_kernel(const __half* __restrict__ yd, const int* __r
 }
 
 // Combine with the decoder's next steps folded in: out = residual + block output (when a residual is given),
-// and normed = rms_norm(out) * weight.  One CTA per token, 8 columns per thread and step, up to 4 steps
-// (H <= 8192); the sum of squares goes through shared memory.
+// and normed = rms_norm(out) * weight.  One CTA per token, 8 columns per thread and step, NS steps
+// (H <= 8192); the sum of squares goes through shared memory.  Bound by the latency of a CTA's few loads: what does not depend
+// on the entries is requested before they are known, and NS is the number of steps, not four, so that twice as many CTAs
+// fit an SM (4096 tokens of 8 rows of 2048: 56 -> 35 us; 512 of 4: 7.2 -> 5.8; 16 of 2 rows of 4096: 6.0 -> 4.7).
+template <int NS>
 __global__ void __launch_bounds__(256) moe_combine_norm_kernel(const __half* __restrict__ yd, const int* __restrict__ tok_entries,
                                                                int n_entries, const int* __restrict__ sel, int k, int H,
                                                                int by_expert, const __half* __restrict__ ysh,
@@ -599,40 +604,33 @@ __global__ void __launch_bounds__(256) moe_combine_norm_kernel(const __half* __r
                                                                const int* __restrict__ epoch, size_t half_elems) {
     const int t = blockIdx.x;
     if (epoch) yd += (size_t)(*epoch & 1) * half_elems;
-    int order[16];
-    for (int s = 0; s < k; ++s) order[s] = s;
-    if (by_expert) {
-        for (int i = 1; i < k; ++i) {
-            const int v = order[i];
-            const int ev = sel[t * k + v];
-            int j = i - 1;
-            while (j >= 0 && sel[t * k + order[j]] > ev) {
-                order[j + 1] = order[j];
-                --j;
-            }
-            order[j + 1] = v;
-        }
+    uint4 sh[NS], rs[NS];
+#pragma unroll
+    for (int step = 0; step < NS; ++step) {
+        const int c0 = (step * 256 + threadIdx.x) * 8;
+        if (ysh && c0 < H) sh[step] = *reinterpret_cast<const uint4*>(ysh + (size_t)t * H + c0);
+        if (residual && c0 < H) rs[step] = *reinterpret_cast<const uint4*>(residual + (size_t)t * H + c0);
     }
+    __shared__ int s_entry[16];
+    ordered_entries(sel + t * k, tok_entries + t * k, k, by_expert != 0, s_entry);
     const float gate = (ysh && gate_col >= 0) ? sigmoid16(__half2float(logits[(size_t)t * ldl + gate_col])) : 1.f;
-    float val[4][8];
+    float val[NS][8];
     float ss = 0.f;
 #pragma unroll
-    for (int step = 0; step < 4; ++step) {
+    for (int step = 0; step < NS; ++step) {
         const int c0 = (step * 256 + threadIdx.x) * 8;
         if (c0 >= H) continue;
         float acc[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-        combine_rows(yd, tok_entries + t * k, order, k, n_entries, H, c0, acc);
+        combine_rows(yd, s_entry, k, n_entries, H, c0, acc);
         if (ysh) {
-            __align__(16) __half v[8];
-            *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(ysh + (size_t)t * H + c0);
+            const __half* v = reinterpret_cast<const __half*>(&sh[step]);
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc[i] = round16(acc[i] + round16(gate * __half2float(v[i])));
         }
         if (residual) {
-            __align__(16) __half v[8];
-            *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(residual + (size_t)t * H + c0);
+            const __half* v = reinterpret_cast<const __half*>(&rs[step]);
 #pragma unroll
             for (int i = 0; i < 8; ++i) acc[i] = round16(__half2float(v[i]) + acc[i]);
         }
@@ -654,7 +652,7 @@ __global__ void __launch_bounds__(256) moe_combine_norm_kernel(const __half* __r
     for (int w = 0; w < 8; ++w) tot += red[w];
     const float r = rsqrtf(tot / H + eps);
 #pragma unroll
-    for (int step = 0; step < 4; ++step) {
+    for (int step = 0; step < NS; ++step) {
         const int c0 = (step * 256 + threadIdx.x) * 8;
         if (c0 >= H) continue;
         __align__(16) __half o[8], wv[8];
@@ -1269,7 +1267,8 @@ extern "C" int glq_moe_forward_ep(const glq_moe_desc_t* d, const void* x, int n,
     // 8. combine
     if (ep && ep->normed_out) {
         if (d->H > 8192) return GLQ_ERR_UNSUPPORTED;
-        moe_combine_norm_kernel<<<n, 256, 0, st>>>(
+        auto kern = d->H <= 2048 ? moe_combine_norm_kernel<1> : d->H <= 4096 ? moe_combine_norm_kernel<2> : moe_combine_norm_kernel<4>;
+        kern<<<n, 256, 0, st>>>(
             reinterpret_cast<const __half*>(p_yd), p_tok, nk, p_sel, k, d->H, n > d->slot_order_max_tokens ? 1 : 0,
             shared ? reinterpret_cast<const __half*>(ws + L.ysh) : nullptr, p_logits, ldl, d->router_rows > d->E ? d->E : -1,
             reinterpret_cast<const __half*>(ep->residual), reinterpret_cast<const __half*>(ep->norm_weight), ep->norm_eps,
