@@ -147,7 +147,7 @@ MoeLayout moe_layout(const glq_moe_desc_t* d, int n) {
 
 // ---- routing plan -----------------------------------------------------------------------------------
 // One CTA; the selection stays in shared memory between the phases (through global memory every scan of an expert's warp waited
-// for L2: 13.4 us for 32 tokens over 60 experts, 12.7 now).  Phase A, warp per token: softmax over the fp16 router logits in fp32, top-k (ties to
+// for L2: 13.4 us for 32 tokens over 60 experts, 12.7 without; 10.6 with softmax_topk).  Phase A, warp per token: softmax over the fp16 router logits in fp32, top-k (ties to
 // the lower expert index), optional renormalisation, weights rounded to fp16.  Phase B, warp per
 // expert: entry counts, offsets and the expert's entry list in token order (ballot scans:
 // deterministic), and the compacted list of live experts.
@@ -158,72 +158,23 @@ __device__ __forceinline__ void route_token(int t, int lane, const __half* __res
                                             int* __restrict__ sel_out, __half* __restrict__ wts_out, int* s_sel = nullptr,
                                             __half* s_wts = nullptr) {
     const __half* row = logits + (size_t)t * ldl;
-    float lv[8], pv[8];
-    float mx = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int e = lane + 32 * i;
-        lv[i] = e < E ? __half2float(row[e]) : -INFINITY;
-        mx = fmaxf(mx, lv[i]);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    float sum = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        pv[i] = (lane + 32 * i) < E ? expf(lv[i] - mx) : 0.f;
-        sum += pv[i];
-    }
-    sum = warp_sum(sum);
-#pragma unroll
-    // a probability that is not a number (non-finite hidden state) counts as zero: the top-k below then
-    // still selects k distinct experts and no index leaves the tables
-    for (int i = 0; i < 8; ++i) {
-        const float pr = pv[i] / sum;
-        pv[i] = (lane + 32 * i) < E ? (pr >= 0.f ? pr : 0.f) : -1.f;
-    }
-    float wk[16];
-    int ek[16];
-    float wsum = 0.f;
-    for (int s = 0; s < k; ++s) {
-        float best = -1.f;
-        int be = 0x7fffffff;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            if (pv[i] > best) {   // increasing i = increasing expert index: first maximum wins
-                best = pv[i];
-                be = lane + 32 * i;
-            }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oe = __shfl_xor_sync(0xffffffffu, be, o);
-            if (ob > best || (ob == best && oe < be)) {
-                best = ob;
-                be = oe;
-            }
+    int e;
+    float pe, wsum;
+    softmax_topk(row, E, k, lane, e, pe, wsum);
+    if (lane < k) {
+        const int i = t * k + lane;
+        const __half wh = __float2half_rn(renorm ? pe / wsum : pe);
+        sel[i] = e;
+        wts[i] = wh;
+        if (s_sel) {
+            s_sel[i] = e;
+            s_wts[i] = wh;
         }
-        wk[s] = best;
-        ek[s] = be;
-        wsum += best;
-        if ((be & 31) == lane) pv[be >> 5] = -1.f;   // taken
-    }
-    if (lane == 0) {
-        for (int s = 0; s < k; ++s) {
-            const float wv = renorm ? wk[s] / wsum : wk[s];
-            const __half wh = __float2half_rn(wv);
-            sel[t * k + s] = ek[s];
-            wts[t * k + s] = wh;
-            if (s_sel) {
-                s_sel[t * k + s] = ek[s];
-                s_wts[t * k + s] = wh;
-            }
-            if (sel_out) sel_out[t * k + s] = ek[s];
-            if (wts_out) wts_out[t * k + s] = wh;
-        }
+        if (sel_out) sel_out[i] = e;
+        if (wts_out) wts_out[i] = wh;
     }
     if (logits_out)
-        for (int e = lane; e < E; e += 32) logits_out[(size_t)t * E + e] = row[e];
+        for (int j = lane; j < E; j += 32) logits_out[(size_t)t * E + j] = row[j];
 }
 
 // Warp 0 of a CTA: exclusive prefix of the per-expert counts in sm_cnt (entry offsets are global: every rank
