@@ -16,6 +16,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <algorithm>
 #include <cstring>
 #include <map>
 #include <unordered_map>
@@ -101,6 +102,13 @@ long integer(PyObject* o) {
 void need_cuda(const at::Tensor& t, const char* name) {
     if (!t.is_cuda()) fail(std::string(name) + " must be a CUDA tensor (glorcq_b200 has no CPU path)");
     if (!t.is_contiguous()) fail(std::string(name) + " must be contiguous");
+}
+// the last dimension is the row: an element count that fits by chance would be read as other rows than it has (no rows: any width)
+void need_rows(const at::Tensor& t, const char* name, int64_t K) {
+    if (t.dim() == 0) fail(std::string(name) + " must have at least one dimension");
+    const auto lead = t.sizes().slice(0, t.dim() - 1);
+    if (t.size(-1) != K && std::find(lead.begin(), lead.end(), 0) == lead.end())
+        fail(std::string(name) + " must have rows of " + std::to_string(K) + " values, got " + std::to_string(t.size(-1)));
 }
 void need(const at::Tensor& t, const char* name, at::ScalarType dtype, const char* dtype_name) {
     if (!t.is_cuda()) fail(std::string(name) + " must be a CUDA tensor");
@@ -208,16 +216,15 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
         const at::Tensor* signs = tensor_or_none(a[3], "signs");
         const at::Tensor* xu = tensor_or_none(a[4], "precomputed x@U");
         if (x.scalar_type() != at::kHalf) fail("x must be fp16");
+        need_rows(x, "x", L->w.K);
         need_cuda(x, "x");
-        const int64_t K = x.dim() == 2 ? x.size(1) : L->w.K, rows = x.dim() == 2 ? x.size(0) : x.numel() / std::max<int64_t>(K, 1);
-        if (x.dim() != 2 && rows * K != x.numel()) fail("x does not hold whole rows of the layer's input size");
+        const int64_t K = L->w.K, rows = x.dim() == 2 ? x.size(0) : x.numel() / std::max<int64_t>(K, 1);
         c10::cuda::OptionalCUDAGuard guard(x.device());
         at::Tensor y;
         if (x.dim() == 2) {
             y = empty({rows, L->w.N}, at::kHalf, x);
         } else {
             auto shape = x.sizes().vec();
-            if (shape.empty()) fail("x must have at least one dimension");
             shape.back() = L->w.N;
             y = empty(shape, at::kHalf, x);
         }

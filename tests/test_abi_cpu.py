@@ -110,3 +110,16 @@ def test_native_host_path_binds_and_refuses_cpu_tensors(libpath):
         nat.linear(layer)
     with pytest.raises(RuntimeError, match="x_rot must be a CUDA tensor"):
         nat.turbo_matmul(*[torch.zeros(1, 4, dtype=torch.float16)] * 4)
+
+
+@pytest.mark.parametrize("shape", [(1, 64), (2, 4, 64), (64,), (2, 256), (4, 192), (2, 0)])
+def test_native_linear_refuses_rows_of_another_width(libpath, shape):
+    """Decided before any look at the device; (2, 4, 64) holds as many values as four rows of 128."""
+    import torch
+    from glorcq_b200 import _lib
+    nat = _lib.native()
+    layer = nat.layer(_lib.FMT_Q2, 128, bytes(_lib.Weight(None, None, None, None, None, None, 16, 128, 0, 0)))
+    with pytest.raises(RuntimeError, match=f"rows of 128 values, got {shape[-1]}"):
+        nat.linear(layer, torch.zeros(shape, dtype=torch.float16), None, None, None)
+    with pytest.raises(RuntimeError, match="at least one dimension"):
+        nat.linear(layer, torch.zeros((), dtype=torch.float16), None, None, None)
