@@ -473,9 +473,12 @@ PyObject* py_moe(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
         const at::Tensor *res = tensor_or_none(a[2], "residual"), *nw = tensor_or_none(a[3], "norm weight");
         const bool norm = a[4] != Py_None;
         const at::Tensor *sel_in = tensor_or_none(a[5], "top_k_index"), *wts_in = tensor_or_none(a[6], "top_k_weights");
+        const int64_t H = d->H;
+        need_rows(x, "hidden_states", H);
         need(x, "hidden_states", at::kHalf, "torch.float16");
-        const int64_t H = d->H, n = x.numel() / H;
-        if (n * H != x.numel()) fail("hidden_states do not hold whole rows");
+        const int64_t n = x.numel() / H;
+        if (norm && res && res->numel() != x.numel()) fail("the residual must have the shape of hidden_states");
+        if (norm && nw && nw->numel() != H) fail("the norm weight must have " + std::to_string(H) + " values");
         c10::cuda::OptionalCUDAGuard guard(x.device());
         const cudaStream_t st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
         at::Tensor out = empty(x.sizes(), at::kHalf, x), logits, normed;

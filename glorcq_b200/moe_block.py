@@ -288,7 +288,7 @@ class GraphCompatibleMoeBlock(nn.Module):
         first result becomes ``residual + block output`` (``residual`` (B, S, H), optional) and a third result
         is its RMS norm times ``weight``: ((B, S, H), logits, (B, S, H))."""
         if self._native is not None and top_k_index is None and residual is None and next_norm is None and self.gate is not None \
-                and self._ep[1] == 1 and hidden_states.dtype is torch.float16 and hidden_states.is_contiguous():
+                and self._ep[1] == 1 and hidden_states.dtype is torch.float16 and hidden_states.dim() == 3 and hidden_states.is_contiguous():
             out, logits, self.last_selected_experts, self.last_routing_weights, _ = _lib.native().moe(
                 self._block(hidden_states.device), hidden_states, None, None, None, None, None)
             return out, logits
@@ -303,6 +303,8 @@ class GraphCompatibleMoeBlock(nn.Module):
             self._build(x.device)
         d = self._desc
         n = x.shape[0]
+        if n > 0 and hidden_dim != d.H:
+            raise RuntimeError(f"hidden_states must have rows of {d.H} values, got {hidden_dim}")
         given = top_k_index is not None
         if given != (self.gate is None):
             raise RuntimeError("routing must be passed exactly when the block has no router")

@@ -123,3 +123,34 @@ def test_native_linear_refuses_rows_of_another_width(libpath, shape):
         nat.linear(layer, torch.zeros(shape, dtype=torch.float16), None, None, None)
     with pytest.raises(RuntimeError, match="at least one dimension"):
         nat.linear(layer, torch.zeros((), dtype=torch.float16), None, None, None)
+
+
+@pytest.mark.parametrize("shape", [(1, 4, 64), (2, 4, 192), (1, 2, 0)])
+def test_native_moe_refuses_rows_of_another_width(libpath, shape):
+    import ctypes as C
+    import torch
+    from glorcq_b200 import _lib
+    d = _lib.MoeDesc()
+    d.H, d.I, d.E, d.top_k = 128, 64, 4, 2
+    nat = _lib.native()
+    block = nat.block(C.addressof(d), 0, 0, 0, 0)
+    with pytest.raises(RuntimeError, match=f"rows of 128 values, got {shape[-1]}"):
+        nat.moe(block, torch.zeros(shape, dtype=torch.float16), None, None, None, None, None)
+    with pytest.raises(RuntimeError, match="must be a CUDA tensor"):
+        nat.moe(block, torch.zeros(1, 4, 128, dtype=torch.float16), None, None, None, None, None)
+
+
+def test_moe_block_takes_three_dimensions_once_built_too(libpath):
+    from types import SimpleNamespace
+    import ctypes as C
+    import torch
+    from glorcq_b200 import _lib
+    from glorcq_b200.moe_block import GraphCompatibleMoeBlock
+    blk = GraphCompatibleMoeBlock(SimpleNamespace(num_experts=4, top_k=2, norm_topk_prob=False, gate=torch.nn.Identity(), experts=None))
+    blk._desc, blk._built = _lib.MoeDesc(), True
+    blk._desc.H, blk._desc.I, blk._desc.E, blk._desc.top_k = 128, 64, 4, 2
+    blk._native = (_lib.native().block(C.addressof(blk._desc), 0, 0, 0, 0), False, (0, 0, 0))
+    with pytest.raises(ValueError):
+        blk(torch.zeros(4, 128, dtype=torch.float16))
+    with pytest.raises(RuntimeError, match="CUDA"):
+        blk(torch.zeros(1, 4, 128, dtype=torch.float16))
