@@ -289,6 +289,7 @@ PyObject* py_grouped_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
         nargs_are(n, 2);
         Group* G = capsule<Group>(args[0], "glq.group");
         const at::Tensor& x = tensor(args[1], "x");
+        if (x.dim() == 2) need_rows(x, "x", G->K);
         if (x.scalar_type() != at::kHalf || x.dim() != 2 || !x.is_cuda() || x.stride(1) != 1) fail("x must be fp16 CUDA rows");
         c10::cuda::OptionalCUDAGuard guard(x.device());
         const int64_t B = x.size(0);

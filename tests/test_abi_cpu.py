@@ -154,3 +154,15 @@ def test_moe_block_takes_three_dimensions_once_built_too(libpath):
         blk(torch.zeros(4, 128, dtype=torch.float16))
     with pytest.raises(RuntimeError, match="CUDA"):
         blk(torch.zeros(1, 4, 128, dtype=torch.float16))
+
+
+@pytest.mark.parametrize("K", [64, 192, 0])
+def test_native_group_refuses_rows_of_another_width(libpath, K):
+    import torch
+    from glorcq_b200 import _lib
+    nat = _lib.native()
+    group = nat.group(_lib.FMT_Q2, 128, 3, 16, 128, 0, 0, 0)
+    with pytest.raises(RuntimeError, match=f"rows of 128 values, got {K}"):
+        nat.grouped_linear(group, torch.zeros(2, K, dtype=torch.float16))
+    with pytest.raises(RuntimeError, match="fp16 CUDA rows"):
+        nat.grouped_linear(group, torch.zeros(2, 128, dtype=torch.float16))
