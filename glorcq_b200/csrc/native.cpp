@@ -4,8 +4,10 @@
 // Why: a decode-sized call runs for 5 to 10 us on the GPU, and the same steps in Python (a ctypes call with
 // twenty arguments, two workspace queries, device and stream look-ups, torch.empty) took 20 to 60 us of host time, so
 // eager calls were bound by the interpreter.  The functions take tensors as they come (METH_FASTCALL, no argument
-// parsing), hold the GIL for the few launches they make -- which also keeps the launches of one call together when
-// several threads share a stream -- and raise RuntimeError exactly where the ctypes path did.
+// parsing) and raise RuntimeError exactly where the ctypes path did.
+//
+// The launches run without the interpreter lock (struct Launching): a launch into a full queue waits for the GPU, and
+// the process's other threads have other GPUs to feed meanwhile.
 //
 // The library itself is not linked: bind() receives the entry points' addresses from the loaded library, so that a
 // checking build selected with GLQ_LIB serves this module too.
@@ -19,6 +21,7 @@
 #include <algorithm>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <unordered_map>
 #include <utility>
 #include <vector>
@@ -99,6 +102,11 @@ long integer(PyObject* o) {
     if (v == -1 && PyErr_Occurred()) throw Error{};
     return v;
 }
+float number(PyObject* o) {
+    const double v = PyFloat_AsDouble(o);
+    if (v == -1 && PyErr_Occurred()) throw Error{};
+    return (float)v;
+}
 void need_cuda(const at::Tensor& t, const char* name) {
     if (!t.is_cuda()) fail(std::string(name) + " must be a CUDA tensor (glorcq_b200 has no CPU path)");
     if (!t.is_contiguous()) fail(std::string(name) + " must be contiguous");
@@ -163,6 +171,35 @@ Scratch& scratch(int dev, cudaStream_t st, size_t nbytes, size_t nctr) {
     }
     if (small_ctr) s.ctr = at::zeros({(int64_t)std::max<size_t>(nctr, 1 << 16)}, opt.dtype(at::kInt));
     return s;
+}
+
+// The launches of one call: the interpreter lock is given back, and one lock per stream keeps the launches of a call
+// together when several threads share the stream, since they also share its scratch.  The locks are taken in this order
+// and given back in the other, so a thread that waits for the stream never holds the interpreter.  Whatever the call
+// launches on is held by references of its own: other threads may grow the scratch or clear the maps meanwhile.
+// Costs 0.1 us a call.
+struct Launching {
+    PyThreadState* state;
+    std::mutex& m;
+    static std::mutex& of(cudaStream_t st) {         // (a few streams may share a lock)
+        static std::mutex* locks = new std::mutex[64];
+        return locks[(reinterpret_cast<uintptr_t>(st) >> 4) % 61];
+    }
+    explicit Launching(cudaStream_t st) : state(PyEval_SaveThread()), m(of(st)) { m.lock(); }
+    ~Launching() {
+        m.unlock();
+        PyEval_RestoreThread(state);
+    }
+    Launching(const Launching&) = delete;
+};
+
+template <class F> void launch(cudaStream_t st, const char* what, F&& f) {
+    int status;
+    {
+        Launching unlocked(st);
+        status = f();
+    }
+    check(status, what);
 }
 
 PyObject* py_workspace(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -252,17 +289,16 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
         }
         const int dev = x.get_device();
         const cudaStream_t st = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
-        Scratch& s = scratch(dev, st, needs.first, needs.second);
+        const Scratch s = scratch(dev, st, needs.first, needs.second);
         void* ws = s.ws.mutable_data_ptr();
         auto* ctr = static_cast<int32_t*>(s.ctr.mutable_data_ptr());
-        if (signs)
-            check(api.glq_linear_rht_forward(L->fmt, L->gs, &L->w, ptr(ut), static_cast<const float*>(signs->const_data_ptr()),
-                                             x.const_data_ptr(), K, ptr(xu), y.mutable_data_ptr(), L->w.N, (int)rows, ws,
-                                             (size_t)s.ws.numel(), ctr, (size_t)s.ctr.numel(), st), "linear_rht_forward");
-        else
-            check(api.glq_linear_forward(L->fmt, L->gs, &L->w, ptr(ut), x.const_data_ptr(), K, ptr(xu), y.mutable_data_ptr(),
-                                         L->w.N, (int)rows, ws, (size_t)s.ws.numel(), ctr, (size_t)s.ctr.numel(), st),
-                  "linear_forward");
+        launch(st, signs ? "linear_rht_forward" : "linear_forward", [&] {
+            return signs ? api.glq_linear_rht_forward(L->fmt, L->gs, &L->w, ptr(ut), static_cast<const float*>(signs->const_data_ptr()),
+                                                      x.const_data_ptr(), K, ptr(xu), y.mutable_data_ptr(), L->w.N, (int)rows, ws,
+                                                      (size_t)s.ws.numel(), ctr, (size_t)s.ctr.numel(), st)
+                         : api.glq_linear_forward(L->fmt, L->gs, &L->w, ptr(ut), x.const_data_ptr(), K, ptr(xu), y.mutable_data_ptr(),
+                                                  L->w.N, (int)rows, ws, (size_t)s.ws.numel(), ctr, (size_t)s.ctr.numel(), st);
+        });
         return wrap(y);
     });
 }
@@ -298,7 +334,7 @@ PyObject* py_grouped_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
         at::Tensor& rows = G->rows[B];
         if (!rows.defined()) rows = at::arange(B, x.options().dtype(at::kInt)).repeat({G->P});
         at::Tensor y = empty({G->P, B, G->N}, at::kHalf, x), a;
-        auto call = [&](int fmt, int gs, const glq_weight_t* table, int N, int rank, at::Tensor& out, const at::Tensor* xu) {
+        auto args = [&](int fmt, int gs, const glq_weight_t* table, int N, int rank, at::Tensor& out, const at::Tensor* xu) {
             glq_mm_args_t m;
             std::memset(&m, 0, sizeof(m));
             m.fmt = fmt;
@@ -320,18 +356,32 @@ PyObject* py_grouped_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
             }
             m.y = out.mutable_data_ptr();
             m.ldy = N;
-            Scratch& s = scratch(dev, st, api.glq_mm_workspace_bytes(&m), api.glq_mm_counters(&m));
-            m.workspace = s.ws.mutable_data_ptr();
-            m.workspace_bytes = (size_t)s.ws.numel();
-            m.counters = static_cast<int32_t*>(s.ctr.mutable_data_ptr());
-            m.n_counters = (size_t)s.ctr.numel();
-            check(api.glq_grouped_matmul(&m, st), "grouped_matmul");
+            return m;
         };
-        if (G->ut_table && G->rank > 0) {
-            a = empty({G->P, B, G->rank}, at::kHalf, x);
-            call(GLQ_FMT_F16, 0, G->ut_table, G->rank, 0, a, nullptr);
+        const bool low_rank = G->ut_table && G->rank > 0;
+        if (low_rank) a = empty({G->P, B, G->rank}, at::kHalf, x);
+        // both products are launched under one lock: nothing of another thread may come between them
+        glq_mm_args_t mm[2];
+        int n_mm = 0;
+        if (low_rank) mm[n_mm++] = args(GLQ_FMT_F16, 0, G->ut_table, G->rank, 0, a, nullptr);
+        mm[n_mm++] = args(G->fmt, G->gs, G->table, G->N, low_rank ? G->rank : 0, y, low_rank ? &a : nullptr);
+        size_t nbytes = 0, nctr = 0;
+        for (int i = 0; i < n_mm; ++i) {
+            nbytes = std::max(nbytes, api.glq_mm_workspace_bytes(&mm[i]));
+            nctr = std::max(nctr, api.glq_mm_counters(&mm[i]));
         }
-        call(G->fmt, G->gs, G->table, G->N, a.defined() ? G->rank : 0, y, a.defined() ? &a : nullptr);
+        const Scratch s = scratch(dev, st, nbytes, nctr);
+        for (int i = 0; i < n_mm; ++i) {
+            mm[i].workspace = s.ws.mutable_data_ptr();
+            mm[i].workspace_bytes = (size_t)s.ws.numel();
+            mm[i].counters = static_cast<int32_t*>(s.ctr.mutable_data_ptr());
+            mm[i].n_counters = (size_t)s.ctr.numel();
+        }
+        launch(st, "grouped_matmul", [&] {
+            int status = GLQ_OK;
+            for (int i = 0; i < n_mm && status == GLQ_OK; ++i) status = api.glq_grouped_matmul(&mm[i], st);
+            return status;
+        });
         return wrap(y);
     });
 }
@@ -354,9 +404,11 @@ PyObject* py_turbo_matmul(PyObject*, PyObject* const* a, Py_ssize_t n) {
         c10::cuda::OptionalCUDAGuard guard(x.device());
         at::Tensor y = empty({B, N}, at::kHalf, x);
         if (B == 0 || N == 0) return wrap(y);
-        check(api.glq_turbo_dequant_matmul(x.const_data_ptr(), static_cast<const uint8_t*>(q.const_data_ptr()), static_cast<const float*>(nrm.const_data_ptr()),
-                                           static_cast<const float*>(cen.const_data_ptr()), y.mutable_data_ptr(), (int)B, (int)N, (int)K,
-                                           c10::cuda::getCurrentCUDAStream(x.device().index()).stream()), "turbo_dequant_matmul");
+        const cudaStream_t st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+        launch(st, "turbo_dequant_matmul", [&] {
+            return api.glq_turbo_dequant_matmul(x.const_data_ptr(), static_cast<const uint8_t*>(q.const_data_ptr()), static_cast<const float*>(nrm.const_data_ptr()),
+                                                static_cast<const float*>(cen.const_data_ptr()), y.mutable_data_ptr(), (int)B, (int)N, (int)K, st);
+        });
         return wrap(y);
     });
 }
@@ -378,9 +430,11 @@ PyObject* py_turbo_grouped_gemv(PyObject*, PyObject* const* a, Py_ssize_t n) {
         c10::cuda::OptionalCUDAGuard guard(x.device());
         at::Tensor y = empty({E * N}, at::kHalf, x);
         if (E == 0 || N == 0) return wrap(y);
-        check(api.glq_turbo_dequant_grouped_gemv(x.const_data_ptr(), static_cast<const uint8_t*>(q.const_data_ptr()), static_cast<const float*>(nrm.const_data_ptr()),
-                                                 static_cast<const float*>(cen.const_data_ptr()), y.mutable_data_ptr(), (int)E, (int)N, (int)K,
-                                                 c10::cuda::getCurrentCUDAStream(x.device().index()).stream()), "turbo_dequant_grouped_gemv");
+        const cudaStream_t st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+        launch(st, "turbo_dequant_grouped_gemv", [&] {
+            return api.glq_turbo_dequant_grouped_gemv(x.const_data_ptr(), static_cast<const uint8_t*>(q.const_data_ptr()), static_cast<const float*>(nrm.const_data_ptr()),
+                                                      static_cast<const float*>(cen.const_data_ptr()), y.mutable_data_ptr(), (int)E, (int)N, (int)K, st);
+        });
         return wrap(y);
     });
 }
@@ -406,9 +460,13 @@ PyObject* py_gptq_matmul(PyObject*, PyObject* const* a, Py_ssize_t n) {
         c10::cuda::OptionalCUDAGuard guard(x.device());
         at::Tensor y = empty({B, N}, at::kFloat, x);
         if (B == 0 || N == 0) return wrap(y);
-        check(api.glq_gptq_dequant_matmul(static_cast<const float*>(x.const_data_ptr()), static_cast<const int8_t*>(q.const_data_ptr()), s.const_data_ptr(), z.const_data_ptr(),
-                                          static_cast<const float*>(ptr(lo)), static_cast<float*>(y.mutable_data_ptr()), (int)B, (int)N, (int)K, (int)integer(a[4]),
-                                          (int)G, PyObject_IsTrue(a[5]), c10::cuda::getCurrentCUDAStream(x.device().index()).stream()), "gptq_dequant_matmul");
+        const int gs = (int)integer(a[4]), sym = PyObject_IsTrue(a[5]);
+        if (sym < 0) throw Error{};
+        const cudaStream_t st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+        launch(st, "gptq_dequant_matmul", [&] {
+            return api.glq_gptq_dequant_matmul(static_cast<const float*>(x.const_data_ptr()), static_cast<const int8_t*>(q.const_data_ptr()), s.const_data_ptr(), z.const_data_ptr(),
+                                               static_cast<const float*>(ptr(lo)), static_cast<float*>(y.mutable_data_ptr()), (int)B, (int)N, (int)K, gs, (int)G, sym, st);
+        });
         return wrap(y);
     });
 }
@@ -487,7 +545,7 @@ PyObject* py_moe(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
         at::Tensor sel = empty({n, d->top_k}, at::kInt, x), wts = empty({n, d->top_k}, at::kHalf, x);
         if (norm) normed = empty(x.sizes(), at::kHalf, x);
         if (n > 0) {
-            Scratch& s = block_scratch(B, n, st);
+            const Scratch s = block_scratch(B, n, st);
             char* ws = static_cast<char*>(s.ws.mutable_data_ptr());
             char* base = reinterpret_cast<char*>(up256(reinterpret_cast<size_t>(ws)));
             glq_moe_ep_t ep;
@@ -500,14 +558,16 @@ PyObject* py_moe(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
             }
             if (norm) {
                 ep.normed_out = normed.mutable_data_ptr();
-                ep.norm_eps = (float)PyFloat_AsDouble(a[4]);
+                ep.norm_eps = number(a[4]);
                 ep.residual = static_cast<decltype(ep.residual)>(ptr(res));
                 ep.norm_weight = static_cast<decltype(ep.norm_weight)>(ptr(nw));
             }
-            check(api.glq_moe_forward_ep(d, x.const_data_ptr(), (int)n, out.mutable_data_ptr(), logits.defined() ? logits.mutable_data_ptr() : nullptr,
-                                         static_cast<int32_t*>(sel.mutable_data_ptr()), wts.mutable_data_ptr(), base,
-                                         (size_t)s.ws.numel() - (size_t)(base - ws), static_cast<int32_t*>(s.ctr.mutable_data_ptr()),
-                                         (size_t)s.ctr.numel(), st, B->side, B->fork, B->join, (sel_in || norm) ? &ep : nullptr), "moe_forward");
+            launch(st, "moe_forward", [&] {
+                return api.glq_moe_forward_ep(d, x.const_data_ptr(), (int)n, out.mutable_data_ptr(), logits.defined() ? logits.mutable_data_ptr() : nullptr,
+                                              static_cast<int32_t*>(sel.mutable_data_ptr()), wts.mutable_data_ptr(), base,
+                                              (size_t)s.ws.numel() - (size_t)(base - ws), static_cast<int32_t*>(s.ctr.mutable_data_ptr()),
+                                              (size_t)s.ctr.numel(), st, B->side, B->fork, B->join, (sel_in || norm) ? &ep : nullptr);
+            });
         }
         auto opt = [](at::Tensor& t) {
             if (t.defined()) return wrap(t);
@@ -528,8 +588,12 @@ PyObject* py_add_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t n) {
         c10::cuda::OptionalCUDAGuard guard(x.device());
         const int64_t H = x.size(-1);
         at::Tensor xo = empty(x.sizes(), at::kHalf, x), ho = empty(x.sizes(), at::kHalf, x);
-        check(api.glq_add_rmsnorm(x.const_data_ptr(), dl.const_data_ptr(), w.const_data_ptr(), (float)PyFloat_AsDouble(a[3]), (int)(x.numel() / H), (int)H,
-                                  xo.mutable_data_ptr(), ho.mutable_data_ptr(), c10::cuda::getCurrentCUDAStream(x.device().index()).stream()), "add_rmsnorm");
+        const float eps = number(a[3]);
+        const cudaStream_t st = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+        launch(st, "add_rmsnorm", [&] {
+            return api.glq_add_rmsnorm(x.const_data_ptr(), dl.const_data_ptr(), w.const_data_ptr(), eps, H > 0 ? (int)(x.numel() / H) : 0, (int)H,
+                                       xo.mutable_data_ptr(), ho.mutable_data_ptr(), st);
+        });
         return Py_BuildValue("NN", wrap(xo), wrap(ho));
     });
 }

@@ -404,3 +404,57 @@ def test_dense_weight_route_dtype_and_reference_op_names(dev):
     assert GK._int8_codes(q32) is a8
     q32 += 0
     assert GK._int8_codes(q32) is not a8
+
+
+# ---- threads ------------------------------------------------------------------------------------------
+def test_launches_run_without_the_interpreter_lock(dev):
+    """The library's entry points are replaced by PyGILState_Check: 0, a success, when the calling thread does not
+    hold the interpreter lock, 1, an unknown status, when it does."""
+    import ctypes as C
+    from glorcq_b200 import _lib, tiled
+    from glorcq_b200.kernels import gptq_dequant_matmul, turbo_dequant_grouped_gemv, turbo_dequant_matmul
+    lin = cases.to_b200_linear(cases.make_linear(3, 64, 128, rank=16), dev)
+    group = tiled.GroupedLinear([lin._tiled] * 2, [lin._ut] * 2)
+    blk = cases.to_b200_moe(cases.make_moe(5, 128, 64, 4, 2, rank=16, experts_per_cluster=2), dev)
+    x = cases.make_x(4, 2, 128).to(dev)
+    blk(x.view(1, 2, 128))
+    q, n, c = torch.zeros(16, 32, dtype=torch.uint8, device=dev), torch.ones(16, device=dev), torch.ones(4, device=dev)
+    s = torch.ones(16, 1, dtype=torch.float16, device=dev)
+    calls = [lambda: lin(x), lambda: group.forward(x), lambda: blk(x.view(1, 2, 128)), lambda: turbo_dequant_matmul(x, q, n, c),
+             lambda: turbo_dequant_grouped_gemv(x, q, n, c, 8), lambda: _lib.native().add_rmsnorm(x, x, s[:1].expand(1, 128).contiguous(), 1e-6),
+             lambda: gptq_dequant_matmul(x.float(), torch.zeros(16, 128, dtype=torch.int8, device=dev), s, s, 128, False, torch.empty(0, device=dev))]
+    for f in calls:
+        f()
+    nat = _lib.native()
+    real = {e: C.cast(getattr(_lib.lib(), e), C.c_void_p).value for e in nat.names()}
+    probe = C.cast(C.pythonapi.PyGILState_Check, C.c_void_p).value
+    launches = ("glq_linear_forward", "glq_grouped_matmul", "glq_moe_forward_ep", "glq_turbo_dequant_matmul",
+                "glq_turbo_dequant_grouped_gemv", "glq_add_rmsnorm", "glq_gptq_dequant_matmul")
+    try:
+        nat.bind({**real, **{e: probe for e in launches}})
+        for f in calls:
+            f()
+    finally:
+        nat.bind(real)
+
+
+def test_threads_on_one_stream_share_its_scratch(dev):
+    """x.U and the product's operands lie in the stream's scratch: calls of several threads must not mix there."""
+    import threading
+    work = []
+    for i, B in enumerate((1, 40, 7, 300)):
+        lin = cases.to_b200_linear(cases.make_linear(50 + i, 256, 512, rank=32), dev)
+        x = cases.make_x(60 + i, B, 512).to(dev)
+        work.append((lin, x, lin(x)))
+    wrong = []
+
+    def many(lin, x, ref):
+        for _ in range(100):
+            if not torch.equal(lin(x), ref):
+                wrong.append(x.shape)
+    threads = [threading.Thread(target=many, args=w) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
