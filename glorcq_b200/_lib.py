@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 # GLQ_LIB selects another build of the same ABI (e.g. one compiled with -DGLQ_CHECKED)
 LIB_PATH = os.environ.get("GLQ_LIB") or os.path.join(HERE, "libglorcq_b200.so")
 
-FMT_Q2, FMT_Q4, FMT_T2, FMT_F16 = 0, 1, 2, 3
+FMT_Q2, FMT_Q4, FMT_T2, FMT_F16, FMT_Q3 = 0, 1, 2, 3, 4
 EPI_LINEAR, EPI_SWIGLU = 0, 1
 
 vp = C.c_void_p

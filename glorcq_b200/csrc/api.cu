@@ -56,10 +56,12 @@ extern "C" int glq_last_cuda_error(void) { return g_last_cuda_error; }
 // ---------------------------------------------------------------------------------------------
 // tiled layout sizes
 // ---------------------------------------------------------------------------------------------
+static inline int tile_fmt(int fmt) { return fmt == GLQ_FMT_Q3 ? GLQ_FMT_Q4 : fmt; }
 static inline int fmt_kb(int fmt) { return (fmt == GLQ_FMT_Q2 || fmt == GLQ_FMT_T2) ? 128 : 64; }
 static inline int dest_pairs(int n_rows, int count) { return (cdiv(n_rows, 16) * count + 1) / 2; }
 
 extern "C" size_t glq_tiled_bytes(int fmt, int n_rows, int K, int count) {
+    fmt = tile_fmt(fmt);
     if (fmt < 0 || fmt > 2 || n_rows <= 0 || K <= 0 || count < 1 || count > 2) return 0;
     return (size_t)dest_pairs(n_rows, count) * cdiv(K, fmt_kb(fmt)) * 2 * block_bytes_of(fmt);
 }
@@ -99,6 +101,7 @@ static int num_sms() {
 
 static int plan_geometry(int fmt, int epilogue, int N, int K, int group_size, int n_problems, int max_rows,
                          bool allow_split, Geometry* out) {
+    fmt = tile_fmt(fmt);
     if (fmt < 0 || fmt > 3 || N <= 0 || K <= 0 || n_problems <= 0 || max_rows <= 0) return GLQ_ERR_ARG;
     Geometry g{};
     g.nw = (epilogue == GLQ_EPI_SWIGLU) ? 2 : 1;
@@ -208,7 +211,7 @@ static int launch_skinny(int fmt, bool rowmajor, const SkinnyParams& p, const Ge
         if (fmt != GLQ_FMT_T2) return GLQ_ERR_UNSUPPORTED;
         return launch_fmt<GLQ_FMT_T2, true>(p, g, (int)grid, st);
     }
-    switch (fmt) {
+    switch (tile_fmt(fmt)) {
         case GLQ_FMT_Q2: return launch_fmt<GLQ_FMT_Q2, false>(p, g, (int)grid, st);
         case GLQ_FMT_Q4: return launch_fmt<GLQ_FMT_Q4, false>(p, g, (int)grid, st);
         case GLQ_FMT_T2: return launch_fmt<GLQ_FMT_T2, false>(p, g, (int)grid, st);
@@ -281,6 +284,8 @@ static int stream_splits(size_t base, size_t stage, int nt, int npairs, int unit
 static bool plan_stream(int fmt, int epilogue, int N, int K, int rank, int group_size, int n_problems, int max_rows,
                         StreamGeom* out, int chunks = 1) {
     if (stream_disabled()) return false;
+    const bool exact = fmt == GLQ_FMT_Q3;
+    fmt = tile_fmt(fmt);
     if (fmt != GLQ_FMT_Q2 && fmt != GLQ_FMT_Q4 && fmt != GLQ_FMT_T2) return false;
     if (N <= 0 || K <= 0 || n_problems <= 0 || max_rows <= 0 || rank < 0 || rank % 16 != 0) return false;
     StreamGeom g{};
@@ -293,7 +298,7 @@ static bool plan_stream(int fmt, int epilogue, int N, int K, int rank, int group
         group_blocks = group_size / kb;
     }
     int rows;
-    if (max_rows <= 8 && !i8_disabled()) {
+    if (max_rows <= 8 && !exact && !i8_disabled()) {
         g.i8 = 1;
         g.nt = max_rows <= 4 ? 1 : 2;
         rows = 4 * g.nt;
@@ -401,6 +406,28 @@ static int launch_stream_fmt(const StreamParams& sp, const StreamGeom& g, cudaSt
     return launch_stream_one<FMT, false, 4>(sp, g, st);
 }
 
+// Rows of a chunk when a product with host-known counts is cut into chunks of its rows, the slots of ONE launch of the
+// streaming kernel; 0 when it is not.
+// 9..32 rows: the integer path stages at most 8 rows (4 when the staged activations of a long reduction leave no room for 8)
+// and streams at a multiple of the fp16 path's rate for many rows (a launch per chunk took 17.7 us for each 8 of 16 rows of a
+// 4-bit 4096 x 4096); the chunks read the weights at about the same time, once from memory and then from L2.
+// (Codebook rows: the fp16 path rounds the levels to fp16.  Error against 64 bits, 9..32 tokens of a 60-expert block behind its
+// Hadamard rotation: 0.82-0.83e-3, fp16 path 0.86-0.94e-3; with 1 in 200 input values 50 times larger 0.75-0.80, 0.79-0.84.)
+// GLQ_FMT_Q3: any number of rows, on the fp16 path.  8 rows take the integer path's time (4096 x 4096: 16.8 us both), 32 rows of
+// 2048 x 2048 21 us instead of 13, 512 rows 111 instead of 210 in launches of 32; error against 64 bits 2.07e-4, the rounding
+// of the result, where block fixed point gives 2.12e-4 and 3.3e-4 with 1 in 200 activations 50 times larger.
+static int plan_chunks(const glq_mm_args_t* a, StreamGeom* sg) {
+    const bool exact = a->fmt == GLQ_FMT_Q3;
+    if (a->slot_count || a->slot_offset || a->slot_index || a->max_rows <= 8 || a->fmt == GLQ_FMT_F16 ||
+        (!exact && (a->max_rows > 32 || i8_disabled())))
+        return 0;
+    for (int c : {8, 4})
+        if (plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, c, sg, cdiv(a->max_rows, c)) &&
+            (exact || sg->i8))
+            return c;
+    return 0;
+}
+
 static int launch_stream(const glq_mm_args_t* a, SkinnyParams& p, const StreamGeom& g, cudaStream_t st, bool a_late = false, bool dependent = false, int cnt_lo = 0,
                          int cnt_hi = 0x7fffffff) {
     const int fmt = a->fmt, N = a->N, K = a->K, rank = a->rank, n_problems = a->n_problems;
@@ -440,7 +467,7 @@ static int launch_stream(const glq_mm_args_t* a, SkinnyParams& p, const StreamGe
     // a concurrent stream runs grouped products too: two thirds of the CTA slots, so that its kernels find room
     // (measured on the MoE block: the shared expert's branch beside the routed experts')
     if (t_share_sm && gl.grid > 4 * num_sms() / 3) gl.grid = 4 * num_sms() / 3;
-    switch (fmt) {
+    switch (tile_fmt(fmt)) {
         case GLQ_FMT_Q2: return launch_stream_fmt<GLQ_FMT_Q2>(sp, gl, st);
         case GLQ_FMT_Q4: return launch_stream_fmt<GLQ_FMT_Q4>(sp, gl, st);
         case GLQ_FMT_T2: return launch_stream_fmt<GLQ_FMT_T2>(sp, gl, st);
@@ -679,7 +706,7 @@ extern "C" size_t glq_mm_workspace_bytes(const glq_mm_args_t* a) {
     TcGeom tg;
     if (plan_tc(a, &tg)) return tg.xp_bytes;
     StreamGeom sg;
-    if (plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, a->max_rows, &sg)) return 0;
+    if (plan_chunks(a, &sg) || plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, a->max_rows, &sg)) return 0;
     Geometry g;
     if (plan_geometry(a->fmt, a->epilogue, a->N, a->K, a->group_size, a->n_problems, a->max_rows, true, &g) != GLQ_OK)
         return 0;
@@ -691,7 +718,7 @@ extern "C" size_t glq_mm_counters(const glq_mm_args_t* a) {
     TcGeom tg;
     if (plan_tc(a, &tg)) return 0;
     StreamGeom sg;
-    if (plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, a->max_rows, &sg)) return 0;
+    if (plan_chunks(a, &sg) || plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, a->max_rows, &sg)) return 0;
     Geometry g;
     if (plan_geometry(a->fmt, a->epilogue, a->N, a->K, a->group_size, a->n_problems, a->max_rows, true, &g) != GLQ_OK)
         return 0;
@@ -725,21 +752,11 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
     // more than 32 rows per slot, else to the fp16 path with four tiles.  Each class is one launch that
     // skips the slots of the others.
     StreamGeom sg8, sg16;
-    // 9..32 rows, counts known on the host: the integer path stages at most 8 rows (4 when the staged activations of a long
-    // reduction leave no room for 8) and streams at a multiple of the fp16 path's rate, so the rows are cut into chunks, the
-    // slots of ONE launch (a launch per chunk took 17.7 us for each 8 of 16 rows of a 4-bit 4096 x 4096); the chunks read
-    // the weights at about the same time, once from memory and then from L2.
-    int cap = use_tc ? 16 : std::min(a->max_rows, 32);
-    bool chunked = false;
-    if (!use_tc && !a->slot_count && !a->slot_offset && !a->slot_index && a->max_rows > 8 && a->max_rows <= 32 && !i8_disabled() &&
-        a->fmt != GLQ_FMT_F16)
-        for (int c : {8, 4})
-            if (!chunked && plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, c, &sg, cdiv(a->max_rows, c)) &&
-                sg.i8) {
-                chunked = true;
-                cap = c;
-            }
-    bool use_stream = chunked || plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, cap, &sg);
+    const int chunk = use_tc ? 0 : plan_chunks(a, &sg);
+    const int cap = chunk ? chunk : use_tc ? 16 : std::min(a->max_rows, 32);
+    // (more rows than a slot of the streaming kernel holds, and no other kernel for them: the general one)
+    const bool use_stream = chunk || ((use_tc || a->max_rows <= cap) &&
+                                      plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, cap, &sg));
     const bool classes = use_stream && a->slot_count != nullptr && a->max_rows > 8 && !hybrid_disabled();
     const bool split8 = classes && plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, 8, &sg8) &&
                         sg8.i8;
@@ -784,7 +801,7 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
     p.rows_stride = a->rows_stride > 0 ? a->rows_stride : a->max_rows;
     p.epilogue = a->epilogue;
     p.x_vec = (aligned16(a->x) && a->ldx % 8 == 0) ? 1 : 0;
-    if (chunked) p.max_rows = cap;
+    if (chunk) p.max_rows = chunk;
     if (use_stream) {
         cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
         const bool a_late = (a->flags & GLQ_MM_A_FROM_PREVIOUS_LAUNCH) != 0, dep = (a->flags & GLQ_MM_AFTER_KERNEL) != 0;
@@ -1172,6 +1189,7 @@ extern "C" int glq_pack_f16(const void* W, long stride_n, long stride_k, int N, 
 extern "C" int glq_dequant_tiled(int fmt, const void* tiled, const float* norms_tiled, const float* centroids, int N,
                                  int K, int slot, int count, void* out, void* stream) {
     if (!tiled || !out || N <= 0 || K <= 0 || !slot_ok(slot, count)) return GLQ_ERR_ARG;
+    fmt = tile_fmt(fmt);
     const size_t elems = (size_t)N * K;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (fmt == GLQ_FMT_Q2 || fmt == GLQ_FMT_Q4) {

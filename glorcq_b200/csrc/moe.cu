@@ -857,7 +857,7 @@ extern "C" int glq_moe_forward_ep(const glq_moe_desc_t* d, const void* x, int n,
     const size_t px_half = px ? px->half_elems : 0;
     if (ep_world > 1 && (phase == GLQ_MOE_PHASE_ALL || !ep->entry_out)) return GLQ_ERR_ARG;   // the exchange is the caller's
     if (n == 0) return GLQ_OK;
-    if (d->top_k < 1 || d->top_k > 16 || d->E < d->top_k || d->E > 256 || d->H % 8 != 0 || d->I % 8 != 0)
+    if (d->fmt == GLQ_FMT_Q3 || d->top_k < 1 || d->top_k > 16 || d->E < d->top_k || d->E > 256 || d->H % 8 != 0 || d->I % 8 != 0)
         return GLQ_ERR_UNSUPPORTED;
     const bool given = ep && ep->sel_in != nullptr;     // routing supplied by the caller: no router, no shared expert
     if (given && (!ep->weight_in || d->I_shared > 0 || router_logits)) return GLQ_ERR_ARG;

@@ -29,10 +29,10 @@ from .tiled import TiledWeight
 def _fuse_tiles(a: TiledWeight, b: TiledWeight) -> TiledWeight:
     """gate|up fused weight from two plain tiled weights of one shape: pair p = (tile p of a, tile p of b).
     Pure re-indexing of the already tiled buffers (load time)."""
-    if (a.fmt, a.N, a.K, a.group_size, a.rank) != (b.fmt, b.N, b.K, b.group_size, b.rank):
+    if (a.tile_fmt, a.N, a.K, a.group_size, a.rank) != (b.tile_fmt, b.N, b.K, b.group_size, b.rank):
         raise RuntimeError("gate_proj and up_proj must share format, shape, group size and rank")
     L = _lib.lib()
-    f = TiledWeight(a.fmt, a.N, a.K, a.group_size, 2, a.device)
+    f = TiledWeight(a.tile_fmt, a.N, a.K, a.group_size, 2, a.device)
     ntiles = (a.N + 15) // 16
     bb = 512 if a.fmt == FMT_T2 else 576
     nkb = a.codes.numel() // (((ntiles + 1) // 2) * 2 * bb)
@@ -114,17 +114,20 @@ class GraphCompatibleMoeBlock(nn.Module):
             for lin in (g, u, dn):
                 if getattr(lin, "_tiled", None) is None:
                     raise RuntimeError("every expert projection must be a GLoRCQLinear in the tiled layout "
-                                       "(2/4-bit codes with group size 128/64 multiples, or 2-bit codebook)")
+                                       "(2-bit codes with a group size that is a multiple of 128, 3- or 4-bit codes with one "
+                                       "that is a multiple of 64, or the 2-bit codebook)")
         g0, _, d0 = lins[mine[0]]
         H, I = g0.in_features, g0.out_features
-        fmt, gs = g0._tiled.fmt, g0._tiled.group_size
+        # 3-bit codes are the block's 4-bit codes: its kernels take activations as block fixed point up to 32 rows of an
+        # expert and fp16((q - z) s) above, as for every format (a layer of its own keeps 3-bit codes unrounded)
+        fmt, gs = g0._tiled.tile_fmt, g0._tiled.group_size
         rank = g0._tiled.rank
         gate_up, down, utg, utu, utd = ([Weight() for _ in range(E)] for _ in range(5))
         rm_gu, rm_d = [0] * (2 * E), [0] * E     # row-major U^T of the persistent decode kernel
         for e, (g, u, dn) in lins.items():
             f = _fuse_tiles(g._tiled, u._tiled)
             if (f.fmt, f.group_size, f.rank, f.N, f.K) != (fmt, gs, rank, I, H) or \
-                    (dn._tiled.fmt, dn._tiled.group_size, dn._tiled.rank, dn._tiled.N, dn._tiled.K) != (fmt, gs, rank, H, I):
+                    (dn._tiled.tile_fmt, dn._tiled.group_size, dn._tiled.rank, dn._tiled.N, dn._tiled.K) != (fmt, gs, rank, H, I):
                 raise RuntimeError("all experts of a block must share format, group size, rank and shapes")
             self._keep += [f, dn._tiled]
             gate_up[e] = f.desc

@@ -72,10 +72,11 @@ class GLoRCQLinear(nn.Module):
     def load_gptq(self, packed_data, device="cuda", keep_raw=False, check_range=True):
         """Integer codes + per-group scale/zero.  2-, 3- and 4-bit codes with a group size that is a
         multiple of 128 (64 for 3- and 4-bit) are re-tiled for the fused kernel; anything else keeps the
-        (N,K) codes and runs through the int8 drop-in kernel.  3-bit codes take the 4-bit fields: half the
-        bytes of the int8 codes, and one launch where the int8 route needs six (2 rows of 2048 x 2048 with
-        rank 64: 117 -> 26 us per eager call).  Their range is checked whatever `check_range` says: codes
-        outside it (the int8 kernel takes any int8 value) keep the int8 route."""
+        (N,K) codes and runs through the int8 drop-in kernel.  3-bit codes take the 4-bit fields, half the
+        bytes of the int8 codes, and are multiplied as exactly as by the int8 kernel (GLQ_FMT_Q3): two launches where
+        that route needs six (2048 x 2048 with rank 64, eager: 2 rows 108 -> 10 us, 512 rows 5656 -> 111).  Their
+        range is checked whatever `check_range` says: codes outside it (the int8 kernel takes any int8 value) keep
+        the int8 route."""
         self.quant_type = "gptq"
         q = packed_data["qweight_int"].to(device)
         self.scales = packed_data["scales"].to(device).to(torch.float16)
@@ -204,7 +205,7 @@ class GLoRCQLinear(nn.Module):
                 signs = self._rht_signs
                 if signs is not None and signs.dtype is torch.float32 and signs.is_cuda:
                     return tiled.linear_forward(t, x, self._ut, None, signs)
-            elif self.gptq_bits != 3 or x.numel() <= 32 * self.in_features:
+            else:
                 return tiled.linear_forward(t, x, self._ut)
         orig_shape = x.shape
         in_dtype = x.dtype
@@ -220,13 +221,8 @@ class GLoRCQLinear(nn.Module):
         if self._tiled is None and self._dense is not None:
             y = self._forward_dense(x, a)
         elif self.quant_type == "gptq":
-            if self._tiled is not None and (self.gptq_bits != 3 or x.shape[0] <= 32):
+            if self._tiled is not None:
                 y = tiled.linear_forward(self._tiled, x, ut=self._ut, a=a)
-            elif self._tiled is not None:
-                # 3-bit codes stay on the integer product, which keeps (q - z) * s unrounded as the int8 kernel does
-                # (the GEMM above 32 rows rounds it to fp16): 32 rows at a time
-                y = torch.cat([tiled.linear_forward(self._tiled, x[i:i + 32], ut=self._ut, a=None if a is None else a[i:i + 32])
-                               for i in range(0, x.shape[0], 32)])
             else:
                 y = gptq_dequant_matmul_fused(x, self.qweight_int, self.scales, self.zeros,
                                               self.gptq_groupsize, self.gptq_sym, lora_USV=None)

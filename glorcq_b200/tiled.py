@@ -15,7 +15,7 @@ from typing import Dict, Optional, Tuple
 import torch
 
 from . import _lib
-from ._lib import FMT_F16, FMT_Q2, FMT_Q4, FMT_T2, Weight
+from ._lib import FMT_F16, FMT_Q2, FMT_Q3, FMT_Q4, FMT_T2, Weight
 
 
 def _stream_ptr(device) -> int:
@@ -125,11 +125,11 @@ class TiledWeight:
         kb = 128 if bits == 2 else 64
         if groupsize <= 0 or groupsize % kb != 0:
             raise RuntimeError(f"group size {groupsize} must be a positive multiple of {kb} for {bits}-bit codes")
-        return FMT_Q2 if bits == 2 else FMT_Q4
+        return {2: FMT_Q2, 3: FMT_Q3, 4: FMT_Q4}[bits]
 
     @classmethod
     def from_gptq(cls, qweight_int, scales, zeros, bits, groupsize, sym=False):
-        """(N,K) int32 codes in [0, 2^bits) + (N,G) fp16 scales/zeros -> Q2 / Q4 tiles."""
+        """(N,K) int32 codes in [0, 2^bits) + (N,G) fp16 scales/zeros -> Q2 / Q3 / Q4 tiles."""
         fmt = cls._gptq_fmt(bits, groupsize)
         N, K = qweight_int.shape
         self = cls(fmt, N, K, groupsize, 1, qweight_int.device)
@@ -162,6 +162,11 @@ class TiledWeight:
                                                _stream_ptr(W.device)), "pack_f16")
         return self
 
+    @property
+    def tile_fmt(self):
+        """The layout alone: Q3 is Q4 tiles whose products are taken unrounded."""
+        return FMT_Q4 if self.fmt == FMT_Q3 else self.fmt
+
     # ---- descriptor ---------------------------------------------------------------------------
     @property
     def desc(self) -> Weight:
@@ -190,7 +195,7 @@ class TiledWeight:
 
     # ---- checks ------------------------------------------------------------------------------
     def dequantize(self, slot: int = 0) -> torch.Tensor:
-        """Dequantised (N,K) weights of the matrix in `slot`: fp16 for Q2/Q4, fp32 for T2."""
+        """Dequantised (N,K) weights of the matrix in `slot`: fp16 for Q2/Q3/Q4, fp32 for T2."""
         L = _lib.lib()
         dt = torch.float32 if self.fmt == FMT_T2 else torch.float16
         out = torch.empty(self.N, self.K, dtype=dt, device=self.device)

@@ -35,6 +35,10 @@ extern "C" {
 #define GLQ_FMT_Q4 1  /* 4-bit integer codes, fp16 scale and zero per (row, group)       */
 #define GLQ_FMT_T2 2  /* 2-bit codebook indices, fp32 norm per row, 4-entry fp32 codebook */
 #define GLQ_FMT_F16 3 /* dense fp16                                                        */
+/* The tiles of Q4, multiplied as they are: activations stay fp16 and (q - z) s is never rounded, whatever the row count,
+ * where Q4 takes 16-bit block fixed point for up to 32 rows and fp16 weights above.  For codes that had neither before
+ * (3-bit codes: the int8 kernel's arithmetic).  Not taken by glq_moe_forward, whose experts are Q4 then. */
+#define GLQ_FMT_Q3 4
 
 /* epilogues of glq_grouped_matmul */
 #define GLQ_EPI_LINEAR 0 /* y = fp16(fp16(q-part) + fp16(low-rank part)) [* entry scale] [+ bias] */
@@ -127,7 +131,7 @@ size_t glq_tiled_bytes(int fmt, int n_rows, int K, int count);       /* codes (+
 size_t glq_sv_bytes(int n_rows, int rank, int count);                /* packed SV buffer         */
 size_t glq_rows_f32_count(int n_rows, int count);                    /* floats of a tile-ordered row vector */
 
-/* codes (N,K) int32 in [0, 2^bits), scales/zeros (N,G) fp16 (zeros NULL: symmetric) -> Q2 / Q4 */
+/* codes (N,K) int32 in [0, 2^bits), scales/zeros (N,G) fp16 (zeros NULL: symmetric) -> Q2 / Q4 (Q3: as 4-bit codes) */
 int glq_pack_gptq(const int32_t* q, const void* scales, const void* zeros, int bits, int N, int K, int group_size,
                   void* tiled, int slot, int count, void* stream);
 /* packed (N,K/4) uint8 2-bit indices -> T2 */
@@ -162,7 +166,7 @@ int glq_dequant_tiled(int fmt, const void* tiled, const float* norms_tiled, cons
  * ------------------------------------------------------------------------------------------ */
 typedef struct glq_mm_args {
     int32_t fmt;         /* GLQ_FMT_* */
-    int32_t group_size;  /* Q2: multiple of 128; Q4: multiple of 64; others ignored */
+    int32_t group_size;  /* Q2: multiple of 128; Q3, Q4: multiple of 64; others ignored */
     int32_t epilogue;    /* GLQ_EPI_* */
     int32_t n_problems;  /* slots covered by the grid */
     int32_t max_rows;    /* upper bound of rows per slot (sizes shared memory and passes) */

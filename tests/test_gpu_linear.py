@@ -135,6 +135,30 @@ def test_integer_path_hostile_activations(dev, N, K, bits, B):
         assert cases.rel_l2(y[b], ref[b]) <= REL, f"row {b}"
 
 
+@pytest.mark.parametrize("B", [1, 8, 9, 33, 300])
+@pytest.mark.parametrize("N,K,gs", [(2048, 2048, 128), (1000, 768, 64), (72, 14336, 128), (72, 24576, 128)])
+def test_3bit_layers_round_their_result_only(dev, N, K, gs, B):
+    """3-bit codes are multiplied as the int8 kernel does it: fp16 activations and unrounded (q - z) s, alone and in a group
+    of layers, on both sides of 32 rows.  What is left is one fp16 rounding of the result: 2.1e-4 for results that are
+    normal values (a uniform error of half a unit over their binades), 2.3e-4 with 8 % for the spread over a few thousand
+    results; block fixed point adds 2e-4 and more on these rows, an fp16 weight 2e-4.  (14336: chunks of four rows,
+    24576: the general kernel.)"""
+    from glorcq_b200 import tiled
+    d = cases.make_linear(N + K + B, N, K, bits=3, groupsize=gs, with_lora=False)
+    lin = cases.to_b200_linear(d, dev)
+    x = (_hostile_rows(B, K, 70 + B) * 0.03125).to(dev)
+    q, s, z = (d[k].to(dev).double() for k in ("qweight_int", "scales", "zeros"))
+    W = ((q - z.repeat_interleave(gs, 1)[:, :K]) * s.repeat_interleave(gs, 1)[:, :K])
+    ref = x.double() @ W.T
+    assert float(ref.abs().max()) < 60000
+    err = lambda y: float((y.double() - ref).norm() / ref.norm())
+    bar = 2.3e-4 * (1 + 1.5 / (N * B) ** 0.5)
+    assert err(lin(x)) <= bar
+    both = tiled.GroupedLinear([lin._tiled, lin._tiled], None).forward(x)
+    assert err(both[0]) <= bar and torch.equal(both[0], both[1])
+    assert tiled.debug_error() is None
+
+
 @pytest.mark.parametrize("N,K,rank,B,int_zeros", [(1408, 2048, 64, 128, True), (2048, 1408, 64, 300, True),
                                                    (100, 392, 16, 200, True), (256, 256, 16, 64, False),
                                                    (24, 128, 0, 40, True), (5632, 2048, 64, 96, True)])

@@ -53,6 +53,14 @@ def test_no_shared_expert_and_top8(dev, N):
     assert cases.rel_l2(y, ref) <= REL_BLOCK
 
 
+@pytest.mark.parametrize("N", [1, 9, 150])
+def test_3bit_block(dev, N):
+    """3-bit experts are 4-bit codes to the block: persistent kernel, streaming products, tensor-core products."""
+    blk = cases.make_moe(37, 256, 128, 6, 2, I_shared=256, rank=16, experts_per_cluster=2, bits=3)
+    mb, y, logits, ref, _ = _run(blk, N, dev, 1037)
+    assert cases.rel_l2(y, ref) <= REL_BLOCK
+
+
 @pytest.mark.parametrize("N", [1, 7, 150])
 def test_codebook_format_block(dev, N):
     blk = cases.make_moe(35, 256, 128, 6, 2, I_shared=256, rank=16, experts_per_cluster=2, fmt="turbo")
