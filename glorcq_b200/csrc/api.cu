@@ -640,21 +640,22 @@ static void fill_tc_operands(const glq_mm_args_t* a, TcParams& p) {
 }
 
 // Dense products with few columns (xu_mm.cuh).  Above 32 rows, where the order of the sums is the tcgen05 kernel's.  Up to 512
-// columns: every 64-column slice reads x again (from L2), and a wide W fills the tcgen05 kernel's tiles.
+// columns: every 64-column slice reads x again (from L2), and a wide W fills the tcgen05 kernel's tiles.  Nothing of x itself
+// decides, so that the workspace query, which may come before there is an x, gives the answer of the call.
 static bool xu_takes(const glq_mm_args_t* a) {
     return a->fmt == GLQ_FMT_F16 && a->max_rows > 32 && a->N > 0 && a->N <= 512 && a->K > 0 && a->K % 8 == 0 && a->n_problems > 0 &&
-           a->epilogue == GLQ_EPI_LINEAR && !a->entry_scale && !(a->rank > 0 && a->a0) && aligned16(a->x) && a->ldx % 8 == 0;
+           a->epilogue == GLQ_EPI_LINEAR && !a->entry_scale && !(a->rank > 0 && a->a0);
 }
 
-template <int NT>
+template <int NT, bool VEC>
 static int launch_xu_t(TcParams& p, const glq_mm_args_t* a, cudaStream_t st) {
     using C = XuCfg<NT>;
     static bool configured[64] = {};
-    const int rc = allow_smem(xu_kernel<NT>, configured, C::SMEM);
+    const int rc = allow_smem(xu_kernel<NT, VEC>, configured, C::SMEM);
     if (rc != GLQ_OK) return rc;
     const bool one = a->n_problems == 1 && !a->slot_offset && !a->n_slots;
     p.tiles_max = one ? cdiv(a->max_rows, C::ROWS) : (int)(total_entries(a) / C::ROWS + a->n_problems + 1);
-    xu_kernel<NT><<<dim3(p.tiles_max, cdiv(a->N, kXuCols)), kXuThreads, C::SMEM, st>>>(p);
+    xu_kernel<NT, VEC><<<dim3(p.tiles_max, cdiv(a->N, kXuCols)), kXuThreads, C::SMEM, st>>>(p);
     GLQ_CUDA(cudaGetLastError());
     return GLQ_OK;
 }
@@ -665,7 +666,8 @@ static int launch_xu(const glq_mm_args_t* a, cudaStream_t st) {
     p.nkb = cdiv(a->K, 64);
     // 64 rows per CTA read W half as often; 32 where the smaller tiles still leave CTA slots free
     const long long total = total_entries(a), tiles = std::max(total / 32, std::min<long long>(a->n_problems, total));
-    return tiles * cdiv(a->N, kXuCols) > 3 * num_sms() ? launch_xu_t<8>(p, a, st) : launch_xu_t<4>(p, a, st);
+    if (tiles * cdiv(a->N, kXuCols) > 3 * num_sms()) return p.x_vec16 ? launch_xu_t<8, true>(p, a, st) : launch_xu_t<8, false>(p, a, st);
+    return p.x_vec16 ? launch_xu_t<4, true>(p, a, st) : launch_xu_t<4, false>(p, a, st);
 }
 
 // output of the x.U product that this thread launched last, if xu_kernel took it and no other product has come since
@@ -702,7 +704,7 @@ static int launch_tc(const glq_mm_args_t* a, const TcGeom& g, cudaStream_t st, c
 }
 
 extern "C" size_t glq_mm_workspace_bytes(const glq_mm_args_t* a) {
-    if (!a) return 0;
+    if (!a || xu_takes(a)) return 0;
     TcGeom tg;
     if (plan_tc(a, &tg)) return tg.xp_bytes;
     StreamGeom sg;

@@ -38,7 +38,7 @@ struct MoeLayout {
     size_t active2, n_active2, slot_count2, slot_offset2;   // gate and up x.U as one launch: 2E slots
     size_t plan_blk;                                        // per-block expert counts of the many-token plan
     size_t a_gu, h, b, yd, a_sg, a_su, hs, bs, ysh, xr, hr, hsr, mm, mm2;
-    size_t total, mm_bytes, mm_counters;
+    size_t total, mm_bytes, mm2_bytes, mm_counters;
 };
 
 // Rows per problem slot of the routed products.  With 9 or more tokens but few rows per expert on
@@ -110,37 +110,52 @@ MoeLayout moe_layout(const glq_moe_desc_t* d, int n) {
     if (d->rot_in || d->rht_in) L.xr = take((size_t)n * d->H * 2);
     if (d->rot_mid || d->rht_mid) L.hr = take(nk * d->I * 2);
     if ((d->sh_rot_mid || d->sh_rht_mid) && d->I_shared > 0) L.hsr = take((size_t)n * d->I_shared * 2);
-    // scratch / counters of the matmul calls: they run one after the other, so they share
+    // scratch / counters of the matmul calls: those of a branch run one after the other, so they share.  The shared expert's
+    // branch may run on a second stream (mm2); without one its calls take the first branch's scratch
     const int P = moe_slots(d, n);
     const int rows = moe_chunk(d, n) ? std::min(n, moe_chunk(d, n)) : n;   // rows per routed slot
     glq_mm_args_t m;
-    size_t wb = 0, wc = 0;
+    size_t wb = 0, wb2 = 0, wc = 0;
+    bool shared = false;
     auto acc = [&]() {
-        wb = std::max(wb, glq_mm_workspace_bytes(&m));
+        const size_t b = glq_mm_workspace_bytes(&m);
+        wb = std::max(wb, b);
+        if (shared) wb2 = std::max(wb2, b);
         wc = std::max(wc, glq_mm_counters(&m));
     };
     set_mm(&m, GLQ_FMT_F16, 0, GLQ_EPI_LINEAR, 1, n, d->dense0_rows, d->H, 0); acc();
     if (d->rot_in) { set_mm(&m, GLQ_FMT_F16, 0, GLQ_EPI_LINEAR, 1, n, d->H, d->H, 0); acc(); }
     if (d->rot_mid) { set_mm(&m, GLQ_FMT_F16, 0, GLQ_EPI_LINEAR, 1, (int)nk, d->I, d->I, 0); acc(); }
-    if (d->sh_rot_mid && d->I_shared > 0) { set_mm(&m, GLQ_FMT_F16, 0, GLQ_EPI_LINEAR, 1, n, d->I_shared, d->I_shared, 0); acc(); }
+    // the routed products are planned by the entries of all slots together, as their calls are: the slot arrays' presence says
+    // so (nothing is read here)
+    static const int32_t present = 0;
+    auto acc_routed = [&]() {
+        m.slot_index = m.slot_count = m.slot_offset = &present;
+        acc();
+    };
     if (d->rank > 0) {
-        set_mm(&m, GLQ_FMT_F16, 0, GLQ_EPI_LINEAR, 2 * P, rows, d->rank, d->H, 0, (int)(2 * nk)); acc();
-        set_mm(&m, GLQ_FMT_F16, 0, GLQ_EPI_LINEAR, P, rows, d->rank, d->I, 0, (int)nk); acc();
+        set_mm(&m, GLQ_FMT_F16, 0, GLQ_EPI_LINEAR, 2 * P, rows, d->rank, d->H, 0, (int)(2 * nk)); acc_routed();
+        set_mm(&m, GLQ_FMT_F16, 0, GLQ_EPI_LINEAR, P, rows, d->rank, d->I, 0, (int)nk); acc_routed();
     }
-    set_mm(&m, d->fmt, d->group_size, GLQ_EPI_SWIGLU, P, rows, d->I, d->H, d->rank, (int)nk); acc();
-    set_mm(&m, d->fmt, d->group_size, GLQ_EPI_LINEAR, P, rows, d->H, d->I, d->rank, (int)nk); acc();
+    set_mm(&m, d->fmt, d->group_size, GLQ_EPI_SWIGLU, P, rows, d->I, d->H, d->rank, (int)nk); acc_routed();
+    set_mm(&m, d->fmt, d->group_size, GLQ_EPI_LINEAR, P, rows, d->H, d->I, d->rank, (int)nk); acc_routed();
     if (d->I_shared > 0) {
+        shared = true;
+        if (d->sh_rot_mid) { set_mm(&m, GLQ_FMT_F16, 0, GLQ_EPI_LINEAR, 1, n, d->I_shared, d->I_shared, 0); acc(); }
         if (d->rank > 0) {
             set_mm(&m, GLQ_FMT_F16, 0, GLQ_EPI_LINEAR, 1, n, d->rank, d->H, 0); acc();
             set_mm(&m, GLQ_FMT_F16, 0, GLQ_EPI_LINEAR, 1, n, d->rank, d->I_shared, 0); acc();
         }
-        set_mm(&m, d->fmt, d->group_size, GLQ_EPI_SWIGLU, 1, n, d->I_shared, d->H, d->rank); acc();
-        set_mm(&m, d->fmt, d->group_size, GLQ_EPI_LINEAR, 1, n, d->H, d->I_shared, d->rank); acc();
+        for (int r : {0, (int)d->rank}) {            // without a low-rank term of its own the tiles may be others
+            set_mm(&m, d->fmt, d->group_size, GLQ_EPI_SWIGLU, 1, n, d->I_shared, d->H, r); acc();
+            set_mm(&m, d->fmt, d->group_size, GLQ_EPI_LINEAR, 1, n, d->H, d->I_shared, r); acc();
+        }
     }
     L.mm_bytes = up256(wb);
     L.mm_counters = wc;
     L.mm = take(L.mm_bytes);
-    L.mm2 = take(L.mm_bytes);   // the shared expert's branch may run concurrently on a second stream
+    L.mm2_bytes = up256(wb2);
+    L.mm2 = take(L.mm2_bytes);
     L.total = off;
     return L;
 }
@@ -966,7 +981,7 @@ extern "C" int glq_moe_forward_ep(const glq_moe_desc_t* d, const void* x, int n,
         if (on_aux && forked && share_sm()) mm.flags |= GLQ_MM_SHARE_SM;      // the routed products run beside it
         after_kernel[on_aux ? 1 : 0] = true;
         mm.workspace = ws + (on_aux ? L.mm2 : L.mm);
-        mm.workspace_bytes = L.mm_bytes;
+        mm.workspace_bytes = on_aux ? L.mm2_bytes : L.mm_bytes;
         mm.counters = counters ? counters + (on_aux ? L.mm_counters : 0) : nullptr;
         mm.n_counters = L.mm_counters;
         return glq_grouped_matmul(&mm, on_aux && forked ? aux_stream : stream);

@@ -146,8 +146,9 @@ using ScratchMap = std::map<std::pair<int, cudaStream_t>, Scratch>;
 ScratchMap& g_scratch = *new ScratchMap;      // never destroyed: the process may end after the driver has gone
 
 // Scratch of calls larger than this is shared by all blocks on a stream: they run one after another, and a private
-// copy for every block and token count of a 32-layer model would not fit.
-constexpr size_t kSharedScratchFrom = 64u << 20;
+// copy for every block and prompt length would not fit.  16 MB lie between the calls that graphs capture (64 tokens of the
+// benchmark's models: 3 to 7 MB) and their prompts (512 tokens: 54 to 128 MB).
+constexpr size_t kSharedScratchFrom = 16u << 20;
 ScratchMap& g_big = *new ScratchMap;
 
 Scratch& scratch(int dev, cudaStream_t st, size_t nbytes, size_t nctr) {
@@ -497,13 +498,11 @@ PyObject* py_block(PyObject*, PyObject* const* a, Py_ssize_t n) {   // descripto
 // streams), and a workspace made by the warm-up call must be the one a later capture finds: an allocation inside a
 // capture would put its zero fill into the graph, once per replay.
 Scratch& block_scratch(Block* B, int64_t n, cudaStream_t st) {
-    auto it = B->scratch.find(n);
-    if (it != B->scratch.end()) return it->second;
     auto& nd = B->needs[n];
     if (!nd.first) nd = {api.glq_moe_workspace_bytes(B->d, (int)n) + 256, std::max<size_t>(api.glq_moe_counters(B->d, (int)n), 1)};
-    const auto opt = at::TensorOptions().device(at::kCUDA, B->device);
     const bool big = nd.first > kSharedScratchFrom && !capturing(st);
     Scratch& s = big ? g_big[{B->device, st}] : B->scratch[n];
+    const auto opt = at::TensorOptions().device(at::kCUDA, B->device);
     if (!s.ws.defined() || (size_t)s.ws.numel() < nd.first) {
         s.ws = at::Tensor();
         s.ws = at::empty({(int64_t)nd.first}, opt.dtype(at::kByte));

@@ -35,8 +35,9 @@ __device__ __forceinline__ void ldsm_x4(uint32_t a, uint32_t (&r)[4]) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a));
 }
 
+// VEC: rows of x start on 16-byte boundaries; others are loaded value by value.
 // grid = (row tiles, 64-column slices)
-template <int NT>
+template <int NT, bool VEC>
 __global__ void __launch_bounds__(kXuThreads) xu_kernel(const TcParams p) {
     using C = XuCfg<NT>;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -75,7 +76,16 @@ __global__ void __launch_bounds__(kXuThreads) xu_kernel(const TcParams p) {
                 for (int i = 0; i < NT / 2; ++i) {
                     const int r = (tid >> 3) + 16 * i;
                     const bool ok = in && src[i] != nullptr;
-                    cp_async16_zfill(dst + (uint32_t)(u * (C::X / 2) + r * 128 + (((tid & 7) ^ (r & 7)) << 4)), ok ? src[i] + k : p.x, ok ? 16 : 0);
+                    const uint32_t d = dst + (uint32_t)(u * (C::X / 2) + r * 128 + (((tid & 7) ^ (r & 7)) << 4));
+                    if constexpr (VEC) {
+                        cp_async16_zfill(d, ok ? src[i] + k : p.x, ok ? 16 : 0);
+                    } else {
+                        __align__(16) __half v[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) v[j] = ok ? __ldg(src[i] + k + j) : __float2half(0.f);
+                        const uint4 q = *reinterpret_cast<const uint4*>(v);
+                        sts128(d, q.x, q.y, q.z, q.w);
+                    }
                 }
 #pragma unroll
                 for (int m = 0; m < 4; ++m) {

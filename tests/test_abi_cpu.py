@@ -166,3 +166,23 @@ def test_native_group_refuses_rows_of_another_width(libpath, K):
         nat.grouped_linear(group, torch.zeros(2, K, dtype=torch.float16))
     with pytest.raises(RuntimeError, match="fp16 CUDA rows"):
         nat.grouped_linear(group, torch.zeros(2, 128, dtype=torch.float16))
+
+
+def test_workspace_of_products_with_few_columns(libpath):
+    """The x.U products of a prompt re-tile nothing: no workspace, whatever x will be; wider products need theirs."""
+    import ctypes as C
+    from glorcq_b200 import _lib
+    L = _lib.lib()
+    m = _lib.MMArgs()
+    m.fmt, m.n_problems, m.max_rows, m.rows_stride, m.N, m.K = _lib.FMT_F16, 1, 333, 333, 64, 4096
+    assert L.glq_mm_workspace_bytes(C.byref(m)) == 0
+    m.x, m.ldx = 2, 4097                        # not on 16-byte boundaries
+    assert L.glq_mm_workspace_bytes(C.byref(m)) == 0
+    m.N = 520
+    assert L.glq_mm_workspace_bytes(C.byref(m)) >= 333 * 4096 * 2
+    # a prompt through a block: the buffers of 512 x 4 entries (h, outputs, x.U: 19 MB; shared expert 9 MB) and one product's
+    # re-tiled rows (at most 2048 + 61 x 256 rows of 2304 channels), not those of 60 experts with 512 rows each
+    d = _lib.MoeDesc()
+    d.H, d.I, d.E, d.top_k, d.rank, d.fmt, d.group_size, d.router_rows, d.dense0_rows = 2048, 1408, 60, 4, 64, _lib.FMT_Q2, 128, 61, 192
+    d.I_shared = 5632
+    assert L.glq_moe_workspace_bytes(C.byref(d), 512) < (19 + 9 + 81 + 10) << 20

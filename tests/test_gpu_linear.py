@@ -380,6 +380,8 @@ def test_dense_few_columns(dev, N, K):
         y = tiled.dense_matmul(tw, x.to(dev))
         assert cases.rel_l2(y.cpu(), x.float() @ W.float().T) <= REL, B
         assert torch.equal(y, tiled.dense_matmul(tw, x.to(dev))), B
+        off = torch.empty(B * K + 1, dtype=torch.float16, device=dev)[1:].view(B, K).copy_(x)       # rows off 16-byte boundaries
+        assert torch.equal(y, tiled.dense_matmul(tw, off)), B
     assert tiled.debug_error() is None
 
 

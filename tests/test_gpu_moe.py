@@ -434,3 +434,20 @@ def test_qwen3_30b_a3b_block_shape(dev):
     assert cases.rel_l2(y, ref) <= REL_BLOCK
     from glorcq_b200 import tiled
     assert tiled.debug_error() is None
+
+
+@pytest.mark.parametrize("N", [33, 64, 100, 129, 200, 257, 400, 515, 700])
+def test_scratch_of_a_prompt_is_planned_as_its_products_are(dev, N):
+    """The workspace query plans each product before its operands exist; a block whose shared expert has no low-rank
+    term plans that one's tiles without it.  A query that asked for less than a launch needs would be refused."""
+    blk = cases.make_moe(600, 256, 384, 8, 2, I_shared=640, rank=64, experts_per_cluster=3)
+    for p in blk["shared_expert"].values():
+        p.pop("U"), p.pop("SV")
+    mb, y, logits, ref, ref_logits = _run(blk, N, dev, 1600 + N)
+    # a token whose second and third logit lie within a rounding of each other may go to either expert
+    sel = mb.last_selected_experts.cpu().long().sort(1).values
+    ref_sel = O.route(cases.to_oracle_moe(blk), cases.make_x(1600 + N, N, 256))[2].sort(1).values
+    same = (sel == ref_sel).all(1)
+    top = ref_logits.view(N, -1).float().topk(3, 1).values
+    assert ((top[~same, 1] - top[~same, 2]) <= 2.0 ** -10 * top[~same, 1].abs()).all()
+    assert int(same.sum()) >= N - 2 and cases.rel_l2(y.view(N, -1)[same], ref.view(N, -1)[same]) <= REL_BLOCK
