@@ -138,12 +138,16 @@ bool capturing(cudaStream_t st) {
 // ---- scratch of a stream -------------------------------------------------------------------------------------
 // One scratch buffer and one array of arrival counters per (device, stream); torch hands out a bounded set of
 // streams, the buffers grow to the largest call and clear_workspaces() gives them back.  The counters must be zero
-// before a call and every kernel leaves them zero, so they are cleared only when the array is made.
+// before a call and every kernel leaves them zero, so they are cleared only when the array is made.  Buffers that a call
+// under capture was given are kept when a larger call outgrows them: the graph goes on using them (asking the stream costs
+// 40 ns a call; at most one buffer per growth is kept).
 struct Scratch {
     at::Tensor ws, ctr;
+    bool captured = false;
 };
 using ScratchMap = std::map<std::pair<int, cudaStream_t>, Scratch>;
 ScratchMap& g_scratch = *new ScratchMap;      // never destroyed: the process may end after the driver has gone
+std::vector<Scratch>& g_outgrown = *new std::vector<Scratch>;
 
 // Scratch of calls larger than this is shared by all blocks on a stream: they run one after another, and a private
 // copy for every block and prompt length would not fit.  16 MB lie between the calls that graphs capture (64 tokens of the
@@ -154,17 +158,24 @@ ScratchMap& g_big = *new ScratchMap;
 Scratch& scratch(int dev, cudaStream_t st, size_t nbytes, size_t nctr) {
     Scratch& s = g_scratch[{dev, st}];
     const bool small_ws = !s.ws.defined() || (size_t)s.ws.numel() < nbytes, small_ctr = !s.ctr.defined() || (size_t)s.ctr.numel() < nctr;
-    if (!small_ws && !small_ctr) return s;
-    if ((!s.ws.defined() || !s.ctr.defined()) && capturing(st)) {
+    const bool capture = capturing(st);
+    if (!small_ws && !small_ctr) {
+        s.captured |= capture;
+        return s;
+    }
+    if ((!s.ws.defined() || !s.ctr.defined()) && capture) {
         // no allocation (and no zero fill) inside a capture: the scratch of the warm-up calls on this device serves
         // the captured calls too (they run in stream order after them)
         for (auto& kv : g_scratch)
             if (kv.first.first == dev && kv.second.ws.defined() && kv.second.ctr.defined() &&
                 (size_t)kv.second.ws.numel() >= nbytes && (size_t)kv.second.ctr.numel() >= nctr) {
+                kv.second.captured = true;
                 s = kv.second;
                 return s;
             }
     }
+    if (s.captured) g_outgrown.push_back(s);
+    s.captured = capture;
     const auto opt = at::TensorOptions().device(at::kCUDA, dev);
     if (small_ws) {
         s.ws = at::Tensor();
@@ -214,6 +225,7 @@ PyObject* py_workspace(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 PyObject* py_clear_workspaces(PyObject*, PyObject*) {
     g_scratch.clear();
+    g_outgrown.clear();
     g_big.clear();
     Py_RETURN_NONE;
 }

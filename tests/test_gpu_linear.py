@@ -484,3 +484,26 @@ def test_threads_on_one_stream_share_its_scratch(dev):
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_scratch_of_a_captured_call_outlives_a_larger_call(dev):
+    """The graph writes x.U and reads it back in the scratch it was captured with."""
+    from glorcq_b200 import _lib
+    small, large = (cases.to_b200_linear(cases.make_linear(90 + i, 256, K, rank=32), dev) for i, K in enumerate((512, 4096)))
+    x, xl = cases.make_x(92, 4, 512).to(dev), cases.make_x(93, 1000, 4096).to(dev)
+    ref = small(x)
+    st, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    _lib.native().clear_workspaces()
+    with torch.cuda.stream(st):
+        small(x)
+        st.synchronize()
+        with torch.cuda.graph(graph, stream=st):
+            y = small(x)
+        before = _lib.native().workspace(0, 0, 0)[0].numel()
+        large(xl)
+        assert _lib.native().workspace(0, 0, 0)[0].numel() > before
+        others = [torch.full((before // 4,), 7, dtype=torch.int32, device=dev) for _ in range(16)]
+        graph.replay()
+    st.synchronize()
+    assert torch.equal(y, ref)
+    assert all(bool((t == 7).all()) for t in others)
