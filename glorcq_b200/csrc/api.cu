@@ -559,7 +559,7 @@ static bool plan_tc(const glq_mm_args_t* a, TcGeom* out) {
     TcGeom g{};
     const long long total = total_entries(a);
     g.nkb = cdiv(a->K, 128);
-    g.ns = a->rank > 0 ? cdiv(a->rank, 64) : 0;
+    g.ns = a->rank > 0 && a->fmt != GLQ_FMT_F16 ? cdiv(a->rank, 64) : 0;      // (dense weights have no low-rank term)
     g.na = a->epilogue == GLQ_EPI_SWIGLU ? 2 : 1;
     choose_tile(a, total, g.nkb + g.ns, &g);
     const long long tiles = total / g.tn + a->n_problems + 1;

@@ -91,9 +91,7 @@ __global__ void __launch_bounds__(kLmThreads, 1) lm_head_kernel(const LmParams p
             qa[d] = ldg_stream(w0 + d * 4);
             qb[d] = ldg_stream(w1 + d * 4);
         }
-    asm volatile("griddepcontrol.wait;" ::: "memory");              // W is nobody's output, x is
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // activations: rows beyond B are zero
+    // activations, staged while the first of W are on their way: rows beyond B are zero
     for (int i = tid; i < 8 * NT * (H / 8); i += kLmThreads) {
         const int row = i / (H / 8), c = i % (H / 8);
         uint4 v = make_uint4(0, 0, 0, 0);

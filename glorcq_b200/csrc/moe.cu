@@ -262,8 +262,6 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const __half* __restrict
     int* sm_off = sm_cnt + E;
     int* s_sel = sm_off + E;
     __half* s_wts = reinterpret_cast<__half*>(s_sel + n * k);
-    asm volatile("griddepcontrol.wait;" ::: "memory");              // no-ops for a plain launch
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // Phase A: one warp per token, lanes over experts (E <= 256)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     if (sel_in) {
@@ -760,8 +758,11 @@ bool plan_fused(const glq_moe_desc_t* d, int n, FusedParams* out, size_t* smem_b
     off = (off + 15) / 16 * 16;
     P.off_red = (int)off;
     off += (size_t)2 * kFSW * 2 * 32 * sizeof(float2);     // k-split sums (two parities)
-    P.off_prob = (int)off;
-    off += (size_t)kFRows * (256 + 16) * sizeof(float);    // the routing's probabilities
+    P.off_seg = (int)off;
+    // sums of the segments of a row of the shared U^T: 16 floats.  The rest is unused and stays: without it the one-token block of
+    // 60 experts takes 31.42 us instead of 31.25, wherever the ring is aligned to (128, 512, 1024 bytes)
+    off += (size_t)kFRows * (256 + 16) * sizeof(float);
+    static_assert(kFW - kFSW <= 256 + 16, "segment sums");
     off = (off + 15) / 16 * 16;
     P.off_plan = (int)off;
     off += sizeof(FusedPlan);
@@ -1045,24 +1046,15 @@ extern "C" int glq_moe_forward_ep(const glq_moe_desc_t* d, const void* x, int n,
         if (cudaGetLastError() != cudaSuccess) return GLQ_ERR_CUDA;
         after_kernel[0] = true;
     } else {
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(1);
-        cfg.blockDim = dim3(1024);
-        cfg.dynamicSmemBytes = 2 * d->E * sizeof(int) + (size_t)nk * (sizeof(int) + sizeof(__half));
-        cfg.stream = st;
-        cudaLaunchAttribute attr{};
-        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr.val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 0;   // plain launch (a dependent launch after the router product measured no faster)
-        if (cudaLaunchKernelEx(&cfg, moe_plan_kernel, (const __half*)p_logits, ldl, n, (int)d->E, k, (int)d->norm_topk_prob,
-                               p_sel, p_wts, p_active, p_nact, p_cnt, p_off, p_erow, p_escale, p_tok,
-                               reinterpret_cast<__half*>(router_logits), (int*)sel_out, reinterpret_cast<__half*>(weight_out),
-                               reinterpret_cast<int*>(ws + L.active2), reinterpret_cast<int*>(ws + L.n_active2),
-                               reinterpret_cast<int*>(ws + L.slot_count2), reinterpret_cast<int*>(ws + L.slot_offset2),
-                               ep_rank, ep_world, given ? (const int*)ep->sel_in : (const int*)nullptr,
-                               given ? reinterpret_cast<const __half*>(ep->weight_in) : (const __half*)nullptr, chunk) != cudaSuccess)
-            return GLQ_ERR_CUDA;
+        // (a programmatically dependent launch after the router product measured no faster)
+        const size_t smem = 2 * d->E * sizeof(int) + (size_t)nk * (sizeof(int) + sizeof(__half));
+        moe_plan_kernel<<<1, 1024, smem, st>>>(
+            p_logits, ldl, n, (int)d->E, k, (int)d->norm_topk_prob, p_sel, p_wts, p_active, p_nact, p_cnt, p_off, p_erow, p_escale, p_tok,
+            reinterpret_cast<__half*>(router_logits), (int*)sel_out, reinterpret_cast<__half*>(weight_out),
+            reinterpret_cast<int*>(ws + L.active2), reinterpret_cast<int*>(ws + L.n_active2),
+            reinterpret_cast<int*>(ws + L.slot_count2), reinterpret_cast<int*>(ws + L.slot_offset2), ep_rank, ep_world,
+            given ? (const int*)ep->sel_in : nullptr, given ? reinterpret_cast<const __half*>(ep->weight_in) : nullptr, chunk);
+        if (cudaGetLastError() != cudaSuccess) return GLQ_ERR_CUDA;
         after_kernel[0] = true;
     }
     // rows of remote experts' entries stay zero, so that summing the ranks' buffers is exact

@@ -91,7 +91,7 @@ struct FusedParams {
     int* flags;
     FusedPhase ph[4];        // 0 shared gate|up, 1 routed gate|up, 2 shared down, 3 routed down
     int stages, stage_bytes;
-    int off_act, off_ox, off_red, off_ring, off_plan, off_tab, off_prob;   // shared memory carve-up (bytes)
+    int off_act, off_ox, off_red, off_ring, off_plan, off_tab, off_seg;   // shared memory carve-up (bytes)
     int g_shared;            // CTAs [0, g_shared) run the shared expert's chain, the others the routed experts' chain
     unsigned long long wait_ns;
     // S10: the combine inside this launch (0: the caller launches it, e.g. after an exchange between ranks)
@@ -385,7 +385,6 @@ __global__ void __launch_bounds__(kFT, 1) moe_fused_kernel(const FusedParams p) 
     uint4* xs = reinterpret_cast<uint4*>(smem + p.off_act);
     float2* ox = reinterpret_cast<float2*>(smem + p.off_ox);
     float2* red = reinterpret_cast<float2*>(smem + p.off_red);
-    float* prob = reinterpret_cast<float*>(smem + p.off_prob);
     FusedPlan& plan = *reinterpret_cast<FusedPlan*>(smem + p.off_plan);
     ExpertPtrs* tab = reinterpret_cast<ExpertPtrs*>(smem + p.off_tab);
     const uint32_t xs_a = smem_u32(xs), ox_a = smem_u32(ox);
@@ -589,7 +588,7 @@ __global__ void __launch_bounds__(kFT, 1) moe_fused_kernel(const FusedParams p) 
             if (p.ph[2].live && p.ph[2].rank > 0) {
                 const int rows_per_cta = kDW / s6_segs;
                 bool waited = false;
-                float* rbuf = prob;      // idle after the plan
+                float* rbuf = reinterpret_cast<float*>(smem + p.off_seg);
 #pragma unroll 1
                 for (int base = sub_cta * rows_per_cta; base < p.R; base += sub_G * rows_per_cta) {
                     if (!waited) warp_wait(flags + FL_HS, p.ph[0].npairs, 202), waited = true;

@@ -1,20 +1,18 @@
-// Grouped dequant-GEMM on the 5th-generation tensor cores (tcgen05.mma, accumulators in TMEM) for
-// problems with many activation rows (prefill, large decode batches).
+// Many activation rows per problem (prompts, large decode batches) on the 5th-generation tensor cores (tcgen05.mma,
+// accumulators in TMEM): what its two kernels share -- the operands, the token tiles and their pre-pass, the
+// primitives -- and the kernel for dense fp16 weights.  Packed codes: tc_ps.cuh.
 //
-//   D[feature, token] = sum_k W[feature, k] * X[token, k]   (+ sum_r SV[feature, r] * a[token, r])
+//   D[feature, token] = sum_k W[feature, k] * X[token, k]
 //
-// The weights are the M operand ("swap AB"): a CTA owns 128 output features of one problem and TN
-// tokens; producer warps unpack the 2-bit codes of the pair-interleaved tiled layout to the exact
-// fp16 values fp16((q - z) * s) and store them as a K-major, 128-byte-swizzled UMMA operand in shared
-// memory; the token operand arrives ready-made: a pre-pass (tc_pack_b_kernel) gathers the problem's
-// activation rows, orders k like the unpack does and writes swizzled tiles, so the main kernel fetches
-// each k stage of it with one bulk copy.  One thread issues the MMAs; the low-rank term is folded in
-// as extra k steps (A = SV rows, B = the entries' x.U rows), so the epilogue only rounds, applies
-// SwiGLU / routing weight / bias and stores.
+// The weights are the M operand ("swap AB"): an item is 128 output features of one problem and TN tokens.  The token
+// operand arrives ready-made: the pre-pass (tc_pack_b_kernel) gathers the problem's activation rows and, for packed
+// codes, those of x.U, orders k as the weight operand has it and writes 128-byte-swizzled tiles, so that each k stage
+// is one bulk copy.  The kernel here (tc_kernel, one item per CTA) stores the tiled fp16 fragments as a K-major,
+// swizzled operand in shared memory; one thread issues the MMAs, and the epilogue only rounds, applies bias and
+// routing weight, and stores.
 //
-// k order inside every group of 16 input channels: position 2j holds channel j, position 2j+1 holds
-// channel j+8 (the order in which one shift-and-mask yields two codes); both operands use it, so the
-// dot products are unchanged.
+// k order inside a group of 16 input channels for dense weights: that of the stored fragments (lane t has channels 2t,
+// 2t+1, 2t+8, 2t+9); both operands use it, so the dot products are unchanged.
 //
 // Every mbarrier wait is bounded (about 2 ms); a wait that runs out records error 100/101, marks the
 // CTA dead, and all roles fall through to the common exit, which frees the tensor memory.

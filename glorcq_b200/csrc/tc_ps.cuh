@@ -62,8 +62,8 @@ __device__ __forceinline__ void tc_st_x2(uint32_t taddr, const uint32_t (&r)[8])
 __device__ __forceinline__ void tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // D (TMEM) += A (TMEM, 128 lanes x 8 columns = 16 fp16 per row) * B (shared memory descriptor), a run of four k steps: A
 // advances by 8 columns, B by 32 bytes.  The whole warp comes here with the same operands and one elected lane issues: in code
-// that one lane runs alone the operands of every instruction go through R2UR, and the issuing warp, not the tensor pipe,
-// set the pace (113 to 117 cycles per MMA of any N up to 128).  One election serves the four (one for each still left 70
+// that one lane runs alone the issuing warp, not the tensor pipe, set the pace (113 to 117 cycles per MMA of any N up to
+// 128).  One election serves the four (one for each still left 70
 // to 90 cycles between MMAs of 64 columns, which the tensor pipe does in 32).
 __device__ __forceinline__ void tc_mma4_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t acc) {
     asm volatile(
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
             if (ok) tc_commit_warp(bar_acc);
         }
     } else if (warp == kTcProducers + 1) {
-        // ================= results: staging tiles -> y, one 256-byte copy per token row =================
+        // ================= results: staging tiles -> y, 16 bytes per lane, two token rows at a time =================
         int pass = 0;
         for (int it = 0; have_item(it); ++it) {
             const volatile PsItem& im = s_item[it % kPsQueue];
