@@ -703,29 +703,28 @@ static int launch_tc(const glq_mm_args_t* a, const TcGeom& g, cudaStream_t st, c
     return GLQ_ERR_UNSUPPORTED;
 }
 
-extern "C" size_t glq_mm_workspace_bytes(const glq_mm_args_t* a) {
-    if (!a || xu_takes(a)) return 0;
+// workspace bytes and arrival counters of a call: one planning for both
+struct MmNeeds {
+    size_t bytes = 0, counters = 0;
+};
+static MmNeeds mm_needs(const glq_mm_args_t* a) {
+    MmNeeds n;
     TcGeom tg;
-    if (plan_tc(a, &tg)) return tg.xp_bytes;
     StreamGeom sg;
-    if (plan_chunks(a, &sg) || plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, a->max_rows, &sg)) return 0;
     Geometry g;
-    if (plan_geometry(a->fmt, a->epilogue, a->N, a->K, a->group_size, a->n_problems, a->max_rows, true, &g) != GLQ_OK)
-        return 0;
-    return g.scratch_bytes;
+    if (!a || xu_takes(a)) return n;
+    if (plan_tc(a, &tg)) {
+        n.bytes = tg.xp_bytes;
+    } else if (!plan_chunks(a, &sg) &&
+               !plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, a->max_rows, &sg) &&
+               plan_geometry(a->fmt, a->epilogue, a->N, a->K, a->group_size, a->n_problems, a->max_rows, true, &g) == GLQ_OK) {
+        n.bytes = g.scratch_bytes;
+        n.counters = g.n_counters;
+    }
+    return n;
 }
-
-extern "C" size_t glq_mm_counters(const glq_mm_args_t* a) {
-    if (!a) return 0;
-    TcGeom tg;
-    if (plan_tc(a, &tg)) return 0;
-    StreamGeom sg;
-    if (plan_chunks(a, &sg) || plan_stream(a->fmt, a->epilogue, a->N, a->K, a->rank, a->group_size, a->n_problems, a->max_rows, &sg)) return 0;
-    Geometry g;
-    if (plan_geometry(a->fmt, a->epilogue, a->N, a->K, a->group_size, a->n_problems, a->max_rows, true, &g) != GLQ_OK)
-        return 0;
-    return g.n_counters;
-}
+extern "C" size_t glq_mm_workspace_bytes(const glq_mm_args_t* a) { return mm_needs(a).bytes; }
+extern "C" size_t glq_mm_counters(const glq_mm_args_t* a) { return mm_needs(a).counters; }
 
 extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
     if (!a || !a->x || !a->y) return GLQ_ERR_ARG;
@@ -899,15 +898,15 @@ static int linear_forward(int fmt, int group_size, const glq_weight_t* w, const 
     glq_mm_args_t m;
     linear_args(fmt, group_size, w, B, &m);
     char* ws = reinterpret_cast<char*>(workspace);
-    const size_t main_ws = up256(glq_mm_workspace_bytes(&m));
-    const size_t main_ctr = glq_mm_counters(&m);
+    const MmNeeds main = mm_needs(&m);
+    const size_t main_ws = up256(main.bytes), main_ctr = main.counters;
     const void* a_use = a;
     if (!a && ut && w->rank > 0 && w->sv) {
         glq_mm_args_t u;
         xu_args(w, ut, B, &u);
         const size_t a_bytes = up256((size_t)B * w->rank * sizeof(__half));
-        const size_t u_ws = up256(glq_mm_workspace_bytes(&u));
-        const size_t u_ctr = glq_mm_counters(&u);
+        const MmNeeds un = mm_needs(&u);
+        const size_t u_ws = up256(un.bytes), u_ctr = un.counters;
         if (!ws || workspace_bytes < main_ws + a_bytes + u_ws) return GLQ_ERR_WORKSPACE;
         if (u_ctr > 0 && (!counters || n_counters < main_ctr + u_ctr)) return GLQ_ERR_WORKSPACE;
         u.x = x;
