@@ -56,7 +56,8 @@ __device__ __forceinline__ void store_row(__half* p, bool vec, const __half (&h)
         for (int i = 0; i < EPL; ++i) p[i] = h[i];
 }
 
-// What bounds it: a warp's chain of positions (few heads), instruction issue (many).  One position at a time, every score
+// What bounds it: the wait for the cached rows, at one CTA per SM (few heads; issue slots 22 % used) as at the two that
+// registers allow (16 sequences of 32 heads; 45 %, a quarter of the HBM rate).  One position at a time, every score
 // waited for five shuffles and every update for two exponentials.  Now eight positions make one step: their partial scores are
 // summed by a transposing butterfly (the same pairs of lanes in the same order, so the same bits), the running maximum is
 // a scan, each exponential is taken once per position instead of by every lane, only l and o are chains, and the rows of

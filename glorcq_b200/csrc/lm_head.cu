@@ -56,7 +56,7 @@ size_t lm_smem_bytes(int nt, int H) {
     return (size_t)nt * 8 * (H + 32) * 2 + (size_t)kLmGroups * (kLmSplit - 1) * nt * 32 * sizeof(float4);
 }
 
-// Bound by the read of W: 98 us for 1 row of 151936 x 2048, 6.3 TB/s (137 before); 16 rows of 32000 x 4096 55 us (148 in two
+// Bound by the read of W: 95 to 98 us for 1 row of 151936 x 2048, the rate of a plain copy (137 before); 16 rows of 32000 x 4096 55 us (148 in two
 // passes), 64 of 151936 x 2048 283 us (1127 in eight).  NT 1, 2, 4: 8, 16, 32 activation rows; D: chunks of 32 channels a warp
 // has in flight.  D 4 is 64 KB per SM and all that the stream needs; 6 and 8 spill and took 102 and 117 us.
 template <int NT, int D>

@@ -17,7 +17,8 @@
 //     fixed point (two int8 digits per value, one power-of-two scale per row and k block) when they
 //     are staged, the 2/4-bit codes become int8 with two bit-ops per four weights, and the s8 x s8
 //     -> s32 tensor-core op (m16n8k32) does the dot products exactly; scale, zero point and the digit
-//     weights are applied in fp32 per k block.  More rows (and the codebook format) use the fp16 op;
+//     weights are applied in fp32 per k block (a codebook as two or three such products, tile_block_t2_i8).  Slots of more
+//     rows, and 3-bit codes whatever the rows (GLQ_FMT_Q3: activations as they are), use the fp16 op;
 //   * k splits of a pair are warps of one CTA, reduced through shared memory in a fixed order
 //     (named barrier per pair): no global scratch, no atomics, deterministic;
 //   * when two CTAs of eight warps with their own copies of the staged activations do not fit an SM (8 rows of 4096

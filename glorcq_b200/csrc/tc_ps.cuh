@@ -34,7 +34,7 @@
 // roundings of the dequantisation computed and one selected, every warp looking up its item): 142 us for the gate|up
 // product of 60 experts x 34 rows (1408 x 2048, 2-bit), scheduler slots 57 % used, DRAM 12 %.  Now 140 instructions
 // and 99 us; 97 -> 60 us for the down product (2048 x 1408).  With one multiply-add per pair of 2-bit codes and one election
-// per four MMAs 95 and 54 us.  No pipe is full (integer 45 %, issue slots 49 %, tensor 40 %): what is left is the latency
+// per four MMAs 95 and 54 us.  No pipe is full (gate|up: integer 49 %, issue slots 53 %, tensor 23 %): what is left is the latency
 // of a warp's own chain through a stage, of which four warps per scheduler cover only a part.
 //
 // Every wait is bounded (tc_wait); a wait that runs out marks the CTA dead, all roles leave their loops
