@@ -205,7 +205,8 @@ typedef struct glq_mm_args {
 /* Scratch bytes / arrival counters a call with these args needs (both 0 when no CTA-level k split is
  * used).  The counters must be zero when a call starts and are zero again when it ends, so one
  * zero-initialised array can serve any sequence of calls on one stream; the scratch needs no
- * initialisation. */
+ * initialisation.  Of the pointers only their presence counts (the slot arrays, entry_scale, a0): set those the call will
+ * have; x, ldx and y may follow later. */
 size_t glq_mm_workspace_bytes(const glq_mm_args_t* args);
 size_t glq_mm_counters(const glq_mm_args_t* args);
 int glq_grouped_matmul(const glq_mm_args_t* args, void* stream);
