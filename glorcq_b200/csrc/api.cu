@@ -592,7 +592,7 @@ static int launch_tc_t(const TcParams& p, cudaStream_t st) {
 // packed codes: one CTA per SM over all (token tile, feature tile) items
 template <int FMT, int TN, int NM, bool SW>
 static int launch_tc_ps_t(TcParams& p, cudaStream_t st) {
-    using C = TcPsCfg<TN, NM, SW>;
+    using C = TcPsCfg<FMT, TN, NM, SW>;
     static bool configured[64] = {};
     const int rc = allow_smem(tc_ps_kernel<FMT, TN, NM, SW>, configured, C::SMEM);
     if (rc != GLQ_OK) return rc;

@@ -17,7 +17,7 @@
 // CTA instead of once per tile.  16 producer warps unpack the codes of a 128-channel stage into the
 // tensor-memory ring, one warp issues the MMAs, one bulk-copies the token operand.
 //
-//  * Work items are drawn from a grid-wide counter (zeroed by the pre-pass) by the loader warp one item ahead;
+//  * Work items are drawn from a grid-wide counter (zeroed by the pre-pass) by a warp of its own, up to four ahead;
 //    it looks the problem up and hands the operands' addresses to the other warps through a small queue in
 //    shared memory, so an SM that runs faster takes more items and nobody else walks the dependent loads.
 //  * The rings run on across item boundaries: the loader fetches the next item's token operand while the
@@ -34,8 +34,10 @@
 // roundings of the dequantisation computed and one selected, every warp looking up its item): 142 us for the gate|up
 // product of 60 experts x 34 rows (1408 x 2048, 2-bit), scheduler slots 57 % used, DRAM 12 %.  Now 140 instructions
 // and 99 us; 97 -> 60 us for the down product (2048 x 1408).  With one multiply-add per pair of 2-bit codes and one election
-// per four MMAs 95 and 54 us.  No pipe is full (gate|up: integer 49 %, issue slots 53 %, tensor 23 %): what is left is the latency
-// of a warp's own chain through a stage, of which four warps per scheduler cover only a part.
+// per four MMAs 95 and 54 us; with the look-ups in a warp of their own, the accumulator released before the epilogue's arithmetic
+// and that arithmetic left out for tokens that do not exist 86 and 55 (codebook codes: 105 -> 95).  No pipe is full (gate|up:
+// integer 49 %, issue slots 53 %, tensor 23 %): what is left is the latency of a warp's own chain through a stage, of which four
+// warps per scheduler cover only a part.
 //
 // Every wait is bounded (tc_wait); a wait that runs out marks the CTA dead, all roles leave their loops
 // and the kernel ends.
@@ -45,7 +47,7 @@
 
 namespace glq {
 
-constexpr int kPsQueue = 4;        // work items the loader may be ahead of the slowest warp
+constexpr int kPsQueue = 4;        // work items that may be handed out ahead of the slowest warp
 
 __device__ __forceinline__ void tc_st_x4(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
@@ -88,9 +90,15 @@ __device__ __forceinline__ void tc_commit_warp(uint32_t bar) {
 
 constexpr int kPsRows = 64;                                      // tokens of a result pass
 constexpr int kPsOut = kPsRows * 256;                            // its staging tile [token][128 features] fp16, two of them
-constexpr int kPsThreads = (kTcProducers + 3) * 32;
+constexpr int kPsThreads = (kTcProducers + 4) * 32;              // and products, results, loader, items
+// Registers of a thread: 96 at launch (640 threads).  With 4-bit codes of two matrices the producers' loop spills; there the
+// warpgroup of the other roles hands some of its own over (gate|up of 60 experts x 34 rows 138 -> 130 us; 2-bit codes fit, and their
+// down product takes 58 us instead of 56 with the others at 64).
+constexpr int kPsRegsProducer = 104, kPsRegsOther = 64;
+static_assert(kTcProducers * 32 * kPsRegsProducer + 4 * 32 * kPsRegsOther <= kPsThreads * 96, "registers");
 
-template <int TN, int NM, bool SW> struct TcPsCfg {
+template <int FMT, int TN, int NM, bool SW> struct TcPsCfg {
+    static constexpr bool SHIFT_REGS = FMT == GLQ_FMT_Q4 && NM == 2;
     static constexpr int NOUT = SW ? 1 : NM;                     // 128-feature output tiles of an item
     static constexpr int ACC = NM * TN;                          // accumulator columns
     static constexpr int B_BYTES = TN * 256;
@@ -107,12 +115,12 @@ __device__ __forceinline__ bool ps_wait_warp(uint32_t bar, uint32_t parity, vola
     return __all_sync(0xffffffffu, mbar_try_wait(bar, parity) || tc_wait(bar, parity, dead, code));
 }
 
-// A work item as the loader hands it out; ft < 0 ends the list.
+// A work item as it is handed out; ft < 0 ends the list.
 struct PsItem {
     const unsigned char *codes, *sv;
     const __half* bias;
     const float *norms, *centroids;
-    int ft, lt, cnt, e0;
+    int ft, lt, cnt, e0, gt;
 };
 
 // One row's 16 codes of a stage -> eight fp16 pairs in K position order (tc_ts_channel_of).
@@ -238,7 +246,7 @@ __device__ __forceinline__ void ps_q2_fast(const uint32_t (&w)[2][1], const PsQ2
 // accumulator fills half of tensor memory): two warps share a tile, one per half of the lanes' channels.
 template <int FMT, int TN, int NM, bool SW>
 __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) {
-    using C = TcPsCfg<TN, NM, SW>;
+    using C = TcPsCfg<FMT, TN, NM, SW>;
     constexpr int S = C::S;
     static_assert(!SW || NM == 2, "gate|up items hold two matrices");
     constexpr bool AFFINE = FMT != GLQ_FMT_T2;
@@ -248,7 +256,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
     __shared__ __align__(8) unsigned long long bars[2 * S + 6 + 2 * kPsQueue];
     __shared__ uint32_t s_tmem;
     __shared__ int s_dead;
-    __shared__ PsItem s_item[kPsQueue];       // work items in the order the loader drew them
+    __shared__ PsItem s_item[kPsQueue];       // work items in the order they were drawn
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t sbase = (smem_u32(tc_smem_raw) + 1023u) & ~1023u;
@@ -272,7 +280,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
         }
         for (int i = 0; i < kPsQueue; ++i) {
             mbar_init(bar_tq_full + 8 * i, 1);
-            mbar_init(bar_tq_empty + 8 * i, kTcProducers + 2);
+            mbar_init(bar_tq_empty + 8 * i, kTcProducers + 3);
         }
         s_dead = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -301,6 +309,7 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
     };
 
     if (warp < kTcProducers) {
+        if constexpr (C::SHIFT_REGS) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPsRegsProducer));
         // ================= producers: unpack into tensor memory, then the tile's epilogue =================
         const int g = lane >> 2, t = lane & 3;
         const int q = warp & 3, sub = warp >> 2;                   // a warp reaches the tensor-memory lanes of its quarter q
@@ -349,12 +358,18 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
                 const int b = pass & 1;
                 if (pass > 1) ok = ps_wait_warp(bar_stored + 8 * b, (uint32_t)((pass >> 1) & 1) ^ 1u, dead, 106) && ok;
                 tc_ld_wait();
+                if (h == C::NPASS - 1) {            // the accumulator is in registers: the next item's products may start
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_acc_free);
+                }
                 const uint32_t dst = orow + (uint32_t)(b * kPsOut);
-                const int r0 = im.lt * TN + c0 + part * 16, cnt = im.cnt;
+                const int live = im.cnt - (im.lt * TN + c0 + part * 16);       // tokens of this warp's 16 that exist
                 const float scv = __half2float(sc_h[h % (TN / kPsRows)]);
-                if (ok && r0 < cnt) {
+                if (ok && live > 0) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
+                        if (j >= live) break;
                         float v = __uint_as_float(vg[j]);
                         if constexpr (!AFFINE) v *= nrm_g;
                         if constexpr (SW) {
@@ -373,9 +388,6 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
                 if (lane == 0) mbar_arrive(bar_staged + 8 * b);
                 ++pass;
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_acc_free);
             release_item(n);
             return ok;
         };
@@ -560,7 +572,9 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
             if (more) open_item(it + 1);
         }
         tc_fence_before();
-    } else if (warp == kTcProducers) {
+    } else {
+    if constexpr (C::SHIFT_REGS) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPsRegsOther));
+    if (warp == kTcProducers) {
         // ================= MMA issuer =================
         constexpr uint32_t idesc = tc_idesc(TN);
         constexpr uint32_t kAtom = TN * 128 / 16;            // an atom of the token operand in descriptor units
@@ -637,59 +651,18 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
             release_item(it);
             if (!ok) break;
         }
-    } else {
+    } else if (warp == kTcProducers + 2) {
         // ================= loader of the token operand =================
+        // launched beside the pre-pass: its tiles are needed from here on (the other warps' first codes are not its work)
         int s = 0;
         uint32_t ph = 0;
         int issued = 0;
-        // Draw work item n (the first one is the CTA's number, the others come from the grid-wide counter), look its
-        // problem up and publish it; returns its token tile, -1 at the end of the list.  Item n + 1 is published before
-        // the copies of item n are issued: these wait for the ring, and the producers want the addresses early.
-        auto publish = [&](int n) -> int {
-            const int qi = n % kPsQueue;
-            const bool room = __all_sync(0xffffffffu, tc_wait(bar_tq_empty + 8 * qi, (uint32_t)(((n / kPsQueue) & 1) ^ 1), dead, 109));
-            PsItem im;
-            im.ft = -1;
-            int gt = -1;
-            for (bool first = n == 0; room; first = false) {
-                int w = blockIdx.x;
-                if (!first) {
-                    if (n == 0) asm volatile("griddepcontrol.wait;" ::: "memory");     // (a padding tile came first)
-                    if (lane == 0) w = atomicAdd(p.tile_ctr, 1) + gridDim.x;
-                    w = __shfl_sync(0xffffffffu, w, 0);
-                }
-                if (w >= n_work) break;
-                const int tile = w / p.n_ft;
-                int slot;
-                if (tc_find_tile<TN>(p, tile, slot, im.lt, im.cnt, im.e0)) {
-                    const int widx = p.slot_index ? __ldg(p.slot_index + slot) : slot;
-                    const glq_weight_t* W = p.table ? p.table + widx : &p.w;
-                    im.codes = reinterpret_cast<const unsigned char*>(W->codes);
-                    im.sv = reinterpret_cast<const unsigned char*>(W->sv);
-                    im.bias = reinterpret_cast<const __half*>(W->bias);
-                    im.norms = W->norms;
-                    im.centroids = W->centroids;
-                    gt = tile;
-                    im.ft = w - tile * p.n_ft;
-                    break;
-                }
-            }
-            if (lane == 0) {
-                s_item[qi] = im;
-                mbar_arrive(bar_tq_full + 8 * qi);
-            }
-            __syncwarp();
-            return gt;
-        };
-        // launched beside the pre-pass: its tiles and the zeroed counter are needed from here on (the other warps' first codes
-        // and addresses are not its work)
-        int gt = publish(0), nxt = -1;
         asm volatile("griddepcontrol.wait;" ::: "memory");
         asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-        for (int n = 0; gt >= 0; ++n, gt = nxt) {
-            nxt = publish(n + 1);
+        for (int it = 0; have_item(it); ++it) {
+            const unsigned char* tile = p.xp + (size_t)static_cast<const volatile PsItem&>(s_item[it % kPsQueue]).gt * p.tile_bytes;
+            release_item(it);
             if (lane == 0) {
-                const unsigned char* tile = p.xp + (size_t)gt * p.tile_bytes;
                 for (int st = 0; st < nst; ++st) {
                     if (!tc_wait(bar_empty + 8 * s, ph ^ 1u, dead, 105)) break;
                     const uint32_t bbase = sbase + (uint32_t)s * C::B_BYTES;
@@ -727,6 +700,48 @@ __global__ void __launch_bounds__(kPsThreads, 1) tc_ps_kernel(const TcParams p) 
             }
         }
         __syncwarp();
+    } else {
+        // ================= items: draw one (the first is the CTA's number, the others come from the grid-wide counter), look its
+        // problem up, hand it out, up to kPsQueue ahead.  The loads of a look-up depend on one another, 3000 cycles in all; as a
+        // part of the loader's loop they stood between the copies of two items and emptied its ring.
+        bool more = true;
+        for (int n = 0; more; ++n) {
+            const int qi = n % kPsQueue;
+            const bool room = __all_sync(0xffffffffu, tc_wait(bar_tq_empty + 8 * qi, (uint32_t)(((n / kPsQueue) & 1) ^ 1), dead, 109, 50000000ull));
+            PsItem im;
+            im.ft = -1;
+            for (bool first = n == 0; room; first = false) {
+                int w = blockIdx.x;
+                if (!first) {
+                    // (the pre-pass, beside which this grid is launched, zeroes the counter)
+                    if (n <= 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+                    if (lane == 0) w = atomicAdd(p.tile_ctr, 1) + gridDim.x;
+                    w = __shfl_sync(0xffffffffu, w, 0);
+                }
+                if (w >= n_work) break;
+                const int tile = w / p.n_ft;
+                int slot;
+                if (tc_find_tile<TN>(p, tile, slot, im.lt, im.cnt, im.e0)) {
+                    const int widx = p.slot_index ? __ldg(p.slot_index + slot) : slot;
+                    const glq_weight_t* W = p.table ? p.table + widx : &p.w;
+                    im.codes = reinterpret_cast<const unsigned char*>(W->codes);
+                    im.sv = reinterpret_cast<const unsigned char*>(W->sv);
+                    im.bias = reinterpret_cast<const __half*>(W->bias);
+                    im.norms = W->norms;
+                    im.centroids = W->centroids;
+                    im.gt = tile;
+                    im.ft = w - tile * p.n_ft;
+                    break;
+                }
+            }
+            if (lane == 0) {
+                s_item[qi] = im;
+                mbar_arrive(bar_tq_full + 8 * qi);
+            }
+            __syncwarp();
+            more = im.ft >= 0;
+        }
+    }
     }
 
     __syncthreads();
