@@ -511,7 +511,15 @@ __global__ void __launch_bounds__(kFT, 1) moe_fused_kernel(const FusedParams p) 
                     first &= !(ej == e && j < dt);
                 }
                 // this rank's chosen experts below e
-                for (int e2 = p.ep_rank; e2 < e; e2 += p.ep_world) slot += (plan.sel_mask[e2 >> 5] >> (e2 & 31)) & 1u;
+                if (p.ep_world == 1) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int below = e - 32 * i;          // bits of word i that stand for experts below e
+                        if (below > 0) slot += __popc(plan.sel_mask[i] & (below >= 32 ? 0xffffffffu : (1u << below) - 1u));
+                    }
+                } else {
+                    for (int e2 = p.ep_rank; e2 < e; e2 += p.ep_world) slot += (plan.sel_mask[e2 >> 5] >> (e2 & 31)) & 1u;
+                }
                 plan.entry_tok[pos] = dt / k;
                 plan.entry_e[pos] = e;
                 plan.entry_w[pos] = plan.wts[dt];
@@ -983,59 +991,83 @@ __global__ void __launch_bounds__(kFT, 1) moe_fused_kernel(const FusedParams p) 
             dead = dead || plan.dead != 0;
         }
         if (p.combine && cta < n) {
+            // What does not depend on the down outputs is fetched before they are waited for, and then the rows of all entries are
+            // requested together: one row after another, with the residual, the norm weight and the output read back behind
+            // them, the combine kept a block 5 of its 29 us.
             const int tok = cta, k = p.k, H = p.H;
-            const int y_target = (p.ph[2].live ? p.ph[2].npairs : 0) + n_slots * p.ph[3].npairs;
-            stream_wait(flags + FL_Y, y_target, 206);
-            int order[16];
-            for (int s = 0; s < k; ++s) order[s] = s;
-            if (p.by_expert)
-                for (int i = 1; i < k; ++i) {
-                    const int v = order[i];
-                    const int ev = plan.sel[tok * k + v];
-                    int j = i - 1;
-                    while (j >= 0 && plan.sel[tok * k + order[j]] > ev) {
-                        order[j + 1] = order[j];
-                        --j;
+            int* s_entry = reinterpret_cast<int*>(smem + p.off_seg) + (kFW - kFSW) * kFRows;     // behind the segment sums
+            if (tid < k) {                     // slot tid's place in the order of the sum: experts ascending, or slots
+                int rank = tid;
+                if (p.by_expert) {
+                    const int e = plan.sel[tok * k + tid];
+                    rank = 0;
+                    for (int s = 0; s < k; ++s) {
+                        const int es = plan.sel[tok * k + s];
+                        rank += es < e || (es == e && s < tid) ? 1 : 0;
                     }
-                    order[j + 1] = v;
                 }
+                s_entry[rank] = plan.tok_entry[tok * k + tid];
+            }
             const float gate = (p.ysh && p.gate_col >= 0)
                                    ? sigmoid16(__half2float(__ldcg(p.logits + (size_t)tok * p.ldl + p.gate_col))) : 1.f;
             // 384 threads x 8 columns per step
+            constexpr int NS = 3;              // steps: H <= 8192
+            uint4 res[NS], nw[NS];
+#pragma unroll
+            for (int st = 0; st < NS; ++st) {
+                const int c0 = (st * kST + tid) * 8;
+                res[st] = nw[st] = make_uint4(0, 0, 0, 0);
+                if (c0 >= H) continue;
+                if (p.residual) res[st] = __ldg(reinterpret_cast<const uint4*>(p.residual + (size_t)tok * H + c0));
+                if (p.normed && p.norm_w) nw[st] = __ldg(reinterpret_cast<const uint4*>(p.norm_w + c0));
+            }
+            const int y_target = (p.ph[2].live ? p.ph[2].npairs : 0) + n_slots * p.ph[3].npairs;
+            stream_wait(flags + FL_Y, y_target, 206);
             float ss = 0.f;
-#pragma unroll 1
-            for (int c0 = tid * 8; c0 < H; c0 += kST * 8) {
+            uint4 outv[NS];
+#pragma unroll
+            for (int st = 0; st < NS; ++st) {
+                const int c0 = (st * kST + tid) * 8;
+                if (c0 >= H) continue;
+                uint4 sh = make_uint4(0, 0, 0, 0);
+                if (p.ysh) sh = __ldcg(reinterpret_cast<const uint4*>(p.ysh + (size_t)tok * H + c0));
                 float acc[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) acc[i] = 0.f;
 #pragma unroll 1
-                for (int s = 0; s < k; ++s) {
-                    const int entry = plan.tok_entry[tok * k + order[s]];
-                    if (entry < 0) continue;     // dropped slot
-                    __align__(16) __half v[8];
-                    *reinterpret_cast<uint4*>(v) = __ldcg(reinterpret_cast<const uint4*>(p.yd + (size_t)entry * H + c0));
+                for (int s0 = 0; s0 < k; s0 += 4) {
+                    uint4 v[4];
+                    int entry[4];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[i] = round16(acc[i] + __half2float(v[i]));
+                    for (int u = 0; u < 4; ++u) {
+                        entry[u] = s0 + u < k ? s_entry[s0 + u] : -1;        // negative: a dropped slot
+                        v[u] = entry[u] >= 0 ? __ldcg(reinterpret_cast<const uint4*>(p.yd + (size_t)entry[u] * H + c0)) : make_uint4(0, 0, 0, 0);
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (entry[u] >= 0) {
+                            const __half* h = reinterpret_cast<const __half*>(&v[u]);
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) acc[i] = round16(acc[i] + __half2float(h[i]));
+                        }
                 }
                 if (p.ysh) {
-                    __align__(16) __half v[8];
-                    *reinterpret_cast<uint4*>(v) = __ldcg(reinterpret_cast<const uint4*>(p.ysh + (size_t)tok * H + c0));
+                    const __half* h = reinterpret_cast<const __half*>(&sh);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[i] = round16(acc[i] + round16(gate * __half2float(v[i])));
+                    for (int i = 0; i < 8; ++i) acc[i] = round16(acc[i] + round16(gate * __half2float(h[i])));
                 }
                 if (p.residual) {
-                    __align__(16) __half v[8];
-                    *reinterpret_cast<uint4*>(v) = __ldg(reinterpret_cast<const uint4*>(p.residual + (size_t)tok * H + c0));
+                    const __half* h = reinterpret_cast<const __half*>(&res[st]);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[i] = round16(__half2float(v[i]) + acc[i]);
+                    for (int i = 0; i < 8; ++i) acc[i] = round16(__half2float(h[i]) + acc[i]);
                 }
-                __align__(16) __half o[8];
+                __half* o = reinterpret_cast<__half*>(&outv[st]);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     o[i] = __float2half_rn(acc[i]);       // exact: the sums above are already rounded to fp16
                     ss += acc[i] * acc[i];
                 }
-                *reinterpret_cast<uint4*>(p.out + (size_t)tok * H + c0) = *reinterpret_cast<const uint4*>(o);
+                *reinterpret_cast<uint4*>(p.out + (size_t)tok * H + c0) = outv[st];
             }
             if (p.normed) {
                 float* rs = reinterpret_cast<float*>(red);
@@ -1047,12 +1079,12 @@ __global__ void __launch_bounds__(kFT, 1) moe_fused_kernel(const FusedParams p) 
 #pragma unroll
                 for (int i = 0; i < kFSW; ++i) tot += rs[i];
                 const float r = rsqrtf(tot / H + p.norm_eps);
-#pragma unroll 1
-                for (int c0 = tid * 8; c0 < H; c0 += kST * 8) {
-                    // this thread's own outputs of the loop above (fp16, exactly the summed values)
-                    __align__(16) __half v[8], o[8], wv[8];
-                    *reinterpret_cast<uint4*>(v) = *reinterpret_cast<const uint4*>(p.out + (size_t)tok * H + c0);
-                    if (p.norm_w) *reinterpret_cast<uint4*>(wv) = __ldg(reinterpret_cast<const uint4*>(p.norm_w + c0));
+#pragma unroll
+                for (int st = 0; st < NS; ++st) {
+                    const int c0 = (st * kST + tid) * 8;
+                    if (c0 >= H) continue;
+                    const __half *v = reinterpret_cast<const __half*>(&outv[st]), *wv = reinterpret_cast<const __half*>(&nw[st]);
+                    __align__(16) __half o[8];
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const float nv = __half2float(v[i]) * r;
