@@ -107,6 +107,7 @@ _SIGS = {
     "glq_mm_workspace_bytes": (C.c_size_t, [C.POINTER(MMArgs)]),
     "glq_mm_counters": (C.c_size_t, [C.POINTER(MMArgs)]),
     "glq_grouped_matmul": (C.c_int, [C.POINTER(MMArgs), vp]),
+    "glq_grouped_matmul_pair": (C.c_int, [C.POINTER(MMArgs), C.POINTER(MMArgs), vp]),
     "glq_linear_counters": (C.c_size_t, [C.c_int, C.c_int, C.POINTER(Weight), C.c_int]),
     "glq_linear_workspace_bytes": (C.c_size_t, [C.c_int, C.c_int, C.POINTER(Weight), C.c_int]),
     "glq_linear_forward": (C.c_int, [C.c_int, C.c_int, C.POINTER(Weight), vp, vp, C.c_int64, vp, vp, C.c_int64,

@@ -406,6 +406,48 @@ static int launch_stream_fmt(const StreamParams& sp, const StreamGeom& g, cudaSt
     return launch_stream_one<FMT, false, 4>(sp, g, st);
 }
 
+template <int FMT, bool I8, int NT, int NW = 8>
+static int launch_stream_pair_t(const StreamParams& sp, const StreamGeom& g, const SkinnyParams& xu, int n_xu, cudaStream_t st) {
+    auto kern = stream_pair_kernel<FMT, I8, NT, NW>;
+    static size_t configured[16] = {0};
+    int dev = 0;
+    GLQ_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 16 || configured[dev] < g.smem) {
+        GLQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+        if (dev >= 0 && dev < 16) configured[dev] = g.smem;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(g.grid + n_xu);
+    cfg.blockDim = dim3(NW * 32);
+    cfg.dynamicSmemBytes = g.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    GLQ_CUDA(cudaLaunchKernelEx(&cfg, kern, sp, xu, n_xu));
+    return GLQ_OK;
+}
+template <int FMT>
+static int launch_stream_pair_fmt(const StreamParams& sp, const StreamGeom& g, const SkinnyParams& xu, int n_xu, cudaStream_t st) {
+    if (!g.i8) {
+        if constexpr (FMT == GLQ_FMT_Q4) return launch_stream_pair_t<FMT, false, 1>(sp, g, xu, n_xu, st);
+        return GLQ_ERR_UNSUPPORTED;
+    }
+    if (g.nw == 16)
+        return g.nt == 1 ? launch_stream_pair_t<FMT, true, 1, 16>(sp, g, xu, n_xu, st) : launch_stream_pair_t<FMT, true, 2, 16>(sp, g, xu, n_xu, st);
+    return g.nt == 1 ? launch_stream_pair_t<FMT, true, 1>(sp, g, xu, n_xu, st) : launch_stream_pair_t<FMT, true, 2>(sp, g, xu, n_xu, st);
+}
+static int launch_stream_pair(int fmt, const StreamParams& sp, const StreamGeom& g, const SkinnyParams& xu, int n_xu, cudaStream_t st) {
+    switch (fmt) {
+        case GLQ_FMT_Q2: return launch_stream_pair_fmt<GLQ_FMT_Q2>(sp, g, xu, n_xu, st);
+        case GLQ_FMT_Q4: return launch_stream_pair_fmt<GLQ_FMT_Q4>(sp, g, xu, n_xu, st);
+        case GLQ_FMT_T2: return launch_stream_pair_fmt<GLQ_FMT_T2>(sp, g, xu, n_xu, st);
+    }
+    return GLQ_ERR_ARG;
+}
+
 // Rows of a chunk when a product with host-known counts is cut into chunks of its rows, the slots of ONE launch of the
 // streaming kernel; 0 when it is not.
 // 9..32 rows: the integer path stages at most 8 rows (4 when the staged activations of a long reduction leave no room for 8)
@@ -428,8 +470,34 @@ static int plan_chunks(const glq_mm_args_t* a, StreamGeom* sg) {
     return 0;
 }
 
+static void fill_operands(const glq_mm_args_t* a, SkinnyParams& p) {
+    p.w = a->w;
+    p.table = a->w_table;
+    p.sv_slices = cdiv(std::max(a->rank, 1), 64);
+    p.slot_index = a->slot_index;
+    p.n_slots = a->n_slots;
+    p.slot_count = a->slot_count;
+    p.slot_offset = a->slot_offset;
+    p.entry_row = a->entry_row;
+    p.entry_scale = reinterpret_cast<const __half*>(a->entry_scale);
+    p.x = reinterpret_cast<const __half*>(a->x);
+    p.ldx = a->ldx;
+    p.a[0] = reinterpret_cast<const __half*>(a->a0);
+    p.a[1] = reinterpret_cast<const __half*>(a->a1);
+    p.lda = a->lda;
+    p.y = reinterpret_cast<__half*>(a->y);
+    p.ldy = a->ldy;
+    p.counters = a->counters;
+    p.scratch = reinterpret_cast<float4*>(a->workspace);
+    p.max_rows = a->max_rows;
+    p.rows_stride = a->rows_stride > 0 ? a->rows_stride : a->max_rows;
+    p.epilogue = a->epilogue;
+    p.x_vec = (aligned16(a->x) && a->ldx % 8 == 0) ? 1 : 0;
+}
+
+// xu, n_xu, pair: x.U in the grid's first n_xu blocks and the two counters it meets the product at (stream_pair_kernel)
 static int launch_stream(const glq_mm_args_t* a, SkinnyParams& p, const StreamGeom& g, cudaStream_t st, bool a_late = false, bool dependent = false, int cnt_lo = 0,
-                         int cnt_hi = 0x7fffffff) {
+                         int cnt_hi = 0x7fffffff, const SkinnyParams* xu = nullptr, int n_xu = 0, int* pair = nullptr, int pair_target = 0) {
     const int fmt = a->fmt, N = a->N, K = a->K, rank = a->rank, n_problems = a->n_problems;
     StreamParams sp{};
     sp.cnt_lo = cnt_lo;
@@ -463,6 +531,12 @@ static int launch_stream(const glq_mm_args_t* a, SkinnyParams& p, const StreamGe
     sp.off_as = g.off_as;
     sp.off_ring = g.off_ring;
     sp.off_red = g.off_red;
+    if (xu) {
+        sp.a_late = 1;
+        sp.pair = pair;
+        sp.pair_target = pair_target;
+        return launch_stream_pair(tile_fmt(fmt), sp, g, *xu, n_xu, st);
+    }
     StreamGeom gl = g;
     // a concurrent stream runs grouped products too: two thirds of the CTA slots, so that its kernels find room
     // (measured on the MoE block: the shared expert's branch beside the routed experts')
@@ -780,28 +854,7 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
     if (!a->w_table && !a->w.codes) return GLQ_ERR_ARG;
 
     SkinnyParams p{};
-    p.w = a->w;
-    p.table = a->w_table;
-    p.sv_slices = cdiv(std::max(a->rank, 1), 64);
-    p.slot_index = a->slot_index;
-    p.n_slots = a->n_slots;
-    p.slot_count = a->slot_count;
-    p.slot_offset = a->slot_offset;
-    p.entry_row = a->entry_row;
-    p.entry_scale = reinterpret_cast<const __half*>(a->entry_scale);
-    p.x = reinterpret_cast<const __half*>(a->x);
-    p.ldx = a->ldx;
-    p.a[0] = reinterpret_cast<const __half*>(a->a0);
-    p.a[1] = reinterpret_cast<const __half*>(a->a1);
-    p.lda = a->lda;
-    p.y = reinterpret_cast<__half*>(a->y);
-    p.ldy = a->ldy;
-    p.counters = a->counters;
-    p.scratch = reinterpret_cast<float4*>(a->workspace);
-    p.max_rows = a->max_rows;
-    p.rows_stride = a->rows_stride > 0 ? a->rows_stride : a->max_rows;
-    p.epilogue = a->epilogue;
-    p.x_vec = (aligned16(a->x) && a->ldx % 8 == 0) ? 1 : 0;
+    fill_operands(a, p);
     if (chunk) p.max_rows = chunk;
     if (use_stream) {
         cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -830,6 +883,45 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
     rc = launch_skinny(a->fmt, false, p, g, a->n_problems, reinterpret_cast<cudaStream_t>(stream));
     t_dependent_launch = false;
     return rc;
+}
+
+// x.U (u) and the product that adds its low-rank term (m): one launch where both are small enough to be resident together, two
+// otherwise.  One launch: at most 8 rows with counts that the host knows, the streaming kernel for m, the general kernel without
+// tile groups for u, a CTA slot for every block of both (where the product fills the slots, blocks behind x.U's would start late
+// and the launch that is saved is a small part), and two counters more than u needs.
+constexpr size_t kPairCounters = 2;
+static int matmul_pair(const glq_mm_args_t* u, const glq_mm_args_t* m, void* stream) {
+    StreamGeom sg;
+    Geometry g;
+    const bool known = !m->slot_index && !m->n_slots && !m->slot_count && !m->slot_offset && !u->slot_index && !u->n_slots && !u->slot_count &&
+                       !u->slot_offset;
+    if (known && !pdl_disabled() && m->max_rows <= 8 && u->max_rows == m->max_rows && u->n_problems == m->n_problems && m->n_problems > 0 && u->fmt == GLQ_FMT_F16 &&
+        u->epilogue == GLQ_EPI_LINEAR && m->epilogue == GLQ_EPI_LINEAR && u->rank == 0 && u->K == m->K && u->y == m->a0 && m->a0 && m->rank > 0 &&
+        m->rank % 16 == 0 && m->lda % 8 == 0 && aligned16(m->a0) && u->x && m->x && m->y && (u->w_table || u->w.codes) && (m->w_table || m->w.codes) &&
+        !u->entry_scale &&
+        plan_stream(m->fmt, m->epilogue, m->N, m->K, m->rank, m->group_size, m->n_problems, m->max_rows, &sg) &&
+        (sg.i8 || (m->fmt == GLQ_FMT_Q3 && sg.nt == 1 && sg.nw == 8)) &&
+        plan_geometry(GLQ_FMT_F16, GLQ_EPI_LINEAR, u->N, u->K, 0, u->n_problems, u->max_rows, true, &g) == GLQ_OK && g.ntt == 1 && g.smem <= sg.smem) {
+        const long n_xu = (long)u->n_problems * g.tile_groups * g.sk;
+        const long slots = (long)num_sms() * (sg.nw == 8 && sg.smem <= 110 * 1024 ? kStreamCtasPerSm : 1);
+        const bool scratch = (g.scratch_bytes == 0 || (u->workspace && u->workspace_bytes >= g.scratch_bytes && aligned16(u->workspace))) && u->counters &&
+                             u->n_counters >= g.n_counters + kPairCounters;
+        if (n_xu + sg.grid <= slots && scratch) {
+            SkinnyParams xp{}, p{};
+            fill_operands(u, xp);
+            fill_geometry(xp, g);
+            fill_operands(m, p);
+            t_xu_out = nullptr;
+            return launch_stream(m, p, sg, reinterpret_cast<cudaStream_t>(stream), false, false, 0, 0x7fffffff, &xp, (int)n_xu,
+                                 u->counters + g.n_counters, u->n_problems * cdiv(u->N, kRowTile));
+        }
+    }
+    const int rc = glq_grouped_matmul(u, stream);
+    return rc != GLQ_OK ? rc : glq_grouped_matmul(m, stream);
+}
+extern "C" int glq_grouped_matmul_pair(const glq_mm_args_t* xu, const glq_mm_args_t* mm, void* stream) {
+    if (!xu || !mm) return GLQ_ERR_ARG;
+    return matmul_pair(xu, mm, stream);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -884,7 +976,7 @@ extern "C" size_t glq_linear_counters(int fmt, int group_size, const glq_weight_
     if (w->rank > 0) {
         glq_mm_args_t u;
         xu_args(w, w->codes, B, &u);
-        total += glq_mm_counters(&u);
+        total += glq_mm_counters(&u) + (B <= 8 ? kPairCounters : 0);
     }
     return total;
 }
@@ -901,8 +993,9 @@ static int linear_forward(int fmt, int group_size, const glq_weight_t* w, const 
     const MmNeeds main = mm_needs(&m);
     const size_t main_ws = up256(main.bytes), main_ctr = main.counters;
     const void* a_use = a;
-    if (!a && ut && w->rank > 0 && w->sv) {
-        glq_mm_args_t u;
+    glq_mm_args_t u;
+    const bool own_xu = !a && ut && w->rank > 0 && w->sv;
+    if (own_xu) {
         xu_args(w, ut, B, &u);
         const size_t a_bytes = up256((size_t)B * w->rank * sizeof(__half));
         const MmNeeds un = mm_needs(&u);
@@ -916,9 +1009,7 @@ static int linear_forward(int fmt, int group_size, const glq_weight_t* w, const 
         u.workspace = ws + main_ws + a_bytes;
         u.workspace_bytes = u_ws;
         u.counters = counters ? counters + main_ctr : nullptr;
-        u.n_counters = u_ctr;
-        int rc = glq_grouped_matmul(&u, stream);
-        if (rc != GLQ_OK) return rc;
+        u.n_counters = counters ? n_counters - main_ctr : 0;
         a_use = ws + main_ws;
     }
     if (main_ws > 0 && (!ws || workspace_bytes < main_ws)) return GLQ_ERR_WORKSPACE;
@@ -934,9 +1025,10 @@ static int linear_forward(int fmt, int group_size, const glq_weight_t* w, const 
     m.counters = counters;
     m.n_counters = main_ctr;
     if (!a_use) m.w.rank = 0, m.rank = 0;
-    // x.U was just launched above and is needed only in the epilogue; x itself is older
-    if (a_use != nullptr && a_use != a) m.flags = GLQ_MM_A_FROM_PREVIOUS_LAUNCH;
-    return glq_grouped_matmul(&m, stream);
+    if (!own_xu) return glq_grouped_matmul(&m, stream);
+    // (as two launches: x.U is the launch before and is needed only in the epilogue; x itself is older)
+    m.flags = GLQ_MM_A_FROM_PREVIOUS_LAUNCH;
+    return matmul_pair(&u, &m, stream);
 }
 
 extern "C" int glq_linear_forward(int fmt, int group_size, const glq_weight_t* w, const void* ut, const void* x,

@@ -43,6 +43,7 @@ struct Api {
     GLQ_FN(glq_mm_workspace_bytes)                                                                                  \
     GLQ_FN(glq_mm_counters)                                                                                         \
     GLQ_FN(glq_grouped_matmul)                                                                                      \
+    GLQ_FN(glq_grouped_matmul_pair)                                                                                 \
     GLQ_FN(glq_turbo_dequant_matmul)                                                                                \
     GLQ_FN(glq_turbo_dequant_grouped_gemv)                                                                          \
     GLQ_FN(glq_gptq_dequant_matmul)                                                                                 \
@@ -381,7 +382,7 @@ PyObject* py_grouped_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
         size_t nbytes = 0, nctr = 0;
         for (int i = 0; i < n_mm; ++i) {
             nbytes = std::max(nbytes, api.glq_mm_workspace_bytes(&mm[i]));
-            nctr = std::max(nctr, api.glq_mm_counters(&mm[i]));
+            nctr = std::max(nctr, api.glq_mm_counters(&mm[i]) + 2);       // (and the two of a pair)
         }
         const Scratch s = scratch(dev, st, nbytes, nctr);
         for (int i = 0; i < n_mm; ++i) {
@@ -391,9 +392,7 @@ PyObject* py_grouped_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
             mm[i].n_counters = (size_t)s.ctr.numel();
         }
         launch(st, "grouped_matmul", [&] {
-            int status = GLQ_OK;
-            for (int i = 0; i < n_mm && status == GLQ_OK; ++i) status = api.glq_grouped_matmul(&mm[i], st);
-            return status;
+            return low_rank ? api.glq_grouped_matmul_pair(&mm[0], &mm[1], st) : api.glq_grouped_matmul(&mm[0], st);
         });
         return wrap(y);
     });

@@ -333,19 +333,18 @@ __device__ __forceinline__ void load_codes(const glq_weight_t& W, int rt, int pa
 // in three chunks; with one group of 32 weight rows per CTA the staging was most of the time: 152 us for the down
 // products of 16 tokens over 8 experts, 107 us with four).  The order of every sum is the same.
 // ---------------------------------------------------------------------------------------------
-template <int FMT, int NW, int NTT, bool RM, int TGN = 1>
-__global__ void __launch_bounds__(kThreads, 2) skinny_kernel(const SkinnyParams p) {
+// PAIRED: the blocks are those of a product that shares its launch with them (stream_mm.cuh): 256 of its threads work, the launch
+// before is waited for once the first codes are on their way, and every row tile that is written counts itself in `arrivals`.
+template <int FMT, int NW, int NTT, bool RM, int TGN, bool PAIRED>
+__device__ __forceinline__ void skinny_body(const SkinnyParams& p, int bid, int* arrivals) {
     using F = Fmt<FMT>;
     constexpr int kDepth = F::DEPTH;
     extern __shared__ uint4 smem_u4[];
     __shared__ int s_last;
-    // Programmatic dependent launch, both no-ops for a plain launch: wait for the preceding grid of the
-    // stream (this kernel reads its results from the first load on), then let the next grid be scheduled
-    // (it waits for this one in the same way before it reads what this one writes).
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-
-    int bid = blockIdx.x;
+    auto sync = [] {
+        if constexpr (PAIRED) asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+        else __syncthreads();
+    };
     const int s = bid % p.sk;
     bid /= p.sk;
     const int n_tg = (p.tile_groups + TGN - 1) / TGN;
@@ -433,9 +432,10 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_kernel(const SkinnyParams 
                     }
                 }
             }
-            if (iter++ > 0) __syncthreads();  // everyone is done with the previous contents of shared memory
+            if (PAIRED && iter == 0) asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
+            if (iter++ > 0) sync();  // everyone is done with the previous contents of shared memory
             stage_x<FMT>(p, xs, ox, kc_lo, nkc, e0, pass0, cnt, K);
-            __syncthreads();
+            sync();
 
 #pragma unroll
             for (int gi = 0; gi < TGN; ++gi) {
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_kernel(const SkinnyParams 
         auto& acc = accs[gi];
         const int rt = rt_of(gi), pr = NW == 2 ? rt : (rt >> 1), pj0 = NW == 2 ? 0 : (rt & 1);
         const bool tile_ok = rt < ntiles;
-        if (gi > 0) __syncthreads();      // the sums of the group before have been read
+        if (gi > 0) sync();      // the sums of the group before have been read
         // ---- reduce the kKW warps of a row tile (fixed order) ----
         if (kw != 0) {
 #pragma unroll
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_kernel(const SkinnyParams 
                     red[((warp * NW + i) * NTT + tt) * 32 + lane] =
                         make_float4(acc[i][tt][0], acc[i][tt][1], acc[i][tt][2], acc[i][tt][3]);
         }
-        __syncthreads();
+        sync();
         if (kw == 0) {
             for (int k2 = 1; k2 < kKW; ++k2)
 #pragma unroll
@@ -544,14 +544,14 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_kernel(const SkinnyParams 
                                make_float4(acc[i][tt][0], acc[i][tt][1], acc[i][tt][2], acc[i][tt][3]));
                 __threadfence();
             }
-            __syncthreads();
+            sync();
             if (tid == 0) {
                 const int old = atomicAdd(&p.counters[tile_id], 1);
                 const int last = (old == p.sk - 1);
                 if (last) p.counters[tile_id] = 0;
                 s_last = last;
             }
-            __syncthreads();
+            sync();
             if (!s_last) continue;
             __threadfence();
             if (kw == 0) {
@@ -664,9 +664,23 @@ __global__ void __launch_bounds__(kThreads, 2) skinny_kernel(const SkinnyParams 
                             p.y[(size_t)(e0 + row) * p.ldy + n] = __float2half_rn(v);
                     }
                 }
+            if constexpr (PAIRED) {
+                __syncwarp();
+                if (lane == 0) asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(arrivals) : "memory");
+            }
         }
         }
     }
+}
+
+template <int FMT, int NW, int NTT, bool RM, int TGN = 1>
+__global__ void __launch_bounds__(kThreads, 2) skinny_kernel(const SkinnyParams p) {
+    // Programmatic dependent launch, both no-ops for a plain launch: wait for the preceding grid of the
+    // stream (this kernel reads its results from the first load on), then let the next grid be scheduled
+    // (it waits for this one in the same way before it reads what this one writes).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    skinny_body<FMT, NW, NTT, RM, TGN, false>(p, blockIdx.x, nullptr);
 }
 
 }  // namespace glq

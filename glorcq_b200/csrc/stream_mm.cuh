@@ -62,6 +62,8 @@ struct StreamParams {
     int cnt_lo, cnt_hi;  // only slots with cnt_lo < rows <= cnt_hi are this launch's (others belong to a sibling launch)
     int dependent;  // 1: launched with programmatic stream serialization
     int a_late;   // 1: the x.U operand is still being written when this kernel starts (programmatic dependent launch)
+    int* pair;    // {row tiles of x.U written, CTAs done}: zero between calls; x.U is computed by the first blocks of this launch
+    int pair_target;
 };
 
 // ---- shared memory, mbarrier and bulk copy primitives ------------------------------------------
@@ -119,6 +121,27 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, bool& d
             return;
         }
     }
+}
+// Bounded wait of a warp for a counter in global memory (about 2 ms, then error 112); what was written before the arrivals is visible.
+__device__ __forceinline__ void pair_wait(const int* f, int target, int lane, bool& dead) {
+    int ok = 1;
+    if (lane == 0 && !dead) {
+        int v;
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
+        if (v < target) {
+            const unsigned long long t0 = global_ns();
+            for (;;) {
+                asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
+                if (v >= target) break;
+                if (global_ns() - t0 > 2000000ull) {
+                    ok = glq_ok(false, 112, (unsigned long long)v, (unsigned long long)target);
+                    break;
+                }
+                __nanosleep(20);
+            }
+        }
+    }
+    if (!__shfl_sync(0xffffffffu, ok, 0)) dead = true;
 }
 __device__ __forceinline__ uint4 ld_global_u4(const uint4* p) {
     uint4 v;
@@ -376,8 +399,9 @@ __device__ __forceinline__ void tile_block_t2_i8(const uint4 q, const uint4 (&bx
 // I8 = true : NT tiles of 4 activation rows (integer path: affine formats and the 2-bit codebook)
 // I8 = false: NT tiles of 8 activation rows (fp16 path)
 // NW = 8: two CTAs per SM; NW = 16 (integer path only): one
-template <int FMT, bool I8, int NT, int NW>
-__global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) stream_kernel(const StreamParams sp) {
+// PAIRED: the grid's first blocks compute x.U (stream_pair_kernel); this is block `block` of the `n_blocks` behind them
+template <int FMT, bool I8, int NT, int NW, bool PAIRED>
+__device__ __forceinline__ void stream_body(const StreamParams& sp, int block, int n_blocks) {
     using F = Fmt<FMT>;
     static_assert(FMT != GLQ_FMT_F16, "dense weights use the fallback kernel");
     static_assert(I8 || NW == 8, "the fp16 path stages with the threads of eight warps");
@@ -399,13 +423,13 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
 
     // Programmatic dependent launch (no-ops for a plain launch).  a_late: only the x.U operand comes from
     // the preceding grid, the wait sits in front of the low-rank term; otherwise wait here.
-    if (!sp.a_late) asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!PAIRED && !sp.a_late) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if constexpr (!PAIRED) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int n_live = p.n_slots ? min(__ldg(p.n_slots), sp.n_problems) : sp.n_problems;
     const long total = (long)n_live * sp.ips;
-    const int it_lo = (int)((long)blockIdx.x * total / gridDim.x);
-    const int it_hi = (int)((long)(blockIdx.x + 1) * total / gridDim.x);
-    if (it_lo >= it_hi) {
+    const int it_lo = (int)((long)block * total / n_blocks);
+    const int it_hi = (int)((long)(block + 1) * total / n_blocks);
+    if (!PAIRED && it_lo >= it_hi) {
         // a dependent launch must not end before the launch it depends on has: later launches of the
         // stream order themselves after this grid only
         if (sp.a_late) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -540,6 +564,9 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
     };
     fetch_seek();
     while (f_live && f_inflight < S) fetch_one();
+    // The weights of a layer are older than the launch before this one: their first stages are requested before it is waited for.
+    // The next launch may come after the wait only, so that all launches before this one are complete when it starts.
+    if constexpr (PAIRED) asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
 
     uint32_t TL[2] = {0, 0}, TH[2] = {0, 0};  // codebook tables of the two tiles of a pair
     // integer path of the codebook format: coefficients of the two tiles' codebooks (tile_block_t2_i8)
@@ -779,8 +806,9 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
                 for (int q = 0; q < 4; ++q) lo[j][m][q] = 0.f;
         const int nsv = im.nch - im.ncode;
         if (sp.a_late && nsv > 0 && !dep_waited) {
-            // programmatic dependent launch: everything up to here overlapped the launch that produces x.U
-            asm volatile("griddepcontrol.wait;" ::: "memory");
+            // everything up to here overlapped the blocks, or the launch, that produce x.U
+            if constexpr (PAIRED) pair_wait(sp.pair, sp.pair_target, lane, dead);
+            else asm volatile("griddepcontrol.wait;" ::: "memory");
             dep_waited = true;
         }
         for (int c = 0; c < nsv; ++c) {
@@ -882,8 +910,34 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
             }
         }
     }
-    // see the early exit above: a dependent grid ends only after the grid it depends on
-    if (sp.a_late && !dep_waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if constexpr (PAIRED) {
+        // the CTA that is done last clears both counters: every other one is past its wait
+        __syncthreads();
+        if (tid == 0 && atomicAdd(sp.pair + 1, 1) == n_blocks - 1) sp.pair[0] = sp.pair[1] = 0;
+    } else {
+        // see the early exit above: a dependent grid ends only after the grid it depends on
+        if (sp.a_late && !dep_waited) asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
+}
+
+template <int FMT, bool I8, int NT, int NW>
+__global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) stream_kernel(const StreamParams sp) {
+    stream_body<FMT, I8, NT, NW, false>(sp, blockIdx.x, gridDim.x);
+}
+
+// A layer of at most 8 rows in one launch: blocks [0, n_xu) compute x.U as skinny_kernel does, the others the product, whose
+// low-rank term waits for the row tiles of x.U behind a counter.  Only blocks of higher numbers wait, and only for lower ones, which
+// are scheduled first and wait for nobody; the host takes this form only where all of them are resident at once.
+// Bound by latency, the host's and the chain's: with two launches (the second programmatically dependent) one row through 1408 x 2048,
+// 2-bit, rank 64 took 11.2 us a call, 7.7 now; 2 rows of 3-bit 2048 x 2048 10.8 and 7.5, 5 rows of codebook 5632 x 2048 16.4 and 14.4.
+template <int FMT, bool I8, int NT, int NW>
+__global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) stream_pair_kernel(const StreamParams sp, const SkinnyParams xp, int n_xu) {
+    if ((int)blockIdx.x < n_xu) {
+        if (NW > kWarpsPerCta && threadIdx.x >= kThreads) return;
+        skinny_body<GLQ_FMT_F16, 1, 1, false, 1, true>(xp, blockIdx.x, sp.pair);
+    } else {
+        stream_body<FMT, I8, NT, NW, true>(sp, blockIdx.x - n_xu, gridDim.x - n_xu);
+    }
 }
 
 }  // namespace glq

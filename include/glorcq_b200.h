@@ -210,6 +210,9 @@ typedef struct glq_mm_args {
 size_t glq_mm_workspace_bytes(const glq_mm_args_t* args);
 size_t glq_mm_counters(const glq_mm_args_t* args);
 int glq_grouped_matmul(const glq_mm_args_t* args, void* stream);
+/* xu, then mm, whose a0 is xu's output (flag GLQ_MM_A_FROM_PREVIOUS_LAUNCH): the same results as the two calls.  Up to 8 rows with
+ * host-known counts run as one launch when xu->counters has two ints more than glq_mm_counters(xu). */
+int glq_grouped_matmul_pair(const glq_mm_args_t* xu, const glq_mm_args_t* mm, void* stream);
 
 /* Randomized Hadamard rotation of activation rows (rht_forward, hadamard_rotation.py:50-65, which
  * multiplies by the signs and calls the third-party fast-hadamard-transform):

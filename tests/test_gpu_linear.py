@@ -507,3 +507,19 @@ def test_scratch_of_a_captured_call_outlives_a_larger_call(dev):
     st.synchronize()
     assert torch.equal(y, ref)
     assert all(bool((t == 7).all()) for t in others)
+
+
+@pytest.mark.parametrize("B", [1, 4, 5, 8])
+@pytest.mark.parametrize("fmt,bits,N,K,rank", [("gptq", 2, 1408, 2048, 64), ("gptq", 4, 520, 896, 16), ("gptq", 3, 40, 192, 128), ("turbo", 2, 1000, 8192, 80),
+                                               ("gptq", 4, 4096, 4096, 64), ("gptq", 2, 72, 14336, 32), ("gptq", 2, 14336, 4096, 64)])
+def test_low_rank_operand_in_the_products_launch(dev, fmt, bits, N, K, rank, B):
+    """x.U computed by the first blocks of the product's launch (or, for the largest, by a launch of its own) gives the bits of x.U
+    computed alone and handed in, call after call, and leaves the arrival counters at zero."""
+    from glorcq_b200 import _lib, tiled
+    lin = cases.to_b200_linear(cases.make_linear(N + K + B, N, K, rank=rank, fmt=fmt, bits=bits), dev)
+    x = cases.make_x(B + N, B, K).to(dev)
+    ref = tiled.linear_forward(lin._tiled, x, a=tiled.dense_matmul(lin._ut, x))
+    for _ in range(3):
+        assert torch.equal(tiled.linear_forward(lin._tiled, x, lin._ut), ref)
+    torch.cuda.synchronize()
+    assert not bool(_lib.native().workspace(0, 0, 0)[1].any()) and tiled.debug_error() is None
