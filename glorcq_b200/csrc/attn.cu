@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <cstdlib>
 
 #include "glq_common.cuh"
 
@@ -76,11 +77,14 @@ __global__ void __launch_bounds__(kAttnWarps * 32, EPL == 4 && G == 1 ? 4 : 1) a
     const int h = blockIdx.x * G, b = blockIdx.y, z = blockIdx.z, nsplit = gridDim.z;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int group = n_heads / n_kv, kvh = h / group;
+    __half* kc = k_cache + ((size_t)b * n_kv + kvh) * max_len * HD;
+    __half* vc = v_cache + ((size_t)b * n_kv + kvh) * max_len * HD;
+    // (launched plainly, after all before it: in the places that the projections leave free beside them the CTAs would lie two to an SM,
+    // 8.9 us instead of 7.5; the output projection behind it may fetch its first weights meanwhile)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     long long pos = *pos_p;
     if (pos < 0) pos = 0;
     if (pos >= max_len) pos = max_len - 1;
-    __half* kc = k_cache + ((size_t)b * n_kv + kvh) * max_len * HD;
-    __half* vc = v_cache + ((size_t)b * n_kv + kvh) * max_len * HD;
     // this CTA's share of the cached positions (the grid's z dimension splits them), interleaved over its warps; a step is
     // kAhead of a warp's positions, its keys and values at constant distances from one row
     const int per = ((int)pos + nsplit - 1) / nsplit;
@@ -564,6 +568,14 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(const __half* __restri
     const size_t row = (size_t)blockIdx.x * H;
     float val[4][8];
     float ss = 0.f;
+    // (launched beside the projection that writes delta, for which it waits; the weight is older: 2.3 -> 1.8 us behind it)
+    __align__(16) __half wv[4][8];
+#pragma unroll
+    for (int step = 0; step < 4; ++step) {
+        const int c0 = (step * 256 + threadIdx.x) * 8;
+        if (w && c0 < H) *reinterpret_cast<uint4*>(wv[step]) = __ldg(reinterpret_cast<const uint4*>(w + c0));
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 #pragma unroll
     for (int step = 0; step < 4; ++step) {
         const int c0 = (step * 256 + threadIdx.x) * 8;
@@ -591,25 +603,40 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(const __half* __restri
     for (int step = 0; step < 4; ++step) {
         const int c0 = (step * 256 + threadIdx.x) * 8;
         if (c0 >= H) continue;
-        __align__(16) __half o[8], wv[8];
-        if (w) *reinterpret_cast<uint4*>(wv) = *reinterpret_cast<const uint4*>(w + c0);
+        __align__(16) __half o[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = __float2half_rn(w ? __half2float(wv[i]) * (val[step][i] * r) : val[step][i] * r);
+        for (int i = 0; i < 8; ++i) o[i] = __float2half_rn(w ? __half2float(wv[step][i]) * (val[step][i] * r) : val[step][i] * r);
         *reinterpret_cast<uint4*>(h_out + row + c0) = *reinterpret_cast<const uint4*>(o);
     }
 }
 
 }  // namespace
 
+// launch with programmatic stream serialization: the grid may start before the launch ahead of it has ended and waits for it itself
+template <typename... P, typename... A>
+static cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    static const bool off = std::getenv("GLQ_NO_PDL") != nullptr;
+    attr.val.programmaticStreamSerializationAllowed = off ? 0 : 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 extern "C" int glq_add_rmsnorm(const void* x, const void* delta, const void* weight, float eps, int rows, int H, void* x_out,
                                void* h_out, void* stream) {
     if (!x || !delta || !x_out || !h_out || rows < 0 || H <= 0) return GLQ_ERR_ARG;
     if (H % 8 != 0 || H > 8192) return GLQ_ERR_UNSUPPORTED;
     if (rows == 0) return GLQ_OK;
-    add_rmsnorm_kernel<<<rows, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-        reinterpret_cast<const __half*>(x), reinterpret_cast<const __half*>(delta), reinterpret_cast<const __half*>(weight), eps,
-        H, reinterpret_cast<__half*>(x_out), reinterpret_cast<__half*>(h_out));
-    return cudaGetLastError() == cudaSuccess ? GLQ_OK : GLQ_ERR_CUDA;
+    return launch_dependent(add_rmsnorm_kernel, dim3(rows), dim3(256), reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const __half*>(x),
+                            reinterpret_cast<const __half*>(delta), reinterpret_cast<const __half*>(weight), eps, H,
+                            reinterpret_cast<__half*>(x_out), reinterpret_cast<__half*>(h_out)) == cudaSuccess
+               ? GLQ_OK : GLQ_ERR_CUDA;
 }
 
 // position splits per head: enough CTAs to fill the device for long caches
