@@ -108,40 +108,48 @@ __host__ __device__ inline size_t skinny_smem_bytes(int fmt, int kb_cta, int ntc
 // Activation staging: x rows -> shared memory in fragment order, plus per k block the two sums the
 // affine formats need: O = sum off(k) x_k (offset carried by the unpack) and X = sum x_k.
 // ---------------------------------------------------------------------------------------------
-template <int FMT>
+// Only live rows are staged; a column of no row keeps what was there, and its sums go nowhere.  Rows come from L2 at a latency of
+// about a microsecond: the loads of BATCH units of 16 channels are on their way together (32 rows of 2048 channels: 13.6 -> 11.5 us
+// a launch with four, 16 rows 7.7 -> 6.6; beside the codes of the packed formats in flight four of them spill, and a thread's one
+// unit of a row or two comes later behind three empty ones).
+template <int FMT, int BATCH = 1>
 __device__ __forceinline__ void stage_x(const SkinnyParams& p, uint4* xs, float2* ox, int kb_lo, int nkb_cta,
                                         int e0, int pass0, int cnt, int K) {
     using F = Fmt<FMT>;
-    const int ntc = p.ntc;
-    const int total = ntc * nkb_cta * F::UPK;
-    for (int base = 0; base < total; base += kThreads) {
-        const int u = base + (int)threadIdx.x;
-        const bool valid = u < total;
-        const int col = valid ? u / (nkb_cta * F::UPK) : 0;
-        const int rem = valid ? u % (nkb_cta * F::UPK) : 0;
-        const int kbl = rem / F::UPK, wi = rem % F::UPK;
-        const int k0 = (kb_lo + kbl) * F::KB + wi * 16;
-        __align__(16) __half v[16];
-        const bool live = valid && (pass0 + col < cnt) && (k0 < K);
-        if (live) {
-            const int entry = e0 + pass0 + col;
-            const long long row = p.entry_row ? p.entry_row[entry] : entry;
-            const __half* src = p.x + row * p.ldx + k0;
-            if (!GLQ_OKAY(p.x_extent == 0 || (row >= 0 && row * p.ldx + k0 + min(16, K - k0) <= p.x_extent), 21,
-                          row * p.ldx + k0, p.x_extent)) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = __float2half(0.f);
-            } else if (p.x_vec && k0 + 16 <= K) {
-                *reinterpret_cast<uint4*>(&v[0]) = __ldg(reinterpret_cast<const uint4*>(src));
-                *reinterpret_cast<uint4*>(&v[8]) = __ldg(reinterpret_cast<const uint4*>(src) + 1);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = (k0 + j < K) ? src[j] : __float2half(0.f);
-            }
+    const int ntc = p.ntc, ncol = min(ntc, cnt - pass0);
+    const int per = nkb_cta * F::UPK, total = ncol * per;
+    const int dcol = kThreads / per, drem = kThreads % per;
+    auto advance = [&](int& col, int& rem) {
+        col += dcol;
+        if ((rem += drem) >= per) rem -= per, ++col;
+    };
+    auto load = [&](int col, int rem, uint4 (&v)[2]) {
+        v[0] = v[1] = make_uint4(0, 0, 0, 0);
+        const int k0 = kb_lo * F::KB + rem * 16;
+        if (col >= ncol || k0 >= K) return;
+        const int entry = e0 + pass0 + col;
+        const long long row = p.entry_row ? p.entry_row[entry] : entry;
+        const __half* src = p.x + row * p.ldx + k0;
+        if (!GLQ_OKAY(p.x_extent == 0 || (row >= 0 && row * p.ldx + k0 + min(16, K - k0) <= p.x_extent), 21,
+                      row * p.ldx + k0, p.x_extent))
+            return;
+        if (p.x_vec && k0 + 16 <= K) {
+            v[0] = __ldg(reinterpret_cast<const uint4*>(src));
+            v[1] = __ldg(reinterpret_cast<const uint4*>(src) + 1);
         } else {
+            __align__(16) __half h[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __float2half(0.f);
+            for (int j = 0; j < 16; ++j) h[j] = (k0 + j < K) ? src[j] : __float2half(0.f);
+            v[0] = reinterpret_cast<const uint4*>(h)[0];
+            v[1] = reinterpret_cast<const uint4*>(h)[1];
         }
+    };
+    auto store = [&](int col, int rem, const uint4 (&raw)[2]) {
+        const bool valid = col < ncol;
+        const int kbl = rem / F::UPK, wi = rem % F::UPK;
+        __align__(16) __half v[16];
+        *reinterpret_cast<uint4*>(&v[0]) = raw[0];
+        *reinterpret_cast<uint4*>(&v[8]) = raw[1];
         __align__(16) __half o[16];
         if constexpr (FMT == GLQ_FMT_Q2) {
             // piece pp holds codes [0,8,1,9,2,10,3,11] (+4 for pp = 1)
@@ -216,6 +224,22 @@ __device__ __forceinline__ void stage_x(const SkinnyParams& p, uint4* xs, float2
             }
             if (valid && wi == 0 && GLQ_OKAY(kbl * ntc + col < p.kb_chunk * ntc, 4, kbl * ntc + col, p.kb_chunk * ntc))
                 ox[kbl * ntc + col] = make_float2(so, sx);
+        }
+    };
+    int col = threadIdx.x / per, rem = threadIdx.x % per;
+    for (int base = 0; base < total; base += BATCH * kThreads) {
+        uint4 v[BATCH][2];
+        int lcol = col, lrem = rem;
+#pragma unroll
+        for (int b = 0; b < BATCH; ++b) {
+            load(lcol, lrem, v[b]);
+            advance(lcol, lrem);
+        }
+#pragma unroll
+        for (int b = 0; b < BATCH; ++b) {
+            if (base + b * kThreads >= total) break;
+            store(col, rem, v[b]);
+            advance(col, rem);
         }
     }
 }
@@ -434,7 +458,7 @@ __device__ __forceinline__ void skinny_body(const SkinnyParams& p, int bid, int*
             }
             if (PAIRED && iter == 0) asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
             if (iter++ > 0) sync();  // everyone is done with the previous contents of shared memory
-            stage_x<FMT>(p, xs, ox, kc_lo, nkc, e0, pass0, cnt, K);
+            stage_x<FMT, FMT == GLQ_FMT_F16 && NTT >= 2 ? 4 : 1>(p, xs, ox, kc_lo, nkc, e0, pass0, cnt, K);
             sync();
 
 #pragma unroll
