@@ -313,6 +313,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) rope_prefill_kernel(
     const bool vec = vec_i != 0;
     const int lane = threadIdx.x & 31;
     const int bt = blockIdx.x, b = bt / T, t = bt - b * T;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     long long pos = positions[t];
     if (pos < 0) pos = 0;
     if (pos >= max_len) pos = max_len - 1;
@@ -404,6 +405,7 @@ __global__ void __launch_bounds__(128, 3) attn_prefill_kernel(const __half* __re
     // launch order = work order: the query blocks with the most keys first, over all heads and batch rows
     const int n_hb = n_heads * B;
     const int qb = (int)(gridDim.x / n_hb) - 1 - (int)(blockIdx.x / n_hb);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int h = (int)(blockIdx.x % n_hb) % n_heads, b = (int)(blockIdx.x % n_hb) / n_heads;
     const int kvh = h / (n_heads / n_kv);
     const int q0 = qb * C::BM + warp * 16;                      // first query row of this warp
@@ -612,28 +614,12 @@ __global__ void __launch_bounds__(256) add_rmsnorm_kernel(const __half* __restri
 
 }  // namespace
 
-// launch with programmatic stream serialization: the grid may start before the launch ahead of it has ended and waits for it itself
-template <typename... P, typename... A>
-static cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    static const bool off = std::getenv("GLQ_NO_PDL") != nullptr;
-    attr.val.programmaticStreamSerializationAllowed = off ? 0 : 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
-}
-
 extern "C" int glq_add_rmsnorm(const void* x, const void* delta, const void* weight, float eps, int rows, int H, void* x_out,
                                void* h_out, void* stream) {
     if (!x || !delta || !x_out || !h_out || rows < 0 || H <= 0) return GLQ_ERR_ARG;
     if (H % 8 != 0 || H > 8192) return GLQ_ERR_UNSUPPORTED;
     if (rows == 0) return GLQ_OK;
-    return launch_dependent(add_rmsnorm_kernel, dim3(rows), dim3(256), reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const __half*>(x),
+    return launch_beside(add_rmsnorm_kernel, dim3(rows), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const __half*>(x),
                             reinterpret_cast<const __half*>(delta), reinterpret_cast<const __half*>(weight), eps, H,
                             reinterpret_cast<__half*>(x_out), reinterpret_cast<__half*>(h_out)) == cudaSuccess
                ? GLQ_OK : GLQ_ERR_CUDA;
@@ -709,8 +695,9 @@ extern "C" int glq_rope_prefill(void* q, void* k, const void* v, const void* cos
     for (const void* ptr : {(const void*)q, (const void*)k, v, cos_t, sin_t, (const void*)k_cache, (const void*)v_cache})
         if (reinterpret_cast<uintptr_t>(ptr) & 7u) vec = 0;
     auto st = reinterpret_cast<cudaStream_t>(stream);
+    cudaError_t rc = cudaSuccess;
 #define GLQ_ROPE_CASE(EPL)                                                                                                  \
-    rope_prefill_kernel<EPL><<<grid, kAttnWarps * 32, 0, st>>>(                                                             \
+    rc = launch_beside(rope_prefill_kernel<EPL>, grid, dim3(kAttnWarps * 32), 0, st,                                        \
         reinterpret_cast<__half*>(q), reinterpret_cast<__half*>(k), reinterpret_cast<const __half*>(v),                     \
         reinterpret_cast<const __half*>(cos_t), reinterpret_cast<const __half*>(sin_t),                                     \
         reinterpret_cast<const long long*>(positions), reinterpret_cast<__half*>(k_cache), reinterpret_cast<__half*>(v_cache), \
@@ -723,7 +710,7 @@ extern "C" int glq_rope_prefill(void* q, void* k, const void* v, const void* cos
         default: return GLQ_ERR_UNSUPPORTED;
     }
 #undef GLQ_ROPE_CASE
-    return cudaGetLastError() == cudaSuccess ? GLQ_OK : GLQ_ERR_CUDA;
+    return rc == cudaSuccess ? GLQ_OK : GLQ_ERR_CUDA;
 }
 
 extern "C" int glq_attn_prefill(const void* q, const void* k, const void* v, void* y, int B, int T, int n_heads, int n_kv,
@@ -737,6 +724,7 @@ extern "C" int glq_attn_prefill(const void* q, const void* k, const void* v, voi
         if ((reinterpret_cast<uintptr_t>(ptr) & 15u) != 0) return GLQ_ERR_ALIGN;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     const dim3 grid((unsigned)((T + 63) / 64 * n_heads * B));     // every (query block, head, batch row), most keys first
+    cudaError_t rc = cudaSuccess;
 #define GLQ_PREFILL(HD)                                                                                                  \
     {                                                                                                                    \
         static bool configured[64] = {};                                                                                 \
@@ -748,11 +736,11 @@ extern "C" int glq_attn_prefill(const void* q, const void* k, const void* v, voi
                 return GLQ_ERR_CUDA;                                                                                     \
             if (dev >= 0 && dev < 64) configured[dev] = true;                                                            \
         }                                                                                                                \
-        attn_prefill_kernel<HD><<<grid, 128, PrefillCfg<HD>::SMEM, st>>>(                                                \
+        rc = launch_beside(attn_prefill_kernel<HD>, grid, dim3(128), PrefillCfg<HD>::SMEM, st,                           \
             reinterpret_cast<const __half*>(q), reinterpret_cast<const __half*>(k), reinterpret_cast<const __half*>(v),  \
             reinterpret_cast<__half*>(y), B, T, n_heads, n_kv);                                                              \
     }
     if (head_dim == 64) GLQ_PREFILL(64) else GLQ_PREFILL(128)
 #undef GLQ_PREFILL
-    return cudaGetLastError() == cudaSuccess ? GLQ_OK : GLQ_ERR_CUDA;
+    return rc == cudaSuccess ? GLQ_OK : GLQ_ERR_CUDA;
 }

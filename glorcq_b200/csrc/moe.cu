@@ -330,6 +330,7 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const __half* __restrict
                                                         int* __restrict__ sel_out, __half* __restrict__ wts_out,
                                                         const int* __restrict__ sel_in, const __half* __restrict__ wts_in) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (sel_in) {   // routing decided by the caller: copy it; an index outside [0, E) marks a dropped slot
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n * k; i += gridDim.x * blockDim.x) {
             const int e = sel_in[i];
@@ -347,6 +348,7 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const __half* __restrict
 __global__ void __launch_bounds__(32) moe_plan_count_kernel(const int* __restrict__ sel, int nk, int E, int* __restrict__ blk) {
     extern __shared__ int sm_c[];
     const int lane = threadIdx.x, b = blockIdx.x;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int e = lane; e < E; e += 32) sm_c[e] = 0;
     __syncwarp();
     const int i_end = min(nk, (b + 1) * kPlanChunk);
@@ -373,6 +375,7 @@ __global__ void __launch_bounds__(1024) moe_plan_lists_kernel(int* __restrict__ 
                                                               int* __restrict__ active2, int* __restrict__ n_active2,
                                                               int* __restrict__ slot_count2, int* __restrict__ slot_offset2) {
     extern __shared__ int sm_cnt[];  // [E] counts, then [E] offsets
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     int* sm_off = sm_cnt + E;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int e = threadIdx.x; e < E; e += blockDim.x) {
@@ -401,6 +404,7 @@ __global__ void __launch_bounds__(32) moe_plan_scatter_kernel(const int* __restr
                                                               int* __restrict__ tok_entries) {
     extern __shared__ int sm_b[];
     const int lane = threadIdx.x, b = blockIdx.x;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const unsigned lt = (1u << lane) - 1u;
     for (int e = lane; e < E; e += 32) sm_b[e] = blk[(size_t)b * E + e];
     __syncwarp();
@@ -1034,16 +1038,19 @@ extern "C" int glq_moe_forward_ep(const glq_moe_desc_t* d, const void* x, int n,
         int* blk = reinterpret_cast<int*>(ws + L.plan_blk);
         const int* s_in = given ? (const int*)ep->sel_in : (const int*)nullptr;
         const __half* w_in = given ? reinterpret_cast<const __half*>(ep->weight_in) : (const __half*)nullptr;
-        moe_route_kernel<<<given ? std::min(1024, (nk + 255) / 256) : (n + 7) / 8, 256, 0, st>>>(
+        cudaError_t e = launch_beside(
+            moe_route_kernel, dim3(given ? std::min(1024, (nk + 255) / 256) : (n + 7) / 8), dim3(256), 0, st,
             (const __half*)p_logits, ldl, n, (int)d->E, k, (int)d->norm_topk_prob, p_sel, p_wts, p_tok,
             reinterpret_cast<__half*>(router_logits), (int*)sel_out, reinterpret_cast<__half*>(weight_out), s_in, w_in);
-        moe_plan_count_kernel<<<nb, 32, d->E * sizeof(int), st>>>(p_sel, nk, (int)d->E, blk);
-        moe_plan_lists_kernel<<<1, 1024, 2 * d->E * sizeof(int), st>>>(
-            blk, nb, nk, (int)d->E, chunk, ep_rank, ep_world, p_active, p_nact, p_cnt, p_off,
-            reinterpret_cast<int*>(ws + L.active2), reinterpret_cast<int*>(ws + L.n_active2),
-            reinterpret_cast<int*>(ws + L.slot_count2), reinterpret_cast<int*>(ws + L.slot_offset2));
-        moe_plan_scatter_kernel<<<nb, 32, d->E * sizeof(int), st>>>(p_sel, p_wts, nk, (int)d->E, k, blk, p_erow, p_escale, p_tok);
-        if (cudaGetLastError() != cudaSuccess) return GLQ_ERR_CUDA;
+        if (e == cudaSuccess) e = launch_beside(moe_plan_count_kernel, dim3(nb), dim3(32), d->E * sizeof(int), st, p_sel, nk, (int)d->E, blk);
+        if (e == cudaSuccess)
+            e = launch_beside(moe_plan_lists_kernel, dim3(1), dim3(1024), 2 * d->E * sizeof(int), st,
+                              blk, nb, nk, (int)d->E, chunk, ep_rank, ep_world, p_active, p_nact, p_cnt, p_off,
+                              reinterpret_cast<int*>(ws + L.active2), reinterpret_cast<int*>(ws + L.n_active2),
+                              reinterpret_cast<int*>(ws + L.slot_count2), reinterpret_cast<int*>(ws + L.slot_offset2));
+        if (e == cudaSuccess)
+            e = launch_beside(moe_plan_scatter_kernel, dim3(nb), dim3(32), d->E * sizeof(int), st, p_sel, p_wts, nk, (int)d->E, k, blk, p_erow, p_escale, p_tok);
+        if (e != cudaSuccess) return GLQ_ERR_CUDA;
         after_kernel[0] = true;
     } else {
         // (a programmatically dependent launch after the router product measured no faster)

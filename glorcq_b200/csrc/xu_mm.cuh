@@ -41,8 +41,8 @@ template <int NT, bool VEC>
 __global__ void __launch_bounds__(kXuThreads) xu_kernel(const TcParams p) {
     using C = XuCfg<NT>;
     extern __shared__ __align__(128) unsigned char smem[];
-    // (launched plainly, after all before it; the pre-pass of the product that takes x.U may start beside it)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // (in this order: the pre-pass of the product that takes x.U may start beside this kernel, but after all before it)
+    asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
     int slot, lt, cnt, e0;
     if (!tc_find_tile<C::ROWS>(p, blockIdx.x, slot, lt, cnt, e0)) return;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t = lane & 3;

@@ -523,3 +523,37 @@ def test_low_rank_operand_in_the_products_launch(dev, fmt, bits, N, K, rank, B):
         assert torch.equal(tiled.linear_forward(lin._tiled, x, lin._ut), ref)
     torch.cuda.synchronize()
     assert not bool(_lib.native().workspace(0, 0, 0)[1].any()) and tiled.debug_error() is None
+
+
+@pytest.mark.parametrize("rows", [1, 8, 33, 300])
+def test_layer_captured_behind_an_event(dev, rows):
+    """A layer's first launch may start beside the launch ahead of it; behind an event of another stream, in a graph and
+    outside, it still sees what that stream wrote."""
+    d = cases.make_linear(4100 + rows, 256, 512, rank=32)
+    lin = cases.to_b200_linear(d, dev)
+    x = cases.make_x(4200 + rows, rows, 512).to(dev)
+    side = torch.cuda.Stream()
+
+    def step():
+        main = torch.cuda.current_stream()
+        big = torch.ones(1 << 24, device=dev).cumsum(0)          # (the writer of the layer's input starts late)
+        x2 = x + x + 0 * big[0].half()
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            y = lin(x2)
+        main.wait_stream(side)
+        return y + 0
+    want = lin(x + x)
+    for _ in range(2):
+        assert torch.equal(step(), want)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = step()
+    for _ in range(3):
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)
+    from glorcq_b200 import tiled
+    assert tiled.debug_error() is None
