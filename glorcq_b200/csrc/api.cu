@@ -1317,6 +1317,12 @@ static int launch_rht_e(const void* x, int64_t ldx, const float* signs, int rows
     auto kern = rht_kernel<E, TI, TO>;
     if (smem > 48 * 1024) GLQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int vec = aligned16(x) && ldx % 8 == 0 ? 1 : 0;
+    // (more rows than SMs gain nothing from waiting beside the launch ahead)
+    if (rows <= num_sms()) {
+        GLQ_CUDA(launch_beside(kern, dim3(rows), dim3(threads), smem, st, reinterpret_cast<const TI*>(x), (long long)ldx, signs, d, n, scale,
+                               reinterpret_cast<TO*>(y), (long long)ldy, vec));
+        return GLQ_OK;
+    }
     kern<<<rows, threads, smem, st>>>(reinterpret_cast<const TI*>(x), ldx, signs, d, n, scale, reinterpret_cast<TO*>(y), ldy, vec);
     GLQ_CUDA(cudaGetLastError());
     return GLQ_OK;

@@ -252,8 +252,8 @@ template <int E, typename TI, typename TO>
 __global__ void __launch_bounds__(E >= 5 ? 1024 : 512) rht_kernel(const TI* __restrict__ x, long long ldx, const float* __restrict__ signs,
                                                                   int d, int n, float scale, TO* __restrict__ y, long long ldy, int vec) {
     extern __shared__ float rht_buf[];
-    // (the product behind it may fetch its weights meanwhile)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // (in this order; the product behind it may fetch its weights meanwhile)
+    asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
     constexpr int V = 1 << E;
     const TI* xr = x + (size_t)blockIdx.x * ldx;
     TO* yr = y + (size_t)blockIdx.x * ldy;

@@ -262,6 +262,7 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const __half* __restrict
     int* sm_off = sm_cnt + E;
     int* s_sel = sm_off + E;
     __half* s_wts = reinterpret_cast<__half*>(s_sel + n * k);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     // Phase A: one warp per token, lanes over experts (E <= 256)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     if (sel_in) {
@@ -980,8 +981,8 @@ extern "C" int glq_moe_forward_ep(const glq_moe_desc_t* d, const void* x, int n,
     // library's launches (not the first launch of the call, not after an event wait)
     bool after_kernel[2] = {false, false};
     auto finish = [&](glq_mm_args_t& mm) {
-        // (chaining every launch this way, GLQ_MM_AFTER_KERNEL, measured no faster than plain launches
-        // inside a graph: only the two x.U edges, whose consumers have real independent work, are used)
+        // (GLQ_MM_AFTER_KERNEL: behind launches of a few CTAs only.  CTAs that wait beside a product for its end take places that the
+        // other stream needs)
         if (!after_kernel[on_aux ? 1 : 0]) mm.flags &= ~GLQ_MM_A_FROM_PREVIOUS_LAUNCH;
         if (on_aux && forked && share_sm()) mm.flags |= GLQ_MM_SHARE_SM;      // the routed products run beside it
         after_kernel[on_aux ? 1 : 0] = true;
@@ -1026,6 +1027,7 @@ extern "C" int glq_moe_forward_ep(const glq_moe_desc_t* d, const void* x, int n,
         m.ldx = d->H;
         m.y = p_logits;
         m.ldy = ldl;
+        if (d->rht_in) m.flags = GLQ_MM_AFTER_KERNEL;
         if ((rc = finish(m)) != GLQ_OK) return rc;
     }
 
@@ -1053,15 +1055,15 @@ extern "C" int glq_moe_forward_ep(const glq_moe_desc_t* d, const void* x, int n,
         if (e != cudaSuccess) return GLQ_ERR_CUDA;
         after_kernel[0] = true;
     } else {
-        // (a programmatically dependent launch after the router product measured no faster)
         const size_t smem = 2 * d->E * sizeof(int) + (size_t)nk * (sizeof(int) + sizeof(__half));
-        moe_plan_kernel<<<1, 1024, smem, st>>>(
-            p_logits, ldl, n, (int)d->E, k, (int)d->norm_topk_prob, p_sel, p_wts, p_active, p_nact, p_cnt, p_off, p_erow, p_escale, p_tok,
+        const cudaError_t e = launch_beside(
+            moe_plan_kernel, dim3(1), dim3(1024), smem, st,
+            (const __half*)p_logits, ldl, n, (int)d->E, k, (int)d->norm_topk_prob, p_sel, p_wts, p_active, p_nact, p_cnt, p_off, p_erow, p_escale, p_tok,
             reinterpret_cast<__half*>(router_logits), (int*)sel_out, reinterpret_cast<__half*>(weight_out),
             reinterpret_cast<int*>(ws + L.active2), reinterpret_cast<int*>(ws + L.n_active2),
             reinterpret_cast<int*>(ws + L.slot_count2), reinterpret_cast<int*>(ws + L.slot_offset2), ep_rank, ep_world,
             given ? (const int*)ep->sel_in : nullptr, given ? reinterpret_cast<const __half*>(ep->weight_in) : nullptr, chunk);
-        if (cudaGetLastError() != cudaSuccess) return GLQ_ERR_CUDA;
+        if (e != cudaSuccess) return GLQ_ERR_CUDA;
         after_kernel[0] = true;
     }
     // rows of remote experts' entries stay zero, so that summing the ranks' buffers is exact
@@ -1092,6 +1094,7 @@ extern "C" int glq_moe_forward_ep(const glq_moe_desc_t* d, const void* x, int n,
         m.ldx = d->H;
         m.y = a_gate;
         m.ldy = R;
+        if (ep_world == 1) m.flags = GLQ_MM_AFTER_KERNEL;       // (else a memset lies in between)
         if ((rc = finish(m)) != GLQ_OK) return rc;
     }
     // 4. h = silu(gate x) * (up x), one row per (token, expert) entry
@@ -1139,6 +1142,7 @@ extern "C" int glq_moe_forward_ep(const glq_moe_desc_t* d, const void* x, int n,
         m.lda = R;
         if (hq == ws + L.h) m.flags = GLQ_MM_A_FROM_PREVIOUS_LAUNCH;   // h.U directly before; not when a rotation sits between
     }
+    if (d->rht_mid) m.flags = GLQ_MM_AFTER_KERNEL;
     m.y = p_yd;
     m.ldy = d->H;
     if ((rc = finish(m)) != GLQ_OK) return rc;
