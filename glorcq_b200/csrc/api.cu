@@ -172,13 +172,8 @@ template <int FMT, int NW, int NTT, bool RM, int TGN = 1>
 static int launch_one(const SkinnyParams& p, int grid, size_t smem, cudaStream_t st) {
     auto kern = skinny_kernel<FMT, NW, NTT, RM, TGN>;
     if (smem > 48 * 1024) {
-        static size_t configured[16] = {0};
-        int dev = 0;
-        GLQ_CUDA(cudaGetDevice(&dev));
-        if (dev < 0 || dev >= 16 || configured[dev] < smem) {
-            GLQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            if (dev >= 0 && dev < 16) configured[dev] = smem;
-        }
+        static SmemLimit limit;
+        GLQ_CUDA(reserve_smem(reinterpret_cast<const void*>(kern), limit, smem));
     }
     if (t_dependent_launch) return launch_dependent(kern, dim3(grid), dim3(kThreads), smem, st, p);
     kern<<<grid, kThreads, smem, st>>>(p);
@@ -380,13 +375,8 @@ static bool plan_stream(int fmt, int epilogue, int N, int K, int rank, int group
 template <int FMT, bool I8, int NT, int NW = 8>
 static int launch_stream_one(const StreamParams& sp, const StreamGeom& g, cudaStream_t st) {
     auto kern = stream_kernel<FMT, I8, NT, NW>;
-    static size_t configured[16] = {0};
-    int dev = 0;
-    GLQ_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 16 || configured[dev] < g.smem) {
-        GLQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
-        if (dev >= 0 && dev < 16) configured[dev] = g.smem;
-    }
+    static SmemLimit limit;
+    GLQ_CUDA(reserve_smem(reinterpret_cast<const void*>(kern), limit, g.smem));
     if (sp.a_late || sp.dependent) return launch_dependent(kern, dim3(g.grid), dim3(NW * 32), g.smem, st, sp);
     kern<<<g.grid, NW * 32, g.smem, st>>>(sp);
     GLQ_CUDA(cudaGetLastError());
@@ -409,13 +399,8 @@ static int launch_stream_fmt(const StreamParams& sp, const StreamGeom& g, cudaSt
 template <int FMT, bool I8, int NT, int NW = 8>
 static int launch_stream_pair_t(const StreamParams& sp, const StreamGeom& g, const SkinnyParams& xu, int n_xu, cudaStream_t st) {
     auto kern = stream_pair_kernel<FMT, I8, NT, NW>;
-    static size_t configured[16] = {0};
-    int dev = 0;
-    GLQ_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 16 || configured[dev] < g.smem) {
-        GLQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
-        if (dev >= 0 && dev < 16) configured[dev] = g.smem;
-    }
+    static SmemLimit limit;
+    GLQ_CUDA(reserve_smem(reinterpret_cast<const void*>(kern), limit, g.smem));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(g.grid + n_xu);
     cfg.blockDim = dim3(NW * 32);
@@ -1125,22 +1110,15 @@ extern "C" int glq_gptq_dequant_matmul(const float* x, const int8_t* q, const vo
     int per = 8;
     while (per > 1 && smem * per > 200 * 1024) per /= 2;
     if (smem > 200 * 1024) return GLQ_ERR_UNSUPPORTED;
-    static size_t configured[2][64] = {{0}, {0}};
-    int dev = 0;
-    GLQ_CUDA(cudaGetDevice(&dev));
+    static SmemLimit limit[2];
     for (int b0 = 0; b0 < B; b0 += per) {
         const int nb = std::min(per, B - b0);
         const int wide = nb > 4 ? 1 : 0;
         const dim3 grid(cdiv(N, kWarpsPerCta));
         const size_t need = smem * nb;
-        if (need > 48 * 1024 && (dev < 0 || dev >= 64 || configured[wide][dev] < need)) {
-            if (wide)
-                GLQ_CUDA(cudaFuncSetAttribute(gptq_i8_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem * per)));
-            else
-                GLQ_CUDA(cudaFuncSetAttribute(gptq_i8_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              (int)(smem * std::min(per, 4))));
-            if (dev >= 0 && dev < 64) configured[wide][dev] = wide ? smem * per : smem * std::min(per, 4);
-        }
+        if (need > 48 * 1024)
+            GLQ_CUDA(reserve_smem(wide ? reinterpret_cast<const void*>(gptq_i8_kernel<8>) : reinterpret_cast<const void*>(gptq_i8_kernel<4>),
+                                  limit[wide], smem * (wide ? per : std::min(per, 4))));
         const float* xb = x + (size_t)b0 * K;
         const float* lb = lora_out ? lora_out + (size_t)b0 * N : nullptr;
         float* yb = y + (size_t)b0 * N;

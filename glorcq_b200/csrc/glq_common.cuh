@@ -7,7 +7,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstdlib>
+#include <mutex>
 
 #include "../../include/glorcq_b200.h"
 
@@ -144,6 +146,25 @@ __device__ __forceinline__ float warp_sum(float v) {
 __device__ __forceinline__ uint32_t pack_half2(float a, float b) {
     __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<uint32_t*>(&h);
+}
+
+// Dynamic shared memory that one kernel may use, raised as calls need it.  Calls of several threads meet here: setting the attribute
+// and noting it is one step, so that no smaller size is set after a larger one was noted.
+struct SmemLimit {
+    std::atomic<size_t> set[64];
+};
+static inline cudaError_t reserve_smem(const void* kern, SmemLimit& l, size_t smem) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const bool known = dev >= 0 && dev < 64;
+    if (known && l.set[dev].load(std::memory_order_acquire) >= smem) return cudaSuccess;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    if (known && l.set[dev].load(std::memory_order_relaxed) >= smem) return cudaSuccess;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && known) l.set[dev].store(smem, std::memory_order_release);
+    return e;
 }
 
 // Launch with programmatic stream serialization: the grid may start before the launch ahead of it has ended and waits for it itself

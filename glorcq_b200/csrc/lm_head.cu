@@ -244,14 +244,8 @@ int lm_grid() {
 template <int NT, int D>
 int lm_pass(const LmParams& p, int grid, cudaStream_t st) {
     const size_t smem = lm_smem_bytes(NT, p.H);
-    static size_t configured[64] = {0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return GLQ_ERR_CUDA;
-    if (smem > 48 * 1024 && (dev < 0 || dev >= 64 || configured[dev] < smem)) {
-        if (cudaFuncSetAttribute(lm_head_kernel<NT, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return GLQ_ERR_CUDA;
-        if (dev >= 0 && dev < 64) configured[dev] = smem;
-    }
+    static glq::SmemLimit limit;
+    if (smem > 48 * 1024 && glq::reserve_smem(reinterpret_cast<const void*>(lm_head_kernel<NT, D>), limit, smem) != cudaSuccess) return GLQ_ERR_CUDA;
     lm_head_kernel<NT, D><<<grid, kLmThreads, smem, st>>>(p);
     return cudaGetLastError() == cudaSuccess ? GLQ_OK : GLQ_ERR_CUDA;
 }

@@ -798,19 +798,19 @@ bool plan_fused(const glq_moe_desc_t* d, int n, FusedParams* out, size_t* smem_b
 template <int FMT>
 int launch_fused_t(const FusedParams& P, size_t smem, cudaStream_t st) {
     auto kern = moe_fused_kernel<FMT>;
-    static size_t configured[64] = {0};
-    static int resident[64] = {0};
+    static SmemLimit limit;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return GLQ_ERR_CUDA;
     if (dev < 0 || dev >= 64) return GLQ_ERR_UNSUPPORTED;
-    if (configured[dev] < smem) {
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return GLQ_ERR_CUDA;
+    // (sizes are a CTA of an SM each: what holds for the first holds for all)
+    static std::atomic<int> resident[64];
+    if (reserve_smem(reinterpret_cast<const void*>(kern), limit, smem) != cudaSuccess) return GLQ_ERR_CUDA;
+    if (resident[dev].load(std::memory_order_relaxed) == 0) {
         int nb = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, kFT, smem) != cudaSuccess) return GLQ_ERR_CUDA;
-        resident[dev] = nb;
-        configured[dev] = smem;
+        resident[dev].store(nb, std::memory_order_relaxed);
     }
-    if (resident[dev] < 1) return GLQ_ERR_UNSUPPORTED;
+    if (resident[dev].load(std::memory_order_relaxed) < 1) return GLQ_ERR_UNSUPPORTED;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(fused_sms());
     cfg.blockDim = dim3(kFT);

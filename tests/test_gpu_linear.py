@@ -557,3 +557,34 @@ def test_layer_captured_behind_an_event(dev, rows):
         assert torch.equal(y, want)
     from glorcq_b200 import tiled
     assert tiled.debug_error() is None
+
+
+def test_threads_on_streams_of_their_own(dev):
+    """Calls of one kernel that need more and less shared memory, from threads on streams of their own."""
+    import threading
+    work = []
+    for i, (B, K) in enumerate(((4, 512), (8, 4096), (6, 2048), (3, 5632))):
+        lin = cases.to_b200_linear(cases.make_linear(150 + i, 256, K, rank=32), dev)
+        x = cases.make_x(160 + i, B, K).to(dev)
+        work.append((lin, x, torch.cuda.Stream()))
+    got, errors = {}, []
+    start = threading.Barrier(len(work))
+
+    def many(i, lin, x, st):
+        try:
+            start.wait()
+            with torch.cuda.stream(st):
+                got[i] = [lin(x) for _ in range(50)]
+        except Exception as e:      # noqa: BLE001
+            errors.append(e)
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=many, args=(i, *w)) for i, w in enumerate(work)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors
+    for i, (lin, x, _) in enumerate(work):
+        ref = lin(x)
+        assert all(torch.equal(y, ref) for y in got[i])
