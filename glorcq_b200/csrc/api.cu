@@ -719,7 +719,10 @@ static int launch_xu_t(TcParams& p, const glq_mm_args_t* a, cudaStream_t st) {
     p.tiles_max = one ? cdiv(a->max_rows, C::ROWS) : (int)(total_entries(a) / C::ROWS + a->n_problems + 1);
     // (not beside a launch that left SMs to another stream: CTAs that wait there would take that stream's places, and a routing plan
     // that starts 90 us later costs a 2000-token block 490 us instead of 470)
-    return launch_maybe_dependent(!pdl_disabled() && !t_share_sm, xu_kernel<NT, VEC>, dim3(p.tiles_max, cdiv(a->N, kXuCols)), dim3(kXuThreads), C::SMEM, st, p);
+    // (nor h.U behind the GEMM of many experts: its few CTAs lay two to an SM in the first places that came free; 300 tokens through eight
+    // Mixtral-shaped experts, codebook: 691 us against 663)
+    const bool beside = !t_share_sm && (!a->n_slots || (a->flags & GLQ_MM_AFTER_KERNEL) != 0);
+    return launch_maybe_dependent(!pdl_disabled() && beside, xu_kernel<NT, VEC>, dim3(p.tiles_max, cdiv(a->N, kXuCols)), dim3(kXuThreads), C::SMEM, st, p);
 }
 static int launch_xu(const glq_mm_args_t* a, cudaStream_t st) {
     if (!a->w_table && !a->w.codes) return GLQ_ERR_ARG;
