@@ -47,7 +47,10 @@
 
 namespace glq {
 
-constexpr int kPsQueue = 4;        // work items that may be handed out ahead of the slowest warp
+// Work items that may be handed out ahead of the slowest warp.  Two hide a look-up; with four a CTA held items back at the end that
+// others had time for (8 Mixtral-shaped experts, codebook, 300 tokens 663 us a block against 607; 2-bit, 600 tokens 803 against 734; a
+// 512-token prompt of 24 layers 8065 against 7905).
+constexpr int kPsQueue = 2;
 
 __device__ __forceinline__ void tc_st_x4(uint32_t taddr, const uint32_t (&r)[16]) {
     asm volatile(
