@@ -16,6 +16,7 @@ LIB_PATH = os.environ.get("GLQ_LIB") or os.path.join(HERE, "libglorcq_b200.so")
 
 FMT_Q2, FMT_Q4, FMT_T2, FMT_F16, FMT_Q3 = 0, 1, 2, 3, 4
 EPI_LINEAR, EPI_SWIGLU = 0, 1
+WEIGHT_SETTLED = 0x53455454
 
 vp = C.c_void_p
 

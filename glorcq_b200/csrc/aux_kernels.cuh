@@ -19,6 +19,9 @@ __device__ __forceinline__ size_t tiled_block_offset(int src_tile, int slot, int
     return (((size_t)(d >> 1) * nkb + kb) * 2 + (d & 1)) * bb;
 }
 
+// launched behind every packing kernel (api.cu, pack_end)
+__global__ void settle_kernel() {}
+
 // one thread per 32-bit word of the destination blocks of one source matrix
 __global__ void pack_gptq_kernel(const int32_t* __restrict__ q, const __half* __restrict__ scales,
                                  const __half* __restrict__ zeros, int bits, int N, int K, int group_size,

@@ -364,7 +364,8 @@ PyObject* py_grouped_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
             m.x = x.const_data_ptr();
             m.ldx = x.stride(0);
             if (xu) {
-                m.flags = GLQ_MM_A_FROM_PREVIOUS_LAUNCH;     // x.U was launched directly before
+                // x.U was launched directly before; the tables came by copies, the weights in them were packed
+                m.flags = GLQ_MM_A_FROM_PREVIOUS_LAUNCH | GLQ_MM_WEIGHTS_SETTLED;
                 m.a0 = xu->const_data_ptr();
                 m.lda = xu->size(2);
             }

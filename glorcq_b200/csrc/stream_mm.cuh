@@ -64,6 +64,7 @@ struct StreamParams {
     int a_late;   // 1: the x.U operand is still being written when this kernel starts (programmatic dependent launch)
     int* pair;    // {row tiles of x.U written, CTAs done}: zero between calls; x.U is computed by the first blocks of this launch
     int pair_target;
+    int settled;  // GLQ_WEIGHT_SETTLED holds: weights may be read before the launch ahead is complete
 };
 
 // ---- shared memory, mbarrier and bulk copy primitives ------------------------------------------
@@ -564,7 +565,7 @@ __device__ __forceinline__ void stream_body(const StreamParams& sp, int block, i
     };
     fetch_seek();
     while (f_live && f_inflight < S) fetch_one();
-    // The weights of a layer are older than the launch before this one: their first stages are requested before it is waited for.
+    // Weights that no launch writes which may still run: their first stages are requested before the launch ahead is waited for.
     // The next launch may come after the wait only, so that all launches before this one are complete when it starts.
     if constexpr (PAIRED) asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;" ::: "memory");
 
@@ -932,6 +933,7 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
 // 2-bit, rank 64 took 11.2 us a call, 7.7 now; 2 rows of 3-bit 2048 x 2048 10.8 and 7.5, 5 rows of codebook 5632 x 2048 16.4 and 14.4.
 template <int FMT, bool I8, int NT, int NW>
 __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) stream_pair_kernel(const StreamParams sp, const SkinnyParams xp, int n_xu) {
+    if (!sp.settled) asm volatile("griddepcontrol.wait;" ::: "memory");
     if ((int)blockIdx.x < n_xu) {
         if (NW > kWarpsPerCta && threadIdx.x >= kThreads) return;
         skinny_body<GLQ_FMT_F16, 1, 1, false, 1, true>(xp, blockIdx.x, sp.pair);

@@ -55,8 +55,14 @@ typedef struct glq_weight {
     int32_t N;              /* output features                                                   */
     int32_t K;              /* input features                                                    */
     int32_t rank;           /* low-rank width (multiple of 16), 0 = none                         */
-    int32_t reserved;
+    int32_t reserved;       /* 0, or GLQ_WEIGHT_SETTLED                                          */
 } glq_weight_t;
+/* In `reserved` of the descriptor given to glq_linear_forward: the call may read the descriptor's buffers and the U^T handed in
+ * with it while the launch issued on this stream immediately before the call still runs.  The caller's word that no kernel
+ * which may then still run writes them: neither that launch nor, if that launch lets dependent launches start before it has
+ * waited for it, the one before.  (Copies, fills and events are ordered in full; glq_pack_* see to it themselves.)  With any
+ * other value, 0 among them, weights are read when all before the call is complete. */
+#define GLQ_WEIGHT_SETTLED 0x53455454
 
 /* ---------------------------------------------------------------------------------------------
  * Library information
@@ -125,7 +131,8 @@ int glq_turbo_dequant_matmul_static(const void* x_rot, const uint8_t* packed, co
  * a pair is (gate tile p, up tile p) and one launch computes silu(gate x) * (up x).  The
  * destination buffers must be zero-filled before packing (padding tiles are not written).
  * These replace the (N,K) int32 / (N,K/4) uint8 / (N,G) fp16 tensors stored by the reference's
- * quantizer (joint_optim.py:319-327; turbo_weight_quantizer.py:149-156).
+ * quantizer (joint_optim.py:319-327; turbo_weight_quantizer.py:149-156).  Each call ends with an empty launch, so that a product
+ * that is started beside the launch ahead of it (GLQ_WEIGHT_SETTLED) finds the packed data complete.
  * ------------------------------------------------------------------------------------------ */
 size_t glq_tiled_bytes(int fmt, int n_rows, int K, int count);       /* codes (+ scales) buffer */
 size_t glq_sv_bytes(int n_rows, int rank, int count);                /* packed SV buffer         */
@@ -193,7 +200,8 @@ typedef struct glq_mm_args {
 } glq_mm_args_t;
 /* a0 / a1 are written by the launch issued on this stream immediately before this call, and nothing
  * else this call reads is: the kernel may then be launched programmatically dependent (it starts while
- * that launch still runs and waits for it only before the low-rank term). */
+ * that launch still runs and waits for it only before the low-rank term).  If that launch is not one of this library's, it
+ * must not let dependent launches start before it has waited for all before it. */
 #define GLQ_MM_A_FROM_PREVIOUS_LAUNCH 1
 /* The operation issued on this stream immediately before this call is a kernel launch of this library
  * (no event wait or foreign work in between): the launch may be programmatically dependent on it; the
@@ -201,6 +209,8 @@ typedef struct glq_mm_args {
 #define GLQ_MM_AFTER_KERNEL 2
 /* Another stream runs grouped products at the same time: use two thirds of the CTA slots, so that both find room. */
 #define GLQ_MM_SHARE_SM 4
+/* GLQ_WEIGHT_SETTLED for the weights, the descriptor tables and the U^T of a pair (glq_grouped_matmul_pair: of mm's flags). */
+#define GLQ_MM_WEIGHTS_SETTLED 8
 
 /* Scratch bytes / arrival counters a call with these args needs (both 0 when no CTA-level k split is
  * used).  The counters must be zero when a call starts and are zero again when it ends, so one

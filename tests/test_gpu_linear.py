@@ -588,3 +588,58 @@ def test_threads_on_streams_of_their_own(dev):
     for i, (lin, x, _) in enumerate(work):
         ref = lin(x)
         assert all(torch.equal(y, ref) for y in got[i])
+
+
+def _programmatic_edges(graph):
+    """[(kernel ahead, kernel started beside it)] of a captured graph of kernels"""
+    import ctypes as C
+    cu, g, n = C.CDLL("libcuda.so.1"), C.c_void_p(graph.raw_cuda_graph()), C.c_size_t(0)
+    assert cu.cuGraphGetEdges_v2(g, None, None, None, C.byref(n)) == 0
+    src, dst, data = (C.c_void_p * n.value)(), (C.c_void_p * n.value)(), (C.c_ubyte * (8 * n.value))()      # data: ports, then the type
+    assert cu.cuGraphGetEdges_v2(g, src, dst, data, C.byref(n)) == 0
+
+    def name(node):
+        p, s = (C.c_void_p * 16)(), C.c_char_p()             # CUDA_KERNEL_NODE_PARAMS_v2: func, seven ints, two pointers, kern
+        assert cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), p) == 0
+        rc = cu.cuFuncGetName(C.byref(s), C.c_void_p(p[0])) if p[0] else cu.cuKernelGetName(C.byref(s), C.c_void_p(p[7]))
+        assert rc == 0
+        return s.value.decode()
+    return [(name(a), name(b)) for a, b, kind in zip(src, dst, data[2::8]) if kind == 1]
+
+
+@pytest.mark.parametrize("fmt,bits", [("gptq", 2), ("gptq", 4), ("gptq", 3), ("turbo", 2)])
+@pytest.mark.parametrize("B", [1, 8])
+def test_layer_directly_behind_its_packing(dev, fmt, bits, B):
+    """A layer's launch reads weights while the launch ahead of it still runs: that is never the kernel which packs them.  Without the
+    caller's word in the descriptor it waits first."""
+    from glorcq_b200 import _lib, tiled
+    lin = cases.to_b200_linear(cases.make_linear(7100 + bits + B, 1408, 2048, rank=64, fmt=fmt, bits=bits), dev)
+    x = cases.make_x(7200 + B, B, 2048).to(dev)
+    pool = [(cases.make_x(7300 + i, 2048, 64).to(dev) * 0.01, cases.make_x(7400 + i, 1408, 64).to(dev) * 0.01) for i in range(2)]
+    refs = []
+    for U, SV in pool:
+        lin.load_sv(U, SV)
+        torch.cuda.synchronize()
+        refs.append(tiled.linear_forward(lin._tiled, x, a=tiled.dense_matmul(lin._ut, x)))
+    assert not torch.equal(*refs)
+    for i in range(20):                                 # the buffer of SV is packed anew, U^T comes from the pool
+        lin.load_sv(*pool[i % 2])
+        assert torch.equal(tiled.linear_forward(lin._tiled, x, lin._ut), refs[i % 2]), i
+    for i in range(20):                                 # and U^T packed last
+        lin.load_sv(pool[i % 2][0].clone(), pool[i % 2][1])
+        assert torch.equal(tiled.linear_forward(lin._tiled, x, lin._ut), refs[i % 2]), i
+    torch.cuda.synchronize()
+    for word in (_lib.WEIGHT_SETTLED, 0):
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            lin._tiled.put_sv(0, pool[1][1])
+            lin._tiled._native = None
+            lin._tiled.desc.reserved = word
+            y = [tiled.linear_forward(lin._tiled, x, lin._ut) for _ in range(2)]
+        edges = _programmatic_edges(graph)
+        assert ["pair" in b for _, b in edges] == [True, True] and not any("pack" in a for a, _ in edges), edges
+        lin._tiled.put_sv(0, pool[0][1])
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y[0], refs[1]) and torch.equal(y[1], refs[1])
+    assert tiled.debug_error() is None
