@@ -155,6 +155,31 @@ def test_decoder_logits_prefill_and_decode(dev, cfg, cache_len):
     assert cases.rel_l2(step.cpu(), ref[:, T:]) <= REL_LOGITS
 
 
+@pytest.mark.parametrize("rows,H", [(1, 8), (3, 2048), (2, 2056), (150, 8192)])
+def test_add_rmsnorm_behind_the_launch_that_writes_its_operands(dev, rows, H):
+    """x + delta and the norm of the sum, with x, delta and the weight written by the launch directly before, anew for each call; a
+    32-bit sum of squares against 64 bits, then one rounding to fp16 (2^-11) and one of the factor."""
+    from glorcq_b200 import _lib, tiled
+    g = torch.Generator().manual_seed(H + rows)
+    src = [torch.randn(2 * rows + 1, H, generator=g).half().to(dev) for _ in range(4)]
+    buf = torch.zeros_like(src[0])
+    x, delta, w = buf[:rows], buf[rows:2 * rows], buf[2 * rows]
+    xo, ho = torch.empty(rows, H, dtype=torch.float16, device=dev), torch.empty(rows, H, dtype=torch.float16, device=dev)
+    got = []
+    for i in range(8):
+        torch.add(src[i % 4], 0.25, out=buf)
+        _lib.check(_lib.lib().glq_add_rmsnorm(x.data_ptr(), delta.data_ptr(), w.data_ptr(), 1e-6, rows, H, xo.data_ptr(), ho.data_ptr(),
+                                              tiled._stream_ptr(dev)), "add_rmsnorm")
+        got.append((xo.clone(), ho.clone()))
+    for i, (gx, gh) in enumerate(got):
+        s = src[i % 4] + 0.25
+        want = s[:rows] + s[rows:2 * rows]
+        assert torch.equal(gx, want)
+        d = want.double()
+        ref = d * torch.rsqrt((d * d).mean(-1, keepdim=True) + 1e-6) * s[2 * rows].double()
+        assert ((gh.double() - ref).abs() <= 2.0 ** -10 * ref.abs() + 2.0 ** -24).all()
+
+
 @pytest.mark.parametrize("B,T,nh,nkv,hd,norms", [(1, 37, 4, 4, 128, False), (2, 19, 8, 2, 64, True), (1, 5, 2, 1, 32, True)])
 def test_rope_prefill_matches_tensor_ops(dev, B, T, nh, nkv, hd, norms):
     """The prompt's norms + rotary embedding + cache write in one launch against the fp16 tensor operations it
