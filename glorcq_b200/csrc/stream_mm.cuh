@@ -62,7 +62,7 @@ struct StreamParams {
     int cnt_lo, cnt_hi;  // only slots with cnt_lo < rows <= cnt_hi are this launch's (others belong to a sibling launch)
     int dependent;  // 1: launched with programmatic stream serialization
     int a_late;   // 1: the x.U operand is still being written when this kernel starts (programmatic dependent launch)
-    int* pair;    // {row tiles of x.U written, CTAs done}: zero between calls; x.U is computed by the first blocks of this launch
+    int* pair;    // {row tiles of x.U written, CTAs done + 2^16 for each that saw them all}: zero between calls; x.U is computed by the first blocks of this launch
     int pair_target;
     int settled;  // GLQ_WEIGHT_SETTLED holds: weights may be read before the launch ahead is complete
 };
@@ -912,9 +912,19 @@ __device__ __forceinline__ void stream_body(const StreamParams& sp, int block, i
         }
     }
     if constexpr (PAIRED) {
-        // the CTA that is done last clears both counters: every other one is past its wait
-        __syncthreads();
-        if (tid == 0 && atomicAdd(sp.pair + 1, 1) == n_blocks - 1) sp.pair[0] = sp.pair[1] = 0;
+        // The CTA that is done last clears both counters.  Once any CTA has seen all row tiles of x.U counted (the upper half of the second
+        // counter) no more come; where none has (every wait ran out, or no weight has a low-rank factor) they are taken off instead, so
+        // that those still to come leave zero too.  (Taking them off always: 0.1 to 0.4 us a call; counting x.U's blocks and
+        // clearing behind them 0.1, with a fence in every CTA 0.6 to 1.)
+        const int seen = __syncthreads_or(dep_waited && !dead) ? 0x10000 : 0;
+        if (tid == 0) {
+            const int done = atomicAdd(sp.pair + 1, 1 + seen) + seen;
+            if ((done & 0xffff) == n_blocks - 1) {
+                if (done >= 0x10000) sp.pair[0] = 0;
+                else atomicSub(sp.pair, sp.pair_target);
+                sp.pair[1] = 0;
+            }
+        }
     } else {
         // see the early exit above: a dependent grid ends only after the grid it depends on
         if (sp.a_late && !dep_waited) asm volatile("griddepcontrol.wait;" ::: "memory");

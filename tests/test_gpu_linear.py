@@ -643,3 +643,56 @@ def test_layer_directly_behind_its_packing(dev, fmt, bits, B):
         torch.cuda.synchronize()
         assert torch.equal(y[0], refs[1]) and torch.equal(y[1], refs[1])
     assert tiled.debug_error() is None
+
+
+@pytest.mark.parametrize("bits,N,K,rank,B", [(2, 32, 128, 16, 1), (2, 1408, 2048, 64, 1), (4, 2048, 2048, 128, 5), (3, 520, 896, 80, 8)])
+def test_counters_of_a_layer_in_one_launch(dev, bits, N, K, rank, B):
+    """The row tiles of x.U are counted in and taken off again, whether the product's wait for them ran out or not (a counter that
+    starts two short stands for tiles that come late: cleared, it would end two too high); the call after it is right."""
+    import ctypes as C
+    from glorcq_b200 import _lib, tiled
+    L = _lib.lib()
+    lin = cases.to_b200_linear(cases.make_linear(7500 + N, N, K, rank=rank, bits=bits), dev)
+    t = lin._tiled
+    x, y = cases.make_x(7600 + N, B, K).to(dev), torch.empty(B, N, dtype=torch.float16, device=dev)
+    ref = tiled.linear_forward(t, x, a=tiled.dense_matmul(lin._ut, x))
+    n_bytes = L.glq_linear_workspace_bytes(t.fmt, t.group_size, C.byref(t.desc), B)
+    n_ctr = L.glq_linear_counters(t.fmt, t.group_size, C.byref(t.desc), B)
+    ws, ctr = torch.empty(n_bytes, dtype=torch.uint8, device=dev), torch.zeros(n_ctr, dtype=torch.int32, device=dev)
+
+    def call():
+        _lib.check(L.glq_linear_forward(t.fmt, t.group_size, C.byref(t.desc), lin._ut.codes.data_ptr(), x.data_ptr(), K, None, y.data_ptr(), N, B,
+                                        ws.data_ptr(), n_bytes, ctr.data_ptr(), n_ctr, tiled._stream_ptr(dev)), "linear_forward")
+    call()
+    assert torch.equal(y, ref) and not ctr.any() and tiled.debug_error() is None
+    ctr[-2] = -2                                        # (the last two are those of x.U and its product)
+    call()
+    assert tiled.debug_error()[0] == 112
+    assert ctr[-2] == -2 and not ctr[:-2].any() and ctr[-1] == 0
+    ctr[-2] += 2                                        # the two that were late
+    y.zero_()
+    call()
+    assert torch.equal(y, ref) and not ctr.any() and tiled.debug_error() is None
+
+
+def test_pair_of_a_weight_without_its_low_rank_factor(dev):
+    """Nobody waits for x.U then: it is computed all the same, and the counters are zero once the launch is complete."""
+    import ctypes as C
+    from glorcq_b200 import _lib, tiled
+    lin = cases.to_b200_linear(cases.make_linear(7701, 64, 4096, rank=64), dev)
+    x = cases.make_x(7702, 3, 4096).to(dev)
+    t, a, y = lin._tiled, torch.empty(3, 64, dtype=torch.float16, device=dev), torch.empty(3, 64, dtype=torch.float16, device=dev)
+    ws, ctr = torch.empty(1 << 20, dtype=torch.uint8, device=dev), torch.zeros(1 << 12, dtype=torch.int32, device=dev)
+    u, m = _lib.MMArgs(), _lib.MMArgs()
+    for g, out, n in ((u, a, 64), (m, y, 64)):
+        g.n_problems, g.max_rows, g.rows_stride, g.N, g.K = 1, 3, 3, n, 4096
+        g.x, g.ldx, g.y, g.ldy = x.data_ptr(), 4096, out.data_ptr(), n
+        g.workspace, g.workspace_bytes, g.counters, g.n_counters = ws.data_ptr(), ws.numel(), ctr.data_ptr(), ctr.numel()
+    u.fmt, u.w = _lib.FMT_F16, lin._ut.desc
+    m.fmt, m.group_size, m.rank, m.a0, m.lda, m.flags = t.fmt, t.group_size, 64, a.data_ptr(), 64, 1
+    m.w = _lib.Weight.from_buffer_copy(bytes(t.desc))
+    m.w.sv = None
+    want, a_want = tiled.linear_forward(t, x, a=torch.zeros_like(a)), tiled.dense_matmul(lin._ut, x)
+    for _ in range(20):
+        _lib.check(_lib.lib().glq_grouped_matmul_pair(C.byref(u), C.byref(m), tiled._stream_ptr(dev)), "pair")
+        assert torch.equal(y, want) and torch.equal(a, a_want) and not ctr.any()
