@@ -474,14 +474,15 @@ __global__ void __launch_bounds__(1024) moe_exchange_kernel(const __half* __rest
         asm volatile("st.release.sys.global.s32 [%0], %1;" ::"l"(theirs), "r"(step) : "memory");
         const int* mine = flags[rank] + threadIdx.x;
         const unsigned long long t0 = global_ns();
-        for (;;) {
+        for (bool late = false;;) {
             int seen;
             asm volatile("ld.acquire.sys.global.s32 %0, [%1];" : "=r"(seen) : "l"(mine) : "memory");
             if (seen - step >= 0) break;
-            if (global_ns() - t0 > limit_ns) {
+            if (late) {
                 atomicCAS(error, 0, step);      // the first wait that ran out stays on record
                 break;
             }
+            late = global_ns() - t0 > limit_ns;
             __nanosleep(100);
         }
     }

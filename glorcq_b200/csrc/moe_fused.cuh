@@ -137,12 +137,14 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
 __device__ __noinline__ bool flag_wait(const int* f, int target, unsigned long long limit_ns, int code) {
     if (ld_acquire(f) >= target) return true;
     const unsigned long long t0 = global_ns();
-    for (;;) {
-        if (ld_acquire(f) >= target) return true;
-        if (global_ns() - t0 > limit_ns) {
-            glq_ok(false, code, (unsigned long long)ld_acquire(f), (unsigned long long)target);
+    for (bool late = false;;) {
+        const int v = ld_acquire(f);
+        if (v >= target) return true;
+        if (late) {
+            glq_ok(false, code, (unsigned long long)v, (unsigned long long)target);
             return false;
         }
+        late = global_ns() - t0 > limit_ns;
         __nanosleep(20);
     }
 }
@@ -418,6 +420,7 @@ __global__ void __launch_bounds__(kFT, 1) moe_fused_kernel(const FusedParams p) 
         int ok = 1;
         if (lane == 0 && !dead) ok = flag_wait(f, target, p.wait_ns, code) ? 1 : 0;
         ok = __shfl_sync(0xffffffffu, ok, 0);
+        __syncwarp();                       // (the shuffle orders no memory)
         if (!ok) dead = true;
     };
     // all stream warps (thread 0 polls); also a barrier of the stream warps before and after
@@ -483,6 +486,7 @@ __global__ void __launch_bounds__(kFT, 1) moe_fused_kernel(const FusedParams p) 
             int ok = 1;
             if (lane == 0) ok = flag_wait(flags + FL_R, p.dense_rows, p.wait_ns, 201) ? 1 : 0;
             ok = __shfl_sync(0xffffffffu, ok, 0);
+            __syncwarp();
             if (!ok) dead = true, plan.dead = 1;
         }
         trace(2);

@@ -110,20 +110,25 @@ __device__ __forceinline__ unsigned long long global_ns() {
 }
 // Bounded wait: polls for at most about 2 ms.  A wait that runs out records error code 100 and
 // marks the warp dead; a dead warp no longer waits, so the kernel always ends within milliseconds.
+// (Here and in the other bounded waits the clock is read before what is waited for, so that time for which the GPU ran something
+// else between the two does not count as a wait that ran out.)
 __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity, bool& dead) {
     if (dead) return;
     if (mbar_try_wait(bar, parity)) return;
     const unsigned long long t0 = global_ns();
     // try_wait suspends the thread in hardware for a bounded time: a waiting warp takes no issue slots
-    while (!mbar_try_wait(bar, parity)) {
-        if (global_ns() - t0 > 2000000ull) {
+    for (bool late = false;;) {
+        if (mbar_try_wait(bar, parity)) return;
+        if (late) {
             glq_ok(false, 100, bar, parity);
             dead = true;
             return;
         }
+        late = global_ns() - t0 > 2000000ull;
     }
 }
-// Bounded wait of a warp for a counter in global memory (about 2 ms, then error 112); what was written before the arrivals is visible.
+// Bounded wait of a warp for a counter in global memory (about 4 ms, as the other waits between CTAs, then error 112); what was
+// written before the arrivals is visible to the whole warp.
 __device__ __forceinline__ void pair_wait(const int* f, int target, int lane, bool& dead) {
     int ok = 1;
     if (lane == 0 && !dead) {
@@ -131,18 +136,20 @@ __device__ __forceinline__ void pair_wait(const int* f, int target, int lane, bo
         asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
         if (v < target) {
             const unsigned long long t0 = global_ns();
-            for (;;) {
+            for (bool late = false;;) {
                 asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
                 if (v >= target) break;
-                if (global_ns() - t0 > 2000000ull) {
+                if (late) {
                     ok = glq_ok(false, 112, (unsigned long long)v, (unsigned long long)target);
                     break;
                 }
+                late = global_ns() - t0 > 4000000ull;
                 __nanosleep(20);
             }
         }
     }
     if (!__shfl_sync(0xffffffffu, ok, 0)) dead = true;
+    __syncwarp();            // (the shuffle orders no memory)
 }
 __device__ __forceinline__ uint4 ld_global_u4(const uint4* p) {
     uint4 v;

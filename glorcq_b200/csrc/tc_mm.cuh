@@ -270,15 +270,16 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, volatile 
     const unsigned long long t0 = global_ns();
     // try_wait suspends the thread in hardware for a bounded time, so a waiting warp takes no issue slots
     // from the working ones; the loop only re-arms it and enforces the overall limit
-    while (!mbar_try_wait(bar, parity)) {
+    for (bool late = false;;) {
+        if (mbar_try_wait(bar, parity)) return true;
         if (*dead) return false;
-        if (global_ns() - t0 > limit_ns) {
+        if (late) {
             glq_ok(false, code, bar, parity);
             *dead = 1;
             return false;
         }
+        late = global_ns() - t0 > limit_ns;
     }
-    return true;
 }
 
 template <int TN> struct TcCfg {
