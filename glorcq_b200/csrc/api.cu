@@ -547,17 +547,6 @@ static int launch_maybe_dependent(bool dependent, Kern kern, dim3 grid, dim3 blo
     return GLQ_OK;
 }
 
-template <typename Kern>
-static int allow_smem(Kern kern, bool (&configured)[64], size_t smem) {
-    int dev = 0;
-    GLQ_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !configured[dev]) {
-        GLQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        if (dev >= 0 && dev < 64) configured[dev] = true;
-    }
-    return GLQ_OK;
-}
-
 // ---------------------------------------------------------------------------------------------
 // tensor-core path (tc_mm.cuh): many rows per problem
 // ---------------------------------------------------------------------------------------------
@@ -639,9 +628,8 @@ static bool plan_tc(const glq_mm_args_t* a, TcGeom* out) {
 template <int TN>
 static int launch_tc_t(const TcParams& p, cudaStream_t st) {
     using C = TcCfg<TN>;
-    static bool configured[64] = {};
-    const int rc = allow_smem(tc_kernel<TN>, configured, C::SMEM);
-    if (rc != GLQ_OK) return rc;
+    static SmemLimit limit;
+    GLQ_CUDA(reserve_smem(reinterpret_cast<const void*>(tc_kernel<TN>), limit, C::SMEM));
     tc_pack_b_kernel<TN><<<dim3(p.tiles_max, p.nkb + p.ns), 256, 0, st>>>(p);
     GLQ_CUDA(cudaGetLastError());
     tc_kernel<TN><<<dim3(p.n_ft, p.tiles_max), kTcThreads, C::SMEM, st>>>(p);
@@ -653,9 +641,8 @@ static int launch_tc_t(const TcParams& p, cudaStream_t st) {
 template <int FMT, int TN, int NM, bool SW>
 static int launch_tc_ps_t(TcParams& p, cudaStream_t st) {
     using C = TcPsCfg<FMT, TN, NM, SW>;
-    static bool configured[64] = {};
-    const int rc = allow_smem(tc_ps_kernel<FMT, TN, NM, SW>, configured, C::SMEM);
-    if (rc != GLQ_OK) return rc;
+    static SmemLimit limit;
+    GLQ_CUDA(reserve_smem(reinterpret_cast<const void*>(tc_ps_kernel<FMT, TN, NM, SW>), limit, C::SMEM));
     p.n_ft = cdiv(p.N, kTcFeat * C::NOUT);
     const int rp = launch_maybe_dependent(p.a_late != 0, tc_pack_b_kernel<TN>, dim3(p.tiles_max, p.nkb + p.ns), dim3(256), 0, st, p);
     if (rp != GLQ_OK) return rp;
@@ -713,9 +700,8 @@ static bool xu_takes(const glq_mm_args_t* a) {
 template <int NT, bool VEC>
 static int launch_xu_t(TcParams& p, const glq_mm_args_t* a, cudaStream_t st) {
     using C = XuCfg<NT>;
-    static bool configured[64] = {};
-    const int rc = allow_smem(xu_kernel<NT, VEC>, configured, C::SMEM);
-    if (rc != GLQ_OK) return rc;
+    static SmemLimit limit;
+    GLQ_CUDA(reserve_smem(reinterpret_cast<const void*>(xu_kernel<NT, VEC>), limit, C::SMEM));
     const bool one = a->n_problems == 1 && !a->slot_offset && !a->n_slots;
     p.tiles_max = one ? cdiv(a->max_rows, C::ROWS) : (int)(total_entries(a) / C::ROWS + a->n_problems + 1);
     // (not beside a launch that left SMs to another stream: CTAs that wait there would take that stream's places, and a routing plan
@@ -1303,7 +1289,10 @@ static int launch_rht_e(const void* x, int64_t ldx, const float* signs, int rows
     const int threads = std::max(32, n >> E);
     const size_t smem = threads > 32 ? (size_t)n * sizeof(float) : 0;
     auto kern = rht_kernel<E, TI, TO>;
-    if (smem > 48 * 1024) GLQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) {
+        static SmemLimit limit;
+        GLQ_CUDA(reserve_smem(reinterpret_cast<const void*>(kern), limit, smem));
+    }
     const int vec = aligned16(x) && ldx % 8 == 0 ? 1 : 0;
     // (more rows than SMs gain nothing from waiting beside the launch ahead)
     if (rows <= num_sms()) {

@@ -724,15 +724,9 @@ extern "C" int glq_attn_prefill(const void* q, const void* k, const void* v, voi
     cudaError_t rc = cudaSuccess;
 #define GLQ_PREFILL(HD)                                                                                                  \
     {                                                                                                                    \
-        static bool configured[64] = {};                                                                                 \
-        int dev = 0;                                                                                                     \
-        if (cudaGetDevice(&dev) != cudaSuccess) return GLQ_ERR_CUDA;                                                     \
-        if (dev < 0 || dev >= 64 || !configured[dev]) {                                                                  \
-            if (cudaFuncSetAttribute(attn_prefill_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,               \
-                                     (int)PrefillCfg<HD>::SMEM) != cudaSuccess)                                          \
-                return GLQ_ERR_CUDA;                                                                                     \
-            if (dev >= 0 && dev < 64) configured[dev] = true;                                                            \
-        }                                                                                                                \
+        static SmemLimit limit;                                                                                          \
+        if (reserve_smem(reinterpret_cast<const void*>(attn_prefill_kernel<HD>), limit, PrefillCfg<HD>::SMEM) != cudaSuccess) \
+            return GLQ_ERR_CUDA;                                                                                         \
         rc = launch_beside(attn_prefill_kernel<HD>, grid, dim3(128), PrefillCfg<HD>::SMEM, st,                           \
             reinterpret_cast<const __half*>(q), reinterpret_cast<const __half*>(k), reinterpret_cast<const __half*>(v),  \
             reinterpret_cast<__half*>(y), B, T, n_heads, n_kv);                                                              \

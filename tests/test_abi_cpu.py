@@ -186,3 +186,11 @@ def test_workspace_of_products_with_few_columns(libpath):
     d.H, d.I, d.E, d.top_k, d.rank, d.fmt, d.group_size, d.router_rows, d.dense0_rows = 2048, 1408, 60, 4, 64, _lib.FMT_Q2, 128, 61, 192
     d.I_shared = 5632
     assert L.glq_moe_workspace_bytes(C.byref(d), 512) < (19 + 9 + 81 + 10) << 20
+
+
+def test_shared_memory_limits_are_set_in_one_place():
+    """A limit that is set without being noted in the same step can be lowered under another thread's launch (glq_common.cuh,
+    reserve_smem)."""
+    csrc = os.path.join(ROOT, "glorcq_b200", "csrc")
+    found = [f for f in sorted(os.listdir(csrc)) for _ in re.findall(r"MaxDynamicSharedMemorySize", open(os.path.join(csrc, f)).read())]
+    assert found == ["glq_common.cuh"]

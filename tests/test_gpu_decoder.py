@@ -155,6 +155,36 @@ def test_decoder_logits_prefill_and_decode(dev, cfg, cache_len):
     assert cases.rel_l2(step.cpu(), ref[:, T:]) <= REL_LOGITS
 
 
+def test_rht_rows_of_two_lengths_from_two_threads(dev):
+    """Both lengths are one kernel that needs 64 and 128 KB of shared memory: neither thread takes the other's back."""
+    import threading
+    from glorcq_b200.hadamard_rotation import generate_rht_signs, rht_forward_half
+    work = []
+    for d in (16384, 32768):
+        x, signs = cases.make_x(d, 2, d).to(dev), generate_rht_signs(d).to(dev)
+        work.append((x, signs, rht_forward_half(x, signs), torch.cuda.Stream()))
+    start, wrong = threading.Barrier(2), []
+
+    def many(x, signs, ref, st):
+        try:
+            start.wait()
+            with torch.cuda.stream(st):
+                for _ in range(400):
+                    y = rht_forward_half(x, signs)
+                st.synchronize()
+            if not torch.equal(y, ref):
+                wrong.append(x.shape)
+        except Exception as e:      # noqa: BLE001
+            wrong.append(e)
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=many, args=w) for w in work]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+
 @pytest.mark.parametrize("rows,H", [(1, 8), (3, 2048), (2, 2056), (150, 8192)])
 def test_add_rmsnorm_behind_the_launch_that_writes_its_operands(dev, rows, H):
     """x + delta and the norm of the sum, with x, delta and the weight written by the launch directly before, anew for each call; a
