@@ -171,6 +171,7 @@ class TiledWeight:
     @property
     def desc(self) -> Weight:
         if self._desc is None:
+            self._native = None
             # (settled: codes, factors and norms are written by the packing calls and by fills before them only)
             self._desc = Weight(_ptr(self.codes), None, _ptr(self.norms), _ptr(self.centroids),
                                 _ptr(self.sv), _ptr(self.bias), self.N, self.K, self.rank, _lib.WEIGHT_SETTLED)

@@ -194,3 +194,17 @@ def test_shared_memory_limits_are_set_in_one_place():
     csrc = os.path.join(ROOT, "glorcq_b200", "csrc")
     found = [f for f in sorted(os.listdir(csrc)) for _ in re.findall(r"MaxDynamicSharedMemorySize", open(os.path.join(csrc, f)).read())]
     assert found == ["glq_common.cuh"]
+
+
+def test_native_descriptor_follows_the_weight(libpath):
+    """The host path's copy of a descriptor is made anew with the descriptor, whoever asked for that first."""
+    import torch
+    from glorcq_b200 import _lib
+    from glorcq_b200.tiled import TiledWeight
+    w = TiledWeight(_lib.FMT_Q2, 16, 128, 128, 1, "cpu")
+    w.set_bias(torch.zeros(16))
+    first = w.native
+    assert w.native is first
+    w.set_bias(None)
+    w.desc_bytes()
+    assert w.native is not first
