@@ -276,7 +276,8 @@ def dense_matmul(w: TiledWeight, x: torch.Tensor) -> torch.Tensor:
 class GroupedLinear:
     """Several quantized layers of one shape applied to the same activation rows in two launches (x.U of
     all of them, then the quantized products with the low-rank term), through ``glq_grouped_matmul``:
-    e.g. the q, k and v projections of an attention layer.  ``forward(x (B,K))`` returns (P, B, N)."""
+    e.g. the q, k and v projections of an attention layer.  ``forward(x (B,K))`` returns (P, B, N).  The layers are taken with the
+    factors and biases that they have when the group is made."""
 
     def __init__(self, weights, uts):
         w0 = weights[0]
@@ -284,6 +285,8 @@ class GroupedLinear:
             if (w.fmt, w.N, w.K, w.group_size, w.rank) != (w0.fmt, w0.N, w0.K, w0.group_size, w0.rank):
                 raise RuntimeError("grouped layers must share format, shape, group size and rank")
         self.weights, self.uts = list(weights), list(uts) if uts else None
+        # the tables are made once: what they point to stays, also when a layer is given other factors or another bias later
+        self._keep = [(w.codes, w.norms, w.centroids, w.sv, w.bias) for w in self.weights + (self.uts or [])]
         dev = w0.device
         self._table = torch.frombuffer(bytearray(b"".join(w.desc_bytes() for w in weights)), dtype=torch.uint8).to(dev)
         self._ut_table = None

@@ -208,3 +208,17 @@ def test_native_descriptor_follows_the_weight(libpath):
     w.set_bias(None)
     w.desc_bytes()
     assert w.native is not first
+
+
+def test_group_keeps_what_its_tables_point_to(libpath):
+    import weakref
+    import torch
+    from glorcq_b200 import _lib
+    from glorcq_b200.tiled import GroupedLinear, TiledWeight
+    w = TiledWeight(_lib.FMT_Q2, 16, 128, 128, 1, "cpu")
+    w.set_bias(torch.zeros(16))
+    bias = weakref.ref(w.bias)
+    group = GroupedLinear([w], None)
+    w.set_bias(None)
+    assert bias() is not None
+    del group
