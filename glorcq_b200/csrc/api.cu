@@ -148,26 +148,8 @@ static int plan_geometry(int fmt, int epilogue, int N, int K, int group_size, in
     return GLQ_OK;
 }
 
-// launch with programmatic stream serialization: the grid may be scheduled while the previous kernel of
-// the stream still runs; the kernels wait for it (griddepcontrol.wait) before they read its results
 static thread_local bool t_dependent_launch = false;
 static thread_local bool t_share_sm = false;
-template <typename Kern, typename Params>
-static int launch_dependent(Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Params& p) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    GLQ_CUDA(cudaLaunchKernelEx(&cfg, kern, p));
-    return GLQ_OK;
-}
-
 template <int FMT, int NW, int NTT, bool RM, int TGN = 1>
 static int launch_one(const SkinnyParams& p, int grid, size_t smem, cudaStream_t st) {
     auto kern = skinny_kernel<FMT, NW, NTT, RM, TGN>;
@@ -175,9 +157,7 @@ static int launch_one(const SkinnyParams& p, int grid, size_t smem, cudaStream_t
         static SmemLimit limit;
         GLQ_CUDA(reserve_smem(reinterpret_cast<const void*>(kern), limit, smem));
     }
-    if (t_dependent_launch) return launch_dependent(kern, dim3(grid), dim3(kThreads), smem, st, p);
-    kern<<<grid, kThreads, smem, st>>>(p);
-    GLQ_CUDA(cudaGetLastError());
+    GLQ_CUDA(launch_kernel(t_dependent_launch, kern, dim3(grid), dim3(kThreads), smem, st, p));
     return GLQ_OK;
 }
 
@@ -236,10 +216,6 @@ struct StreamGeom {
     int grid;
 };
 
-static bool pdl_disabled() {
-    static const bool v = std::getenv("GLQ_NO_PDL") != nullptr;
-    return v;
-}
 static bool stream_disabled() {
     static int v = -1;
     if (v < 0) {
@@ -377,9 +353,7 @@ static int launch_stream_one(const StreamParams& sp, const StreamGeom& g, cudaSt
     auto kern = stream_kernel<FMT, I8, NT, NW>;
     static SmemLimit limit;
     GLQ_CUDA(reserve_smem(reinterpret_cast<const void*>(kern), limit, g.smem));
-    if (sp.a_late || sp.dependent) return launch_dependent(kern, dim3(g.grid), dim3(NW * 32), g.smem, st, sp);
-    kern<<<g.grid, NW * 32, g.smem, st>>>(sp);
-    GLQ_CUDA(cudaGetLastError());
+    GLQ_CUDA(launch_kernel(sp.a_late || sp.dependent, kern, dim3(g.grid), dim3(NW * 32), g.smem, st, sp));
     return GLQ_OK;
 }
 
@@ -401,17 +375,7 @@ static int launch_stream_pair_t(const StreamParams& sp, const StreamGeom& g, con
     auto kern = stream_pair_kernel<FMT, I8, NT, NW>;
     static SmemLimit limit;
     GLQ_CUDA(reserve_smem(reinterpret_cast<const void*>(kern), limit, g.smem));
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(g.grid + n_xu);
-    cfg.blockDim = dim3(NW * 32);
-    cfg.dynamicSmemBytes = g.smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    GLQ_CUDA(cudaLaunchKernelEx(&cfg, kern, sp, xu, n_xu));
+    GLQ_CUDA(launch_kernel(true, kern, dim3(g.grid + n_xu), dim3(NW * 32), g.smem, st, sp, xu, n_xu));
     return GLQ_OK;
 }
 template <int FMT>
@@ -536,18 +500,6 @@ static int launch_stream(const glq_mm_args_t* a, SkinnyParams& p, const StreamGe
 }
 
 // ---------------------------------------------------------------------------------------------
-// glq_grouped_matmul
-// ---------------------------------------------------------------------------------------------
-// <<<>>> with programmatic stream serialization when `dependent`
-template <typename Kern, typename Params>
-static int launch_maybe_dependent(bool dependent, Kern kern, dim3 grid, dim3 block, size_t smem, cudaStream_t st, const Params& p) {
-    if (dependent) return launch_dependent(kern, grid, block, smem, st, p);
-    kern<<<grid, block, smem, st>>>(p);
-    GLQ_CUDA(cudaGetLastError());
-    return GLQ_OK;
-}
-
-// ---------------------------------------------------------------------------------------------
 // tensor-core path (tc_mm.cuh): many rows per problem
 // ---------------------------------------------------------------------------------------------
 struct TcGeom {
@@ -644,14 +596,14 @@ static int launch_tc_ps_t(TcParams& p, cudaStream_t st) {
     static SmemLimit limit;
     GLQ_CUDA(reserve_smem(reinterpret_cast<const void*>(tc_ps_kernel<FMT, TN, NM, SW>), limit, C::SMEM));
     p.n_ft = cdiv(p.N, kTcFeat * C::NOUT);
-    const int rp = launch_maybe_dependent(p.a_late != 0, tc_pack_b_kernel<TN>, dim3(p.tiles_max, p.nkb + p.ns), dim3(256), 0, st, p);
-    if (rp != GLQ_OK) return rp;
+    GLQ_CUDA(launch_kernel(p.a_late != 0, tc_pack_b_kernel<TN>, dim3(p.tiles_max, p.nkb + p.ns), dim3(256), 0, st, p));
     const long work = (long)p.n_ft * p.tiles_max;
     // A CTA of this kernel fills its SM.  Where another stream has launches at the same time, no more of them than the rounds of
     // items need: the shared expert's gate|up for 512 tokens has 176 items, two rounds on 148 SMs and on 88, and on the other 60 the
     // routing plan and the routed x.U now run beside it (24-layer prompt 8840 -> 8485 us).
     const long rounds = (work + num_sms() - 1) / num_sms(), grid = t_share_sm ? (work + rounds - 1) / rounds : std::min<long>(work, num_sms());
-    return launch_maybe_dependent(!pdl_disabled(), tc_ps_kernel<FMT, TN, NM, SW>, dim3((int)grid), dim3(kPsThreads), C::SMEM, st, p);
+    GLQ_CUDA(launch_kernel(true, tc_ps_kernel<FMT, TN, NM, SW>, dim3((int)grid), dim3(kPsThreads), C::SMEM, st, p));
+    return GLQ_OK;
 }
 template <int FMT>
 static int launch_tc_ps(TcParams& p, const TcGeom& g, bool sw, cudaStream_t st) {
@@ -709,7 +661,8 @@ static int launch_xu_t(TcParams& p, const glq_mm_args_t* a, cudaStream_t st) {
     // (nor h.U behind the GEMM of many experts: its few CTAs lay two to an SM in the first places that came free; 300 tokens through eight
     // Mixtral-shaped experts, codebook: 691 us against 663)
     const bool beside = !t_share_sm && (!a->n_slots || (a->flags & GLQ_MM_AFTER_KERNEL) != 0);
-    return launch_maybe_dependent(!pdl_disabled() && beside, xu_kernel<NT, VEC>, dim3(p.tiles_max, cdiv(a->N, kXuCols)), dim3(kXuThreads), C::SMEM, st, p);
+    GLQ_CUDA(launch_kernel(beside, xu_kernel<NT, VEC>, dim3(p.tiles_max, cdiv(a->N, kXuCols)), dim3(kXuThreads), C::SMEM, st, p));
+    return GLQ_OK;
 }
 static int launch_xu(const glq_mm_args_t* a, cudaStream_t st) {
     if (!a->w_table && !a->w.codes) return GLQ_ERR_ARG;
@@ -857,7 +810,7 @@ extern "C" int glq_grouped_matmul(const glq_mm_args_t* a, void* stream) {
         return GLQ_OK;
     }
     fill_geometry(p, g);
-    t_dependent_launch = (a->flags & (GLQ_MM_AFTER_KERNEL | GLQ_MM_A_FROM_PREVIOUS_LAUNCH)) != 0 && !pdl_disabled();
+    t_dependent_launch = (a->flags & (GLQ_MM_AFTER_KERNEL | GLQ_MM_A_FROM_PREVIOUS_LAUNCH)) != 0;
     rc = launch_skinny(a->fmt, false, p, g, a->n_problems, reinterpret_cast<cudaStream_t>(stream));
     t_dependent_launch = false;
     return rc;
@@ -1278,10 +1231,6 @@ extern "C" int glq_dequant_tiled(int fmt, const void* tiled, const float* norms_
 }
 
 // ---------------------------------------------------------------------------------------------
-// First bounds violation recorded by a self-checking kernel: {code, index, limit, block<<32|thread};
-// all zero when there was none.  Synchronises the device.
-// ---------------------------------------------------------------------------------------------
-// ---------------------------------------------------------------------------------------------
 // randomized Hadamard rotation
 // ---------------------------------------------------------------------------------------------
 template <int E, typename TI, typename TO>
@@ -1295,13 +1244,8 @@ static int launch_rht_e(const void* x, int64_t ldx, const float* signs, int rows
     }
     const int vec = aligned16(x) && ldx % 8 == 0 ? 1 : 0;
     // (more rows than SMs gain nothing from waiting beside the launch ahead)
-    if (rows <= num_sms()) {
-        GLQ_CUDA(launch_beside(kern, dim3(rows), dim3(threads), smem, st, reinterpret_cast<const TI*>(x), (long long)ldx, signs, d, n, scale,
-                               reinterpret_cast<TO*>(y), (long long)ldy, vec));
-        return GLQ_OK;
-    }
-    kern<<<rows, threads, smem, st>>>(reinterpret_cast<const TI*>(x), ldx, signs, d, n, scale, reinterpret_cast<TO*>(y), ldy, vec);
-    GLQ_CUDA(cudaGetLastError());
+    GLQ_CUDA(launch_kernel(rows <= num_sms(), kern, dim3(rows), dim3(threads), smem, st, reinterpret_cast<const TI*>(x), (long long)ldx, signs, d, n,
+                           scale, reinterpret_cast<TO*>(y), (long long)ldy, vec));
     return GLQ_OK;
 }
 // values per thread: the smallest power whose exponent covers the stages between warps (log2(n) <= 2 E + 5)
@@ -1331,6 +1275,8 @@ extern "C" int glq_rht_forward(const void* x, int x_is_f32, int64_t ldx, const f
 
 int glq_moe_error_words(unsigned long long* out4, int clear);   // moe.cu: the error word of that translation unit
 
+// First bounds violation or timed-out wait recorded by a kernel: {code, index, limit, block<<32|thread};
+// all zero when there was none.  Synchronises the device.
 extern "C" int glq_debug_error(unsigned long long* out4, int clear) {
     if (!out4) return GLQ_ERR_ARG;
     GLQ_CUDA(cudaMemcpyFromSymbol(out4, g_glq_err, 4 * sizeof(unsigned long long)));

@@ -616,7 +616,7 @@ extern "C" int glq_add_rmsnorm(const void* x, const void* delta, const void* wei
     if (!x || !delta || !x_out || !h_out || rows < 0 || H <= 0) return GLQ_ERR_ARG;
     if (H % 8 != 0 || H > 8192) return GLQ_ERR_UNSUPPORTED;
     if (rows == 0) return GLQ_OK;
-    return launch_beside(add_rmsnorm_kernel, dim3(rows), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const __half*>(x),
+    return launch_kernel(true, add_rmsnorm_kernel, dim3(rows), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream), reinterpret_cast<const __half*>(x),
                             reinterpret_cast<const __half*>(delta), reinterpret_cast<const __half*>(weight), eps, H,
                             reinterpret_cast<__half*>(x_out), reinterpret_cast<__half*>(h_out)) == cudaSuccess
                ? GLQ_OK : GLQ_ERR_CUDA;
@@ -694,7 +694,7 @@ extern "C" int glq_rope_prefill(void* q, void* k, const void* v, const void* cos
     auto st = reinterpret_cast<cudaStream_t>(stream);
     cudaError_t rc = cudaSuccess;
 #define GLQ_ROPE_CASE(EPL)                                                                                                  \
-    rc = launch_beside(rope_prefill_kernel<EPL>, grid, dim3(kAttnWarps * 32), 0, st,                                        \
+    rc = launch_kernel(true, rope_prefill_kernel<EPL>, grid, dim3(kAttnWarps * 32), 0, st,                                        \
         reinterpret_cast<__half*>(q), reinterpret_cast<__half*>(k), reinterpret_cast<const __half*>(v),                     \
         reinterpret_cast<const __half*>(cos_t), reinterpret_cast<const __half*>(sin_t),                                     \
         reinterpret_cast<const long long*>(positions), reinterpret_cast<__half*>(k_cache), reinterpret_cast<__half*>(v_cache), \
@@ -727,7 +727,7 @@ extern "C" int glq_attn_prefill(const void* q, const void* k, const void* v, voi
         static SmemLimit limit;                                                                                          \
         if (reserve_smem(reinterpret_cast<const void*>(attn_prefill_kernel<HD>), limit, PrefillCfg<HD>::SMEM) != cudaSuccess) \
             return GLQ_ERR_CUDA;                                                                                         \
-        rc = launch_beside(attn_prefill_kernel<HD>, grid, dim3(128), PrefillCfg<HD>::SMEM, st,                           \
+        rc = launch_kernel(true, attn_prefill_kernel<HD>, grid, dim3(128), PrefillCfg<HD>::SMEM, st,                           \
             reinterpret_cast<const __half*>(q), reinterpret_cast<const __half*>(k), reinterpret_cast<const __half*>(v),  \
             reinterpret_cast<__half*>(y), B, T, n_heads, n_kv);                                                              \
     }

@@ -167,10 +167,16 @@ static inline cudaError_t reserve_smem(const void* kern, SmemLimit& l, size_t sm
     return e;
 }
 
-// Launch with programmatic stream serialization: the grid may start before the launch ahead of it has ended and waits for it itself
-// (griddepcontrol.wait).  A kernel that waits first thing gains the launch alone: 1.5 us of the 2 between dependent launches of a prompt.
+// GLQ_NO_PDL in the environment: every launch starts when all before it is complete
+static inline bool pdl_disabled() {
+    static const bool off = std::getenv("GLQ_NO_PDL") != nullptr;
+    return off;
+}
+// A launch.  beside: with programmatic stream serialization, the grid may start before the launch ahead of it has ended and waits for it
+// itself (griddepcontrol.wait).  A kernel that waits first thing gains the launch alone: 1.5 us of the 2 between dependent launches
+// of a prompt.
 template <typename... P, typename... A>
-static inline cudaError_t launch_beside(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+static inline cudaError_t launch_kernel(bool beside, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, const A&... args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -178,10 +184,9 @@ static inline cudaError_t launch_beside(void (*kern)(P...), dim3 grid, dim3 bloc
     cfg.stream = st;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    static const bool off = std::getenv("GLQ_NO_PDL") != nullptr;
-    attr.val.programmaticStreamSerializationAllowed = off ? 0 : 1;
+    attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = beside && !pdl_disabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 

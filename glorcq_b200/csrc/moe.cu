@@ -1041,24 +1041,24 @@ extern "C" int glq_moe_forward_ep(const glq_moe_desc_t* d, const void* x, int n,
         int* blk = reinterpret_cast<int*>(ws + L.plan_blk);
         const int* s_in = given ? (const int*)ep->sel_in : (const int*)nullptr;
         const __half* w_in = given ? reinterpret_cast<const __half*>(ep->weight_in) : (const __half*)nullptr;
-        cudaError_t e = launch_beside(
-            moe_route_kernel, dim3(given ? std::min(1024, (nk + 255) / 256) : (n + 7) / 8), dim3(256), 0, st,
+        cudaError_t e = launch_kernel(
+            true, moe_route_kernel, dim3(given ? std::min(1024, (nk + 255) / 256) : (n + 7) / 8), dim3(256), 0, st,
             (const __half*)p_logits, ldl, n, (int)d->E, k, (int)d->norm_topk_prob, p_sel, p_wts, p_tok,
             reinterpret_cast<__half*>(router_logits), (int*)sel_out, reinterpret_cast<__half*>(weight_out), s_in, w_in);
-        if (e == cudaSuccess) e = launch_beside(moe_plan_count_kernel, dim3(nb), dim3(32), d->E * sizeof(int), st, p_sel, nk, (int)d->E, blk);
+        if (e == cudaSuccess) e = launch_kernel(true, moe_plan_count_kernel, dim3(nb), dim3(32), d->E * sizeof(int), st, p_sel, nk, (int)d->E, blk);
         if (e == cudaSuccess)
-            e = launch_beside(moe_plan_lists_kernel, dim3(1), dim3(1024), 2 * d->E * sizeof(int), st,
+            e = launch_kernel(true, moe_plan_lists_kernel, dim3(1), dim3(1024), 2 * d->E * sizeof(int), st,
                               blk, nb, nk, (int)d->E, chunk, ep_rank, ep_world, p_active, p_nact, p_cnt, p_off,
                               reinterpret_cast<int*>(ws + L.active2), reinterpret_cast<int*>(ws + L.n_active2),
                               reinterpret_cast<int*>(ws + L.slot_count2), reinterpret_cast<int*>(ws + L.slot_offset2));
         if (e == cudaSuccess)
-            e = launch_beside(moe_plan_scatter_kernel, dim3(nb), dim3(32), d->E * sizeof(int), st, p_sel, p_wts, nk, (int)d->E, k, blk, p_erow, p_escale, p_tok);
+            e = launch_kernel(true, moe_plan_scatter_kernel, dim3(nb), dim3(32), d->E * sizeof(int), st, p_sel, p_wts, nk, (int)d->E, k, blk, p_erow, p_escale, p_tok);
         if (e != cudaSuccess) return GLQ_ERR_CUDA;
         after_kernel[0] = true;
     } else {
         const size_t smem = 2 * d->E * sizeof(int) + (size_t)nk * (sizeof(int) + sizeof(__half));
-        const cudaError_t e = launch_beside(
-            moe_plan_kernel, dim3(1), dim3(1024), smem, st,
+        const cudaError_t e = launch_kernel(
+            true, moe_plan_kernel, dim3(1), dim3(1024), smem, st,
             (const __half*)p_logits, ldl, n, (int)d->E, k, (int)d->norm_topk_prob, p_sel, p_wts, p_active, p_nact, p_cnt, p_off, p_erow, p_escale, p_tok,
             reinterpret_cast<__half*>(router_logits), (int*)sel_out, reinterpret_cast<__half*>(weight_out),
             reinterpret_cast<int*>(ws + L.active2), reinterpret_cast<int*>(ws + L.n_active2),
