@@ -435,7 +435,8 @@ def test_dense_weight_route_dtype_and_reference_op_names(dev):
 # ---- threads ------------------------------------------------------------------------------------------
 def test_launches_run_without_the_interpreter_lock(dev):
     """The library's entry points are replaced by PyGILState_Check: 0, a success, when the calling thread does not
-    hold the interpreter lock, 1, an unknown status, when it does."""
+    hold the interpreter lock, 1, an unknown status, when it does.  Each is reached by one of the calls: replaced by
+    Py_IsInitialized, which is 1, one of them fails."""
     import ctypes as C
     from glorcq_b200 import _lib, tiled
     from glorcq_b200.kernels import gptq_dequant_matmul, turbo_dequant_grouped_gemv, turbo_dequant_matmul
@@ -446,7 +447,9 @@ def test_launches_run_without_the_interpreter_lock(dev):
     blk(x.view(1, 2, 128))
     q, n, c = torch.zeros(16, 32, dtype=torch.uint8, device=dev), torch.ones(16, device=dev), torch.ones(4, device=dev)
     s = torch.ones(16, 1, dtype=torch.float16, device=dev)
-    calls = [lambda: lin(x), lambda: group.forward(x), lambda: blk(x.view(1, 2, 128)), lambda: turbo_dequant_matmul(x, q, n, c),
+    plain, signs = tiled.GroupedLinear([lin._tiled] * 2, None), torch.ones(128, device=dev)
+    calls = [lambda: lin(x), lambda: group.forward(x), lambda: plain.forward(x), lambda: tiled.linear_forward(lin._tiled, x, lin._ut, signs=signs),
+             lambda: blk(x.view(1, 2, 128)), lambda: turbo_dequant_matmul(x, q, n, c),
              lambda: turbo_dequant_grouped_gemv(x, q, n, c, 8), lambda: _lib.native().add_rmsnorm(x, x, s[:1].expand(1, 128).contiguous(), 1e-6),
              lambda: gptq_dequant_matmul(x.float(), torch.zeros(16, 128, dtype=torch.int8, device=dev), s, s, 128, False, torch.empty(0, device=dev))]
     for f in calls:
@@ -454,12 +457,24 @@ def test_launches_run_without_the_interpreter_lock(dev):
     nat = _lib.native()
     real = {e: C.cast(getattr(_lib.lib(), e), C.c_void_p).value for e in nat.names()}
     probe = C.cast(C.pythonapi.PyGILState_Check, C.c_void_p).value
-    launches = ("glq_linear_forward", "glq_grouped_matmul", "glq_moe_forward_ep", "glq_turbo_dequant_matmul",
-                "glq_turbo_dequant_grouped_gemv", "glq_add_rmsnorm", "glq_gptq_dequant_matmul")
+    fails = C.cast(C.pythonapi.Py_IsInitialized, C.c_void_p).value
+    launches = [e for e in nat.names() if not e.endswith(("_bytes", "_counters")) and e not in ("glq_status_string", "glq_last_cuda_error")]
+
+    def failing():
+        out = 0
+        for f in calls:
+            try:
+                f()
+            except RuntimeError:
+                out += 1
+        return out
     try:
         nat.bind({**real, **{e: probe for e in launches}})
         for f in calls:
             f()
+        for e in launches:
+            nat.bind({**real, **{o: probe for o in launches}, e: fails})
+            assert failing() > 0, e
     finally:
         nat.bind(real)
 
@@ -510,17 +525,47 @@ def test_scratch_of_a_captured_call_outlives_a_larger_call(dev):
 
 
 @pytest.mark.parametrize("B", [1, 4, 5, 8])
-@pytest.mark.parametrize("fmt,bits,N,K,rank", [("gptq", 2, 1408, 2048, 64), ("gptq", 4, 520, 896, 16), ("gptq", 3, 40, 192, 128), ("turbo", 2, 1000, 8192, 80),
-                                               ("gptq", 4, 4096, 4096, 64), ("gptq", 2, 72, 14336, 32), ("gptq", 2, 14336, 4096, 64)])
-def test_low_rank_operand_in_the_products_launch(dev, fmt, bits, N, K, rank, B):
-    """x.U computed by the first blocks of the product's launch (or, for the largest, by a launch of its own) gives the bits of x.U
-    computed alone and handed in, call after call, and leaves the arrival counters at zero."""
+@pytest.mark.parametrize("fmt,bits,N,K,rank,one_launch", [
+    ("gptq", 2, 1408, 2048, 64, 8), ("gptq", 4, 520, 896, 16, 8), ("gptq", 3, 40, 192, 128, 8), ("turbo", 2, 1000, 8192, 80, 8),
+    # (8 rows of 4096 channels leave an SM one CTA, and the product has one for every SM; 8 of 14336 are the general kernel's; the
+    # product of 14336 features has a CTA for every slot)
+    ("gptq", 4, 4096, 4096, 64, 4), ("gptq", 2, 72, 14336, 32, 4), ("gptq", 2, 14336, 4096, 64, 0)])
+def test_low_rank_operand_in_the_products_launch(dev, fmt, bits, N, K, rank, one_launch, B):
+    """x.U computed by the first blocks of the product's launch (up to `one_launch` rows, by a launch of its own above) gives the bits of
+    x.U computed alone and handed in, call after call, and leaves the arrival counters at zero."""
     from glorcq_b200 import _lib, tiled
     lin = cases.to_b200_linear(cases.make_linear(N + K + B, N, K, rank=rank, fmt=fmt, bits=bits), dev)
-    x = cases.make_x(B + N, B, K).to(dev)
-    ref = tiled.linear_forward(lin._tiled, x, a=tiled.dense_matmul(lin._ut, x))
-    for _ in range(3):
-        assert torch.equal(tiled.linear_forward(lin._tiled, x, lin._ut), ref)
+    # (two inputs in turn: the scratch holds the other one's x.U when a call begins)
+    xs = [cases.make_x(B + N + i, B, K).to(dev) for i in range(2)]
+    refs = [tiled.linear_forward(lin._tiled, x, a=tiled.dense_matmul(lin._ut, x)) for x in xs]
+    for i in range(6):
+        assert torch.equal(tiled.linear_forward(lin._tiled, xs[i % 2], lin._ut), refs[i % 2])
+    torch.cuda.synchronize()
+    assert not bool(_lib.native().workspace(0, 0, 0)[1].any()) and tiled.debug_error() is None
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        for x in xs:
+            tiled.linear_forward(lin._tiled, x, lin._ut)
+    names = [n for edge in _programmatic_edges(graph) for n in edge]
+    assert all("stream_pair_kernel" in n for n in names) if B <= one_launch else not any("stream_pair_kernel" in n for n in names), names
+    assert names
+
+
+@pytest.mark.parametrize("B", [1, 5, 8, 9])
+@pytest.mark.parametrize("P,fmt,bits,N,K,rank", [(2, "gptq", 2, 520, 896, 16), (3, "gptq", 4, 2048, 2048, 64), (3, "gptq", 3, 40, 192, 80),
+                                                 (2, "turbo", 2, 1000, 2048, 64)])
+def test_group_with_low_rank_factors(dev, P, fmt, bits, N, K, rank, B):
+    """Layers of their own weights and factors, several in a launch (up to 8 rows with their x.U in its first blocks): the results of the layers
+    one by one within the rounding of two fp16 results, the same bits call after call, and zero arrival counters."""
+    from glorcq_b200 import _lib, tiled
+    lins = [cases.to_b200_linear(cases.make_linear(8000 + N + B + i, N, K, rank=rank, fmt=fmt, bits=bits), dev) for i in range(P)]
+    group = tiled.GroupedLinear([m._tiled for m in lins], [m._ut for m in lins])
+    xs = [cases.make_x(8100 + N + i, B, K).to(dev) for i in range(2)]
+    refs = [torch.stack([m(x) for m in lins]) for x in xs]
+    got = [group.forward(xs[i % 2]) for i in range(6)]
+    for i, y in enumerate(got):
+        assert torch.equal(y, got[i % 2])
+        assert cases.rel_l2(y.cpu(), refs[i % 2].cpu()) <= REL
     torch.cuda.synchronize()
     assert not bool(_lib.native().workspace(0, 0, 0)[1].any()) and tiled.debug_error() is None
 
@@ -565,16 +610,16 @@ def test_threads_on_streams_of_their_own(dev):
     work = []
     for i, (B, K) in enumerate(((4, 512), (8, 4096), (6, 2048), (3, 5632))):
         lin = cases.to_b200_linear(cases.make_linear(150 + i, 256, K, rank=32), dev)
-        x = cases.make_x(160 + i, B, K).to(dev)
-        work.append((lin, x, torch.cuda.Stream()))
+        xs = [cases.make_x(160 + i + 10 * j, B, K).to(dev) for j in range(2)]
+        work.append((lin, xs, torch.cuda.Stream()))
     got, errors = {}, []
     start = threading.Barrier(len(work))
 
-    def many(i, lin, x, st):
+    def many(i, lin, xs, st):
         try:
             start.wait()
             with torch.cuda.stream(st):
-                got[i] = [lin(x) for _ in range(50)]
+                got[i] = [lin(xs[j % 2]) for j in range(50)]
         except Exception as e:      # noqa: BLE001
             errors.append(e)
     torch.cuda.synchronize()
@@ -585,9 +630,9 @@ def test_threads_on_streams_of_their_own(dev):
         t.join()
     torch.cuda.synchronize()
     assert not errors
-    for i, (lin, x, _) in enumerate(work):
-        ref = lin(x)
-        assert all(torch.equal(y, ref) for y in got[i])
+    for i, (lin, xs, _) in enumerate(work):
+        refs = [lin(x) for x in xs]
+        assert all(torch.equal(y, refs[j % 2]) for j, y in enumerate(got[i]))
 
 
 def _programmatic_edges(graph):
