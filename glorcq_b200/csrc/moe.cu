@@ -765,10 +765,11 @@ bool plan_fused(const glq_moe_desc_t* d, int n, FusedParams* out, size_t* smem_b
     P.off_red = (int)off;
     off += (size_t)2 * kFSW * 2 * 32 * sizeof(float2);     // k-split sums (two parities)
     P.off_seg = (int)off;
-    // sums of the segments of a row of the shared U^T: 16 floats.  The rest is unused and stays: without it the one-token block of
-    // 60 experts takes 31.42 us instead of 31.25, wherever the ring is aligned to (128, 512, 1024 bytes)
+    // sums of the segments of a row of the shared U^T (16 floats), then the combine's list of a token's entries (top_k, at most 16, ints).  The rest
+    // is unused and stays: without it the one-token block of 60 experts takes 31.42 us instead of 31.25, wherever the ring is
+    // aligned to (128, 512, 1024 bytes)
     off += (size_t)kFRows * (256 + 16) * sizeof(float);
-    static_assert(kFW - kFSW <= 256 + 16, "segment sums");
+    static_assert((kFW - kFSW) * kFRows * sizeof(float) + 16 * sizeof(int) <= kFRows * (256 + 16) * sizeof(float), "segment sums, entries");
     off = (off + 15) / 16 * 16;
     P.off_plan = (int)off;
     off += sizeof(FusedPlan);

@@ -3,7 +3,7 @@
 //
 // The op is bound by the HBM stream of packed codes, so the kernel is a copy pipeline with compute
 // attached:
-//   * one CTA per SM walks a contiguous range of work items (problem, tile pair, k split); the
+//   * a CTA (two per SM, or one: see below) walks a contiguous range of work items (problem, tile pair, k split); the
 //     activations of a problem are staged once per CTA, not once per tile;
 //   * every warp owns a ring of shared-memory stages filled by bulk asynchronous copies
 //     (cp.async.bulk global -> shared, completion counted on an mbarrier) that the warp issues itself,
@@ -61,7 +61,7 @@ struct StreamParams {
     int off_xs, off_ox, off_as, off_ring, off_red;  // shared memory carve-up (bytes)
     int cnt_lo, cnt_hi;  // only slots with cnt_lo < rows <= cnt_hi are this launch's (others belong to a sibling launch)
     int dependent;  // 1: launched with programmatic stream serialization
-    int a_late;   // 1: the x.U operand is still being written when this kernel starts (programmatic dependent launch)
+    int a_late;   // 1: the x.U operand is still being written when this kernel starts (by the launch ahead, or by its own first blocks)
     int* pair;    // {row tiles of x.U written, CTAs done + 2^16 for each that saw them all}: zero between calls; x.U is computed by the first blocks of this launch
     int pair_target;
     int settled;  // GLQ_WEIGHT_SETTLED holds: weights may be read before the launch ahead is complete
@@ -840,7 +840,7 @@ __device__ __forceinline__ void stream_body(const StreamParams& sp, int block, i
                             as + ((size_t)(swiglu ? j : 0) * kRows + (ok ? row : 0)) * rank + (ok ? cc0 : 0));
                         if (ok) av0 = pav[0], av1 = pav[1];
                     } else if (ok && row < cnt) {
-                        // written by the launch before this one, which has completed by now (see the wait above)
+                        // written by the launch before this one, or by this one's first blocks: complete by now (see the wait above)
                         const uint4* pav = reinterpret_cast<const uint4*>(p.a[swiglu ? j : 0] + (size_t)(e0 + row) * p.lda + cc0);
                         av0 = ld_global_u4(pav);
                         av1 = ld_global_u4(pav + 1);

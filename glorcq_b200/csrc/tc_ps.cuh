@@ -17,7 +17,7 @@
 // CTA instead of once per tile.  16 producer warps unpack the codes of a 128-channel stage into the
 // tensor-memory ring, one warp issues the MMAs, one bulk-copies the token operand.
 //
-//  * Work items are drawn from a grid-wide counter (zeroed by the pre-pass) by a warp of its own, up to four ahead;
+//  * Work items are drawn from a grid-wide counter (zeroed by the pre-pass) by a warp of its own, up to kPsQueue ahead;
 //    it looks the problem up and hands the operands' addresses to the other warps through a small queue in
 //    shared memory, so an SM that runs faster takes more items and nobody else walks the dependent loads.
 //  * The rings run on across item boundaries: the loader fetches the next item's token operand while the
@@ -35,7 +35,8 @@
 // product of 60 experts x 34 rows (1408 x 2048, 2-bit), scheduler slots 57 % used, DRAM 12 %.  Now 140 instructions
 // and 99 us; 97 -> 60 us for the down product (2048 x 1408).  With one multiply-add per pair of 2-bit codes and one election
 // per four MMAs 95 and 54 us; with the look-ups in a warp of their own, the accumulator released before the epilogue's arithmetic
-// and that arithmetic left out for tokens that do not exist 86 and 55 (codebook codes: 105 -> 95).  No pipe is full (gate|up:
+// and that arithmetic left out for tokens that do not exist 86 and 55 (codebook codes: 105 -> 95; prompts of few large experts gain nothing
+// by it: 600 tokens through 8 Mixtral-shaped experts 740 us a block before, 734 now).  No pipe is full (gate|up:
 // integer 49 %, issue slots 53 %, tensor 23 %): what is left is the latency of a warp's own chain through a stage, of which four
 // warps per scheduler cover only a part.
 //

@@ -274,8 +274,8 @@ def dense_matmul(w: TiledWeight, x: torch.Tensor) -> torch.Tensor:
 
 
 class GroupedLinear:
-    """Several quantized layers of one shape applied to the same activation rows in two launches (x.U of
-    all of them, then the quantized products with the low-rank term), through ``glq_grouped_matmul``:
+    """Several quantized layers of one shape applied to the same activation rows: x.U of all of them, then the quantized products with
+    the low-rank term, one launch where both fit the GPU together (up to 8 rows) and two otherwise (``glq_grouped_matmul_pair``),
     e.g. the q, k and v projections of an attention layer.  ``forward(x (B,K))`` returns (P, B, N).  The layers are taken with the
     factors and biases that they have when the group is made."""
 
