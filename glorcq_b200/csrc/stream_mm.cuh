@@ -946,8 +946,9 @@ __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) strea
 // A layer of at most 8 rows in one launch: blocks [0, n_xu) compute x.U as skinny_kernel does, the others the product, whose
 // low-rank term waits for the row tiles of x.U behind a counter.  Only blocks of higher numbers wait, and only for lower ones, which
 // are scheduled first and wait for nobody; the host takes this form only where all of them are resident at once.
-// Bound by latency, the host's and the chain's: with two launches (the second programmatically dependent) one row through 1408 x 2048,
-// 2-bit, rank 64 took 11.2 us a call, 7.7 now; 2 rows of 3-bit 2048 x 2048 10.8 and 7.5, 5 rows of codebook 5632 x 2048 16.4 and 14.4.
+// Bound by latency, the host's and the chain's.  Back to back, with two launches (the second programmatically dependent) and now: one row
+// through 1408 x 2048, 2-bit, rank 64 10.9 and 7.6 us a call (6.5 in a graph), 2 rows of 3-bit 2048 x 2048 10.9 and 7.4, 5 rows of codebook
+// 5632 x 2048 behind their rotation 16.4 and 12.0.  A call that is waited for alone gains 2 to 3 us, and as little on weights seen first.
 template <int FMT, bool I8, int NT, int NW>
 __global__ void __launch_bounds__(NW * 32, NW == 8 ? kStreamCtasPerSm : 1) stream_pair_kernel(const StreamParams sp, const SkinnyParams xp, int n_xu) {
     if (!sp.settled) asm volatile("griddepcontrol.wait;" ::: "memory");
