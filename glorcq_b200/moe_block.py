@@ -129,7 +129,7 @@ class GraphCompatibleMoeBlock(nn.Module):
             if (f.fmt, f.group_size, f.rank, f.N, f.K) != (fmt, gs, rank, I, H) or \
                     (dn._tiled.tile_fmt, dn._tiled.group_size, dn._tiled.rank, dn._tiled.N, dn._tiled.K) != (fmt, gs, rank, H, I):
                 raise RuntimeError("all experts of a block must share format, group size, rank and shapes")
-            self._keep += [f, dn._tiled]
+            self._keep += [f, dn._tiled.buffers()]
             gate_up[e] = f.desc
             down[e] = dn._tiled.desc
             if rank > 0:
@@ -208,7 +208,7 @@ class GraphCompatibleMoeBlock(nn.Module):
             f = _fuse_tiles(sg._tiled, su._tiled)
             if (f.fmt, f.group_size, f.K) != (fmt, gs, H) or f.rank not in (0, rank) or sd._tiled.rank != f.rank:
                 raise RuntimeError("the shared expert must share format, group size and rank with the routed experts")
-            self._keep += [f, sd._tiled]
+            self._keep += [f, sd._tiled.buffers()]
             d.I_shared = sg.out_features
             d.sh_gate_up, d.sh_down = f.desc, sd._tiled.desc
             if f.rank > 0:

@@ -187,6 +187,11 @@ class TiledWeight:
     def desc_bytes(self) -> bytes:
         return bytes(self.desc)
 
+    def buffers(self):
+        """What the descriptor points to.  A table that is made of it once keeps these: the weight itself lets go of factors of
+        another rank and of another bias."""
+        return self.codes, self.norms, self.centroids, self.sv, self.bias
+
     @property
     def device(self):
         return self.codes.device
@@ -286,7 +291,7 @@ class GroupedLinear:
                 raise RuntimeError("grouped layers must share format, shape, group size and rank")
         self.weights, self.uts = list(weights), list(uts) if uts else None
         # the tables are made once: what they point to stays, also when a layer is given other factors or another bias later
-        self._keep = [(w.codes, w.norms, w.centroids, w.sv, w.bias) for w in self.weights + (self.uts or [])]
+        self._keep = [w.buffers() for w in self.weights + (self.uts or [])]
         dev = w0.device
         self._table = torch.frombuffer(bytearray(b"".join(w.desc_bytes() for w in weights)), dtype=torch.uint8).to(dev)
         self._ut_table = None

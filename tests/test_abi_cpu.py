@@ -222,3 +222,27 @@ def test_group_keeps_what_its_tables_point_to(libpath):
     w.set_bias(None)
     assert bias() is not None
     del group
+
+
+def test_block_keeps_what_its_tables_point_to(libpath):
+    import weakref
+    from types import SimpleNamespace
+    import torch
+    from glorcq_b200 import _lib
+    from glorcq_b200.moe_block import GraphCompatibleMoeBlock
+    from glorcq_b200.quantized_linear import GLoRCQLinear
+    from glorcq_b200.tiled import TiledWeight
+
+    def layer(N, K):
+        lin = GLoRCQLinear(K, N)
+        lin._tiled = TiledWeight(_lib.FMT_Q2, N, K, 128, 1, "cpu")
+        return lin
+    experts = [SimpleNamespace(gate_proj=layer(128, 256), up_proj=layer(128, 256), down_proj=layer(256, 128)) for _ in range(2)]
+    down = experts[1].down_proj._tiled
+    down.set_bias(torch.zeros(256))
+    bias = weakref.ref(down.bias)
+    blk = GraphCompatibleMoeBlock(SimpleNamespace(num_experts=2, top_k=1, norm_topk_prob=False, gate=None, experts=experts))
+    blk._build(torch.device("cpu"))
+    down.set_bias(None)
+    assert bias() is not None
+    del blk
